@@ -795,6 +795,49 @@ void grid_from_params(const hbt_params &p, Grid &g) {
     g.cph = make_cos_scale(g.hbarC_inv);
 }
 
+// The margins of the tile screen (hbt_screen.cuh derives them).
+static void fill_tile_screen(const Grid &g, Screen &s) {
+    const double u = 5.9604644775390625e-8, up = 1.0 + 1e-5;  // 2^-24; rounding up
+    auto f = [](double v) { return static_cast<float>(v); };
+    const double n = g.qnpts, inv = 1.0 / g.delta_q, Q = std::max(-g.q_lo, g.q_hi) + 1e-7;
+    const double c0 = -g.q_base * inv - 0.5;
+    const double edge = std::max(std::fabs(g.q_lo - g.q_base),
+                                 std::fabs(g.q_base + n * g.delta_q - g.q_hi)) * inv;
+    const double k0 = 2.0 * inv * Q * (5.6 + 8.3) * u +
+                      3.0 * u * (Q * inv + std::fabs(c0) + n + 2.0) + 8.0 * u + 1.001 * edge +
+                      1e-9 * n + 8.0 * u * (n + 1.0);
+    s.sc_c0 = f(c0);
+    s.sc_nk1 = f(-8.3 * u * std::max(2.0 * inv * Q * 0.53 * 1.06, 10.0) * up);
+    s.sc_nk2 = f(-2.0 * inv * 4.1 * u * up);
+    s.sc_nk3 = f(-2.0 * inv * (g.boost ? 4.1 : 2.1) * u * up);
+    // the outer limits lie 8 u (n + 1) inside the margin, so that a
+    // coordinate they keep, however they round, has its rint on the grid or
+    // is undecided
+    s.sc_top = f(n - 8.0 * u * (n + 1.0));
+    s.sc_bot = f(-1.0 + 8.0 * u);
+    s.sc_n2 = (unsigned)g.qnpts * (unsigned)g.qnpts;
+    s.sc_q3 = s.sc_n2 * (unsigned)g.qnpts;
+    s.sc_bin0 = 0x4b400000u * (s.sc_n2 + (unsigned)g.qnpts + 1u);
+    // a grid without a positive bin width is left to the reference chain
+    s.sc_h0 = g.delta_q > 0.0 ? f(0.5 - k0 * up) : -INFINITY;
+    const double nk = g.n_KT - 1, ik = 1.0 / g.dKT, ck = -g.KT_min * ik - 0.5;
+    s.sk_half_inv = f(0.5 * ik);
+    s.sk_c0 = f(ck);
+    s.sk_nkA = f(-2.01 * u * ik * up);
+    s.sk_nkk = f(-8.0 * u * ik * up);
+    s.sk_top = f(nk - 8.0 * u * (nk + 1.0));
+    const double kk0 = 12.0 * u * (nk + std::fabs(ck) + 2.0) + 1e-9 * (nk + 1.0);
+    s.sk_h0 = g.dKT > 0.0 && g.KT_min >= 0.0 ? f(0.5 - kk0 * up) : -INFINITY;
+    const double ip = g.n_Kphi / g.two_pi;
+    s.sp_cos = f(std::cos(g.psi_ref));
+    s.sp_sin = f(std::sin(g.psi_ref));
+    s.sp_scale = f(ip);
+    s.sp_quarter = f(0.25 * g.n_Kphi);
+    s.sp_nkA = f(-2.0 * 2.01 * u * ip * up);
+    s.sp_h0 = f(0.5 - (2.0 * ip * (2e-6 + 20.0 * u) + ip * g.kphi_tol + 8.0 * u * (g.n_Kphi + 1.0) +
+                       1e-9) * up);
+}
+
 void screen_from_grid(const Grid &g, Screen &s) {
     auto f = [](double v) { return static_cast<float>(v); };
     auto slack = [](double v, float v32) { return std::fabs(v - static_cast<double>(v32)); };
@@ -820,6 +863,7 @@ void screen_from_grid(const Grid &g, Screen &s) {
     s.n_KT = g.n_KT;
     s.n_Kphi = g.n_Kphi;
     fill_prefilter(s);
+    fill_tile_screen(g, s);
 }
 
 bool params_valid(const hbt_params &p) {

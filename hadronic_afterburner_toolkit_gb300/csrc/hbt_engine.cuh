@@ -119,6 +119,17 @@ struct Screen {
     // screened kernels and the pair-by-pair cut rows of cap admission)
     // decides it the same way
     float kphi_tol;
+    // tile screen (hbt_screen.cuh screen_two): bin coordinate q / bin width +
+    // sc_c0, its margin 0.5 - et = sc_h0 + w (sc_nk1 / k + sc_nk2) + e_long
+    // sc_nk3, the grid's outer limits sc_top - h and sc_bot + h, qnpts^2,
+    // the offset of the flat bin and qnpts^3 (bins a decided pair can have)
+    float sc_c0, sc_h0, sc_nk1, sc_nk2, sc_nk3, sc_top, sc_bot;
+    unsigned sc_n2, sc_bin0, sc_q3;
+    // K_T (slot_of): bin coordinate 2 K_T sk_half_inv + sk_c0 and its margin
+    float sk_half_inv, sk_c0, sk_h0, sk_nkA, sk_nkk, sk_top;
+    // K_phi (slot_of): cosine and sine of psi_ref, bins per radian and per
+    // quarter turn, margin
+    float sp_cos, sp_sin, sp_scale, sp_quarter, sp_h0, sp_nkA;
 };
 
 // Host: the prefilter constants of a screen whose window is filled in.

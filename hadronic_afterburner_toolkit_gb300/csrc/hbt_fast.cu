@@ -16,7 +16,7 @@ using namespace tile;
 
 template <bool AZ, bool BOOST, int PREC>
 __global__ void __launch_bounds__(FT) k_same_screened(Device d, long long n, Cols8 c) {
-    __shared__ TileSmem sm;
+    __shared__ SameSmem sm;
     __shared__ double2 cs[COS_TABLE];
     if (PREC == 0) fill_cos_table(cs);
     if (PREC == 2) fill_df_table(reinterpret_cast<float4 *>(cs));
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(FT) k_same_screened(Device d, long long n, Col
 template <bool AZ, bool BOOST>
 __global__ void __launch_bounds__(FT) k_mixed_screened(Device d, long long n1, Cols4 l1,
                                                        long long n2, Cols4 l2, long long tiles1) {
-    __shared__ TileSmem sm;
+    __shared__ MixedSmem sm;
     const long long ti = blockIdx.x % tiles1, tj = blockIdx.x / tiles1;
     mixed_tile_pair<AZ, BOOST>(d, sm, l1.p, n1, l2.p, n2, ti * FT, tj * FT);
 }

@@ -78,13 +78,48 @@ struct SameCtas {
 #endif
 constexpr int kMixedCtas = HBT_MIXED_CTAS;
 
+// One item: the tile pair, with or without the q_inv histograms by the type
+// of its shared memory.
+template <bool AZ, bool BOOST, int PREC, int MODE>
+__device__ __forceinline__ void same_item(const Device &d, SameSmem &sm, const double2 *cs,
+                                          const double *const *c, const unsigned *orig,
+                                          long long n, const Item &it) {
+    same_tile_pair<AZ, BOOST, PREC, MODE>(d, sm, cs, c, orig, n, (long long)it.ti * FT,
+                                          (long long)it.tj * FT);
+}
+template <bool AZ, bool BOOST, int PREC, int MODE>
+__device__ __forceinline__ void same_item(const Device &d, QinvSmem &sm, const double2 *cs,
+                                          const double *const *c, const unsigned *orig,
+                                          long long n, const Item &it) {
+    same_tile_pair_qinv<AZ, BOOST, PREC, MODE>(d, sm, cs, c, orig, n, (long long)it.ti * FT,
+                                               (long long)it.tj * FT);
+}
+template <bool AZ, bool BOOST, int MODE>
+__device__ __forceinline__ void mixed_item(const Device &d, MixedSmem &sm,
+                                           const double *const *l1, long long n1,
+                                           const double *const *l2, long long n2, const Item &it,
+                                           const unsigned *o1, const unsigned *o2,
+                                           long long row_base) {
+    mixed_tile_pair<AZ, BOOST, MODE>(d, sm, l1, n1, l2, n2, (long long)it.ti * FT,
+                                     (long long)it.tj * FT, o1, o2, row_base);
+}
+template <bool AZ, bool BOOST, int MODE>
+__device__ __forceinline__ void mixed_item(const Device &d, QinvSmem &sm,
+                                           const double *const *l1, long long n1,
+                                           const double *const *l2, long long n2, const Item &it,
+                                           const unsigned *o1, const unsigned *o2,
+                                           long long row_base) {
+    mixed_tile_pair_qinv<AZ, BOOST, MODE>(d, sm, l1, n1, l2, n2, (long long)it.ti * FT,
+                                          (long long)it.tj * FT, o1, o2, row_base);
+}
+
 // Same-event items [base, min(end, queued)) pulled by persistent CTAs.
 // MODE: fast binning, or one pass of ordered cap admission; MANY: the items
 // of many analyses (b.devs), fast binning only.
 template <bool AZ, bool BOOST, int PREC, int MODE, bool QINV, bool MANY>
 __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(Device d, BatchDev b, unsigned base,
                                                            unsigned end) {
-    __shared__ SmemFor<QINV> sm;
+    __shared__ typename std::conditional<QINV, QinvSmem, SameSmem>::type sm;
     __shared__ unsigned item;
     __shared__ double2 cs[COS_TABLE];
     if (PREC == 0) fill_cos_table(cs);
@@ -104,13 +139,9 @@ __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(D
         if constexpr (MANY) {
             __shared__ Device dsm;
             load_device(b, job, dsm);
-            same_tile_pair<AZ, BOOST, PREC, MODE, QINV>(dsm, sm, cs, c, b.orig + la.off, la.n,
-                                                        (long long)it.ti * FT,
-                                                        (long long)it.tj * FT);
+            same_item<AZ, BOOST, PREC, MODE>(dsm, sm, cs, c, b.orig + la.off, la.n, it);
         } else {
-            same_tile_pair<AZ, BOOST, PREC, MODE, QINV>(d, sm, cs, c, b.orig + la.off, la.n,
-                                                        (long long)it.ti * FT,
-                                                        (long long)it.tj * FT);
+            same_item<AZ, BOOST, PREC, MODE>(d, sm, cs, c, b.orig + la.off, la.n, it);
         }
         __syncthreads();
     }
@@ -119,7 +150,7 @@ __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(D
 // Mixed-event items, all in one launch.
 template <bool AZ, bool BOOST, int MODE, bool QINV, bool MANY>
 __global__ void __launch_bounds__(FT, kMixedCtas) k_persistent_mixed(Device d, BatchDev b) {
-    __shared__ TileSmem sm;
+    __shared__ typename std::conditional<QINV, QinvSmem, MixedSmem>::type sm;
     __shared__ unsigned item;
     const unsigned stop = min(b.n_items[1], b.mixed_cap);
     for (;;) {
@@ -139,15 +170,11 @@ __global__ void __launch_bounds__(FT, kMixedCtas) k_persistent_mixed(Device d, B
         if constexpr (MANY) {
             __shared__ Device dsm;
             load_device(b, job, dsm);
-            mixed_tile_pair<AZ, BOOST, MODE, QINV>(dsm, sm, c1, la.n, c2, lb.n,
-                                                   (long long)it.ti * FT, (long long)it.tj * FT,
-                                                   b.orig + la.off, b.orig + lb.off,
-                                                   job.row_base);
+            mixed_item<AZ, BOOST, MODE>(dsm, sm, c1, la.n, c2, lb.n, it, b.orig + la.off,
+                                        b.orig + lb.off, job.row_base);
         } else {
-            mixed_tile_pair<AZ, BOOST, MODE, QINV>(d, sm, c1, la.n, c2, lb.n,
-                                                   (long long)it.ti * FT, (long long)it.tj * FT,
-                                                   b.orig + la.off, b.orig + lb.off,
-                                                   job.row_base);
+            mixed_item<AZ, BOOST, MODE>(d, sm, c1, la.n, c2, lb.n, it, b.orig + la.off,
+                                        b.orig + lb.off, job.row_base);
         }
         __syncthreads();
     }

@@ -1,27 +1,14 @@
 // Screened pair binning of one tile pair (device code shared by the grid
-// kernels of hbt_fast.cu and the persistent batch kernel of hbt_batch.cu).
+// kernels of hbt_fast.cu and the persistent batch kernels of
+// hbt_persist.cuh).
 //
 // GB300 runs FP64 at 1/58 of its FP32 rate, so every pair is first screened
 // in FP32 and only the pairs that are binned pay for more work:
 //
-//  A. Prefilter (every pair, ~30 FP32 operations).  Rejects only pairs
-//     certainly outside the window: q_out^2 + q_side^2 = q_x^2 + q_y^2 in
-//     real arithmetic, so a binned pair has q_x^2 + q_y^2 <= 2 Q^2, and
-//     |q_long| <= Q (with the boost: |S_E dq_z - S_z dq_E| <= Q sqrt(M^2),
-//     no division), Q = max(-lo, hi); each test carries the FP32 rounding of
-//     its inputs (2.01 u per sum) and a relative margin.  Other pairs are
-//     queued.
-//  B. Window screen and bins, per warp on 32 queued pairs with all lanes
-//     active.  From FP32 copies of the momenta: K_perp^2, q_out, q_side,
-//     q_long and a rigorous bound on how far each lies from the value the
-//     reference computes in FP64 (error analysis below).  A pair is dropped
-//     when a window check fails by more than its bound; the bin indices are
-//     decided in FP32 when every truncation is farther from its edge than
-//     its bound (they are then the reference's indices exactly), K_phi
-//     likewise with atan2f; any pair with an undecided window, index or
-//     angle runs the reference-order FP64 chain of hbt_chain.cuh instead.
-//     Same-event pairs that pass go to a second per-warp queue, so the FP64
-//     work of stage C again runs on 32 pairs at a time.
+//  A. Screen (hbt_screen.cuh, every pair): certainly outside the window, its
+//     q bin certain, or undecided.  Pairs not outside go to a per-warp queue.
+//  B. Slot (32 queued pairs, all lanes active): the K_T and K_phi bins in
+//     FP32 with error bounds (slot_of).
 //  C. Histogram update.  Mixed pairs add 1 to their denominator bin.
 //     Same-event pairs add q_out, q_side, q_long and cos(q.dx / hbarC):
 //       FP64 form  - the phase q.dx and its cos in FP64 (table_cos,
@@ -43,24 +30,33 @@
 //     and position difference, so it negates q_out, q_side, q_long exactly
 //     (IEEE rounding is symmetric in sign) and leaves the phase and its cos
 //     unchanged.
-//  D. Pairs left undecided in B go to a third per-warp queue; the reference
-//     chain runs on them 32 at a time.
+//  D. Pairs left undecided by A or B go to another per-warp queue; the
+//     reference chain runs on them 32 at a time.
 //
-// Error analysis (u = 2^-24).  Inputs are FP64 values v rounded once to
-// FP32: |v32 - v| <= u|v|.  For s = a +- b in FP32, |s - S| <= 2.01 u A with
-// A = |a| + |b| and S the exact sum of the FP64 inputs.  Products, sums, the
-// reciprocal square root (rsqrtf: at most 2 ulp) and the approximate
-// divisions used only inside the bounds (__fdividef: at most 2 ulp, the
-// bounds carry a 1e-4 relative margin for it) propagate this as coded in
-// screen_windows() and decide_bins(); every bound is then doubled and widened
-// by the rounding of the FP32 copies of the constants, which also covers the
-// FP64 reference's own rounding (2^-29 times smaller).
+// Measured on the central group (150k pions, 5.4e9 pairs in the kept tile
+// pairs, 1.94e9 binned), whole passes, against a scalar prefilter, a queue
+// and a scalar window test with per-component bounds: FP32-weight form 118.0
+// -> 70.6 ms, FP64 form 143.6 -> 134.7 ms (bound by the FP64 pipe, so the
+// issue slots saved show less), double-float kaons 18.3 -> 16.1 ms.
+//
+// The forms with q_inv histograms (same_tile_pair_qinv,
+// mixed_tile_pair_qinv) screen in two steps, a prefilter and a window test
+// on queued pairs, in scalar FP32.  Error analysis of that screen (u = 2^-24).  Inputs are FP64 values v
+// rounded once to FP32: |v32 - v| <= u|v|.  For s = a +- b in FP32, |s - S|
+// <= 2.01 u A with A = |a| + |b| and S the exact sum of the FP64 inputs.
+// Products, sums, the reciprocal square root (rsqrtf: at most 2 ulp) and the
+// approximate divisions used only inside the bounds (__fdividef: at most 2
+// ulp, the bounds carry a 1e-4 relative margin for it) propagate this as
+// coded in screen_lcms() and decide_bins(); every bound is then doubled and
+// widened by the rounding of the FP32 copies of the constants, which also
+// covers the FP64 reference's own rounding (2^-29 times smaller).
 #pragma once
 
 #include <type_traits>
 
 #include "hbt_chain.cuh"
 #include "hbt_math.cuh"
+#include "hbt_screen.cuh"
 
 namespace hbt {
 namespace tile {
@@ -68,7 +64,6 @@ namespace tile {
 using namespace chain;
 
 constexpr float U = 5.9604645e-8f;  // 2^-24
-constexpr int FT = 128;             // tile edge (particles) for both lists
 constexpr int QCAP = 64;            // per-warp compaction queue
 
 // FP32 screen quantities of one pair and their error bounds.
@@ -171,64 +166,6 @@ __device__ __forceinline__ int screen_lcms(const Screen &S, float4 a, float4 b, 
     if (wo == 0 || ws == 0 || wl == 0) return 0;
     if (wo == 2 || ws == 2 || wl == 2) return 2;
     return 1;
-}
-
-// Stage B: window checks.  Returns 0 (reject), 1 (all windows certainly
-// passed), 2 (undecided).  The K_T and LCMS parts of screen_kt and
-// screen_lcms in one function (the forms without q_inv histograms keep it
-// whole: split, their register allocation spilled more).
-template <bool BOOST>
-__device__ __forceinline__ int screen_windows(const Screen &S, float4 a, float4 b, Q &q) {
-    q.sx = a.x + b.x;
-    q.sy = a.y + b.y;
-    const float dx = a.x - b.x, dy = a.y - b.y;
-    q.Ax = fabsf(a.x) + fabsf(b.x);
-    q.Ay = fabsf(a.y) + fabsf(b.y);
-    q.k2 = __fmaf_rn(q.sx, q.sx, q.sy * q.sy);
-    const float AA = __fmaf_rn(q.Ax, q.Ax, q.Ay * q.Ay);
-    // |k2 - (S_x^2 + S_y^2)|
-    q.ek2 = 6.1f * U * __fmaf_rn(q.Ax, fabsf(q.sx), q.Ay * fabsf(q.sy)) + 3.1f * U * q.k2 +
-            1e-13f * AA;
-    // K_T window (reference rejects Kp2 < KT_min^2 or Kp2 > KT_max^2)
-    const float ekt = 2.0f * q.ek2 + S.kt_slack;
-    if ((S.kt_lo4 > 0.0f && q.k2 + ekt < S.kt_lo4) || q.k2 - ekt > S.kt_hi4) return 0;
-    int cls = ((S.kt_lo4 == 0.0f || q.k2 - ekt > S.kt_lo4) && q.k2 + ekt < S.kt_hi4) ? 1 : 2;
-    const float rel_k2 = __fdividef(q.ek2, q.k2) * 1.0001f;
-    if (!(q.k2 > 0.0f) || !(rel_k2 <= 0.05f)) return 2;  // |S| too small for the bounds
-    const float inv = rsqrtf(q.k2);
-    const float rel_inv = 0.53f * rel_k2 + 4.5f * U;
-    const float eN = 9.0f * U * AA;
-    const float no = __fmaf_rn(dx, q.sx, dy * q.sy);
-    const float ns = __fmaf_rn(dy, q.sx, -(dx * q.sy));
-    q.qo = no * inv;
-    q.eqo = __fmaf_rn(fabsf(no), rel_inv, eN) * inv + U * fabsf(q.qo);
-    q.qs = ns * inv;
-    q.eqs = __fmaf_rn(fabsf(ns), rel_inv, eN) * inv + U * fabsf(q.qs);
-    const float dz = a.z - b.z;
-    const float Az = fabsf(a.z) + fabsf(b.z);
-    if (BOOST) {
-        const float sE = a.w + b.w, sz = a.z + b.z, dE = a.w - b.w;
-        const float AE = fabsf(a.w) + fabsf(b.w);
-        const float m = sE - sz, p = sE + sz;
-        const float e0 = 2.01f * U * (AE + Az);
-        const float rel_m2 =
-            (__fdividef(e0 + U * fabsf(m), m) + __fdividef(e0 + U * fabsf(p), p)) * 1.0001f +
-            1.01f * U;
-        if (!(m > 0.0f) || !(p > 0.0f) || !(rel_m2 <= 0.05f)) return 2;
-        const float rl = rsqrtf(m * p);
-        const float rel_rl = 0.53f * rel_m2 + 4.5f * U;
-        const float nl = __fmaf_rn(sE, dz, -(sz * dE));
-        q.ql = nl * rl;
-        q.eql = __fmaf_rn(fabsf(nl), rel_rl, 17.0f * U * AE * Az) * rl + U * fabsf(q.ql);
-    } else {
-        q.ql = dz;
-        q.eql = 2.1f * U * Az;
-    }
-    const int wo = window_class(S, q.qo, q.eqo), ws = window_class(S, q.qs, q.eqs),
-              wl = window_class(S, q.ql, q.eql);
-    if (wo == 0 || ws == 0 || wl == 0) return 0;
-    if (wo == 2 || ws == 2 || wl == 2) return 2;
-    return cls;
 }
 
 // floor((v - base) / delta_q) when certain, else -1.
@@ -742,10 +679,40 @@ __device__ __forceinline__ void values64(const Grid &g, const double2 *cs, const
     w = table_cos(cs, g.cph, ph);
 }
 
-// Shared memory of one tile pair; E2 is the entry of the second same-event
-// queue (uint2, or uint4 when q_inv histograms are binned too).
-template <class E2>
-struct TileSmemT {
+// Shared memory of a same-event tile pair.
+struct SameSmem {
+    // FP64 columns px py pz E x y z t (FP64 form) or split columns ((hi, lo)
+    // FP32 pairs, the other forms)
+    double si[8][FT];
+    double sj[8][FT];
+    // FP64 form with the boost: p_z and E as (hi, lo) FP32 pairs, for the
+    // longitudinal sums in double-float
+    float4 zi[FT], zj[FT];
+    TermsPair ti[FT / 2], tj[FT / 2];  // screen terms
+    // pairs past the screen (screen_loop): up to 31 left over and 64 of a step
+    uint2 queue[FT / 32][96];
+    // undecided pairs, (i, j) bits: the reference chain runs on them 32 at a
+    // time (inline, a warp would run it for the one or two lanes holding one)
+    unsigned queue3[FT / 32][QCAP];
+    __align__(8) unsigned oi[FT], oj[FT];  // original list positions (pair orientation)
+    float offi[4], offj[4];  // double-float form: the tiles' momentum offsets
+};
+
+// Shared memory of a mixed-event tile pair.
+struct MixedSmem {
+    TermsPair ti[FT / 2], tj[FT / 2];
+    uint2 queue[FT / 32][96];
+    unsigned queue3[FT / 32][QCAP];
+};
+
+__device__ __forceinline__ Terms terms_at(const TermsPair *b, int k) {
+    const TermsPair &d = b[k >> 1];
+    const int h = k & 1;
+    return Terms{d.x[h], d.y[h], d.m[h], d.p[h], d.r2[h], d.t2[h]};
+}
+
+// Shared memory of the forms with q_inv histograms.
+struct QinvSmem {
     // same-event tiles: FP64 columns (FP64 form) or split columns (hi, lo
     // FP32 pairs, FP32-weight form), px py pz E x y z t
     double si[8][FT];
@@ -758,27 +725,15 @@ struct TileSmemT {
     // z and w), for the longitudinal sums in double-float
     float2 li[FT], lj[FT];
     unsigned queue[FT / 32][QCAP];
-    // same-event pairs that passed the window screen: x = (i, j, swap,
-    // undecided, slot) bits, y = q bin (bin_entry); with q_inv, x = (i, j,
-    // swap, undecided, 3-D event, q_inv event) bits, y = q bin, z = slot |
-    // K_T bin << 16, w = q_inv bin
-    E2 queue2[FT / 32][QCAP];
-    // pairs the screen left undecided, (i, j, swap) bits: the reference
-    // chain runs on them 32 at a time (inline, a warp would run it for the
-    // one or two lanes holding such a pair)
+    // same-event pairs that passed the screen: x = (i, j, swap, undecided,
+    // 3-D event, q_inv event) bits, y = q bin, z = slot | K_T bin << 16, w =
+    // q_inv bin
+    uint4 queue2[FT / 32][QCAP];
+    // undecided pairs, (i, j, swap) bits
     unsigned queue3[FT / 32][QCAP];
     unsigned oi[FT], oj[FT];  // original list positions (pair orientation)
     float offi[4], offj[4];   // double-float form: the tiles' momentum offsets
 };
-using TileSmem = TileSmemT<uint2>;
-template <bool QINV>
-using SmemFor = TileSmemT<typename std::conditional<QINV, uint4, uint2>::type>;
-
-// Entry of the second same-event queue.
-__device__ __forceinline__ uint2 bin_entry(unsigned e, bool undecided, int slot, int bin) {
-    return make_uint2((e & 0x1ffffu) | (undecided ? 1u << 17 : 0u) | ((unsigned)slot << 18),
-                      (unsigned)bin);
-}
 
 // Appends this lane's entry to the warp queue when `take`, and runs
 // `process(entry, true)` on 32 queued entries whenever 32 are waiting (all
@@ -916,6 +871,321 @@ __device__ __forceinline__ bool admit(const Device &d, int slot, long long row, 
     return row < d.caps.row_cut[slot];
 }
 
+// Loads a tile's screen terms: row `tid` of the tile at k0 of a list of n
+// particles with columns c, or padding past its end.
+template <bool BOOST>
+__device__ __forceinline__ Terms load_terms(const double *const *c, long long k, long long n,
+                                            float pad) {
+    return k < n ? screen_terms<BOOST>(c[0][k], c[1][k], c[2][k], c[3][k]) : pad_terms(pad);
+}
+
+// The pair loop: screens this lane's row against particles [0, jend) of the
+// j-tile, pairs with jj <= jmin left out, and collects the pairs that are
+// not certainly outside in the warp's queue; `process(entry, valid)` runs on
+// 32 of them at a time, all lanes in step.  An entry is x = row | particle
+// << 8 | undecided << 16, y = q bin.  ORIENT: the pair's first particle is
+// the one with the smaller original position (oa, oj).
+template <bool BOOST, bool ORIENT, class F>
+__device__ __forceinline__ void screen_loop(const Screen &S, const Terms &terms, int il,
+                                            const TermsPair *tj, unsigned oa, const unsigned *oj,
+                                            int jmin, int jend, uint2 *q, F &process) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const Row a = row_of(terms);
+    const f2 plus = both(S.inv_dq);
+    const int steps = (jend + 1) >> 1;
+    int count = 0;
+    for (int jp = 0;; jp++) {
+        const bool last = jp >= steps;
+        if (!last) {
+            f2 inv_dq = plus;
+            if (ORIENT) {
+                const uint2 o = *reinterpret_cast<const uint2 *>(oj + 2 * jp);
+                inv_dq = pack2(oa > o.x ? -S.inv_dq : S.inv_dq, oa > o.y ? -S.inv_dq : S.inv_dq);
+            }
+            Screened r;
+            if (!screen_two<BOOST>(S, a, tj[jp], inv_dq, r)) continue;
+            const int jj = 2 * jp;
+            const bool t0 = r.take[0] && jj > jmin;
+            const bool t1 = r.take[1] && jj + 1 > jmin && jj + 1 < jend;
+            const unsigned m0 = __ballot_sync(0xffffffffu, t0);
+            const unsigned m1 = __ballot_sync(0xffffffffu, t1);
+            if (!(m0 | m1)) continue;
+            const unsigned e = (unsigned)il | ((unsigned)jj << 8);
+            if (t0)
+                q[count + __popc(m0 & below)] =
+                    make_uint2(e | (r.und[0] ? 1u << 16 : 0u), r.bin[0]);
+            count += __popc(m0);
+            if (t1)
+                q[count + __popc(m1 & below)] =
+                    make_uint2((e + 256u) | (r.und[1] ? 1u << 16 : 0u), r.bin[1]);
+            count += __popc(m1);
+            __syncwarp();
+        }
+        // full groups of 32 from the queue's end; at the end of the tile the
+        // rest
+        while (count >= (last ? 1 : 32)) {
+            const int take = min(count, 32);
+            count -= take;
+            process(q[count + min(lane, take - 1)], lane < take);
+            __syncwarp();
+        }
+        if (last) break;
+    }
+}
+
+// Same-event pairs of the tiles starting at i0 and j0 (i0 <= j0) of one list
+// of n particles with columns c = px py pz E x y z t.  Every unordered pair
+// is visited once (position j > i); it is oriented as the reference orients
+// it, q = p_first - p_second with `first` the particle earlier in the
+// caller's list: orig[k] is that original index of row k, or nullptr when
+// the rows are in the caller's order.  MODE selects the admission: FAST bins
+// every pair; COUNT and ORDER are the two passes of ordered cap admission,
+// which see each pair at its row (the earlier of its two positions in the
+// caller's list).
+// Called by all FT threads of the CTA; the caller syncs before reusing `sm`.
+template <bool AZ, bool BOOST, int PREC, int MODE = MODE_FAST>
+__device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, const double2 *cs,
+                                               const double *const *c, const unsigned *orig,
+                                               long long n, long long i0, long long j0) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    // split columns of the FP32-weight and double-float forms, in the FP64
+    // tiles' place
+    float2(*spi)[FT] = reinterpret_cast<float2(*)[FT]>(&sm.si[0][0]);
+    float2(*spj)[FT] = reinterpret_cast<float2(*)[FT]>(&sm.sj[0][0]);
+    if (PREC == 0) {
+        for (int f = 0; f < 8; f++) {
+            sm.si[f][tid] = (i0 + tid < n) ? c[f][i0 + tid] : 0.0;
+            sm.sj[f][tid] = (j0 + tid < n) ? c[f][j0 + tid] : 0.0;
+        }
+        if (BOOST) {
+            const float2 iz = split(sm.si[2][tid]), iE = split(sm.si[3][tid]);
+            const float2 jz = split(sm.sj[2][tid]), jE = split(sm.sj[3][tid]);
+            sm.zi[tid] = make_float4(iz.x, iz.y, iE.x, iE.y);
+            sm.zj[tid] = make_float4(jz.x, jz.y, jE.x, jE.y);
+        }
+    } else if (PREC == 1) {
+        for (int f = 0; f < 8; f++) {
+            spi[f][tid] = split((i0 + tid < n) ? c[f][i0 + tid] : 0.0);
+            spj[f][tid] = split((j0 + tid < n) ? c[f][j0 + tid] : 0.0);
+        }
+    } else {
+        // double-float form: momenta split relative to the tile's first row
+        for (int f = 0; f < 8; f++) {
+            const double vi = (i0 + tid < n) ? c[f][i0 + tid] : 0.0;
+            const double vj = (j0 + tid < n) ? c[f][j0 + tid] : 0.0;
+            float oi = 0.0f, oj = 0.0f;
+            if (f < 4) {
+                oi = (float)c[f][i0];
+                oj = (float)c[f][j0];
+                if (tid == 0) {
+                    sm.offi[f] = oi;
+                    sm.offj[f] = oj;
+                }
+            }
+            spi[f][tid] = split(vi - (double)oi);
+            spj[f][tid] = split(vj - (double)oj);
+        }
+    }
+    sm.oi[tid] = orig ? (i0 + tid < n ? orig[i0 + tid] : 0u) : (unsigned)(i0 + tid);
+    sm.oj[tid] = orig ? (j0 + tid < n ? orig[j0 + tid] : 0u) : (unsigned)(j0 + tid);
+    put_terms(sm.ti, tid, load_terms<BOOST>(c, i0 + tid, n, -1e15f));
+    put_terms(sm.tj, tid, load_terms<BOOST>(c, j0 + tid, n, 1e15f));
+    __syncthreads();
+    const Screen &S = d.s;
+    // warp w takes the tile's rows w, w + 4, w + 8, ...: the rows are sorted
+    // in momentum space, so interleaving spreads each warp's rows over the
+    // tile and evens out the binned pairs between warps
+    const int il = lane * (FT / 32) + w;
+    const int jend = (int)min((long long)FT, n - j0);
+    // each unordered pair once; none for rows past the list's end
+    const int jmin = i0 + il >= n ? FT : (i0 == j0 ? il : -1);
+    unsigned *q3 = sm.queue3[w];
+    int count3 = 0;
+
+    // pairs left undecided, 32 at a time: the reference chain decides them
+    // (and may hand a K_phi edge to the host), from the FP64 tile or
+    // (FP32-weight and double-float forms) the FP64 columns
+    auto chains = [&](unsigned e, bool valid) {
+        if (!valid) return;
+        const int qi = e & 0xff, qj = (e >> 8) & 0xff;
+        const long long oa = sm.oi[qi], ob = sm.oj[qj];
+        const bool swap = oa > ob;
+        double A[8], B[8];  // first and second particle of the pair
+#pragma unroll
+        for (int f = 0; f < 8; f++) {
+            const double u = PREC == 0 ? sm.si[f][qi] : c[f][i0 + qi];
+            const double v = PREC == 0 ? sm.sj[f][qj] : c[f][j0 + qj];
+            A[f] = swap ? v : u;
+            B[f] = swap ? u : v;
+        }
+        if (MODE != MODE_FAST) {
+            const long long row = swap ? ob : oa, col = swap ? oa : ob;
+            undecided_pair_ordered<false, MODE>(d, A, B, row, col, n, n);
+            return;
+        }
+        if (PREC == 1)
+            undecided_pair32<BOOST>(d, A, B, i0 + qi, j0 + qj, n);
+        else
+            undecided_pair64(d, A, B, i0 + qi, j0 + qj, n);
+    };
+
+    // one pair with its q bin and slot decided: its values into its bin
+    auto decided = [&](unsigned e, int slot, unsigned bin) {
+        const int qi = e & 0xff, qj = (e >> 8) & 0xff;
+        const unsigned oa = sm.oi[qi], ob = sm.oj[qj];
+        const bool swap = oa > ob;
+        if (MODE != MODE_FAST) {
+            if (!admit<MODE>(d, slot, (long long)min(oa, ob), n)) return;
+        }
+        const long long at = (long long)slot * d.g.q3 + bin;
+        if (PREC == 1) {
+            // the pair as stored (i, j); swapping first and second negates
+            // q_out, q_side, q_long exactly and leaves the phase unchanged
+            float2 a[8], b[8];
+#pragma unroll
+            for (int f = 0; f < 8; f++) {
+                a[f] = spi[f][qi];
+                b[f] = spj[f][qj];
+            }
+            float4 v = values32_split<BOOST>(d.s, a, b);
+            if (swap) {
+                v.x = -v.x;
+                v.y = -v.y;
+                v.z = -v.z;
+            }
+            atomicAdd(partials_of(d) + at, v);
+            atomicAdd(d.h.cnt + at, 1ull);
+            return;
+        }
+        double vo, vs, vl, vw;
+        if (PREC == 2) {
+            float2 a[8], b[8];
+#pragma unroll
+            for (int f = 0; f < 8; f++) {
+                a[f] = spi[f][qi];
+                b[f] = spj[f][qj];
+            }
+            values_df<BOOST>(d.s, reinterpret_cast<const float4 *>(cs), a, b, sm.offi, sm.offj,
+                             swap, vo, vs, vl, vw);
+        } else {
+            // the pair in the reference's orientation, from the FP64 tile
+            // (the two rows chosen once, then read column by column)
+            const double *ra = swap ? &sm.sj[0][qj] : &sm.si[0][qi];
+            const double *rb = swap ? &sm.si[0][qi] : &sm.sj[0][qj];
+            double A[8], B[8];
+#pragma unroll
+            for (int f = 0; f < 8; f++) {
+                A[f] = ra[f * FT];
+                B[f] = rb[f * FT];
+            }
+            FF sz = {0.0f, 0.0f}, sE = {0.0f, 0.0f};
+            if (BOOST) {
+                const float4 za = sm.zi[qi], zb = sm.zj[qj];
+                sz = ff_sum(make_float2(za.x, za.y), make_float2(zb.x, zb.y));
+                sE = ff_sum(make_float2(za.z, za.w), make_float2(zb.z, zb.w));
+            }
+            values64<BOOST>(d.g, cs, A, B, sz, sE, vo, vs, vl, vw);
+        }
+        Sums *h = d.h.sums + at;
+        atomicAdd(&h->qo, vo);
+        atomicAdd(&h->qs, vs);
+        atomicAdd(&h->ql, vl);
+        atomicAdd(&h->w, vw);
+        atomicAdd(d.h.cnt + at, 1ull);
+    };
+
+    // 32 pairs that passed the screen (all lanes of the warp in step): their
+    // slot, the decided pairs' values, then the undecided ones to the last
+    // queue (last, so that the chain runs with nothing of the values live)
+    auto process = [&](uint2 e2, bool valid) {
+        const unsigned e = e2.x & 0xffffu;
+        int slot = -2;
+        if (valid) {
+            const int qi = e & 0xff, qj = e >> 8;
+            const TermsPair &a = sm.ti[qi >> 1], &b = sm.tj[qj >> 1];
+            slot = slot_of<AZ>(S, a.x[qi & 1], a.y[qi & 1], b.x[qj & 1], b.y[qj & 1]);
+            if (slot != -2 && ((e2.x >> 16) || e2.y >= S.sc_q3)) slot = -1;
+        }
+        if (slot >= 0) decided(e, slot, e2.y);
+        enqueue(q3, count3, slot == -1, e, lane, chains);
+    };
+
+    // (the orientation is by original position)
+    const Terms row = terms_at(sm.ti, il);
+    screen_loop<BOOST, true>(S, row, il, sm.tj, sm.oi[il], sm.oj, jmin, jend, sm.queue[w],
+                             process);
+    drain(q3, count3, lane, chains);
+}
+
+// Mixed-event pairs of the list-1 tile at i0 (n1 particles, columns l1 =
+// px py pz E) and the list-2 tile at j0 (n2 particles, columns l2).  Under
+// ordered cap admission (MODE COUNT / ORDER) a pair's row and column are
+// its positions in the caller's lists, orig1 / orig2 (nullptr: the rows are
+// in the caller's order).
+template <bool AZ, bool BOOST, int MODE = MODE_FAST>
+__device__ __forceinline__ void mixed_tile_pair(const Device &d, MixedSmem &sm,
+                                                const double *const *l1, long long n1,
+                                                const double *const *l2, long long n2,
+                                                long long i0, long long j0,
+                                                const unsigned *orig1 = nullptr,
+                                                const unsigned *orig2 = nullptr,
+                                                long long row_base = 0) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    put_terms(sm.ti, tid, load_terms<BOOST>(l1, i0 + tid, n1, -1e15f));
+    put_terms(sm.tj, tid, load_terms<BOOST>(l2, j0 + tid, n2, 1e15f));
+    __syncthreads();
+    const Screen &S = d.s;
+    const int il = lane * (FT / 32) + w;  // interleaved rows, as in same_tile_pair
+    const int jend = (int)min((long long)FT, n2 - j0);
+    const int jmin = i0 + il >= n1 ? FT : -1;
+    // ordered admission: row stride of the survivor counts and key stride of
+    // the deferrals (several jobs admitted together, or this job alone)
+    const long long rows = d.caps.rows_total ? d.caps.rows_total : n1;
+    const long long cols = d.caps.cols_key ? d.caps.cols_key : n2;
+    unsigned *q3 = sm.queue3[w];
+    int count3 = 0;
+
+    // pairs the screen left undecided, 32 at a time: the reference chain
+    // decides (inline, a warp would run it for one or two lanes)
+    auto chains = [&](unsigned e, bool valid) {
+        if (!valid) return;
+        const int qi = e & 0xff, qj = (e >> 8) & 0xff;
+        if (MODE != MODE_FAST) {
+            const long long row = row_base + (orig1 ? (long long)orig1[i0 + qi] : i0 + qi);
+            const long long col = orig2 ? (long long)orig2[j0 + qj] : j0 + qj;
+            const double A[4] = {l1[0][i0 + qi], l1[1][i0 + qi], l1[2][i0 + qi], l1[3][i0 + qi]};
+            const double B[4] = {l2[0][j0 + qj], l2[1][j0 + qj], l2[2][j0 + qj], l2[3][j0 + qj]};
+            undecided_pair_ordered<true, MODE>(d, A, B, row, col, rows, cols);
+        } else {
+            undecided_mixed_pair(d, l1, l2, i0 + qi, j0 + qj, n1, n2);
+        }
+    };
+
+    // 32 pairs that passed the screen (all lanes of the warp in step)
+    auto process = [&](uint2 e2, bool valid) {
+        const unsigned e = e2.x & 0xffffu;
+        int slot = -2;
+        if (valid) {
+            const int qi = e & 0xff, qj = e >> 8;
+            const TermsPair &a = sm.ti[qi >> 1], &b = sm.tj[qj >> 1];
+            slot = slot_of<AZ>(S, a.x[qi & 1], a.y[qi & 1], b.x[qj & 1], b.y[qj & 1]);
+            if (slot != -2 && ((e2.x >> 16) || e2.y >= S.sc_q3)) slot = -1;
+            bool admitted = slot >= 0;
+            if (MODE != MODE_FAST && admitted) {
+                const long long row = row_base + (orig1 ? (long long)orig1[i0 + qi] : i0 + qi);
+                admitted = admit<MODE>(d, slot, row, rows);
+            }
+            if (admitted) atomicAdd(d.h.den + (long long)slot * d.g.q3 + e2.y, 1ull);
+        }
+        enqueue(q3, count3, slot == -1, e, lane, chains);
+    };
+
+    const Terms row = terms_at(sm.ti, il);
+    screen_loop<BOOST, false>(S, row, il, sm.tj, 0u, nullptr, jmin, jend, sm.queue[w], process);
+    drain(q3, count3, lane, chains);
+}
+
 // Same-event pairs of the tiles starting at i0 and j0 (i0 <= j0) of one list
 // of n particles with columns c = px py pz E x y z t.  Every unordered pair
 // is visited once (position j > i); it is oriented as the reference orients
@@ -929,8 +1199,8 @@ __device__ __forceinline__ bool admit(const Device &d, int slot, long long row, 
 // when its 3-D window or its q_inv window can pass, and its q_inv bin is
 // decided in FP32 with an error bound like the 3-D bins (qinv_class).
 // Called by all FT threads of the CTA; the caller syncs before reusing `sm`.
-template <bool AZ, bool BOOST, int PREC, int MODE = MODE_FAST, bool QINV = false>
-__device__ __forceinline__ void same_tile_pair(const Device &d, SmemFor<QINV> &sm,
+template <bool AZ, bool BOOST, int PREC, int MODE = MODE_FAST>
+__device__ __forceinline__ void same_tile_pair_qinv(const Device &d, QinvSmem &sm,
                                                const double2 *cs,
                                                const double *const *c, const unsigned *orig,
                                                long long n, long long i0, long long j0) {
@@ -1003,229 +1273,63 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SmemFor<QINV> &s
     auto *q2 = sm.queue2[w];
     int count = 0, count2 = 0;
 
-    // the q_inv form's stages exist only in its instantiation: a lambda that
-    // captures the queue counters by reference, even unused, would take
-    // their addresses and push them to local memory in the other forms
-    if constexpr (QINV) {
-        // stage C with q_inv histograms, for 32 screened pairs: the 3-D event
-        // and the q_inv event of each pair (cos(q.dx) computed once for both)
-        unsigned *q3 = sm.queue3[w];
-        int count3 = 0;
-        // the pairs left undecided, 32 at a time: the reference chain
-        // decides both events
-        auto chains_q = [&](unsigned e, bool valid) {
-            if (!valid) return;
-            const int qi = e & 0xff, qj = (e >> 8) & 0xff;
-            const bool swap = (e >> 16) & 1u;
-            double A[8], B[8];  // first and second particle of the pair
+    // stage C with q_inv histograms, for 32 screened pairs: the 3-D event
+    // and the q_inv event of each pair (cos(q.dx) computed once for both)
+    unsigned *q3 = sm.queue3[w];
+    int count3 = 0;
+    // the pairs left undecided, 32 at a time: the reference chain
+    // decides both events
+    auto chains_q = [&](unsigned e, bool valid) {
+        if (!valid) return;
+        const int qi = e & 0xff, qj = (e >> 8) & 0xff;
+        const bool swap = (e >> 16) & 1u;
+        double A[8], B[8];  // first and second particle of the pair
 #pragma unroll
-            for (int f = 0; f < 8; f++) {
-                const double u = PREC == 0 ? sm.si[f][qi] : c[f][i0 + qi];
-                const double v = PREC == 0 ? sm.sj[f][qj] : c[f][j0 + qj];
-                A[f] = swap ? v : u;
-                B[f] = swap ? u : v;
-            }
-            if (MODE == MODE_FAST) {
-                undecided_pair_ordered<false, MODE_FAST>(d, A, B, i0 + qi, j0 + qj, n, n);
-            } else {
-                const long long oa = sm.oi[qi], ob = sm.oj[qj];
-                const long long row = oa < ob ? oa : ob, col = oa < ob ? ob : oa;
-                undecided_pair_ordered<false, MODE>(d, A, B, row, col, n, n);
-            }
-        };
-        auto values_q = [&](uint4 e4, bool valid) {
-            // this lane's q_inv event, added per group of lanes at the end
-            unsigned qkey = 0xffffffffu;
-            double qsum = 0.0, qw = 0.0;
-            const unsigned e = e4.x;
-            const int qi = e & 0xff, qj = (e >> 8) & 0xff;
-            const bool swap = (e >> 16) & 1u;
-            bool has3 = valid && ((e >> 18) & 1u), hasq = valid && ((e >> 19) & 1u);
-            const int bin = (int)e4.y, slot = (int)(e4.z & 0xffffu), iK = (int)(e4.z >> 16);
-            const int kq = (int)e4.w;
-            double A[8], B[8];  // first and second particle of the pair
-#pragma unroll
-            for (int f = 0; f < 8; f++) {
-                const double u = PREC == 0 ? sm.si[f][qi] : c[f][i0 + qi];
-                const double v = PREC == 0 ? sm.sj[f][qj] : c[f][j0 + qj];
-                A[f] = swap ? v : u;
-                B[f] = swap ? u : v;
-            }
-            const long long oa = sm.oi[qi], ob = sm.oj[qj];
-            const long long row = oa < ob ? oa : ob;
-            // undecided: both events wait for the reference chain (stage D)
-            const bool undecided = valid && ((e >> 17) & 1u);
-            if (undecided) has3 = hasq = false;
-            if (MODE != MODE_FAST) {
-                has3 = has3 && admit<MODE>(d, slot, row, n);
-                hasq = hasq && admit<MODE>(d, d.g.n_slots + iK, row, n);
-            }
-            if (has3 || hasq) {
-                const long long at = (long long)slot * d.g.q3 + bin;
-                double wq;
-                if (PREC == 1) {
-                    float2 a[8], b[8];
-#pragma unroll
-                    for (int f = 0; f < 8; f++) {
-                        a[f] = spi[f][qi];
-                        b[f] = spj[f][qj];
-                    }
-                    float4 v = values32_split<BOOST>(d.s, a, b);
-                    if (swap) {
-                        v.x = -v.x;
-                        v.y = -v.y;
-                        v.z = -v.z;
-                    }
-                    if (has3) {
-                        atomicAdd(partials_of(d) + at, v);
-                        atomicAdd(d.h.cnt + at, 1ull);
-                    }
-                    wq = v.w;
-                } else {
-                    double vo, vs, vl;
-                    if (PREC == 0) {
-                        FF sz = {0.0f, 0.0f}, sE = {0.0f, 0.0f};
-                        if (BOOST) {
-                            const float4 fa = sm.fi[qi], fb = sm.fj[qj];
-                            const float2 la = sm.li[qi], lb = sm.lj[qj];
-                            sz = ff_sum(make_float2(fa.z, la.x), make_float2(fb.z, lb.x));
-                            sE = ff_sum(make_float2(fa.w, la.y), make_float2(fb.w, lb.y));
-                        }
-                        values64<BOOST>(d.g, cs, A, B, sz, sE, vo, vs, vl, wq);
-                    } else {
-                        float2 a[8], b[8];
-#pragma unroll
-                        for (int f = 0; f < 8; f++) {
-                            a[f] = spi[f][qi];
-                            b[f] = spj[f][qj];
-                        }
-                        values_df<BOOST>(d.s, reinterpret_cast<const float4 *>(cs), a, b,
-                                         sm.offi, sm.offj, swap, vo, vs, vl, wq);
-                    }
-                    if (has3) {
-                        Sums *h = d.h.sums + at;
-                        atomicAdd(&h->qo, vo);
-                        atomicAdd(&h->qs, vs);
-                        atomicAdd(&h->ql, vl);
-                        atomicAdd(&h->w, wq);
-                        atomicAdd(d.h.cnt + at, 1ull);
-                    }
-                }
-                if (hasq) {
-                    // the reference's q_inv expression (FP64, same order, no
-                    // contraction): the summed value equals the oracle's
-                    const double q_x = A[0] - B[0], q_y = A[1] - B[1], q_z = A[2] - B[2];
-                    const double q_E = A[3] - B[3];
-                    qsum = sqrt(-(q_E * q_E - q_x * q_x - q_y * q_y - q_z * q_z));
-                    qw = wq;
-                    qkey = (unsigned)(iK * d.g.qnpts + kq);
-                }
-            }
-            qinv_update(d, qkey, qsum, qw, true);
-            enqueue(q3, count3, undecided, e & 0x1ffffu, lane, chains_q);
-        };
-
-        // stage B with q_inv histograms: the K_T window and bin, the 3-D
-        // windows and bins, and the q_inv window and bin of each pair; a pair
-        // with any of them undecided goes to the reference chain as a whole
-        auto screen_q = [&](unsigned e, bool valid) {
-            const int qi = e & 0xff, qj = (e >> 8) & 0xff;
-            const bool swap = (e >> 16) & 1u;
-            const float4 fa = swap ? sm.fj[qj] : sm.fi[qi], fb = swap ? sm.fi[qi] : sm.fj[qj];
-            Q s;
-            int c3 = 0, cq = 0, iK = -1, bin = 0, slot = -1, kq = 0;
-            bool und = false;
-            if (valid) {
-                const int kt = screen_kt(S, fa, fb, s);
-                if (kt != 0) {
-                    c3 = screen_lcms<BOOST>(S, fa, fb, s);
-                    cq = qinv_class(S, fa, fb, kq);
-                    if (c3 == 1 || cq == 1) {
-                        iK = kt == 1 ? kt_index(S, s) : -1;
-                        und = iK < 0;
-                    }
-                    if (c3 == 1 && !und) {
-                        int iK2 = 0;
-                        if (decide_bins(S, s, iK2, bin)) {
-                            slot = iK2;
-                            if (AZ) {
-                                const int ip = kphi_screen(S, s);
-                                slot = ip < 0 ? -1 : iK2 * d.g.n_Kphi + ip;
-                            }
-                        }
-                        und = slot < 0;
-                    }
-                    und = und || c3 == 2 || cq == 2;
-                }
-            }
-            const bool take = valid && (und || c3 == 1 || cq == 1);
-            const unsigned x = e | (und ? 1u << 17 : 0u) | (!und && c3 == 1 ? 1u << 18 : 0u) |
-                               (!und && cq == 1 ? 1u << 19 : 0u);
-            const uint4 ent = make_uint4(x, (unsigned)bin,
-                                         (unsigned)(slot < 0 ? 0 : slot) |
-                                             ((unsigned)(iK < 0 ? 0 : iK) << 16),
-                                         (unsigned)kq);
-            enqueue(q2, count2, take, ent, lane, values_q);
-        };
-
-        for (int jj = 0; jj < jend; jj++) {
-            const long long j = j0 + jj;
-            const bool swap = oa > sm.oj[jj];
-            const bool take = i < n && j > i &&
-                              (prefilter<BOOST>(S, a, ga, sm.fj[jj], sm.gj[jj]) ||
-                               prefilter_qinv(S, a, sm.fj[jj]));
-            enqueue(q, count, take,
-                    (unsigned)il | ((unsigned)jj << 8) | ((swap ? 1u : 0u) << 16), lane,
-                    screen_q);
+        for (int f = 0; f < 8; f++) {
+            const double u = PREC == 0 ? sm.si[f][qi] : c[f][i0 + qi];
+            const double v = PREC == 0 ? sm.sj[f][qj] : c[f][j0 + qj];
+            A[f] = swap ? v : u;
+            B[f] = swap ? u : v;
         }
-        drain(q, count, lane, screen_q);
-        drain(q2, count2, lane, values_q);
-        drain(q3, count3, lane, chains_q);
-    } else {
-        unsigned *q3 = sm.queue3[w];
-        int count3 = 0;
-        // stage D for 32 pairs the screen left undecided: the reference chain
-        // decides them (and may hand a K_phi edge to the host), from the FP64
-        // tile or (FP32-weight and double-float forms) the FP64 columns
-        auto chains = [&](unsigned e, bool valid) {
-            if (!valid) return;
-            const int qi = e & 0xff, qj = (e >> 8) & 0xff;
-            const bool swap = (e >> 16) & 1u;
-            double A[8], B[8];  // first and second particle of the pair
+        if (MODE == MODE_FAST) {
+            undecided_pair_ordered<false, MODE_FAST>(d, A, B, i0 + qi, j0 + qj, n, n);
+        } else {
+            const long long oa = sm.oi[qi], ob = sm.oj[qj];
+            const long long row = oa < ob ? oa : ob, col = oa < ob ? ob : oa;
+            undecided_pair_ordered<false, MODE>(d, A, B, row, col, n, n);
+        }
+    };
+    auto values_q = [&](uint4 e4, bool valid) {
+        // this lane's q_inv event, added per group of lanes at the end
+        unsigned qkey = 0xffffffffu;
+        double qsum = 0.0, qw = 0.0;
+        const unsigned e = e4.x;
+        const int qi = e & 0xff, qj = (e >> 8) & 0xff;
+        const bool swap = (e >> 16) & 1u;
+        bool has3 = valid && ((e >> 18) & 1u), hasq = valid && ((e >> 19) & 1u);
+        const int bin = (int)e4.y, slot = (int)(e4.z & 0xffffu), iK = (int)(e4.z >> 16);
+        const int kq = (int)e4.w;
+        double A[8], B[8];  // first and second particle of the pair
 #pragma unroll
-            for (int f = 0; f < 8; f++) {
-                const double u = PREC == 0 ? sm.si[f][qi] : c[f][i0 + qi];
-                const double v = PREC == 0 ? sm.sj[f][qj] : c[f][j0 + qj];
-                A[f] = swap ? v : u;
-                B[f] = swap ? u : v;
-            }
-            if (MODE != MODE_FAST) {
-                const long long oa = sm.oi[qi], ob = sm.oj[qj];
-                const long long row = oa < ob ? oa : ob, col = oa < ob ? ob : oa;
-                undecided_pair_ordered<false, MODE>(d, A, B, row, col, n, n);
-                return;
-            }
-            if (PREC == 1)
-                undecided_pair32<BOOST>(d, A, B, i0 + qi, j0 + qj, n);
-            else
-                undecided_pair64(d, A, B, i0 + qi, j0 + qj, n);
-        };
-
-        // stage C for one decided pair: its values into its bin
-        auto decided = [&](uint2 e2) {
-            const unsigned e = e2.x;
-            const int qi = e & 0xff, qj = (e >> 8) & 0xff;
-            const bool swap = (e >> 16) & 1u;
-            const int slot = (int)(e >> 18);
-            const int bin = (int)e2.y;
-            if (MODE != MODE_FAST) {
-                const long long oa = sm.oi[qi], ob = sm.oj[qj];
-                const long long row = oa < ob ? oa : ob;
-                if (!admit<MODE>(d, slot, row, n)) return;
-            }
+        for (int f = 0; f < 8; f++) {
+            const double u = PREC == 0 ? sm.si[f][qi] : c[f][i0 + qi];
+            const double v = PREC == 0 ? sm.sj[f][qj] : c[f][j0 + qj];
+            A[f] = swap ? v : u;
+            B[f] = swap ? u : v;
+        }
+        const long long oa = sm.oi[qi], ob = sm.oj[qj];
+        const long long row = oa < ob ? oa : ob;
+        // undecided: both events wait for the reference chain (stage D)
+        const bool undecided = valid && ((e >> 17) & 1u);
+        if (undecided) has3 = hasq = false;
+        if (MODE != MODE_FAST) {
+            has3 = has3 && admit<MODE>(d, slot, row, n);
+            hasq = hasq && admit<MODE>(d, d.g.n_slots + iK, row, n);
+        }
+        if (has3 || hasq) {
+            const long long at = (long long)slot * d.g.q3 + bin;
+            double wq;
             if (PREC == 1) {
-                // the pair as stored (i, j); swapping first and second negates
-                // q_out, q_side, q_long exactly and leaves the phase unchanged
                 float2 a[8], b[8];
 #pragma unroll
                 for (int f = 0; f < 8; f++) {
@@ -1238,92 +1342,111 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SmemFor<QINV> &s
                     v.y = -v.y;
                     v.z = -v.z;
                 }
-                const long long at = (long long)slot * d.g.q3 + bin;
-                atomicAdd(partials_of(d) + at, v);
-                atomicAdd(d.h.cnt + at, 1ull);
-                return;
-            }
-            double vo, vs, vl, vw;
-            if (PREC == 2) {
-                float2 a[8], b[8];
-#pragma unroll
-                for (int f = 0; f < 8; f++) {
-                    a[f] = spi[f][qi];
-                    b[f] = spj[f][qj];
+                if (has3) {
+                    atomicAdd(partials_of(d) + at, v);
+                    atomicAdd(d.h.cnt + at, 1ull);
                 }
-                values_df<BOOST>(d.s, reinterpret_cast<const float4 *>(cs), a, b, sm.offi, sm.offj,
-                                 swap, vo, vs, vl, vw);
+                wq = v.w;
             } else {
-                // the pair in the reference's orientation, from the FP64 tile
-                // (the two rows chosen once, then read column by column)
-                const double *ra = swap ? &sm.sj[0][qj] : &sm.si[0][qi];
-                const double *rb = swap ? &sm.si[0][qi] : &sm.sj[0][qj];
-                double A[8], B[8];
+                double vo, vs, vl;
+                if (PREC == 0) {
+                    FF sz = {0.0f, 0.0f}, sE = {0.0f, 0.0f};
+                    if (BOOST) {
+                        const float4 fa = sm.fi[qi], fb = sm.fj[qj];
+                        const float2 la = sm.li[qi], lb = sm.lj[qj];
+                        sz = ff_sum(make_float2(fa.z, la.x), make_float2(fb.z, lb.x));
+                        sE = ff_sum(make_float2(fa.w, la.y), make_float2(fb.w, lb.y));
+                    }
+                    values64<BOOST>(d.g, cs, A, B, sz, sE, vo, vs, vl, wq);
+                } else {
+                    float2 a[8], b[8];
 #pragma unroll
-                for (int f = 0; f < 8; f++) {
-                    A[f] = ra[f * FT];
-                    B[f] = rb[f * FT];
+                    for (int f = 0; f < 8; f++) {
+                        a[f] = spi[f][qi];
+                        b[f] = spj[f][qj];
+                    }
+                    values_df<BOOST>(d.s, reinterpret_cast<const float4 *>(cs), a, b,
+                                     sm.offi, sm.offj, swap, vo, vs, vl, wq);
                 }
-                FF sz = {0.0f, 0.0f}, sE = {0.0f, 0.0f};
-                if (BOOST) {
-                    const float4 fa = sm.fi[qi], fb = sm.fj[qj];
-                    const float2 la = sm.li[qi], lb = sm.lj[qj];
-                    sz = ff_sum(make_float2(fa.z, la.x), make_float2(fb.z, lb.x));
-                    sE = ff_sum(make_float2(fa.w, la.y), make_float2(fb.w, lb.y));
-                }
-                values64<BOOST>(d.g, cs, A, B, sz, sE, vo, vs, vl, vw);
-            }
-            const long long at = (long long)slot * d.g.q3 + bin;
-            Sums *h = d.h.sums + at;
-            atomicAdd(&h->qo, vo);
-            atomicAdd(&h->qs, vs);
-            atomicAdd(&h->ql, vl);
-            atomicAdd(&h->w, vw);
-            atomicAdd(d.h.cnt + at, 1ull);
-        };
-
-        // stage C for 32 screened pairs (all lanes of the warp in step): the
-        // decided pairs' values, then the undecided ones to stage D's queue
-        // (last, so that stage D runs with nothing of stage C live)
-        auto values = [&](uint2 e2, bool valid) {
-            const bool undecided = valid && ((e2.x >> 17) & 1u);
-            if (valid && !undecided) decided(e2);
-            enqueue(q3, count3, undecided, e2.x & 0x1ffffu, lane, chains);
-        };
-
-        // stage B for 32 prefiltered pairs: window screen and bins; the pairs
-        // inside the window (or undecided) go to the second queue
-        auto screen = [&](unsigned e, bool valid) {
-            const int qi = e & 0xff, qj = (e >> 8) & 0xff;
-            const bool swap = (e >> 16) & 1u;
-            Q s;
-            int wcls = 0;
-            if (valid)
-                wcls = swap ? screen_windows<BOOST>(S, sm.fj[qj], sm.fi[qi], s)
-                            : screen_windows<BOOST>(S, sm.fi[qi], sm.fj[qj], s);
-            int iK = 0, bin = 0, slot = -1;
-            if (wcls == 1 && decide_bins(S, s, iK, bin)) {
-                slot = iK;
-                if (AZ) {
-                    const int ip = kphi_screen(S, s);
-                    slot = ip < 0 ? -1 : iK * d.g.n_Kphi + ip;
+                if (has3) {
+                    Sums *h = d.h.sums + at;
+                    atomicAdd(&h->qo, vo);
+                    atomicAdd(&h->qs, vs);
+                    atomicAdd(&h->ql, vl);
+                    atomicAdd(&h->w, wq);
+                    atomicAdd(d.h.cnt + at, 1ull);
                 }
             }
-            enqueue(q2, count2, wcls != 0, bin_entry(e, slot < 0, slot < 0 ? 0 : slot, bin), lane,
-                    values);
-        };
-
-        for (int jj = 0; jj < jend; jj++) {
-            const long long j = j0 + jj;
-            const bool swap = oa > sm.oj[jj];
-            const bool take = i < n && j > i && prefilter<BOOST>(S, a, ga, sm.fj[jj], sm.gj[jj]);
-            enqueue(q, count, take,
-                    (unsigned)il | ((unsigned)jj << 8) | ((swap ? 1u : 0u) << 16), lane, screen);
+            if (hasq) {
+                // the reference's q_inv expression (FP64, same order, no
+                // contraction): the summed value equals the oracle's
+                const double q_x = A[0] - B[0], q_y = A[1] - B[1], q_z = A[2] - B[2];
+                const double q_E = A[3] - B[3];
+                qsum = sqrt(-(q_E * q_E - q_x * q_x - q_y * q_y - q_z * q_z));
+                qw = wq;
+                qkey = (unsigned)(iK * d.g.qnpts + kq);
+            }
         }
-        drain(q, count, lane, screen);
-        drain(q2, count2, lane, values);
-        drain(q3, count3, lane, chains);
+        qinv_update(d, qkey, qsum, qw, true);
+        enqueue(q3, count3, undecided, e & 0x1ffffu, lane, chains_q);
+    };
+
+    // stage B with q_inv histograms: the K_T window and bin, the 3-D
+    // windows and bins, and the q_inv window and bin of each pair; a pair
+    // with any of them undecided goes to the reference chain as a whole
+    auto screen_q = [&](unsigned e, bool valid) {
+        const int qi = e & 0xff, qj = (e >> 8) & 0xff;
+        const bool swap = (e >> 16) & 1u;
+        const float4 fa = swap ? sm.fj[qj] : sm.fi[qi], fb = swap ? sm.fi[qi] : sm.fj[qj];
+        Q s;
+        int c3 = 0, cq = 0, iK = -1, bin = 0, slot = -1, kq = 0;
+        bool und = false;
+        if (valid) {
+            const int kt = screen_kt(S, fa, fb, s);
+            if (kt != 0) {
+                c3 = screen_lcms<BOOST>(S, fa, fb, s);
+                cq = qinv_class(S, fa, fb, kq);
+                if (c3 == 1 || cq == 1) {
+                    iK = kt == 1 ? kt_index(S, s) : -1;
+                    und = iK < 0;
+                }
+                if (c3 == 1 && !und) {
+                    int iK2 = 0;
+                    if (decide_bins(S, s, iK2, bin)) {
+                        slot = iK2;
+                        if (AZ) {
+                            const int ip = kphi_screen(S, s);
+                            slot = ip < 0 ? -1 : iK2 * d.g.n_Kphi + ip;
+                        }
+                    }
+                    und = slot < 0;
+                }
+                und = und || c3 == 2 || cq == 2;
+            }
+        }
+        const bool take = valid && (und || c3 == 1 || cq == 1);
+        const unsigned x = e | (und ? 1u << 17 : 0u) | (!und && c3 == 1 ? 1u << 18 : 0u) |
+                           (!und && cq == 1 ? 1u << 19 : 0u);
+        const uint4 ent = make_uint4(x, (unsigned)bin,
+                                     (unsigned)(slot < 0 ? 0 : slot) |
+                                         ((unsigned)(iK < 0 ? 0 : iK) << 16),
+                                     (unsigned)kq);
+        enqueue(q2, count2, take, ent, lane, values_q);
+    };
+
+    for (int jj = 0; jj < jend; jj++) {
+        const long long j = j0 + jj;
+        const bool swap = oa > sm.oj[jj];
+        const bool take = i < n && j > i &&
+                          (prefilter<BOOST>(S, a, ga, sm.fj[jj], sm.gj[jj]) ||
+                           prefilter_qinv(S, a, sm.fj[jj]));
+        enqueue(q, count, take,
+                (unsigned)il | ((unsigned)jj << 8) | ((swap ? 1u : 0u) << 16), lane,
+                screen_q);
     }
+    drain(q, count, lane, screen_q);
+    drain(q2, count2, lane, values_q);
+    drain(q3, count3, lane, chains_q);
 }
 
 // Mixed-event pairs of the list-1 tile at i0 (n1 particles, columns l1 =
@@ -1331,8 +1454,8 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SmemFor<QINV> &s
 // ordered cap admission (MODE COUNT / ORDER) a pair's row and column are
 // its positions in the caller's lists, orig1 / orig2 (nullptr: the rows are
 // in the caller's order).
-template <bool AZ, bool BOOST, int MODE = MODE_FAST, bool QINV = false, class SM = TileSmem>
-__device__ __forceinline__ void mixed_tile_pair(const Device &d, SM &sm,
+template <bool AZ, bool BOOST, int MODE = MODE_FAST>
+__device__ __forceinline__ void mixed_tile_pair_qinv(const Device &d, QinvSmem &sm,
                                                 const double *const *l1, long long n1,
                                                 const double *const *l2, long long n2,
                                                 long long i0, long long j0,
@@ -1380,97 +1503,59 @@ __device__ __forceinline__ void mixed_tile_pair(const Device &d, SM &sm,
         }
     };
 
-    // one screened pair: its denominator bin, or undecided (true)
-    auto screened = [&](unsigned e) -> bool {
+    // with q_inv histograms: the 3-D and the q_inv denominator events
+    auto process_q = [&](unsigned e, bool valid) {
         const int qi = e & 0xff, qj = (e >> 8) & 0xff;
-        Q s;
-        const int wcls = screen_windows<BOOST>(S, sm.fi[qi], sm.fj[qj], s);
-        if (wcls == 0) return false;
-        int iK = 0, bin = 0, slot = -1;
-        if (wcls == 1 && decide_bins(S, s, iK, bin)) {
-            slot = iK;
-            if (AZ) {
-                const int ip = kphi_screen(S, s);
-                slot = ip < 0 ? -1 : iK * d.g.n_Kphi + ip;
+        unsigned qkey = 0xffffffffu;  // this lane's q_inv denominator bin
+        bool undecided = false;       // both events wait for the chain
+        if (valid) {
+            Q s;
+            const int kt = screen_kt(S, sm.fi[qi], sm.fj[qj], s);
+            int c3 = 0, cq = 0, kq = 0, iK = -1, bin = 0, slot = -1;
+            if (kt != 0) {
+                c3 = screen_lcms<BOOST>(S, sm.fi[qi], sm.fj[qj], s);
+                cq = qinv_class(S, sm.fi[qi], sm.fj[qj], kq);
+            }
+            bool und = false;
+            if (c3 == 1 || cq == 1) {
+                iK = kt == 1 ? kt_index(S, s) : -1;
+                und = iK < 0;
+            }
+            if (c3 == 1 && !und) {
+                int iK2 = 0;
+                if (decide_bins(S, s, iK2, bin)) {
+                    slot = iK2;
+                    if (AZ) {
+                        const int ip = kphi_screen(S, s);
+                        slot = ip < 0 ? -1 : iK2 * d.g.n_Kphi + ip;
+                    }
+                }
+                und = slot < 0;
+            }
+            und = und || c3 == 2 || cq == 2;
+            const long long row = row_base + (orig1 ? (long long)orig1[i0 + qi] : i0 + qi);
+            undecided = und;
+            if (!und) {
+                bool h3 = c3 == 1, hq = cq == 1;
+                if (MODE != MODE_FAST) {
+                    h3 = h3 && admit<MODE>(d, slot, row, rows);
+                    hq = hq && admit<MODE>(d, d.g.n_slots + iK, row, rows);
+                }
+                if (h3) atomicAdd(d.h.den + (long long)slot * d.g.q3 + bin, 1ull);
+                if (hq) qkey = (unsigned)(iK * d.g.qnpts + kq);
             }
         }
-        if (slot < 0) return true;
-        if (MODE != MODE_FAST) {
-            const long long row = row_base + (orig1 ? (long long)orig1[i0 + qi] : i0 + qi);
-            if (!admit<MODE>(d, slot, row, rows)) return false;
-        }
-        atomicAdd(d.h.den + (long long)slot * d.g.q3 + bin, 1ull);
-        return false;
-    };
-
-    // 32 prefiltered pairs (all lanes of the warp in step)
-    auto process = [&](unsigned e, bool valid) {
-        const bool undecided = valid && screened(e);
+        qinv_update(d, qkey, 0.0, 0.0, false);
         enqueue(q3, count3, undecided, e, lane, chains);
     };
 
-    if constexpr (QINV) {
-        // with q_inv histograms: the 3-D and the q_inv denominator events
-        auto process_q = [&](unsigned e, bool valid) {
-            const int qi = e & 0xff, qj = (e >> 8) & 0xff;
-            unsigned qkey = 0xffffffffu;  // this lane's q_inv denominator bin
-            bool undecided = false;       // both events wait for the chain
-            if (valid) {
-                Q s;
-                const int kt = screen_kt(S, sm.fi[qi], sm.fj[qj], s);
-                int c3 = 0, cq = 0, kq = 0, iK = -1, bin = 0, slot = -1;
-                if (kt != 0) {
-                    c3 = screen_lcms<BOOST>(S, sm.fi[qi], sm.fj[qj], s);
-                    cq = qinv_class(S, sm.fi[qi], sm.fj[qj], kq);
-                }
-                bool und = false;
-                if (c3 == 1 || cq == 1) {
-                    iK = kt == 1 ? kt_index(S, s) : -1;
-                    und = iK < 0;
-                }
-                if (c3 == 1 && !und) {
-                    int iK2 = 0;
-                    if (decide_bins(S, s, iK2, bin)) {
-                        slot = iK2;
-                        if (AZ) {
-                            const int ip = kphi_screen(S, s);
-                            slot = ip < 0 ? -1 : iK2 * d.g.n_Kphi + ip;
-                        }
-                    }
-                    und = slot < 0;
-                }
-                und = und || c3 == 2 || cq == 2;
-                const long long row = row_base + (orig1 ? (long long)orig1[i0 + qi] : i0 + qi);
-                undecided = und;
-                if (!und) {
-                    bool h3 = c3 == 1, hq = cq == 1;
-                    if (MODE != MODE_FAST) {
-                        h3 = h3 && admit<MODE>(d, slot, row, rows);
-                        hq = hq && admit<MODE>(d, d.g.n_slots + iK, row, rows);
-                    }
-                    if (h3) atomicAdd(d.h.den + (long long)slot * d.g.q3 + bin, 1ull);
-                    if (hq) qkey = (unsigned)(iK * d.g.qnpts + kq);
-                }
-            }
-            qinv_update(d, qkey, 0.0, 0.0, false);
-            enqueue(q3, count3, undecided, e, lane, chains);
-        };
-
-        for (int jj = 0; jj < jend; jj++) {
-            const bool take = active && (prefilter<BOOST>(S, a, ga, sm.fj[jj], sm.gj[jj]) ||
-                                         prefilter_qinv(S, a, sm.fj[jj]));
-            enqueue(q, count, take, (unsigned)il | ((unsigned)jj << 8), lane, process_q);
-        }
-        drain(q, count, lane, process_q);
-        drain(q3, count3, lane, chains);
-    } else {
-        for (int jj = 0; jj < jend; jj++) {
-            const bool take = active && prefilter<BOOST>(S, a, ga, sm.fj[jj], sm.gj[jj]);
-            enqueue(q, count, take, (unsigned)il | ((unsigned)jj << 8), lane, process);
-        }
-        drain(q, count, lane, process);
-        drain(q3, count3, lane, chains);
+    for (int jj = 0; jj < jend; jj++) {
+        const bool take = active && (prefilter<BOOST>(S, a, ga, sm.fj[jj], sm.gj[jj]) ||
+                                     prefilter_qinv(S, a, sm.fj[jj]));
+        enqueue(q, count, take, (unsigned)il | ((unsigned)jj << 8), lane, process_q);
     }
+    drain(q, count, lane, process_q);
+    drain(q3, count3, lane, chains);
 }
 
 }  // namespace tile
