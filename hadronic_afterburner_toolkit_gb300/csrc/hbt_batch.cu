@@ -83,13 +83,31 @@ __global__ void k_keys(BatchDev b) {
     }
 }
 
-__global__ void k_gather(BatchDev b) {
+// Sorted rows, and each row's screen terms and fixed-point columns (once per
+// particle here; a tile pair would convert its 256 particles again each time
+// it is taken).
+template <bool BOOST>
+__global__ void k_gather(BatchDev b, Grid g) {
     for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < b.total;
          s += (long long)gridDim.x * blockDim.x) {
         const int L = (int)(b.keys_out[s] >> 32);
         const BatchList &l = b.lists[L];
         const long long k = (long long)b.vals_out[s] - l.off;
-        for (int f = 0; f < l.ncols; f++) b.table[(long long)f * b.cap + s] = l.src[f][k];
+        double v[8];
+#pragma unroll
+        for (int f = 0; f < 8; f++)
+            if (f < l.ncols) {
+                v[f] = l.src[f][k];
+                b.table[(long long)f * b.cap + s] = v[f];
+            }
+        const Terms t = screen_terms<BOOST>(v[0], v[1], v[2], v[3]);
+        b.terms4[s] = make_float4(t.x, t.y, t.m, t.p);
+        b.terms2[s] = make_float2(t.r2, t.t2);
+        if (l.ncols == 8) {
+            const FixedCols c = fixed_cols(g, v);
+#pragma unroll
+            for (int f = 0; f < 4; f++) b.fixed[(long long)f * b.cap + s] = c.c[f];
+        }
         b.orig[s] = (unsigned)k;  // position in the caller's list (pair orientation)
     }
 }
@@ -342,7 +360,10 @@ cudaError_t run_batch(const Device &d, const BatchDev &b, int grid, unsigned chu
         e = cub::DeviceRadixSort::SortPairs(b.sort_temp, bytes, b.keys_in, b.keys_out, b.vals_in,
                                             b.vals_out, (int)b.total, 0, end_bit, st);
         if (e != cudaSuccess) return e;
-        k_gather<<<gs, 256, 0, st>>>(b);
+        if (d.g.boost)
+            k_gather<true><<<gs, 256, 0, st>>>(b, d.g);
+        else
+            k_gather<false><<<gs, 256, 0, st>>>(b, d.g);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         k_boxes<<<(unsigned)((b.total_tiles * 32 + 255) / 256), 256, 0, st>>>(b);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;

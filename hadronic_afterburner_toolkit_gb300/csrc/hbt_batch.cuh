@@ -64,6 +64,12 @@ struct BatchDev {
     long long cap;          // row capacity of the sorted table
     double *table;          // [8][cap] sorted particle table
     unsigned *orig;         // [cap] each row's position in the caller's list
+    // per row: the fixed-point columns of same-event lists ([4][cap],
+    // hbt_fixed.cuh) and the screen's terms (x, y, m, p) and (r2, t2)
+    // (hbt_screen.cuh), converted once per batch
+    int4 *fixed;
+    float4 *terms4;
+    float2 *terms2;
     unsigned long long *keys_in, *keys_out;
     unsigned *vals_in, *vals_out;
     void *sort_temp;

@@ -793,6 +793,12 @@ void grid_from_params(const hbt_params &p, Grid &g) {
     g.kphi_tol = p.kphi_defer_tol > 0 ? p.kphi_defer_tol : 1e-13;
     g.hbarC_inv = 1. / hbt::kHbarC;
     g.cph = make_cos_scale(g.hbarC_inv);
+    const double turn_h = 0.15915494309189535, turn_l = -9.839338337591243e-18;  // 1 / (2 pi)
+    const double turns = g.hbarC_inv * turn_h;
+    const double rest = std::fma(g.hbarC_inv, turn_h, -turns) + g.hbarC_inv * turn_l;
+    g.pos_h = std::ldexp(turns, 20);
+    g.pos_l = std::ldexp(rest, 20);
+    g.cfx = make_cos_scale(std::ldexp(6.283185307179586 / 512.0, -52));
 }
 
 // The margins of the tile screen (hbt_screen.cuh derives them).

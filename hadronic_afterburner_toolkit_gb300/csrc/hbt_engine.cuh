@@ -25,6 +25,10 @@ struct Grid {
     double dKphi, two_pi, psi_ref, kphi_tol;
     double hbarC_inv;
     CosScale cph;  // table_cos constants for cos(q.dx / hbarC)
+    // fixed-point pair values (hbt_fixed.cuh): 2^20 / (2 pi hbarC) in two
+    // parts, and the cosine's coefficients in 2^-52 table steps
+    double pos_h, pos_l;
+    CosScale cfx;
 };
 
 // Per-bin numerator sums, one 32-byte L2 sector per bin.

@@ -22,7 +22,8 @@ __global__ void __launch_bounds__(FT) k_same_screened(Device d, long long n, Col
     if (PREC == 2) fill_df_table(reinterpret_cast<float4 *>(cs));
     long long ti, tj;
     tri_tile((long long)blockIdx.x + d.block_offset, ti, tj);
-    same_tile_pair<AZ, BOOST, PREC>(d, sm, cs, c.p, nullptr, n, ti * FT, tj * FT);
+    const ListRows l = {c.p, nullptr, nullptr, nullptr, nullptr, 0, n};
+    same_tile_pair<AZ, BOOST, PREC>(d, sm, cs, l, ti * FT, tj * FT);
 }
 
 template <bool AZ, bool BOOST>
@@ -30,7 +31,9 @@ __global__ void __launch_bounds__(FT) k_mixed_screened(Device d, long long n1, C
                                                        long long n2, Cols4 l2, long long tiles1) {
     __shared__ MixedSmem sm;
     const long long ti = blockIdx.x % tiles1, tj = blockIdx.x / tiles1;
-    mixed_tile_pair<AZ, BOOST>(d, sm, l1.p, n1, l2.p, n2, ti * FT, tj * FT);
+    const ListRows a = {l1.p, nullptr, nullptr, nullptr, nullptr, 0, n1};
+    const ListRows b = {l2.p, nullptr, nullptr, nullptr, nullptr, 0, n2};
+    mixed_tile_pair<AZ, BOOST>(d, sm, a, b, ti * FT, tj * FT);
 }
 
 }  // namespace

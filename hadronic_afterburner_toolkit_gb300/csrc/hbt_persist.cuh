@@ -82,35 +82,36 @@ constexpr int kMixedCtas = HBT_MIXED_CTAS;
 // of its shared memory.
 template <bool AZ, bool BOOST, int PREC, int MODE>
 __device__ __forceinline__ void same_item(const Device &d, SameSmem &sm, const double2 *cs,
-                                          const double *const *c, const unsigned *orig,
-                                          long long n, const Item &it) {
-    same_tile_pair<AZ, BOOST, PREC, MODE>(d, sm, cs, c, orig, n, (long long)it.ti * FT,
+                                          const ListRows &l, const Item &it) {
+    same_tile_pair<AZ, BOOST, PREC, MODE>(d, sm, cs, l, (long long)it.ti * FT,
                                           (long long)it.tj * FT);
 }
 template <bool AZ, bool BOOST, int PREC, int MODE>
 __device__ __forceinline__ void same_item(const Device &d, QinvSmem &sm, const double2 *cs,
-                                          const double *const *c, const unsigned *orig,
-                                          long long n, const Item &it) {
-    same_tile_pair_qinv<AZ, BOOST, PREC, MODE>(d, sm, cs, c, orig, n, (long long)it.ti * FT,
-                                               (long long)it.tj * FT);
+                                          const ListRows &l, const Item &it) {
+    same_tile_pair_qinv<AZ, BOOST, PREC, MODE>(d, sm, cs, l.c, l.orig, l.n,
+                                               (long long)it.ti * FT, (long long)it.tj * FT);
 }
 template <bool AZ, bool BOOST, int MODE>
-__device__ __forceinline__ void mixed_item(const Device &d, MixedSmem &sm,
-                                           const double *const *l1, long long n1,
-                                           const double *const *l2, long long n2, const Item &it,
-                                           const unsigned *o1, const unsigned *o2,
+__device__ __forceinline__ void mixed_item(const Device &d, MixedSmem &sm, const ListRows &l1,
+                                           const ListRows &l2, const Item &it,
                                            long long row_base) {
-    mixed_tile_pair<AZ, BOOST, MODE>(d, sm, l1, n1, l2, n2, (long long)it.ti * FT,
-                                     (long long)it.tj * FT, o1, o2, row_base);
+    mixed_tile_pair<AZ, BOOST, MODE>(d, sm, l1, l2, (long long)it.ti * FT, (long long)it.tj * FT,
+                                     row_base);
 }
 template <bool AZ, bool BOOST, int MODE>
-__device__ __forceinline__ void mixed_item(const Device &d, QinvSmem &sm,
-                                           const double *const *l1, long long n1,
-                                           const double *const *l2, long long n2, const Item &it,
-                                           const unsigned *o1, const unsigned *o2,
+__device__ __forceinline__ void mixed_item(const Device &d, QinvSmem &sm, const ListRows &l1,
+                                           const ListRows &l2, const Item &it,
                                            long long row_base) {
-    mixed_tile_pair_qinv<AZ, BOOST, MODE>(d, sm, l1, n1, l2, n2, (long long)it.ti * FT,
-                                          (long long)it.tj * FT, o1, o2, row_base);
+    mixed_tile_pair_qinv<AZ, BOOST, MODE>(d, sm, l1.c, l1.n, l2.c, l2.n, (long long)it.ti * FT,
+                                          (long long)it.tj * FT, l1.orig, l2.orig, row_base);
+}
+
+// A list of the batch as the tile kernels read it (c: its column pointers).
+__device__ __forceinline__ ListRows rows_of(const BatchDev &b, const BatchList &l,
+                                            const double *const *c) {
+    return ListRows{c,    b.orig + l.off, b.fixed + l.off, b.terms4 + l.off, b.terms2 + l.off,
+                    b.cap, l.n};
 }
 
 // Same-event items [base, min(end, queued)) pulled by persistent CTAs.
@@ -139,9 +140,9 @@ __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(D
         if constexpr (MANY) {
             __shared__ Device dsm;
             load_device(b, job, dsm);
-            same_item<AZ, BOOST, PREC, MODE>(dsm, sm, cs, c, b.orig + la.off, la.n, it);
+            same_item<AZ, BOOST, PREC, MODE>(dsm, sm, cs, rows_of(b, la, c), it);
         } else {
-            same_item<AZ, BOOST, PREC, MODE>(d, sm, cs, c, b.orig + la.off, la.n, it);
+            same_item<AZ, BOOST, PREC, MODE>(d, sm, cs, rows_of(b, la, c), it);
         }
         __syncthreads();
     }
@@ -170,11 +171,11 @@ __global__ void __launch_bounds__(FT, kMixedCtas) k_persistent_mixed(Device d, B
         if constexpr (MANY) {
             __shared__ Device dsm;
             load_device(b, job, dsm);
-            mixed_item<AZ, BOOST, MODE>(dsm, sm, c1, la.n, c2, lb.n, it, b.orig + la.off,
-                                        b.orig + lb.off, job.row_base);
+            mixed_item<AZ, BOOST, MODE>(dsm, sm, rows_of(b, la, c1), rows_of(b, lb, c2), it,
+                                        job.row_base);
         } else {
-            mixed_item<AZ, BOOST, MODE>(d, sm, c1, la.n, c2, lb.n, it, b.orig + la.off,
-                                        b.orig + lb.off, job.row_base);
+            mixed_item<AZ, BOOST, MODE>(d, sm, rows_of(b, la, c1), rows_of(b, lb, c2), it,
+                                        job.row_base);
         }
         __syncthreads();
     }

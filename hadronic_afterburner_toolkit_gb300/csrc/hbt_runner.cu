@@ -12,7 +12,7 @@ BatchRunner::~BatchRunner() {
     for (cudaEvent_t e : marks_)
         if (e) cudaEventDestroy(e);
     Buf *all[] = {&lists_, &jobs_, &offs_, &table_, &keys_, &vals_, &sort_temp_, &boxes_,
-                  &items_, &counters_, &devs_, &item_order_, &item_sort_temp_};
+                  &items_, &counters_, &devs_, &item_order_, &item_sort_temp_, &fixed_, &terms_};
     for (Buf *b : all)
         if (b->p) cudaFree(b->p);
 }
@@ -229,6 +229,8 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
         !grow(jobs_, bj.size() * sizeof(BatchJob), err) ||
         !grow(offs_, (2 * lists.size() + bj.size()) * sizeof(long long), err) ||
         !grow(table_, (size_t)8 * total * sizeof(double), err) ||
+        !grow(fixed_, (size_t)4 * total * sizeof(int4), err) ||
+        !grow(terms_, (size_t)total * (sizeof(float4) + sizeof(float2)), err) ||
         !grow(keys_, (size_t)2 * total * sizeof(unsigned long long), err) ||
         !grow(vals_, (size_t)3 * total * sizeof(unsigned), err) ||
         !grow(sort_temp_, sort_bytes, err) || !grow(boxes_, (size_t)tiles * sizeof(Box), err) ||
@@ -266,6 +268,9 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
     b.total_pairs = pairs;
     b.cap = total;
     b.table = static_cast<double *>(table_.p);
+    b.fixed = static_cast<int4 *>(fixed_.p);
+    b.terms4 = static_cast<float4 *>(terms_.p);
+    b.terms2 = reinterpret_cast<float2 *>(b.terms4 + total);
     b.keys_in = static_cast<unsigned long long *>(keys_.p);
     b.keys_out = b.keys_in + total;
     b.vals_in = static_cast<unsigned *>(vals_.p);

@@ -11,12 +11,13 @@
 //     FP32 with error bounds (slot_of).
 //  C. Histogram update.  Mixed pairs add 1 to their denominator bin.
 //     Same-event pairs add q_out, q_side, q_long and cos(q.dx / hbarC):
-//       FP64 form  - the phase q.dx and its cos in FP64 (table_cos,
-//                    hbt_math.cuh, of the unrounded product with 1/hbarC);
-//                    q_out, q_side, q_long from algebraically identical
-//                    expressions (q_out = (q_x S_x + q_y S_y) / |S|, ...) in
-//                    double-float on the FP32 pipe, from the FP64 sums and
-//                    differences (values64);
+//       FP64 form  - differences, sums and the phase q.dx exactly from
+//                    fixed-point columns (hbt_fixed.cuh, values_fixed), the
+//                    cos of its remainder to a table point in FP64; q_out,
+//                    q_side, q_long from algebraically identical expressions
+//                    (q_out = (q_x S_x + q_y S_y) / |S|, ...) in double-float
+//                    on the FP32 pipe; pairs of particles outside the
+//                    columns' range in FP64 (values64);
 //       FP32W form - each FP64 column split once per tile into hi + lo
 //                    FP32 parts; differences and the phase in double-float
 //                    arithmetic on the FP32 pipe, q values in FP32, cos by
@@ -36,8 +37,8 @@
 // Measured on the central group (150k pions, 5.4e9 pairs in the kept tile
 // pairs, 1.94e9 binned), whole passes, against a scalar prefilter, a queue
 // and a scalar window test with per-component bounds: FP32-weight form 118.0
-// -> 70.6 ms, FP64 form 143.6 -> 134.7 ms (bound by the FP64 pipe, so the
-// issue slots saved show less), double-float kaons 18.3 -> 16.1 ms.
+// -> 70.6 ms, FP64 form (still with FP64 values) 143.6 -> 134.7 ms, bound by
+// the FP64 pipe, so the issue slots saved showed less.
 //
 // The forms with q_inv histograms (same_tile_pair_qinv,
 // mixed_tile_pair_qinv) screen in two steps, a prefilter and a window test
@@ -55,6 +56,7 @@
 #include <type_traits>
 
 #include "hbt_chain.cuh"
+#include "hbt_fixed.cuh"
 #include "hbt_math.cuh"
 #include "hbt_screen.cuh"
 
@@ -679,37 +681,160 @@ __device__ __forceinline__ void values64(const Grid &g, const double2 *cs, const
     w = table_cos(cs, g.cph, ph);
 }
 
-// Shared memory of a same-event tile pair.
-struct SameSmem {
-    // FP64 columns px py pz E x y z t (FP64 form) or split columns ((hi, lo)
-    // FP32 pairs, the other forms)
+// values64 from the FP64 columns of rows i and j, in the reference's
+// orientation (`swap`: j first).  For the pairs of particles whose values do
+// not fit the fixed-point columns; out of line to keep its registers out of
+// the pair loop.
+template <bool BOOST>
+__device__ __noinline__ void values64_rows(const Grid &g, const double2 *cs,
+                                           const double *const *c, long long i, long long j,
+                                           bool swap, double &qo, double &qs, double &ql,
+                                           double &w) {
+    double a[8], b[8];
+#pragma unroll
+    for (int f = 0; f < 8; f++) {
+        const double u = c[f][i], v = c[f][j];
+        a[f] = swap ? v : u;
+        b[f] = swap ? u : v;
+    }
+    FF sz = {0.0f, 0.0f}, sE = {0.0f, 0.0f};
+    if (BOOST) {
+        sz = ff_sum(split(a[2]), split(b[2]));
+        sE = ff_sum(split(a[3]), split(b[3]));
+    }
+    values64<BOOST>(g, cs, a, b, sz, sE, qo, qs, ql, w);
+}
+
+// Limbs (h, l) of a difference or sum as a double-float in units of h: h in
+// two exact conversions, l below, normalised (of a small h, l is not below
+// the last bit, and ff_mul drops the product of the low parts).
+__device__ __forceinline__ FF limbs_ff(int h, int l) {
+    const float f = __int2float_rn(h);
+    const float r = __int2float_rn(h - __float2int_rn(f));
+    return fast_two_sum(f, __fmaf_rn(__int2float_rn(l), 0x1p-30f, r));
+}
+
+// hi + lo, in units of 2^-26 GeV, rounded once to FP64 in GeV, negated when
+// `neg` is the sign bit: both parts converted on the integer pipe (exponent
+// rebiased by 896 - 26; a zero part becomes a number below 1e-45, far under
+// the rounding of any sum it enters).
+__device__ __forceinline__ double ff_gev(FF a, unsigned neg) {
+    auto conv = [&](float x) {
+        const unsigned u = __float_as_uint(x) ^ neg;
+        return __hiloint2double((int)(((unsigned)((int)u >> 3) & 0x8fffffffu) + (870u << 20)),
+                                (int)(u << 29));
+    };
+    return conv(a.h) + conv(a.l);
+}
+
+// Summed values of an accepted same-event pair from its fixed-point columns
+// (hbt_fixed.cuh), a from the i-tile, b from the j-tile, negated in q when
+// `swap` (b is the pair's first particle).  The differences and sums are
+// exact; q_out, q_side and the boosted q_long, which are only summed, follow
+// in double-float (ff_lcms, about 1e-14 relative) and come back as FP64 with
+// one addition each.  The phase is summed from 32 x 32 bit products: with
+// the limbs (h, l) of a difference, sum of h h' (unit 2^-37 table steps),
+// h l' + l h' (2^-67) and l l' (2^-97).
+template <bool BOOST>
+__device__ __forceinline__ void values_fixed(const Grid &g, const double2 *cs, const FixedCols &a,
+                                             const FixedCols &b, bool swap, double &qo,
+                                             double &qs, double &ql, double &w) {
+    int h[8], l[8];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        h[2 * k] = a.c[k].x - b.c[k].x;
+        l[2 * k] = a.c[k].y - b.c[k].y;
+        h[2 * k + 1] = a.c[k].z - b.c[k].z;
+        l[2 * k + 1] = a.c[k].w - b.c[k].w;
+    }
+    long long hh = 0, hl = 0, ll = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        hh += (long long)h[k] * h[k + 4];
+        hl += (long long)h[k] * l[k + 4];
+        hl += (long long)l[k] * h[k + 4];
+        ll += (long long)l[k] * l[k + 4];
+    }
+    const unsigned neg = swap ? 0x80000000u : 0u;
+    {
+        FF dp[4], sp[4], vo, vs, vl;
+#pragma unroll
+        for (int f = 0; f < 4; f++) dp[f] = limbs_ff(h[f], l[f]);
+        sp[0] = limbs_ff(a.c[0].x + b.c[0].x, a.c[0].y + b.c[0].y);
+        sp[1] = limbs_ff(a.c[0].z + b.c[0].z, a.c[0].w + b.c[0].w);
+        if (BOOST) {
+            sp[2] = limbs_ff(a.c[1].x + b.c[1].x, a.c[1].y + b.c[1].y);
+            sp[3] = limbs_ff(a.c[1].z + b.c[1].z, a.c[1].w + b.c[1].w);
+        }
+        ff_lcms<BOOST>(dp, sp, vo, vs, vl);
+        qo = ff_gev(vo, neg);
+        qs = ff_gev(vs, neg);
+        ql = ff_gev(vl, neg);
+    }
+    // high part in 2^-37 steps, the rest in the low 30 bits of hl
+    hl += ll >> 30;
+    hh += hl >> 30;
+    const unsigned low = (unsigned)hl << 2;
+    const unsigned fl = (unsigned)hh;
+    const int top = (int)(hh >> 32) + 16;  // + half a step
+    const double2 e = cs[(top >> 5) & (COS_TABLE - 1)];
+    // the remainder, 37 + 15 bits signed, as an FP64 integer (2^-52 steps)
+    const int r = (top & 31) - 16;
+    const double t = __hiloint2double(0x43380000 + (int)__funnelshift_r(fl, (unsigned)r, 17),
+                                      (int)__funnelshift_l(low, fl, 15));
+    const double f = t - 6755399441055744.0;
+    const double f2 = f * f;
+    const double cd = __fma_rn(f2, __fma_rn(f2, g.cfx.c4, g.cfx.c2), 1.0);
+    const double sd = f * __fma_rn(f2, __fma_rn(f2, g.cfx.s5, g.cfx.s3), g.cfx.h);
+    w = __fma_rn(e.x, cd, -(e.y * sd));
+}
+
+// Shared memory of a same-event tile pair.  The i-tile's arrays hold row r at
+// place (r >> 2) + 32 (r & 3): warp w screens the rows w, w + 4, ... (sorted in
+// momentum space, so interleaving evens out the binned pairs between warps),
+// and lane k of it finds its row, and later the rows of neighbouring queue
+// entries, at consecutive places, without bank conflicts.
+struct __align__(16) SameSmem {
+    // FP64 form: fixed-point columns ([4][FT] of int4, FixedCols); the other
+    // forms: split columns ([8][FT] (hi, lo) FP32 pairs px py pz E x y z t)
     double si[8][FT];
     double sj[8][FT];
-    // FP64 form with the boost: p_z and E as (hi, lo) FP32 pairs, for the
-    // longitudinal sums in double-float
-    float4 zi[FT], zj[FT];
-    TermsPair ti[FT / 2], tj[FT / 2];  // screen terms
+    float4 ta[FT];  // the i-tile's screen terms x, y, m, p
+    float2 tb[FT];  // and r2, t2
+    TermsPair tj[FT / 2];
     // pairs past the screen (screen_loop): up to 31 left over and 64 of a step
     uint2 queue[FT / 32][96];
     // undecided pairs, (i, j) bits: the reference chain runs on them 32 at a
     // time (inline, a warp would run it for the one or two lanes holding one)
     unsigned queue3[FT / 32][QCAP];
-    __align__(8) unsigned oi[FT], oj[FT];  // original list positions (pair orientation)
-    float offi[4], offj[4];  // double-float form: the tiles' momentum offsets
+    unsigned oi[FT], oj[FT];  // original list positions (pair orientation)
+    float offi[4], offj[4];   // double-float form: the tiles' momentum offsets
+};
+// Place of row r in the i-tile's arrays, and back.
+__device__ __forceinline__ int place_of(int r) { return (r >> 2) | ((r & 3) << 5); }
+__device__ __forceinline__ int row_at(int s) { return ((s & 31) << 2) | (s >> 5); }
+
+// A particle list as the tile kernels read it: columns (px py pz E, and x y
+// z t of same-event lists), each row's position in the caller's list
+// (nullptr: the rows are in the caller's order) and, on the batched path, the
+// rows' fixed-point columns and screen terms (nullptr: converted here).
+struct ListRows {
+    const double *const *c;
+    const unsigned *orig;
+    const int4 *fixed;
+    const float4 *terms4;
+    const float2 *terms2;
+    long long stride, n;
 };
 
 // Shared memory of a mixed-event tile pair.
-struct MixedSmem {
-    TermsPair ti[FT / 2], tj[FT / 2];
+struct __align__(16) MixedSmem {
+    float4 ta[FT];  // as in SameSmem
+    float2 tb[FT];
+    TermsPair tj[FT / 2];
     uint2 queue[FT / 32][96];
     unsigned queue3[FT / 32][QCAP];
 };
-
-__device__ __forceinline__ Terms terms_at(const TermsPair *b, int k) {
-    const TermsPair &d = b[k >> 1];
-    const int h = k & 1;
-    return Terms{d.x[h], d.y[h], d.m[h], d.p[h], d.r2[h], d.t2[h]};
-}
 
 // Shared memory of the forms with q_inv histograms.
 struct QinvSmem {
@@ -871,22 +996,39 @@ __device__ __forceinline__ bool admit(const Device &d, int slot, long long row, 
     return row < d.caps.row_cut[slot];
 }
 
-// Loads a tile's screen terms: row `tid` of the tile at k0 of a list of n
-// particles with columns c, or padding past its end.
+// Screen terms of row k of a list, padding past its end.
 template <bool BOOST>
-__device__ __forceinline__ Terms load_terms(const double *const *c, long long k, long long n,
-                                            float pad) {
-    return k < n ? screen_terms<BOOST>(c[0][k], c[1][k], c[2][k], c[3][k]) : pad_terms(pad);
+__device__ __forceinline__ Terms load_terms(const ListRows &l, long long k, float pad) {
+    if (k >= l.n) return pad_terms(pad);
+    if (!l.terms4) return screen_terms<BOOST>(l.c[0][k], l.c[1][k], l.c[2][k], l.c[3][k]);
+    const float4 a = l.terms4[k];
+    const float2 b = l.terms2[k];
+    return Terms{a.x, a.y, a.z, a.w, b.x, b.y};
+}
+
+// Fixed-point columns of row k.
+__device__ __forceinline__ FixedCols load_fixed(const Grid &g, const ListRows &l, long long k) {
+    FixedCols r = {};
+    if (k >= l.n) return r;
+    if (l.fixed) {
+#pragma unroll
+        for (int f = 0; f < 4; f++) r.c[f] = l.fixed[f * l.stride + k];
+        return r;
+    }
+    double v[8];
+#pragma unroll
+    for (int f = 0; f < 8; f++) v[f] = l.c[f][k];
+    return fixed_cols(g, v);
 }
 
 // The pair loop: screens this lane's row against particles [0, jend) of the
 // j-tile, pairs with jj <= jmin left out, and collects the pairs that are
 // not certainly outside in the warp's queue; `process(entry, valid)` runs on
-// 32 of them at a time, all lanes in step.  An entry is x = row | particle
-// << 8 | undecided << 16, y = q bin.  ORIENT: the pair's first particle is
+// 32 of them at a time, all lanes in step.  An entry is x = place | particle
+// << 8 | undecided << 16, y = q bin (place: the row's, place_of).  ORIENT: the pair's first particle is
 // the one with the smaller original position (oa, oj).
 template <bool BOOST, bool ORIENT, class F>
-__device__ __forceinline__ void screen_loop(const Screen &S, const Terms &terms, int il,
+__device__ __forceinline__ void screen_loop(const Screen &S, const Terms &terms,
                                             const TermsPair *tj, unsigned oa, const unsigned *oj,
                                             int jmin, int jend, uint2 *q, F &process) {
     const int lane = threadIdx.x & 31;
@@ -911,7 +1053,7 @@ __device__ __forceinline__ void screen_loop(const Screen &S, const Terms &terms,
             const unsigned m0 = __ballot_sync(0xffffffffu, t0);
             const unsigned m1 = __ballot_sync(0xffffffffu, t1);
             if (!(m0 | m1)) continue;
-            const unsigned e = (unsigned)il | ((unsigned)jj << 8);
+            const unsigned e = threadIdx.x | ((unsigned)jj << 8);
             if (t0)
                 q[count + __popc(m0 & below)] =
                     make_uint2(e | (r.und[0] ? 1u << 16 : 0u), r.bin[0]);
@@ -935,38 +1077,36 @@ __device__ __forceinline__ void screen_loop(const Screen &S, const Terms &terms,
 }
 
 // Same-event pairs of the tiles starting at i0 and j0 (i0 <= j0) of one list
-// of n particles with columns c = px py pz E x y z t.  Every unordered pair
+// of particles.  Every unordered pair
 // is visited once (position j > i); it is oriented as the reference orients
 // it, q = p_first - p_second with `first` the particle earlier in the
-// caller's list: orig[k] is that original index of row k, or nullptr when
-// the rows are in the caller's order.  MODE selects the admission: FAST bins
+// caller's list.  MODE selects the admission: FAST bins
 // every pair; COUNT and ORDER are the two passes of ordered cap admission,
 // which see each pair at its row (the earlier of its two positions in the
 // caller's list).
 // Called by all FT threads of the CTA; the caller syncs before reusing `sm`.
 template <bool AZ, bool BOOST, int PREC, int MODE = MODE_FAST>
 __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, const double2 *cs,
-                                               const double *const *c, const unsigned *orig,
-                                               long long n, long long i0, long long j0) {
+                                               const ListRows &l, long long i0, long long j0) {
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    // split columns of the FP32-weight and double-float forms, in the FP64
-    // tiles' place
+    const int at_i = place_of(tid);  // this thread loads row tid of each tile
+    const long long n = l.n;
+    const double *const *c = l.c;
+    int4(*xi)[FT] = reinterpret_cast<int4(*)[FT]>(&sm.si[0][0]);
+    int4(*xj)[FT] = reinterpret_cast<int4(*)[FT]>(&sm.sj[0][0]);
+    // split columns of the FP32-weight and double-float forms, in their place
     float2(*spi)[FT] = reinterpret_cast<float2(*)[FT]>(&sm.si[0][0]);
     float2(*spj)[FT] = reinterpret_cast<float2(*)[FT]>(&sm.sj[0][0]);
     if (PREC == 0) {
-        for (int f = 0; f < 8; f++) {
-            sm.si[f][tid] = (i0 + tid < n) ? c[f][i0 + tid] : 0.0;
-            sm.sj[f][tid] = (j0 + tid < n) ? c[f][j0 + tid] : 0.0;
-        }
-        if (BOOST) {
-            const float2 iz = split(sm.si[2][tid]), iE = split(sm.si[3][tid]);
-            const float2 jz = split(sm.sj[2][tid]), jE = split(sm.sj[3][tid]);
-            sm.zi[tid] = make_float4(iz.x, iz.y, iE.x, iE.y);
-            sm.zj[tid] = make_float4(jz.x, jz.y, jE.x, jE.y);
+        const FixedCols a = load_fixed(d.g, l, i0 + tid), b = load_fixed(d.g, l, j0 + tid);
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            xi[f][at_i] = a.c[f];
+            xj[f][tid] = b.c[f];
         }
     } else if (PREC == 1) {
         for (int f = 0; f < 8; f++) {
-            spi[f][tid] = split((i0 + tid < n) ? c[f][i0 + tid] : 0.0);
+            spi[f][at_i] = split((i0 + tid < n) ? c[f][i0 + tid] : 0.0);
             spj[f][tid] = split((j0 + tid < n) ? c[f][j0 + tid] : 0.0);
         }
     } else {
@@ -983,20 +1123,19 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
                     sm.offj[f] = oj;
                 }
             }
-            spi[f][tid] = split(vi - (double)oi);
+            spi[f][at_i] = split(vi - (double)oi);
             spj[f][tid] = split(vj - (double)oj);
         }
     }
-    sm.oi[tid] = orig ? (i0 + tid < n ? orig[i0 + tid] : 0u) : (unsigned)(i0 + tid);
-    sm.oj[tid] = orig ? (j0 + tid < n ? orig[j0 + tid] : 0u) : (unsigned)(j0 + tid);
-    put_terms(sm.ti, tid, load_terms<BOOST>(c, i0 + tid, n, -1e15f));
-    put_terms(sm.tj, tid, load_terms<BOOST>(c, j0 + tid, n, 1e15f));
+    sm.oi[at_i] = l.orig ? (i0 + tid < n ? l.orig[i0 + tid] : 0u) : (unsigned)(i0 + tid);
+    sm.oj[tid] = l.orig ? (j0 + tid < n ? l.orig[j0 + tid] : 0u) : (unsigned)(j0 + tid);
+    const Terms ti = load_terms<BOOST>(l, i0 + tid, -1e15f);
+    sm.ta[at_i] = make_float4(ti.x, ti.y, ti.m, ti.p);
+    sm.tb[at_i] = make_float2(ti.r2, ti.t2);
+    put_terms(sm.tj, tid, load_terms<BOOST>(l, j0 + tid, 1e15f));
     __syncthreads();
     const Screen &S = d.s;
-    // warp w takes the tile's rows w, w + 4, w + 8, ...: the rows are sorted
-    // in momentum space, so interleaving spreads each warp's rows over the
-    // tile and evens out the binned pairs between warps
-    const int il = lane * (FT / 32) + w;
+    const int il = row_at(tid);  // this lane's row, at place tid
     const int jend = (int)min((long long)FT, n - j0);
     // each unordered pair once; none for rows past the list's end
     const int jmin = i0 + il >= n ? FT : (i0 == j0 ? il : -1);
@@ -1004,18 +1143,17 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
     int count3 = 0;
 
     // pairs left undecided, 32 at a time: the reference chain decides them
-    // (and may hand a K_phi edge to the host), from the FP64 tile or
-    // (FP32-weight and double-float forms) the FP64 columns
+    // (and may hand a K_phi edge to the host), from the FP64 columns
     auto chains = [&](unsigned e, bool valid) {
         if (!valid) return;
         const int qi = e & 0xff, qj = (e >> 8) & 0xff;
+        const int ri = row_at(qi);
         const long long oa = sm.oi[qi], ob = sm.oj[qj];
         const bool swap = oa > ob;
         double A[8], B[8];  // first and second particle of the pair
 #pragma unroll
         for (int f = 0; f < 8; f++) {
-            const double u = PREC == 0 ? sm.si[f][qi] : c[f][i0 + qi];
-            const double v = PREC == 0 ? sm.sj[f][qj] : c[f][j0 + qj];
+            const double u = c[f][i0 + ri], v = c[f][j0 + qj];
             A[f] = swap ? v : u;
             B[f] = swap ? u : v;
         }
@@ -1025,9 +1163,9 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
             return;
         }
         if (PREC == 1)
-            undecided_pair32<BOOST>(d, A, B, i0 + qi, j0 + qj, n);
+            undecided_pair32<BOOST>(d, A, B, i0 + ri, j0 + qj, n);
         else
-            undecided_pair64(d, A, B, i0 + qi, j0 + qj, n);
+            undecided_pair64(d, A, B, i0 + ri, j0 + qj, n);
     };
 
     // one pair with its q bin and slot decided: its values into its bin
@@ -1069,23 +1207,16 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
             values_df<BOOST>(d.s, reinterpret_cast<const float4 *>(cs), a, b, sm.offi, sm.offj,
                              swap, vo, vs, vl, vw);
         } else {
-            // the pair in the reference's orientation, from the FP64 tile
-            // (the two rows chosen once, then read column by column)
-            const double *ra = swap ? &sm.sj[0][qj] : &sm.si[0][qi];
-            const double *rb = swap ? &sm.si[0][qi] : &sm.sj[0][qj];
-            double A[8], B[8];
+            FixedCols a, b;
 #pragma unroll
-            for (int f = 0; f < 8; f++) {
-                A[f] = ra[f * FT];
-                B[f] = rb[f * FT];
+            for (int f = 0; f < 4; f++) {
+                a.c[f] = xi[f][qi];
+                b.c[f] = xj[f][qj];
             }
-            FF sz = {0.0f, 0.0f}, sE = {0.0f, 0.0f};
-            if (BOOST) {
-                const float4 za = sm.zi[qi], zb = sm.zj[qj];
-                sz = ff_sum(make_float2(za.x, za.y), make_float2(zb.x, zb.y));
-                sE = ff_sum(make_float2(za.z, za.w), make_float2(zb.z, zb.w));
-            }
-            values64<BOOST>(d.g, cs, A, B, sz, sE, vo, vs, vl, vw);
+            if (a.c[1].z == kFar || b.c[1].z == kFar)
+                values64_rows<BOOST>(d.g, cs, c, i0 + row_at(qi), j0 + qj, swap, vo, vs, vl, vw);
+            else
+                values_fixed<BOOST>(d.g, cs, a, b, swap, vo, vs, vl, vw);
         }
         Sums *h = d.h.sums + at;
         atomicAdd(&h->qo, vo);
@@ -1103,8 +1234,9 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
         int slot = -2;
         if (valid) {
             const int qi = e & 0xff, qj = e >> 8;
-            const TermsPair &a = sm.ti[qi >> 1], &b = sm.tj[qj >> 1];
-            slot = slot_of<AZ>(S, a.x[qi & 1], a.y[qi & 1], b.x[qj & 1], b.y[qj & 1]);
+            const float4 a = sm.ta[qi];
+            const TermsPair &b = sm.tj[qj >> 1];
+            slot = slot_of<AZ>(S, a.x, a.y, b.x[qj & 1], b.y[qj & 1]);
             if (slot != -2 && ((e2.x >> 16) || e2.y >= S.sc_q3)) slot = -1;
         }
         if (slot >= 0) decided(e, slot, e2.y);
@@ -1112,31 +1244,33 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
     };
 
     // (the orientation is by original position)
-    const Terms row = terms_at(sm.ti, il);
-    screen_loop<BOOST, true>(S, row, il, sm.tj, sm.oi[il], sm.oj, jmin, jend, sm.queue[w],
-                             process);
+    const float4 ta = sm.ta[tid];
+    const float2 tb = sm.tb[tid];
+    screen_loop<BOOST, true>(S, Terms{ta.x, ta.y, ta.z, ta.w, tb.x, tb.y}, sm.tj, sm.oi[tid],
+                             sm.oj, jmin, jend, sm.queue[w], process);
     drain(q3, count3, lane, chains);
 }
 
-// Mixed-event pairs of the list-1 tile at i0 (n1 particles, columns l1 =
-// px py pz E) and the list-2 tile at j0 (n2 particles, columns l2).  Under
-// ordered cap admission (MODE COUNT / ORDER) a pair's row and column are
-// its positions in the caller's lists, orig1 / orig2 (nullptr: the rows are
-// in the caller's order).
+// Mixed-event pairs of the list-1 tile at i0 and the list-2 tile at j0.
+// Under ordered cap admission (MODE COUNT / ORDER) a pair's row and column
+// are its positions in the caller's lists.
 template <bool AZ, bool BOOST, int MODE = MODE_FAST>
 __device__ __forceinline__ void mixed_tile_pair(const Device &d, MixedSmem &sm,
-                                                const double *const *l1, long long n1,
-                                                const double *const *l2, long long n2,
+                                                const ListRows &la, const ListRows &lb,
                                                 long long i0, long long j0,
-                                                const unsigned *orig1 = nullptr,
-                                                const unsigned *orig2 = nullptr,
                                                 long long row_base = 0) {
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    put_terms(sm.ti, tid, load_terms<BOOST>(l1, i0 + tid, n1, -1e15f));
-    put_terms(sm.tj, tid, load_terms<BOOST>(l2, j0 + tid, n2, 1e15f));
+    const long long n1 = la.n, n2 = lb.n;
+    const double *const *l1 = la.c, *const *l2 = lb.c;
+    const unsigned *orig1 = la.orig, *orig2 = lb.orig;
+    const int at_i = place_of(tid);
+    const Terms ti = load_terms<BOOST>(la, i0 + tid, -1e15f);
+    sm.ta[at_i] = make_float4(ti.x, ti.y, ti.m, ti.p);
+    sm.tb[at_i] = make_float2(ti.r2, ti.t2);
+    put_terms(sm.tj, tid, load_terms<BOOST>(lb, j0 + tid, 1e15f));
     __syncthreads();
     const Screen &S = d.s;
-    const int il = lane * (FT / 32) + w;  // interleaved rows, as in same_tile_pair
+    const int il = row_at(tid);  // this lane's row, at place tid
     const int jend = (int)min((long long)FT, n2 - j0);
     const int jmin = i0 + il >= n1 ? FT : -1;
     // ordered admission: row stride of the survivor counts and key stride of
@@ -1150,7 +1284,7 @@ __device__ __forceinline__ void mixed_tile_pair(const Device &d, MixedSmem &sm,
     // decides (inline, a warp would run it for one or two lanes)
     auto chains = [&](unsigned e, bool valid) {
         if (!valid) return;
-        const int qi = e & 0xff, qj = (e >> 8) & 0xff;
+        const int qi = row_at(e & 0xff), qj = (e >> 8) & 0xff;
         if (MODE != MODE_FAST) {
             const long long row = row_base + (orig1 ? (long long)orig1[i0 + qi] : i0 + qi);
             const long long col = orig2 ? (long long)orig2[j0 + qj] : j0 + qj;
@@ -1167,9 +1301,10 @@ __device__ __forceinline__ void mixed_tile_pair(const Device &d, MixedSmem &sm,
         const unsigned e = e2.x & 0xffffu;
         int slot = -2;
         if (valid) {
-            const int qi = e & 0xff, qj = e >> 8;
-            const TermsPair &a = sm.ti[qi >> 1], &b = sm.tj[qj >> 1];
-            slot = slot_of<AZ>(S, a.x[qi & 1], a.y[qi & 1], b.x[qj & 1], b.y[qj & 1]);
+            const int qi = row_at(e & 0xff), qj = e >> 8;
+            const float4 a = sm.ta[e & 0xff];
+            const TermsPair &b = sm.tj[qj >> 1];
+            slot = slot_of<AZ>(S, a.x, a.y, b.x[qj & 1], b.y[qj & 1]);
             if (slot != -2 && ((e2.x >> 16) || e2.y >= S.sc_q3)) slot = -1;
             bool admitted = slot >= 0;
             if (MODE != MODE_FAST && admitted) {
@@ -1181,8 +1316,10 @@ __device__ __forceinline__ void mixed_tile_pair(const Device &d, MixedSmem &sm,
         enqueue(q3, count3, slot == -1, e, lane, chains);
     };
 
-    const Terms row = terms_at(sm.ti, il);
-    screen_loop<BOOST, false>(S, row, il, sm.tj, 0u, nullptr, jmin, jend, sm.queue[w], process);
+    const float4 ta = sm.ta[tid];
+    const float2 tb = sm.tb[tid];
+    screen_loop<BOOST, false>(S, Terms{ta.x, ta.y, ta.z, ta.w, tb.x, tb.y}, sm.tj, 0u, nullptr,
+                              jmin, jend, sm.queue[w], process);
     drain(q3, count3, lane, chains);
 }
 
