@@ -37,6 +37,8 @@ namespace {
 
 using namespace tile;
 
+static_assert(kFixedCols == kFixedEntries, "row size of BatchDev::fixed");
+
 // Morton interleave of three 10-bit cell coordinates.
 __device__ __forceinline__ unsigned spread10(unsigned v) {
     v &= 0x3ffu;
@@ -106,7 +108,7 @@ __global__ void k_gather(BatchDev b, Grid g) {
         if (l.ncols == 8) {
             const FixedCols c = fixed_cols(g, v);
 #pragma unroll
-            for (int f = 0; f < 4; f++) b.fixed[(long long)f * b.cap + s] = c.c[f];
+            for (int f = 0; f < kFixedCols; f++) b.fixed[(long long)f * b.cap + s] = c.c[f];
         }
         b.orig[s] = (unsigned)k;  // position in the caller's list (pair orientation)
     }

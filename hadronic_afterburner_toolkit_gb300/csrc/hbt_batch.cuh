@@ -6,6 +6,9 @@
 
 namespace hbt {
 
+// Fixed-point columns of a same-event row, in entries of two (hbt_fixed.cuh).
+constexpr int kFixedEntries = 4;
+
 // One particle list of a batch, as the caller passed it.
 struct BatchList {
     const double *src[8];  // caller columns px py pz E (x y z t for same-event)
@@ -64,7 +67,7 @@ struct BatchDev {
     long long cap;          // row capacity of the sorted table
     double *table;          // [8][cap] sorted particle table
     unsigned *orig;         // [cap] each row's position in the caller's list
-    // per row: the fixed-point columns of same-event lists ([4][cap],
+    // per row: the fixed-point columns of same-event lists ([kFixedEntries][cap],
     // hbt_fixed.cuh) and the screen's terms (x, y, m, p) and (r2, t2)
     // (hbt_screen.cuh), converted once per batch
     int4 *fixed;

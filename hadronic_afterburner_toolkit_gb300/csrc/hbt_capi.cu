@@ -798,7 +798,7 @@ void grid_from_params(const hbt_params &p, Grid &g) {
     const double rest = std::fma(g.hbarC_inv, turn_h, -turns) + g.hbarC_inv * turn_l;
     g.pos_h = std::ldexp(turns, 20);
     g.pos_l = std::ldexp(rest, 20);
-    g.cfx = make_cos_scale(std::ldexp(6.283185307179586 / 512.0, -52));
+    g.cfx_half = std::ldexp(6.283185307179586 / 2048.0, -53);
 }
 
 // The margins of the tile screen (hbt_screen.cuh derives them).

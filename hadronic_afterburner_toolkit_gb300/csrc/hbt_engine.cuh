@@ -26,9 +26,8 @@ struct Grid {
     double hbarC_inv;
     CosScale cph;  // table_cos constants for cos(q.dx / hbarC)
     // fixed-point pair values (hbt_fixed.cuh): 2^20 / (2 pi hbarC) in two
-    // parts, and the cosine's coefficients in 2^-52 table steps
-    double pos_h, pos_l;
-    CosScale cfx;
+    // parts, and half a 2^-52 of the cos table's step in rad
+    double pos_h, pos_l, cfx_half;
 };
 
 // Per-bin numerator sums, one 32-byte L2 sector per bin.

@@ -6,33 +6,30 @@
 // integers give exactly.  Each column of a same-event list is kept as a
 // 60-bit integer in two signed limbs, value = (h 2^30 + l) / scale with l in
 // [-2^29, 2^29):
-//   momenta    scale 2^56 / GeV (h in 2^-26 GeV): exact for |p| >= 2^-4 GeV,
-//              within 2^-57 GeV below;
-//   positions  times 512 / (2 pi hbarC), scale 2^41 (h in 2^-11 table steps
-//              per GeV): q.dx comes out in steps of the cos table's 512
-//              points per period.  x, y and z are stored negated, so that
-//              q.dx = q_E dt - q_x dx - q_y dy - q_z dz is a sum of four
-//              products.
-// Differences of limbs stay below 2^30 (l) and, for |p| < 8 GeV and
-// positions within 2^18 steps per GeV (634 fm), below 2^30 (h), so the four
-// products' high, cross and low parts accumulate in 64 bits without
-// overflow: 16 multiply-adds of 32 x 32 -> 64 bits for the phase, whose
-// rounding is that of the two stored values alone (2^-42 |q| + 2^-57 |dx|
-// steps: about 1e-15 rad for |q| = 0.2 GeV, dx = 50 fm; the FP64 sum of
-// four rounded products has about 5e-15).  Whole periods drop out as high
-// bits, the table point and the remainder are bit fields, and the remainder
-// enters the table's polynomials as an exact FP64 integer.  A particle
-// outside those ranges (or not finite) carries kFar, and its pairs take the
-// FP64 values (values64).
+//   p_x, p_y, m = E - p_z, p = E + p_z   scale 2^56 / GeV (h in 2^-26 GeV):
+//              exact for p_x, p_y of 2^-4 GeV and more, within 2^-57 GeV;
+//   -x, -y, v = (t + z) / 2, u = (t - z) / 2   times 512 / (2 pi hbarC),
+//              scale 2^41 (h in 2^-11 steps of a 512-point cos table, per
+//              GeV).
+// In these, with d the difference of a column over the pair,
+//   q.dx = d(p_x) d(-x) + d(p_y) d(-y) + d(m) d(v) + d(p) d(u)
+// is a sum of four products, and q_long = (s(m) d(p) - s(p) d(m)) /
+// (2 sqrt(s(m) s(p))) needs no sums of E and p_z (s: sums over the pair).
+// (q_out as the difference of p_x^2 + p_y^2 over |s_T| loses its digits for
+// small |s_T|: it is formed from the differences and sums.)  Differences of limbs stay below 2^30 (l) and, for
+// |p_x|, |p_y|, E < 8 GeV and positions within 2^18 steps per GeV (634 fm),
+// below 2^30 (h), so the products' high, cross and low parts accumulate in
+// 64 bits without overflow: 16 multiply-adds of 32 x 32 -> 64 bits for the
+// phase, whose rounding is that of the stored values alone (2^-42 |q| +
+// 2^-57 |dx| steps: about 1e-15 rad for |q| = 0.2 GeV, dx = 50 fm; the FP64
+// sum of four rounded products has about 5e-15).  Whole periods drop out as
+// high bits, the table point and the remainder are bit fields, and the
+// remainder enters the cosine as an exact FP64 integer.  A particle outside
+// those ranges (or not finite) carries kFar, and its pairs take the FP64
+// values (values64).
 //
-// Of the FP64 pipe a binned pair then takes 9 instructions for the cosine
-// and one addition per q component, where the FP64 differences, phase and
-// table reduction took 29 (with the undecided pairs' chain 13.7 against 31.3
-// measured).  Same-event kernel, central group (150k pions): 109 -> 60.8 ms,
-// FP64 pipe 73 % busy instead of 84 %; 45k-particle group 10.96 -> 5.52 ms.
-// The numerator's distance from the 64-bit sums is unchanged on that group
-// (4.7e-15) and halves on small ones (2.3e-15 -> 1.2e-15), where rounding
-// averages less.
+// Of the FP64 pipe a binned pair takes 5 instructions, all for the cosine,
+// where the FP64 differences, phase, table reduction and sums took 29.
 #pragma once
 
 #include "hbt_engine.cuh"
@@ -50,12 +47,23 @@ __device__ __forceinline__ int2 to_limbs(double hi, double lo) {
     return make_int2(__double2loint(t), min(__double2loint(s), (1 << 29) - 1));
 }
 
-// The eight columns of a same-event particle, two to an entry: (px, py),
-// (pz, E), (-x, -y), (-z, t), each (h, l).
+// Limbs as one integer, and back.
+__device__ __forceinline__ long long join_limbs(int2 a) {
+    return (long long)a.x * (1 << 30) + a.y;
+}
+__device__ __forceinline__ int2 split_limbs(long long v) {
+    const long long h = (v + (1 << 29)) >> 30;
+    return make_int2((int)h, (int)(v - h * (1 << 30)));
+}
+
+// The columns of a same-event particle, two to an entry, each (h, l):
+// (px, py), (m, p), (-x, -y), (v, u).
+constexpr int kFixedCols = 4;
 struct FixedCols {
-    int4 c[4];
+    int4 c[kFixedCols];
 };
 
+// v: px py pz E x y z t.
 __device__ __forceinline__ FixedCols fixed_cols(const Grid &g, const double *v) {
     int2 q[8];
     bool near = true;
@@ -64,21 +72,80 @@ __device__ __forceinline__ FixedCols fixed_cols(const Grid &g, const double *v) 
         double hi, lo = 0.0;
         if (f < 4) {
             near = near && fabs(v[f]) < 8.0;
-            hi = v[f] * 67108864.0;
+            hi = v[f] * 67108864.0;  // 2^26
         } else {
-            const double x = f < 7 ? -v[f] : v[f];
-            hi = x * g.pos_h;
-            lo = __fma_rn(x, g.pos_h, -hi) + x * g.pos_l;
+            hi = v[f] * g.pos_h;
+            lo = __fma_rn(v[f], g.pos_h, -hi) + v[f] * g.pos_l;
             near = near && fabs(hi) < 536870912.0;  // 2^18 2^11
         }
         q[f] = to_limbs(hi, lo);
     }
-    if (!near) q[3].x = kFar;
+    // E > |p_z|: m and p positive, their sums below 2^31 as unsigned h
+    near = near && v[3] > fabs(v[2]);
+    const long long E = join_limbs(q[3]), z = join_limbs(q[2]);
+    const long long T = join_limbs(q[7]), Z = join_limbs(q[6]);
+    const int2 m = split_limbs(E - z), p = split_limbs(E + z);
+    const int2 vv = split_limbs((T + Z) >> 1), uu = split_limbs((T - Z) >> 1);
+    const int2 X = split_limbs(-join_limbs(q[4])), Y = split_limbs(-join_limbs(q[5]));
     FixedCols r;
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-        r.c[k] = make_int4(q[2 * k].x, q[2 * k].y, q[2 * k + 1].x, q[2 * k + 1].y);
+    r.c[0] = make_int4(q[0].x, q[0].y, q[1].x, q[1].y);
+    r.c[1] = make_int4(near ? m.x : kFar, m.y, p.x, p.y);
+    r.c[2] = make_int4(X.x, X.y, Y.x, Y.y);
+    r.c[3] = make_int4(vv.x, vv.y, uu.x, uu.y);
     return r;
+}
+
+// Cosine table of the fixed-point values: cos(2 pi k / 2048) for a quarter
+// period, k = 0..512, in FP64 and a sixth of it in FP32, filled by each CTA.
+struct __align__(16) CosEntry {
+    double c;
+    float sixth;
+    float pad;
+};
+constexpr int kCosEntries = 513;
+__device__ __forceinline__ void fill_cos_entries(CosEntry *t) {
+    for (int k = threadIdx.x; k < kCosEntries; k += blockDim.x) {
+        t[k].c = cospi(k / 1024.0);
+        t[k].sixth = (float)(t[k].c * (1.0 / 6.0));
+    }
+}
+
+// cos of a phase given as hh 2^-37 + (low 30 bits of hl) 2^-67 steps of
+// 2 pi / 512.  In steps of 2 pi / 2048 (hh counts 2^-35): the nearest table
+// point j, of which the quarter period gives signs and the roles of U = cos
+// and V = sin of its place, and the remainder d, |d| <= pi / 2048:
+//   cos(j + d) = U - V d - U d^2 / 2 + V d^3 / 6 + U d^4 / 24,
+// the first three terms in FP64 (d exact but for one rounding), the last
+// two, below 6e-10, in FP32 (the next, V d^5 / 120, is below 7e-17).  Error
+// below 4e-16.
+__device__ __forceinline__ double cos_fixed(const Grid &g, const CosEntry *t, long long hh,
+                                            unsigned hl) {
+    const unsigned fl = (unsigned)hh, low = hl << 2;
+    const int top = (int)(hh >> 32) + 4;  // + half a step
+    const int r = (top & 7) - 4;          // remainder: r, fl, low as one signed number
+    const int j = top >> 3, odd = j & 512, idx = j & 511;
+    const int iu = odd ? 512 - idx : idx;
+    const CosEntry eu = t[iu], ev = t[512 - iu];
+    const unsigned sv = (unsigned)odd << 22;              // V's sign, as a sign bit
+    const unsigned sr = (unsigned)((j + 512) & 1024) << 21;  // the result's
+    const double V = __hiloint2double(__double2hiint(ev.c) ^ (int)sv, __double2loint(ev.c));
+    // 52-bit signed integer remainder (2^-52 steps) as FP64
+    const double z = __hiloint2double(0x43380000 + (int)__funnelshift_r(fl, (unsigned)r, 15),
+                                      (int)__funnelshift_l(low, fl, 17)) -
+                     6755399441055744.0;
+    const double hd = z * g.cfx_half;  // d / 2
+    const double d = __hiloint2double(__double2hiint(hd) + (1 << 20), __double2loint(hd));
+    const double main = __fma_rn(-d, __fma_rn(hd, eu.c, V), eu.c);
+    const float x = __int2float_rn((int)__funnelshift_r(fl, (unsigned)r, 3)) *
+                    (float)(6.283185307179586 / 2048.0 / 4294967296.0);
+    const float x2 = x * x;
+    const float vf = __uint_as_float(__float_as_uint(ev.sixth) ^ sv);
+    const float b = x2 * __fmaf_rn(x, vf, 0.25f * (x2 * eu.sixth));
+    // b as FP64 through its bits (a zero becomes a number below 1e-38)
+    const int bi = __float_as_int(b);
+    const double bd = __hiloint2double(((bi >> 3) & (int)0x8fffffff) + (896 << 20), bi << 29);
+    const double w = main + bd;
+    return __hiloint2double(__double2hiint(w) ^ (int)sr, __double2loint(w));
 }
 
 }  // namespace tile

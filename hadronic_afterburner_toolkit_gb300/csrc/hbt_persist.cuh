@@ -81,15 +81,15 @@ constexpr int kMixedCtas = HBT_MIXED_CTAS;
 // One item: the tile pair, with or without the q_inv histograms by the type
 // of its shared memory.
 template <bool AZ, bool BOOST, int PREC, int MODE>
-__device__ __forceinline__ void same_item(const Device &d, SameSmem &sm, const double2 *cs,
+__device__ __forceinline__ void same_item(const Device &d, SameSmem &sm, const void *cs,
                                           const ListRows &l, const Item &it) {
     same_tile_pair<AZ, BOOST, PREC, MODE>(d, sm, cs, l, (long long)it.ti * FT,
                                           (long long)it.tj * FT);
 }
 template <bool AZ, bool BOOST, int PREC, int MODE>
-__device__ __forceinline__ void same_item(const Device &d, QinvSmem &sm, const double2 *cs,
+__device__ __forceinline__ void same_item(const Device &d, QinvSmem &sm, const void *cs,
                                           const ListRows &l, const Item &it) {
-    same_tile_pair_qinv<AZ, BOOST, PREC, MODE>(d, sm, cs, l.c, l.orig, l.n,
+    same_tile_pair_qinv<AZ, BOOST, PREC, MODE>(d, sm, static_cast<const double2 *>(cs), l.c, l.orig, l.n,
                                                (long long)it.ti * FT, (long long)it.tj * FT);
 }
 template <bool AZ, bool BOOST, int MODE>
@@ -122,8 +122,11 @@ __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(D
                                                            unsigned end) {
     __shared__ typename std::conditional<QINV, QinvSmem, SameSmem>::type sm;
     __shared__ unsigned item;
-    __shared__ double2 cs[COS_TABLE];
-    if (PREC == 0) fill_cos_table(cs);
+    // the form's cos table
+    constexpr int kTable = PREC == 0 ? (QINV ? COS_TABLE : kCosEntries) : (PREC == 2 ? DF_TABLE : 1);
+    __shared__ double2 cs[kTable];
+    if (PREC == 0 && QINV) fill_cos_table(cs);
+    if (PREC == 0 && !QINV) fill_cos_entries(reinterpret_cast<CosEntry *>(cs));
     if (PREC == 2) fill_df_table(reinterpret_cast<float4 *>(cs));
     const unsigned stop = min(end, min(b.n_items[0], b.same_cap));
     for (;;) {

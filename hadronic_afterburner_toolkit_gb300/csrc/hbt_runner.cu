@@ -229,7 +229,7 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
         !grow(jobs_, bj.size() * sizeof(BatchJob), err) ||
         !grow(offs_, (2 * lists.size() + bj.size()) * sizeof(long long), err) ||
         !grow(table_, (size_t)8 * total * sizeof(double), err) ||
-        !grow(fixed_, (size_t)4 * total * sizeof(int4), err) ||
+        !grow(fixed_, (size_t)kFixedEntries * total * sizeof(int4), err) ||
         !grow(terms_, (size_t)total * (sizeof(float4) + sizeof(float2)), err) ||
         !grow(keys_, (size_t)2 * total * sizeof(unsigned long long), err) ||
         !grow(vals_, (size_t)3 * total * sizeof(unsigned), err) ||

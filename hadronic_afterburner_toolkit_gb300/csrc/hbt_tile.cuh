@@ -656,9 +656,8 @@ __device__ __forceinline__ void values_df(const Screen &S, const float4 *tab, co
 // stays below 1e-14 GeV).  Of the FP64 pipe, which bounds this form, a
 // binned pair then takes 27 to 29 instructions instead of 55.
 template <bool BOOST>
-__device__ __forceinline__ void values64(const Grid &g, const double2 *cs, const double *a,
-                                         const double *b, FF sz, FF sE, double &qo, double &qs,
-                                         double &ql, double &w) {
+__device__ __forceinline__ void lcms64(const double *a, const double *b, FF sz, FF sE, double &qo,
+                                       double &qs, double &ql, double &ph) {
     const double dx = a[0] - b[0], dy = a[1] - b[1];
     const double dz = a[2] - b[2], dE = a[3] - b[3];
     FF dp[4] = {f64_to_ff_bits(dx), f64_to_ff_bits(dy), f64_to_ff_bits(dz), f64_to_ff_bits(dE)};
@@ -674,22 +673,30 @@ __device__ __forceinline__ void values64(const Grid &g, const double2 *cs, const
     ql = BOOST ? ff_double_bits(vl) : dz;
     // q.dx = dE dt - dx dX - dy dY - dz dZ, accumulated with fused
     // multiply-adds (one rounding per term)
-    double ph = dE * (a[7] - b[7]);
+    ph = dE * (a[7] - b[7]);
     ph = __fma_rn(-dx, a[4] - b[4], ph);
     ph = __fma_rn(-dy, a[5] - b[5], ph);
     ph = __fma_rn(-dz, a[6] - b[6], ph);
+}
+template <bool BOOST>
+__device__ __forceinline__ void values64(const Grid &g, const double2 *cs, const double *a,
+                                         const double *b, FF sz, FF sE, double &qo, double &qs,
+                                         double &ql, double &w) {
+    double ph;
+    lcms64<BOOST>(a, b, sz, sE, qo, qs, ql, ph);
     w = table_cos(cs, g.cph, ph);
 }
 
-// values64 from the FP64 columns of rows i and j, in the reference's
-// orientation (`swap`: j first).  For the pairs of particles whose values do
-// not fit the fixed-point columns; out of line to keep its registers out of
-// the pair loop.
+// The values of a pair from the FP64 columns of rows i and j, in the
+// reference's orientation (`swap`: j first): momentum sums and differences
+// and the phase in FP64, q_out, q_side and q_long in double-float (ff_lcms).
+// For the pairs of particles whose values do not fit the fixed-point
+// columns; out of line to keep its registers out of the pair loop.  The
+// product of the phase with 1 / hbarC enters the cosine unrounded.
 template <bool BOOST>
-__device__ __noinline__ void values64_rows(const Grid &g, const double2 *cs,
-                                           const double *const *c, long long i, long long j,
-                                           bool swap, double &qo, double &qs, double &ql,
-                                           double &w) {
+__device__ __noinline__ void values64_rows(const Grid &g, const double *const *c, long long i,
+                                           long long j, bool swap, double &qo, double &qs,
+                                           double &ql, double &w) {
     double a[8], b[8];
 #pragma unroll
     for (int f = 0; f < 8; f++) {
@@ -697,46 +704,75 @@ __device__ __noinline__ void values64_rows(const Grid &g, const double2 *cs,
         a[f] = swap ? v : u;
         b[f] = swap ? u : v;
     }
-    FF sz = {0.0f, 0.0f}, sE = {0.0f, 0.0f};
-    if (BOOST) {
-        sz = ff_sum(split(a[2]), split(b[2]));
-        sE = ff_sum(split(a[3]), split(b[3]));
-    }
-    values64<BOOST>(g, cs, a, b, sz, sE, qo, qs, ql, w);
+    double ph;
+    lcms64<BOOST>(a, b, ff_sum(split(a[2]), split(b[2])), ff_sum(split(a[3]), split(b[3])), qo, qs,
+                  ql, ph);
+    const double p = g.hbarC_inv * ph, e = __fma_rn(g.hbarC_inv, ph, -p);
+    double sn, cn;
+    sincos(p, &sn, &cn);
+    w = __fma_rn(-e, sn, cn);
 }
 
 // Limbs (h, l) of a difference or sum as a double-float in units of h: h in
 // two exact conversions, l below, normalised (of a small h, l is not below
-// the last bit, and ff_mul drops the product of the low parts).
+// the last bit, and ff_mul drops the product of the low parts).  The second
+// for an h in [0, 2^32).
 __device__ __forceinline__ FF limbs_ff(int h, int l) {
     const float f = __int2float_rn(h);
     const float r = __int2float_rn(h - __float2int_rn(f));
     return fast_two_sum(f, __fmaf_rn(__int2float_rn(l), 0x1p-30f, r));
 }
+__device__ __forceinline__ FF limbs_ff(unsigned h, int l) {
+    const float f = __uint2float_rn(h);
+    const float r = __int2float_rn((int)(h - __float2uint_rn(f)));
+    return fast_two_sum(f, __fmaf_rn(__int2float_rn(l), 0x1p-30f, r));
+}
 
-// hi + lo, in units of 2^-26 GeV, rounded once to FP64 in GeV, negated when
-// `neg` is the sign bit: both parts converted on the integer pipe (exponent
-// rebiased by 896 - 26; a zero part becomes a number below 1e-45, far under
-// the rounding of any sum it enters).
-__device__ __forceinline__ double ff_gev(FF a, unsigned neg) {
-    auto conv = [&](float x) {
-        const unsigned u = __float_as_uint(x) ^ neg;
-        return __hiloint2double((int)(((unsigned)((int)u >> 3) & 0x8fffffffu) + (870u << 20)),
-                                (int)(u << 29));
-    };
-    return conv(a.h) + conv(a.l);
+// a b + c d: the two products and their sum error-free, the terms below in
+// FP32, normalised.
+__device__ __forceinline__ FF ff_dot(FF a, FF b, FF c, FF d) {
+    const float p = __fmul_rn(a.h, b.h), q = __fmul_rn(c.h, d.h);
+    float e = __fmaf_rn(a.h, b.h, -p), f = __fmaf_rn(c.h, d.h, -q);
+    e = __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.l, e));
+    f = __fmaf_rn(c.l, d.h, __fmaf_rn(c.h, d.l, f));
+    const FF s = two_sum(p, q);
+    return fast_two_sum(s.h, __fadd_rn(s.l, __fadd_rn(e, f)));
+}
+
+// 1 / sqrt(x): with y0 the hardware estimate and x y0^2 = 1 + e formed to
+// 2^-46, y0 (1 - e / 2 + 3 e^2 / 8), the correction left as the low part.
+__device__ __forceinline__ FF ff_rsqrt_fast(FF x) {
+    const float y = rsqrt_approx(x.h);
+    const float p = __fmul_rn(y, y), ep = __fmaf_rn(y, y, -p);
+    const float e = __fmaf_rn(x.h, ep, __fmaf_rn(x.l, p, __fmaf_rn(x.h, p, -1.0f)));
+    return FF{y, __fmul_rn(y, __fmul_rn(e, __fmaf_rn(0.375f, e, -0.5f)))};
+}
+
+// hi + lo rounded to FP64, its sign changed by `neg` (a sign bit), times
+// 2^shift, on the integer pipe: hi's bits as FP64, then lo in units of hi's
+// last FP64 place added to them as a signed integer (twice that count below
+// a power of two, whose places are half as wide).
+__device__ __forceinline__ double ff_scaled(FF a, unsigned neg, int shift) {
+    const unsigned u = __float_as_uint(a.h);
+    const float unit = __uint_as_float((306u << 23) - (u & 0x7f800000u));
+    int lo = __float2int_rn(__uint_as_float(__float_as_uint(a.l) ^ (u & 0x80000000u)) * unit);
+    if ((u & 0x7fffffu) == 0u && lo < 0) lo *= 2;
+    const unsigned s = u ^ neg;
+    const long long hi =
+        ((long long)(((int)s >> 3) & (int)0x8fffffff) + ((long long)(896 + shift) << 20)) << 32 |
+        (s << 29);
+    return __longlong_as_double(hi + lo);
 }
 
 // Summed values of an accepted same-event pair from its fixed-point columns
 // (hbt_fixed.cuh), a from the i-tile, b from the j-tile, negated in q when
 // `swap` (b is the pair's first particle).  The differences and sums are
 // exact; q_out, q_side and the boosted q_long, which are only summed, follow
-// in double-float (ff_lcms, about 1e-14 relative) and come back as FP64 with
-// one addition each.  The phase is summed from 32 x 32 bit products: with
-// the limbs (h, l) of a difference, sum of h h' (unit 2^-37 table steps),
-// h l' + l h' (2^-67) and l l' (2^-97).
+// in double-float (about 1e-14 relative).  The phase is summed from 32 x 32
+// bit products: with the limbs (h, l) of a difference, sum of h h' (unit
+// 2^-37 table steps), h l' + l h' (2^-67) and l l' (2^-97).
 template <bool BOOST>
-__device__ __forceinline__ void values_fixed(const Grid &g, const double2 *cs, const FixedCols &a,
+__device__ __forceinline__ void values_fixed(const Grid &g, const CosEntry *t, const FixedCols &a,
                                              const FixedCols &b, bool swap, double &qo,
                                              double &qs, double &ql, double &w) {
     int h[8], l[8];
@@ -757,36 +793,26 @@ __device__ __forceinline__ void values_fixed(const Grid &g, const double2 *cs, c
     }
     const unsigned neg = swap ? 0x80000000u : 0u;
     {
-        FF dp[4], sp[4], vo, vs, vl;
-#pragma unroll
-        for (int f = 0; f < 4; f++) dp[f] = limbs_ff(h[f], l[f]);
-        sp[0] = limbs_ff(a.c[0].x + b.c[0].x, a.c[0].y + b.c[0].y);
-        sp[1] = limbs_ff(a.c[0].z + b.c[0].z, a.c[0].w + b.c[0].w);
+        const FF dx = limbs_ff(h[0], l[0]), dy = limbs_ff(h[1], l[1]);
+        const FF sx = limbs_ff(a.c[0].x + b.c[0].x, a.c[0].y + b.c[0].y);
+        const FF sy = limbs_ff(a.c[0].z + b.c[0].z, a.c[0].w + b.c[0].w);
+        const FF inv = ff_rsqrt_fast(ff_dot(sx, sx, sy, sy));
+        qo = ff_scaled(ff_mul(ff_dot(dx, sx, dy, sy), inv), neg, -26);
+        qs = ff_scaled(ff_mul(ff_dot(dy, sx, ff_neg(dx), sy), inv), neg, -26);
+        const FF dm = limbs_ff(h[2], l[2]), dp = limbs_ff(h[3], l[3]);
         if (BOOST) {
-            sp[2] = limbs_ff(a.c[1].x + b.c[1].x, a.c[1].y + b.c[1].y);
-            sp[3] = limbs_ff(a.c[1].z + b.c[1].z, a.c[1].w + b.c[1].w);
+            const FF sm = limbs_ff((unsigned)a.c[1].x + (unsigned)b.c[1].x,
+                                   a.c[1].y + b.c[1].y);
+            const FF sp = limbs_ff((unsigned)a.c[1].z + (unsigned)b.c[1].z,
+                                   a.c[1].w + b.c[1].w);
+            const FF n = ff_dot(sm, dp, ff_neg(sp), dm);
+            ql = ff_scaled(ff_mul(n, ff_rsqrt_fast(ff_mul(sm, sp))), neg, -27);
+        } else {
+            ql = ff_scaled(ff_add(dp, ff_neg(dm)), neg, -27);
         }
-        ff_lcms<BOOST>(dp, sp, vo, vs, vl);
-        qo = ff_gev(vo, neg);
-        qs = ff_gev(vs, neg);
-        ql = ff_gev(vl, neg);
     }
-    // high part in 2^-37 steps, the rest in the low 30 bits of hl
     hl += ll >> 30;
-    hh += hl >> 30;
-    const unsigned low = (unsigned)hl << 2;
-    const unsigned fl = (unsigned)hh;
-    const int top = (int)(hh >> 32) + 16;  // + half a step
-    const double2 e = cs[(top >> 5) & (COS_TABLE - 1)];
-    // the remainder, 37 + 15 bits signed, as an FP64 integer (2^-52 steps)
-    const int r = (top & 31) - 16;
-    const double t = __hiloint2double(0x43380000 + (int)__funnelshift_r(fl, (unsigned)r, 17),
-                                      (int)__funnelshift_l(low, fl, 15));
-    const double f = t - 6755399441055744.0;
-    const double f2 = f * f;
-    const double cd = __fma_rn(f2, __fma_rn(f2, g.cfx.c4, g.cfx.c2), 1.0);
-    const double sd = f * __fma_rn(f2, __fma_rn(f2, g.cfx.s5, g.cfx.s3), g.cfx.h);
-    w = __fma_rn(e.x, cd, -(e.y * sd));
+    w = cos_fixed(g, t, hh + (hl >> 30), (unsigned)hl);
 }
 
 // Shared memory of a same-event tile pair.  The i-tile's arrays hold row r at
@@ -795,10 +821,10 @@ __device__ __forceinline__ void values_fixed(const Grid &g, const double2 *cs, c
 // and lane k of it finds its row, and later the rows of neighbouring queue
 // entries, at consecutive places, without bank conflicts.
 struct __align__(16) SameSmem {
-    // FP64 form: fixed-point columns ([4][FT] of int4, FixedCols); the other
-    // forms: split columns ([8][FT] (hi, lo) FP32 pairs px py pz E x y z t)
-    double si[8][FT];
-    double sj[8][FT];
+    // FP64 form: fixed-point columns; the other forms: split columns ([8][FT]
+    // (hi, lo) FP32 pairs px py pz E x y z t) in their place
+    int4 xi[kFixedCols][FT];
+    int4 xj[kFixedCols][FT];
     float4 ta[FT];  // the i-tile's screen terms x, y, m, p
     float2 tb[FT];  // and r2, t2
     TermsPair tj[FT / 2];
@@ -1012,7 +1038,7 @@ __device__ __forceinline__ FixedCols load_fixed(const Grid &g, const ListRows &l
     if (k >= l.n) return r;
     if (l.fixed) {
 #pragma unroll
-        for (int f = 0; f < 4; f++) r.c[f] = l.fixed[f * l.stride + k];
+            for (int f = 0; f < kFixedCols; f++) r.c[f] = l.fixed[f * l.stride + k];
         return r;
     }
     double v[8];
@@ -1086,23 +1112,21 @@ __device__ __forceinline__ void screen_loop(const Screen &S, const Terms &terms,
 // caller's list).
 // Called by all FT threads of the CTA; the caller syncs before reusing `sm`.
 template <bool AZ, bool BOOST, int PREC, int MODE = MODE_FAST>
-__device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, const double2 *cs,
+__device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, const void *cs,
                                                const ListRows &l, long long i0, long long j0) {
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int at_i = place_of(tid);  // this thread loads row tid of each tile
     const long long n = l.n;
     const double *const *c = l.c;
-    int4(*xi)[FT] = reinterpret_cast<int4(*)[FT]>(&sm.si[0][0]);
-    int4(*xj)[FT] = reinterpret_cast<int4(*)[FT]>(&sm.sj[0][0]);
     // split columns of the FP32-weight and double-float forms, in their place
-    float2(*spi)[FT] = reinterpret_cast<float2(*)[FT]>(&sm.si[0][0]);
-    float2(*spj)[FT] = reinterpret_cast<float2(*)[FT]>(&sm.sj[0][0]);
+    float2(*spi)[FT] = reinterpret_cast<float2(*)[FT]>(&sm.xi[0][0]);
+    float2(*spj)[FT] = reinterpret_cast<float2(*)[FT]>(&sm.xj[0][0]);
     if (PREC == 0) {
         const FixedCols a = load_fixed(d.g, l, i0 + tid), b = load_fixed(d.g, l, j0 + tid);
 #pragma unroll
-        for (int f = 0; f < 4; f++) {
-            xi[f][at_i] = a.c[f];
-            xj[f][tid] = b.c[f];
+        for (int f = 0; f < kFixedCols; f++) {
+            sm.xi[f][at_i] = a.c[f];
+            sm.xj[f][tid] = b.c[f];
         }
     } else if (PREC == 1) {
         for (int f = 0; f < 8; f++) {
@@ -1204,19 +1228,20 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
                 a[f] = spi[f][qi];
                 b[f] = spj[f][qj];
             }
-            values_df<BOOST>(d.s, reinterpret_cast<const float4 *>(cs), a, b, sm.offi, sm.offj,
+            values_df<BOOST>(d.s, static_cast<const float4 *>(cs), a, b, sm.offi, sm.offj,
                              swap, vo, vs, vl, vw);
         } else {
             FixedCols a, b;
 #pragma unroll
-            for (int f = 0; f < 4; f++) {
-                a.c[f] = xi[f][qi];
-                b.c[f] = xj[f][qj];
+            for (int f = 0; f < kFixedCols; f++) {
+                a.c[f] = sm.xi[f][qi];
+                b.c[f] = sm.xj[f][qj];
             }
-            if (a.c[1].z == kFar || b.c[1].z == kFar)
-                values64_rows<BOOST>(d.g, cs, c, i0 + row_at(qi), j0 + qj, swap, vo, vs, vl, vw);
+            if (a.c[1].x == kFar || b.c[1].x == kFar)
+                values64_rows<BOOST>(d.g, c, i0 + row_at(qi), j0 + qj, swap, vo, vs, vl, vw);
             else
-                values_fixed<BOOST>(d.g, cs, a, b, swap, vo, vs, vl, vw);
+                values_fixed<BOOST>(d.g, static_cast<const CosEntry *>(cs), a, b, swap, vo, vs,
+                                    vl, vw);
         }
         Sums *h = d.h.sums + at;
         atomicAdd(&h->qo, vo);
