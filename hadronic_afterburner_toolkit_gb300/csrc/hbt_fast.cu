@@ -18,7 +18,7 @@ template <bool AZ, bool BOOST, int PREC>
 __global__ void __launch_bounds__(FT) k_same_screened(Device d, long long n, Cols8 c) {
     __shared__ SameSmem sm;
     __shared__ double2 cs[kCosEntries];
-    if (PREC == 0) fill_cos_entries(reinterpret_cast<CosEntry *>(cs));
+    if (PREC == 0) fill_cos_entries(reinterpret_cast<double *>(cs));
     if (PREC == 2) fill_df_table(reinterpret_cast<float4 *>(cs));
     long long ti, tj;
     tri_tile((long long)blockIdx.x + d.block_offset, ti, tj);

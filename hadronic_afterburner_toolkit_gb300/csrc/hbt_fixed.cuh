@@ -96,18 +96,21 @@ __device__ __forceinline__ FixedCols fixed_cols(const Grid &g, const double *v) 
 }
 
 // Cosine table of the fixed-point values: cos(2 pi k / 2048) for a quarter
-// period, k = 0..512, in FP64 and a sixth of it in FP32, filled by each CTA.
-struct __align__(16) CosEntry {
-    double c;
-    float sixth;
-    float pad;
-};
+// period, k = 0..512, filled by each CTA (FP64 alone: with an FP32 copy beside
+// each entry, the random reads took twice the shared-memory wavefronts).  The
+// last entry, zero, is a number too small to matter whose exponent fits FP32
+// (cos_fixed takes FP32 values from the bits).
 constexpr int kCosEntries = 513;
-__device__ __forceinline__ void fill_cos_entries(CosEntry *t) {
-    for (int k = threadIdx.x; k < kCosEntries; k += blockDim.x) {
-        t[k].c = cospi(k / 1024.0);
-        t[k].sixth = (float)(t[k].c * (1.0 / 6.0));
-    }
+__device__ __forceinline__ void fill_cos_entries(double *t) {
+    for (int k = threadIdx.x; k < kCosEntries; k += blockDim.x)
+        t[k] = k < kCosEntries - 1 ? cospi(k / 1024.0) : 0x1p-100;
+}
+
+// The FP32 value of the leading 24 bits of a normal FP64 one within FP32's
+// exponent range.
+__device__ __forceinline__ float f64_top_bits(double x) {
+    const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+    return __uint_as_float(__funnelshift_l(l, h - (896u << 20), 3) & 0x7fffffffu | h & 0x80000000u);
 }
 
 // cos of a phase given as hh 2^-37 + (low 30 bits of hl) 2^-67 steps of
@@ -118,29 +121,30 @@ __device__ __forceinline__ void fill_cos_entries(CosEntry *t) {
 // the first three terms in FP64 (d exact but for one rounding), the last
 // two, below 6e-10, in FP32 (the next, V d^5 / 120, is below 7e-17).  Error
 // below 4e-16.
-__device__ __forceinline__ double cos_fixed(const Grid &g, const CosEntry *t, long long hh,
+__device__ __forceinline__ double cos_fixed(const Grid &g, const double *t, long long hh,
                                             unsigned hl) {
     const unsigned fl = (unsigned)hh, low = hl << 2;
     const int top = (int)(hh >> 32) + 4;  // + half a step
     const int r = (top & 7) - 4;          // remainder: r, fl, low as one signed number
     const int j = top >> 3, odd = j & 512, idx = j & 511;
     const int iu = odd ? 512 - idx : idx;
-    const CosEntry eu = t[iu], ev = t[512 - iu];
+    const double U = t[iu], tv = t[512 - iu];
     const unsigned sv = (unsigned)odd << 22;              // V's sign, as a sign bit
     const unsigned sr = (unsigned)((j + 512) & 1024) << 21;  // the result's
-    const double V = __hiloint2double(__double2hiint(ev.c) ^ (int)sv, __double2loint(ev.c));
+    const double V = __hiloint2double(__double2hiint(tv) ^ (int)sv, __double2loint(tv));
     // 52-bit signed integer remainder (2^-52 steps) as FP64
     const double z = __hiloint2double(0x43380000 + (int)__funnelshift_r(fl, (unsigned)r, 15),
                                       (int)__funnelshift_l(low, fl, 17)) -
                      6755399441055744.0;
     const double hd = z * g.cfx_half;  // d / 2
     const double d = __hiloint2double(__double2hiint(hd) + (1 << 20), __double2loint(hd));
-    const double main = __fma_rn(-d, __fma_rn(hd, eu.c, V), eu.c);
+    const double main = __fma_rn(-d, __fma_rn(hd, U, V), U);
     const float x = __int2float_rn((int)__funnelshift_r(fl, (unsigned)r, 3)) *
                     (float)(6.283185307179586 / 2048.0 / 4294967296.0);
     const float x2 = x * x;
-    const float vf = __uint_as_float(__float_as_uint(ev.sixth) ^ sv);
-    const float b = x2 * __fmaf_rn(x, vf, 0.25f * (x2 * eu.sixth));
+    // d^3 V / 6 + d^4 U / 24
+    const float b = (x2 * (1.0f / 6.0f)) *
+                    __fmaf_rn(x, f64_top_bits(V), 0.25f * (x2 * f64_top_bits(U)));
     // b as FP64 through its bits (a zero becomes a number below 1e-38)
     const int bi = __float_as_int(b);
     const double bd = __hiloint2double(((bi >> 3) & (int)0x8fffffff) + (896 << 20), bi << 29);

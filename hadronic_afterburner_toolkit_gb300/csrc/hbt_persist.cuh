@@ -123,10 +123,11 @@ __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(D
     __shared__ typename std::conditional<QINV, QinvSmem, SameSmem>::type sm;
     __shared__ unsigned item;
     // the form's cos table
-    constexpr int kTable = PREC == 0 ? (QINV ? COS_TABLE : kCosEntries) : (PREC == 2 ? DF_TABLE : 1);
+    constexpr int kTable =
+        PREC == 0 ? (QINV ? COS_TABLE : (kCosEntries + 1) / 2) : (PREC == 2 ? DF_TABLE : 1);
     __shared__ double2 cs[kTable];
     if (PREC == 0 && QINV) fill_cos_table(cs);
-    if (PREC == 0 && !QINV) fill_cos_entries(reinterpret_cast<CosEntry *>(cs));
+    if (PREC == 0 && !QINV) fill_cos_entries(reinterpret_cast<double *>(cs));
     if (PREC == 2) fill_df_table(reinterpret_cast<float4 *>(cs));
     const unsigned stop = min(end, min(b.n_items[0], b.same_cap));
     for (;;) {

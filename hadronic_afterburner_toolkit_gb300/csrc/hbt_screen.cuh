@@ -96,6 +96,12 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+// 1 / x, relative error 1 ulp (as 1 / sqrt(x): no subnormals).
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 __device__ __forceinline__ f2 rsqrt2(f2 v) {
     float a, b;
     unpack2(v, a, b);
@@ -273,7 +279,7 @@ __device__ __forceinline__ int slot_of(const Screen &S, float ax, float ay, floa
         const float cx = __fmaf_rn(sy, S.sp_sin, sx * S.sp_cos);
         const float cy = __fmaf_rn(sy, S.sp_cos, -(sx * S.sp_sin));
         const float ux = fabsf(cx), uy = fabsf(cy);
-        const float z = __fdividef(fminf(ux, uy), fmaxf(ux, uy));
+        const float z = fminf(ux, uy) * rcp_approx(fmaxf(ux, uy));
         const float z2 = z * z;
         // arctan z / z, times n_Kphi / (2 pi) at the end
         const float pl = __fmaf_rn(

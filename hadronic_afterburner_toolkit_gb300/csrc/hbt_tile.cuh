@@ -749,19 +749,16 @@ __device__ __forceinline__ FF ff_rsqrt_fast(FF x) {
 }
 
 // hi + lo rounded to FP64, its sign changed by `neg` (a sign bit), times
-// 2^shift, on the integer pipe: hi's bits as FP64, then lo in units of hi's
-// last FP64 place added to them as a signed integer (twice that count below
-// a power of two, whose places are half as wide).
+// 2^shift: both parts converted on the integer pipe (a zero part becomes a
+// number below 1e-38, far under the rounding of any sum it enters) and added
+// in FP64.
 __device__ __forceinline__ double ff_scaled(FF a, unsigned neg, int shift) {
-    const unsigned u = __float_as_uint(a.h);
-    const float unit = __uint_as_float((306u << 23) - (u & 0x7f800000u));
-    int lo = __float2int_rn(__uint_as_float(__float_as_uint(a.l) ^ (u & 0x80000000u)) * unit);
-    if ((u & 0x7fffffu) == 0u && lo < 0) lo *= 2;
-    const unsigned s = u ^ neg;
-    const long long hi =
-        ((long long)(((int)s >> 3) & (int)0x8fffffff) + ((long long)(896 + shift) << 20)) << 32 |
-        (s << 29);
-    return __longlong_as_double(hi + lo);
+    auto conv = [&](float x) {
+        const unsigned u = __float_as_uint(x) ^ neg;
+        return __hiloint2double((((int)u >> 3) & (int)0x8fffffff) + ((896 + shift) << 20),
+                                (int)(u << 29));
+    };
+    return conv(a.h) + conv(a.l);
 }
 
 // Summed values of an accepted same-event pair from its fixed-point columns
@@ -772,7 +769,7 @@ __device__ __forceinline__ double ff_scaled(FF a, unsigned neg, int shift) {
 // bit products: with the limbs (h, l) of a difference, sum of h h' (unit
 // 2^-37 table steps), h l' + l h' (2^-67) and l l' (2^-97).
 template <bool BOOST>
-__device__ __forceinline__ void values_fixed(const Grid &g, const CosEntry *t, const FixedCols &a,
+__device__ __forceinline__ void values_fixed(const Grid &g, const double *t, const FixedCols &a,
                                              const FixedCols &b, bool swap, double &qo,
                                              double &qs, double &ql, double &w) {
     int h[8], l[8];
@@ -835,6 +832,10 @@ struct __align__(16) SameSmem {
     unsigned queue3[FT / 32][QCAP];
     unsigned oi[FT], oj[FT];  // original list positions (pair orientation)
     float offi[4], offj[4];   // double-float form: the tiles' momentum offsets
+    // FP64 and double-float forms: 32 pairs' sums and bins on their way out
+    // (add_sums)
+    double2 sums[FT / 32][2][32];
+    Sums *bins[FT / 32][32];
 };
 // Place of row r in the i-tile's arrays, and back.
 __device__ __forceinline__ int place_of(int r) { return (r >> 2) | ((r & 3) << 5); }
@@ -1102,6 +1103,30 @@ __device__ __forceinline__ void screen_loop(const Screen &S, const Terms &terms,
     }
 }
 
+// Adds 32 pairs' sums to their bins (bin: nullptr, none), all lanes of the
+// warp in step.  The four sums of a pair are added by four neighbouring lanes,
+// so that each of the four instructions touches 8 sectors of 32 bytes: with
+// each lane adding its own pair's sums one after another, every instruction
+// touches 32, and the L1 pipe that splits them bounded the kernel (79 % busy;
+// central group 58.5 ms, 56.6 ms with the values left out and 47.2 ms with
+// the additions left out; 52.3 ms this way).
+__device__ __forceinline__ void add_sums(double2 (*sums)[32], Sums **bins, Sums *bin, double qo,
+                                         double qs, double ql, double w) {
+    const int lane = threadIdx.x & 31, c = lane & 3;
+    sums[0][lane] = make_double2(qo, qs);
+    sums[1][lane] = make_double2(ql, w);
+    bins[lane] = bin;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const int p = 8 * r + (lane >> 2);
+        Sums *b = bins[p];
+        const double v = reinterpret_cast<const double *>(&sums[c >> 1][p])[c & 1];
+        if (b) atomicAdd(reinterpret_cast<double *>(b) + c, v);
+    }
+    __syncwarp();
+}
+
 // Same-event pairs of the tiles starting at i0 and j0 (i0 <= j0) of one list
 // of particles.  Every unordered pair
 // is visited once (position j > i); it is oriented as the reference orients
@@ -1192,15 +1217,18 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
             undecided_pair64(d, A, B, i0 + ri, j0 + qj, n);
     };
 
-    // one pair with its q bin and slot decided: its values into its bin
-    auto decided = [&](unsigned e, int slot, unsigned bin) {
+    // one pair with its q bin and slot decided: its values, and its bin (the
+    // FP32-weight form adds them here and returns no bin)
+    auto decided = [&](unsigned e, int slot, unsigned bin, double &vo, double &vs, double &vl,
+                       double &vw) -> Sums * {
         const int qi = e & 0xff, qj = (e >> 8) & 0xff;
         const unsigned oa = sm.oi[qi], ob = sm.oj[qj];
         const bool swap = oa > ob;
         if (MODE != MODE_FAST) {
-            if (!admit<MODE>(d, slot, (long long)min(oa, ob), n)) return;
+            if (!admit<MODE>(d, slot, (long long)min(oa, ob), n)) return nullptr;
         }
         const long long at = (long long)slot * d.g.q3 + bin;
+        atomicAdd(d.h.cnt + at, 1ull);
         if (PREC == 1) {
             // the pair as stored (i, j); swapping first and second negates
             // q_out, q_side, q_long exactly and leaves the phase unchanged
@@ -1217,10 +1245,8 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
                 v.z = -v.z;
             }
             atomicAdd(partials_of(d) + at, v);
-            atomicAdd(d.h.cnt + at, 1ull);
-            return;
+            return nullptr;
         }
-        double vo, vs, vl, vw;
         if (PREC == 2) {
             float2 a[8], b[8];
 #pragma unroll
@@ -1240,15 +1266,10 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
             if (a.c[1].x == kFar || b.c[1].x == kFar)
                 values64_rows<BOOST>(d.g, c, i0 + row_at(qi), j0 + qj, swap, vo, vs, vl, vw);
             else
-                values_fixed<BOOST>(d.g, static_cast<const CosEntry *>(cs), a, b, swap, vo, vs,
+                values_fixed<BOOST>(d.g, static_cast<const double *>(cs), a, b, swap, vo, vs,
                                     vl, vw);
         }
-        Sums *h = d.h.sums + at;
-        atomicAdd(&h->qo, vo);
-        atomicAdd(&h->qs, vs);
-        atomicAdd(&h->ql, vl);
-        atomicAdd(&h->w, vw);
-        atomicAdd(d.h.cnt + at, 1ull);
+        return d.h.sums + at;
     };
 
     // 32 pairs that passed the screen (all lanes of the warp in step): their
@@ -1264,7 +1285,11 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
             slot = slot_of<AZ>(S, a.x, a.y, b.x[qj & 1], b.y[qj & 1]);
             if (slot != -2 && ((e2.x >> 16) || e2.y >= S.sc_q3)) slot = -1;
         }
-        if (slot >= 0) decided(e, slot, e2.y);
+        double vo = 0.0, vs = 0.0, vl = 0.0, vw = 0.0;
+        Sums *bin = nullptr;
+        if (slot >= 0) bin = decided(e, slot, e2.y, vo, vs, vl, vw);
+        if (PREC != 1 && MODE != MODE_COUNT)
+            add_sums(sm.sums[w], sm.bins[w], bin, vo, vs, vl, vw);
         enqueue(q3, count3, slot == -1, e, lane, chains);
     };
 
