@@ -17,9 +17,8 @@ using namespace tile;
 template <bool AZ, bool BOOST, int PREC>
 __global__ void __launch_bounds__(FT) k_same_screened(Device d, long long n, Cols8 c) {
     __shared__ SameSmem sm;
-    __shared__ double2 cs[kCosEntries];
-    if (PREC == 0) fill_cos_entries(reinterpret_cast<double *>(cs));
-    if (PREC == 2) fill_df_table(reinterpret_cast<float4 *>(cs));
+    __shared__ double cs[PREC == 0 ? kCosEntries : 1];
+    if (PREC == 0) fill_cos_entries(cs);
     long long ti, tj;
     tri_tile((long long)blockIdx.x + d.block_offset, ti, tj);
     const ListRows l = {c.p, nullptr, nullptr, nullptr, nullptr, 0, n};
@@ -88,7 +87,8 @@ cudaError_t launch_same_fast(const Device &d0, long long n, const double *const 
     Cols8 c;
     for (int f = 0; f < 8; f++) c.p[f] = c8[f];
     const bool az = d0.g.azimuthal, boost = d0.g.boost;
-    const int prec = d0.precision;
+    // the double-float form runs the FP64 form's kernel (launch_same_mode)
+    const int prec = d0.precision == 1 ? 1 : 0;
     // FP32 partials are merged every `chunk` CTAs to bound the number of
     // terms an FP32 partial bin accumulates
     long long chunk = prec == 1 ? (d0.merge_chunk_blocks > 0 ? d0.merge_chunk_blocks : blocks)
@@ -104,16 +104,11 @@ cudaError_t launch_same_fast(const Device &d0, long long n, const double *const 
             else if (az) HBT_SAME(true, false, 0);
             else if (boost) HBT_SAME(false, true, 0);
             else HBT_SAME(false, false, 0);
-        } else if (prec == 1) {
+        } else {
             if (az && boost) HBT_SAME(true, true, 1);
             else if (az) HBT_SAME(true, false, 1);
             else if (boost) HBT_SAME(false, true, 1);
             else HBT_SAME(false, false, 1);
-        } else {
-            if (az && boost) HBT_SAME(true, true, 2);
-            else if (az) HBT_SAME(true, false, 2);
-            else if (boost) HBT_SAME(false, true, 2);
-            else HBT_SAME(false, false, 2);
         }
 #undef HBT_SAME
         cudaError_t e = cudaGetLastError();

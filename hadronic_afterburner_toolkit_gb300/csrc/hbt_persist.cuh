@@ -83,7 +83,7 @@ constexpr int kMixedCtas = HBT_MIXED_CTAS;
 template <bool AZ, bool BOOST, int PREC, int MODE>
 __device__ __forceinline__ void same_item(const Device &d, SameSmem &sm, const void *cs,
                                           const ListRows &l, const Item &it) {
-    same_tile_pair<AZ, BOOST, PREC, MODE>(d, sm, cs, l, (long long)it.ti * FT,
+    same_tile_pair<AZ, BOOST, PREC, MODE>(d, sm, static_cast<const double *>(cs), l, (long long)it.ti * FT,
                                           (long long)it.tj * FT);
 }
 template <bool AZ, bool BOOST, int PREC, int MODE>
@@ -246,9 +246,12 @@ template <int MODE, bool QINV>
 cudaError_t launch_same_mode(const Device &d, const BatchDev &b, unsigned base, unsigned end,
                              int grid, cudaStream_t st) {
     const bool az = d.g.azimuthal, boost = d.g.boost;
-    // the forms this mode instantiates: FP64 only for COUNT
-    constexpr int P1 = MODE == MODE_COUNT ? 0 : 1, P2 = MODE == MODE_COUNT ? 0 : 2;
-    const int prec = MODE == MODE_COUNT ? 0 : d.precision;
+    // the forms this mode instantiates: FP64 only for COUNT; the double-float
+    // form runs the FP64 form's kernel (same bins, closer values, and faster
+    // than double-float arithmetic since those come from fixed-point columns:
+    // central group 50.7 against 79.7 ms), except with q_inv histograms
+    constexpr int P1 = MODE == MODE_COUNT ? 0 : 1, P2 = QINV && MODE != MODE_COUNT ? 2 : 0;
+    const int prec = MODE == MODE_COUNT ? 0 : (d.precision == 2 ? P2 : d.precision);
 #define HBT_P(AZ_, BO_, PR_) \
     return launch_same_items<AZ_, BO_, PR_, MODE, QINV>(d, b, base, end, grid, st)
     if (prec == 0) {

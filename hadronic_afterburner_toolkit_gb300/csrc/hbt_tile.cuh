@@ -812,14 +812,98 @@ __device__ __forceinline__ void values_fixed(const Grid &g, const double *t, con
     w = cos_fixed(g, t, hh + (hl >> 30), (unsigned)hl);
 }
 
+// Limbs (h, l) of a difference or sum in FP32, in units of h.
+__device__ __forceinline__ float limbs_f(int h, int l) {
+    return __fmaf_rn(__int2float_rn(l), 0x1p-30f, __int2float_rn(h));
+}
+
+// Summed values of the FP32-weight form from the fixed-point columns, for
+// the pair as stored, negated in q when `swap`: q_out, q_side, q_long in FP32
+// from exact differences and sums (a few 1e-7 relative; q_long = (s(m) d(p) -
+// s(p) d(m)) / (2 sqrt(s(m) s(p))), whose two terms add up); the phase as in
+// values_fixed without the products of the low limbs (below 1e-13 rad), its
+// cos by the quarter period's Taylor polynomials of ff_cos (below 2e-7).
+template <bool BOOST>
+__device__ __forceinline__ float4 values32_fixed(const FixedCols &a, const FixedCols &b,
+                                                 bool swap) {
+    int h[8], l[8];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        h[2 * k] = a.c[k].x - b.c[k].x;
+        l[2 * k] = a.c[k].y - b.c[k].y;
+        h[2 * k + 1] = a.c[k].z - b.c[k].z;
+        l[2 * k + 1] = a.c[k].w - b.c[k].w;
+    }
+    long long hh = 0, hl = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        hh += (long long)h[k] * h[k + 4];
+        hl += (long long)h[k] * l[k + 4];
+        hl += (long long)l[k] * h[k + 4];
+    }
+    hh += hl >> 30;
+    const float unit = swap ? -0x1p-26f : 0x1p-26f;  // GeV
+    const float dx = limbs_f(h[0], l[0]), dy = limbs_f(h[1], l[1]);
+    const float dm = limbs_f(h[2], l[2]), dp = limbs_f(h[3], l[3]);
+    const float sx = limbs_f(a.c[0].x + b.c[0].x, a.c[0].y + b.c[0].y);
+    const float sy = limbs_f(a.c[0].z + b.c[0].z, a.c[0].w + b.c[0].w);
+    const float inv = rsqrt_approx(__fmaf_rn(sx, sx, sy * sy)) * unit;
+    float4 v;
+    v.x = __fmaf_rn(dx, sx, dy * sy) * inv;
+    v.y = __fmaf_rn(dy, sx, -(dx * sy)) * inv;
+    if (BOOST) {
+        // (the low limbs change these sums by 2^-27 GeV at most)
+        const float sm = __uint2float_rn((unsigned)a.c[1].x + (unsigned)b.c[1].x);
+        const float sp = __uint2float_rn((unsigned)a.c[1].z + (unsigned)b.c[1].z);
+        v.z = __fmaf_rn(sm, dp, -(sp * dm)) * (rsqrt_approx(sm * sp) * (0.5f * unit));
+    } else {
+        v.z = (dp - dm) * (0.5f * unit);
+    }
+    // period 2^46 units of hh: quarter and remainder, the latter in 2^-34
+    // periods
+    const int top = (int)(hh >> 32) + 2048;  // + half a quarter
+    const int r = (top & 4095) - 2048, quad = top >> 12;
+    const float x = __int2float_rn((int)__funnelshift_r((unsigned)hh, (unsigned)r, 12)) *
+                    (float)(6.283185307179586 / 17179869184.0);
+    const float x2 = x * x;
+    const float c = __fmaf_rn(x2, __fmaf_rn(x2, __fmaf_rn(x2, __fmaf_rn(x2, 2.48015873e-5f,
+                                                                      -1.38888889e-3f),
+                                                          4.16666667e-2f),
+                                            -0.5f),
+                              1.0f);
+    const float s = x * __fmaf_rn(x2, __fmaf_rn(x2, __fmaf_rn(x2, __fmaf_rn(x2, 2.75573192e-6f,
+                                                                          -1.98412698e-4f),
+                                                              8.33333333e-3f),
+                                                -1.66666667e-1f),
+                                  1.0f);
+    // cos(x + quad pi / 2): c, -s, -c, s
+    v.w = __uint_as_float(__float_as_uint(quad & 1 ? s : c) ^
+                          ((unsigned)((quad + 1) & 2) << 30));
+    return v;
+}
+
+// values32 from the FP64 columns of rows i and j (pairs of particles that do
+// not fit the fixed-point columns; out of line, as values64_rows).
+template <bool BOOST>
+__device__ __noinline__ float4 values32_rows(const Grid &g, const double *const *c, long long i,
+                                             long long j, bool swap) {
+    double a[8], b[8];
+#pragma unroll
+    for (int f = 0; f < 8; f++) {
+        const double u = c[f][i], v = c[f][j];
+        a[f] = swap ? v : u;
+        b[f] = swap ? u : v;
+    }
+    return values32<BOOST>(g, a, b);
+}
+
 // Shared memory of a same-event tile pair.  The i-tile's arrays hold row r at
 // place (r >> 2) + 32 (r & 3): warp w screens the rows w, w + 4, ... (sorted in
 // momentum space, so interleaving evens out the binned pairs between warps),
 // and lane k of it finds its row, and later the rows of neighbouring queue
 // entries, at consecutive places, without bank conflicts.
 struct __align__(16) SameSmem {
-    // FP64 form: fixed-point columns; the other forms: split columns ([8][FT]
-    // (hi, lo) FP32 pairs px py pz E x y z t) in their place
+    // fixed-point columns
     int4 xi[kFixedCols][FT];
     int4 xj[kFixedCols][FT];
     float4 ta[FT];  // the i-tile's screen terms x, y, m, p
@@ -831,8 +915,7 @@ struct __align__(16) SameSmem {
     // time (inline, a warp would run it for the one or two lanes holding one)
     unsigned queue3[FT / 32][QCAP];
     unsigned oi[FT], oj[FT];  // original list positions (pair orientation)
-    float offi[4], offj[4];   // double-float form: the tiles' momentum offsets
-    // FP64 and double-float forms: 32 pairs' sums and bins on their way out
+    // FP64 form: 32 pairs' sums and bins on their way out
     // (add_sums)
     double2 sums[FT / 32][2][32];
     Sums *bins[FT / 32][32];
@@ -1137,43 +1220,18 @@ __device__ __forceinline__ void add_sums(double2 (*sums)[32], Sums **bins, Sums 
 // caller's list).
 // Called by all FT threads of the CTA; the caller syncs before reusing `sm`.
 template <bool AZ, bool BOOST, int PREC, int MODE = MODE_FAST>
-__device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, const void *cs,
+__device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, const double *cs,
                                                const ListRows &l, long long i0, long long j0) {
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int at_i = place_of(tid);  // this thread loads row tid of each tile
     const long long n = l.n;
     const double *const *c = l.c;
-    // split columns of the FP32-weight and double-float forms, in their place
-    float2(*spi)[FT] = reinterpret_cast<float2(*)[FT]>(&sm.xi[0][0]);
-    float2(*spj)[FT] = reinterpret_cast<float2(*)[FT]>(&sm.xj[0][0]);
-    if (PREC == 0) {
+    {
         const FixedCols a = load_fixed(d.g, l, i0 + tid), b = load_fixed(d.g, l, j0 + tid);
 #pragma unroll
         for (int f = 0; f < kFixedCols; f++) {
             sm.xi[f][at_i] = a.c[f];
             sm.xj[f][tid] = b.c[f];
-        }
-    } else if (PREC == 1) {
-        for (int f = 0; f < 8; f++) {
-            spi[f][at_i] = split((i0 + tid < n) ? c[f][i0 + tid] : 0.0);
-            spj[f][tid] = split((j0 + tid < n) ? c[f][j0 + tid] : 0.0);
-        }
-    } else {
-        // double-float form: momenta split relative to the tile's first row
-        for (int f = 0; f < 8; f++) {
-            const double vi = (i0 + tid < n) ? c[f][i0 + tid] : 0.0;
-            const double vj = (j0 + tid < n) ? c[f][j0 + tid] : 0.0;
-            float oi = 0.0f, oj = 0.0f;
-            if (f < 4) {
-                oi = (float)c[f][i0];
-                oj = (float)c[f][j0];
-                if (tid == 0) {
-                    sm.offi[f] = oi;
-                    sm.offj[f] = oj;
-                }
-            }
-            spi[f][at_i] = split(vi - (double)oi);
-            spj[f][tid] = split(vj - (double)oj);
         }
     }
     sm.oi[at_i] = l.orig ? (i0 + tid < n ? l.orig[i0 + tid] : 0u) : (unsigned)(i0 + tid);
@@ -1229,46 +1287,26 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
         }
         const long long at = (long long)slot * d.g.q3 + bin;
         atomicAdd(d.h.cnt + at, 1ull);
-        if (PREC == 1) {
-            // the pair as stored (i, j); swapping first and second negates
-            // q_out, q_side, q_long exactly and leaves the phase unchanged
-            float2 a[8], b[8];
+        FixedCols a, b;
 #pragma unroll
-            for (int f = 0; f < 8; f++) {
-                a[f] = spi[f][qi];
-                b[f] = spj[f][qj];
-            }
-            float4 v = values32_split<BOOST>(d.s, a, b);
-            if (swap) {
-                v.x = -v.x;
-                v.y = -v.y;
-                v.z = -v.z;
-            }
+        for (int f = 0; f < kFixedCols; f++) {
+            a.c[f] = sm.xi[f][qi];
+            b.c[f] = sm.xj[f][qj];
+        }
+        const bool far = a.c[1].x == kFar || b.c[1].x == kFar;
+        if (PREC == 1) {
+            float4 v;
+            if (far)
+                v = values32_rows<BOOST>(d.g, c, i0 + row_at(qi), j0 + qj, swap);
+            else
+                v = values32_fixed<BOOST>(a, b, swap);
             atomicAdd(partials_of(d) + at, v);
             return nullptr;
         }
-        if (PREC == 2) {
-            float2 a[8], b[8];
-#pragma unroll
-            for (int f = 0; f < 8; f++) {
-                a[f] = spi[f][qi];
-                b[f] = spj[f][qj];
-            }
-            values_df<BOOST>(d.s, static_cast<const float4 *>(cs), a, b, sm.offi, sm.offj,
-                             swap, vo, vs, vl, vw);
-        } else {
-            FixedCols a, b;
-#pragma unroll
-            for (int f = 0; f < kFixedCols; f++) {
-                a.c[f] = sm.xi[f][qi];
-                b.c[f] = sm.xj[f][qj];
-            }
-            if (a.c[1].x == kFar || b.c[1].x == kFar)
-                values64_rows<BOOST>(d.g, c, i0 + row_at(qi), j0 + qj, swap, vo, vs, vl, vw);
-            else
-                values_fixed<BOOST>(d.g, static_cast<const double *>(cs), a, b, swap, vo, vs,
-                                    vl, vw);
-        }
+        if (far)
+            values64_rows<BOOST>(d.g, c, i0 + row_at(qi), j0 + qj, swap, vo, vs, vl, vw);
+        else
+            values_fixed<BOOST>(d.g, cs, a, b, swap, vo, vs, vl, vw);
         return d.h.sums + at;
     };
 

@@ -28,7 +28,8 @@ def particles(n, seed, x_scale, p_scale):
     return [px, py, pz, E] + pos
 
 
-@pytest.mark.parametrize("precision", [engine.PRECISION_FP64, engine.PRECISION_DF64])
+@pytest.mark.parametrize("precision", [engine.PRECISION_FP64, engine.PRECISION_DF64,
+                                       engine.PRECISION_FP32W])
 @pytest.mark.parametrize("boost", [0, 1])
 @pytest.mark.parametrize("x_scale,p_scale", [(3.0, 0.0), (3.0, 7.9), (300.0, 0.4), (5000.0, 8.0)])
 def test_values_equal_the_oracle(x_scale, p_scale, boost, precision):
@@ -47,6 +48,8 @@ def test_values_equal_the_oracle(x_scale, p_scale, boost, precision):
     if precision == engine.PRECISION_DF64:
         phase *= 64.0  # its stated accuracy allows 48-bit values
     n = np.maximum(o["count"], 1.0)
-    assert np.all(np.abs(h["num"] - o["num"]) <= n * (1e-15 + phase))
+    # FP32 weights: the form's stated bound
+    fp32 = precision == engine.PRECISION_FP32W
+    assert np.all(np.abs(h["num"] - o["num"]) <= n * ((1e-5 if fp32 else 1e-15) + phase))
     for k in ("q_out", "q_side", "q_long"):
-        assert np.all(np.abs(h[k] - o[k]) <= 1e-12 * 0.225 * n), k
+        assert np.all(np.abs(h[k] - o[k]) <= (1e-5 if fp32 else 1e-12) * 0.225 * n), k
