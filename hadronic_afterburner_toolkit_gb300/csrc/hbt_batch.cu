@@ -26,6 +26,7 @@
 //     same-event and mixed-event queues and run the screened tile-pair
 //     bodies of hbt_tile.cuh.  The FP32-weight form runs the same-event
 //     queue in chunks and merges the FP32 partials between them.
+#include <cub/block/block_radix_sort.cuh>
 #include <cub/device/device_radix_sort.cuh>
 
 #include "hbt_batch.cuh"
@@ -69,7 +70,16 @@ __device__ __forceinline__ unsigned cell(double v, double origin, double inv_h) 
     return (unsigned)c;
 }
 
+// The queues start empty (the first kernel of a batch clears their counters).
+__device__ __forceinline__ void clear_queues(const BatchDev &b) {
+    if (blockIdx.x == 0 && threadIdx.x < 2) {
+        b.n_items[threadIdx.x] = 0u;
+        b.item_next[threadIdx.x] = 0u;
+    }
+}
+
 __global__ void k_keys(BatchDev b) {
+    clear_queues(b);
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < b.total;
          g += (long long)gridDim.x * blockDim.x) {
         const int L = find_range(b.list_off, b.n_lists, g);
@@ -85,43 +95,44 @@ __global__ void k_keys(BatchDev b) {
     }
 }
 
-// Sorted rows, and each row's screen terms and fixed-point columns (once per
-// particle here; a tile pair would convert its 256 particles again each time
-// it is taken).
-template <bool BOOST>
+// Row s of the sorted table from row k of list l: its columns, screen terms
+// and fixed-point columns (once per particle here; a tile pair would convert
+// its 256 particles again each time it is taken) and its position in the
+// caller's list.
+template <bool LC>
+__device__ __forceinline__ void put_row(const BatchDev &b, const Grid &g, const BatchList &l,
+                                        long long s, long long k) {
+    double v[8];
+#pragma unroll
+    for (int f = 0; f < 8; f++)
+        if (f < l.ncols) {
+            v[f] = l.src[f][k];
+            b.table[(long long)f * b.cap + s] = v[f];
+        }
+    const Terms t = screen_terms<LC>(v[0], v[1], v[2], v[3]);
+    b.terms4[s] = make_float4(t.x, t.y, t.m, t.p);
+    b.terms2[s] = make_float2(t.r2, t.t2);
+    if (l.ncols == 8) {
+        const FixedCols c = fixed_cols(g, v);
+#pragma unroll
+        for (int f = 0; f < kFixedCols; f++) b.fixed[(long long)f * b.cap + s] = c.c[f];
+    }
+    b.orig[s] = (unsigned)k;
+}
+
+template <bool LC>
 __global__ void k_gather(BatchDev b, Grid g) {
     for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < b.total;
          s += (long long)gridDim.x * blockDim.x) {
         const int L = (int)(b.keys_out[s] >> 32);
         const BatchList &l = b.lists[L];
-        const long long k = (long long)b.vals_out[s] - l.off;
-        double v[8];
-#pragma unroll
-        for (int f = 0; f < 8; f++)
-            if (f < l.ncols) {
-                v[f] = l.src[f][k];
-                b.table[(long long)f * b.cap + s] = v[f];
-            }
-        const Terms t = screen_terms<BOOST>(v[0], v[1], v[2], v[3]);
-        b.terms4[s] = make_float4(t.x, t.y, t.m, t.p);
-        b.terms2[s] = make_float2(t.r2, t.t2);
-        if (l.ncols == 8) {
-            const FixedCols c = fixed_cols(g, v);
-#pragma unroll
-            for (int f = 0; f < kFixedCols; f++) b.fixed[(long long)f * b.cap + s] = c.c[f];
-        }
-        b.orig[s] = (unsigned)k;  // position in the caller's list (pair orientation)
+        put_row<LC>(b, g, l, s, (long long)b.vals_out[s] - l.off);
     }
 }
 
-// One warp per tile: momentum-space box of its particles.
-__global__ void k_boxes(BatchDev b) {
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// Momentum-space box of tile t of list l, by one warp.
+__device__ __forceinline__ void put_box(const BatchDev &b, const BatchList &l, long long t) {
     const int lane = threadIdx.x & 31;
-    if (warp >= b.total_tiles) return;
-    const int L = find_range(b.tile_off, b.n_lists, warp);
-    const BatchList &l = b.lists[L];
-    const long long t = warp - l.tile_off;
     const long long s0 = l.off + t * FT, s1 = min(l.off + (t + 1) * FT, l.off + l.n);
     double x0 = 1e300, x1 = -1e300, y0 = 1e300, y1 = -1e300, Y0 = 1e300, Y1 = -1e300, m0 = 1e300;
     double z0 = 1e300, z1 = -1e300, mm0 = 1e300, mm1 = -1e300;
@@ -166,7 +177,63 @@ __global__ void k_boxes(BatchDev b) {
         mm0 = fmin(mm0, __shfl_xor_sync(0xffffffffu, mm0, o));
         mm1 = fmax(mm1, __shfl_xor_sync(0xffffffffu, mm1, o));
     }
-    if (lane == 0) b.boxes[warp] = Box{x0, x1, y0, y1, Y0, Y1, m0, z0, z1, mm0, mm1};
+    if (lane == 0) b.boxes[l.tile_off + t] = Box{x0, x1, y0, y1, Y0, Y1, m0, z0, z1, mm0, mm1};
+}
+
+// One warp per tile.
+__global__ void k_boxes(BatchDev b) {
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (warp >= b.total_tiles) return;
+    const BatchList &l = b.lists[find_range(b.tile_off, b.n_lists, warp)];
+    put_box(b, l, warp - l.tile_off);
+}
+
+// Sort, gather and boxes of one list of at most kThreads x kItems particles
+// by one block, for batches of short lists: one launch in the place of keys,
+// the device-wide radix sort's 6 to 8, gather and boxes, whose launches and
+// gaps cost such a batch more than its pairs do.  The key is k_keys' with 8
+// bits to a dimension (cells 2.56 GeV and 6.4 units of rapidity either side
+// of zero at the default sizes, values beyond in the outermost), which orders
+// the list alike: 6 passes of the block's sort.  (Cells scaled to the list's
+// own ranges, which the few largest momenta set, made tiles wide in p_x, p_y
+// and culled less.)
+template <bool LC, int kThreads, int kItems>
+__global__ void __launch_bounds__(kThreads) k_prepare(BatchDev b, Grid g) {
+    typedef cub::BlockRadixSort<unsigned, kThreads, kItems, unsigned short> Sort;
+    __shared__ typename Sort::TempStorage tmp;
+    clear_queues(b);
+    const BatchList &l = b.lists[blockIdx.x];
+    const int n = (int)l.n;
+    unsigned key[kItems];
+    unsigned short row[kItems];
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        const int k = i * kThreads + threadIdx.x;
+        row[i] = (unsigned short)k;
+        key[i] = 0xffffffffu;  // past the end: sorts behind every row
+        if (k < n) {
+            const double pz = l.src[2][k], E = l.src[3][k];
+            const double y = 0.5 * log((E + pz) / (E - pz));
+            const double c[3] = {l.src[0][k] * b.inv_cell_pt, l.src[1][k] * b.inv_cell_pt,
+                                 (y == y ? y : 0.0) * b.inv_cell_y};
+            unsigned v = 0;
+#pragma unroll
+            for (int f = 0; f < 3; f++) {
+                // (254 at most: no key equals the padding's 24 bits)
+                const double x = c[f] + 128.0;
+                v |= spread10(x > 0.0 ? (unsigned)fmin(x, 254.0) : 0u) << f;
+            }
+            key[i] = v;
+        }
+    }
+    Sort(tmp).SortBlockedToStriped(key, row, 0, 24);
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        const int s = i * kThreads + threadIdx.x;
+        if (s < n) put_row<LC>(b, g, l, l.off + s, row[i]);
+    }
+    __syncthreads();  // the boxes read this block's rows
+    for (long long t = threadIdx.x >> 5; t < l.tiles; t += kThreads / 32) put_box(b, l, t);
 }
 
 // Can a pair with one particle in box a and one in box b pass the windows?
@@ -353,7 +420,22 @@ cudaError_t run_batch(const Device &d, const BatchDev &b, int grid, unsigned chu
                       cudaEvent_t *marks, int mode) {
     cudaError_t e;
     const int gs = 152 * 8;
-    if (b.total > 0) {
+    const bool lc = d.g.boost || d.g.qinv;  // light-cone screen terms
+    if (b.max_list <= kSmallList) {
+        // (1024-particle lists: 64 threads of 16 rows would leave the sort's
+        // latency bare; 256 of 4 measured fastest)
+        if (b.max_list <= 1024) {
+            if (lc)
+                k_prepare<true, 256, 4><<<b.n_lists, 256, 0, st>>>(b, d.g);
+            else
+                k_prepare<false, 256, 4><<<b.n_lists, 256, 0, st>>>(b, d.g);
+        } else if (lc) {
+            k_prepare<true, 1024, 8><<<b.n_lists, 1024, 0, st>>>(b, d.g);
+        } else {
+            k_prepare<false, 1024, 8><<<b.n_lists, 1024, 0, st>>>(b, d.g);
+        }
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    } else {
         k_keys<<<gs, 256, 0, st>>>(b);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         int end_bit = 32;
@@ -362,7 +444,7 @@ cudaError_t run_batch(const Device &d, const BatchDev &b, int grid, unsigned chu
         e = cub::DeviceRadixSort::SortPairs(b.sort_temp, bytes, b.keys_in, b.keys_out, b.vals_in,
                                             b.vals_out, (int)b.total, 0, end_bit, st);
         if (e != cudaSuccess) return e;
-        if (d.g.boost)
+        if (lc)
             k_gather<true><<<gs, 256, 0, st>>>(b, d.g);
         else
             k_gather<false><<<gs, 256, 0, st>>>(b, d.g);
@@ -370,8 +452,6 @@ cudaError_t run_batch(const Device &d, const BatchDev &b, int grid, unsigned chu
         k_boxes<<<(unsigned)((b.total_tiles * 32 + 255) / 256), 256, 0, st>>>(b);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    if ((e = cudaMemsetAsync(b.n_items, 0, 2 * sizeof(unsigned), st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(b.item_next, 0, 2 * sizeof(unsigned), st)) != cudaSuccess) return e;
     if (b.order_items && b.same_cap > 0 &&
         (e = cudaMemsetAsync(b.item_key_in, 0xff, (size_t)b.same_cap * sizeof(unsigned), st)) !=
             cudaSuccess)
@@ -391,7 +471,7 @@ cudaError_t run_batch(const Device &d, const BatchDev &b, int grid, unsigned chu
             sc.n_Kphi = d.g.n_Kphi;
             sc.az = d.g.azimuthal;
         }
-        k_cull<<<gs, 256, 0, st>>>(b, sc);
+        k_cull<<<(unsigned)min((long long)gs, (b.total_pairs + 255) / 256), 256, 0, st>>>(b, sc);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if (b.order_items && b.same_cap > 0) {

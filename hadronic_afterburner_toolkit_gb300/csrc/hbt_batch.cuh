@@ -9,6 +9,9 @@ namespace hbt {
 // Fixed-point columns of a same-event row, in entries of two (hbt_fixed.cuh).
 constexpr int kFixedEntries = 4;
 
+// Lists up to this length are sorted by one block each (k_prepare).
+constexpr long long kSmallList = 8192;
+
 // One particle list of a batch, as the caller passed it.
 struct BatchList {
     const double *src[8];  // caller columns px py pz E (x y z t for same-event)
@@ -65,6 +68,7 @@ struct BatchDev {
     long long total_tiles;  // tiles in the batch
     long long total_pairs;  // candidate tile pairs
     long long cap;          // row capacity of the sorted table
+    long long max_list;     // particles of the longest list
     double *table;          // [8][cap] sorted particle table
     unsigned *orig;         // [cap] each row's position in the caller's list
     // per row: the fixed-point columns of same-event lists ([kFixedEntries][cap],

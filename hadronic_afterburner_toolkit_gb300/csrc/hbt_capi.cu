@@ -65,6 +65,7 @@ struct hbt_ctx {
     // batched path: tables, sorted particle table, sort scratch, boxes, queue
     hbt::BatchRunner runner;
     int persistent_grid = 152 * 4;
+    bool reads_host = false;  // the GPU reads pageable host memory through the host's page tables
     int sms = 152, max_blocks_per_sm = 5;
     hbt_tuning tune = {0, 0.02, 0.05, kMergeChunk, 1, 0, 1};
     // ordered admission scratch
@@ -75,6 +76,7 @@ struct hbt_ctx {
     // the other buffer (in_free: recorded on `stream` after that binning)
     DevBuf in[2];
     int in_next = 0, in_cur = -1;
+    std::vector<hbt::CopySeg> segs;  // segments of the copy under way (read by the GPU)
     bool in_used[2] = {false, false};
     cudaStream_t copy_in = nullptr;
     cudaEvent_t in_free[2] = {nullptr, nullptr};
@@ -698,9 +700,9 @@ hbt_status bin_mixed_device(hbt_ctx *c, long long n1, const double *const *l1, l
 }
 
 // Copies host columns into a staging buffer; returns device pointers.  The
-// copies run on the context's copy stream into the buffer the previous call
-// did not use, so they overlap that call's binning; the call returns once
-// the copies are done (the caller may then reuse its arrays).  Serving
+// copy (one kernel, or one copy per run of columns) runs on the context's
+// copy stream into the buffer the previous call did not use, so it overlaps
+// that call's binning; the call returns once the copy is done (the caller may then reuse its arrays).  Serving
 // contexts, whose memory comes stream-ordered from a pool, copy on their
 // own stream.
 hbt_status stage(hbt_ctx *c, const double *const *src, const long long *len, int ncols,
@@ -723,9 +725,24 @@ hbt_status stage(hbt_ctx *c, const double *const *src, const long long *len, int
         if (len[f] > 0 && !src[f]) return fail(c, HBT_ERR_INVALID, "null particle array");
         off += (size_t)((len[f] + 31) / 32 * 32);
     }
-    // columns laid out in host memory as they will be on the device (each a
-    // multiple of 32 doubles, back to back) go over in one copy per run
-    for (int f = 0; f < ncols;) {
+    // where the GPU reads host memory itself, one kernel takes all columns
+    if (c->reads_host) {
+        c->segs.clear();
+        for (int f = 0; f < ncols; f++) {
+            if (len[f] <= 0) continue;
+            // a bad pointer fails here, on the host
+            const volatile double *v = src[f];
+            (void)v[0];
+            (void)v[len[f] - 1];
+            for (long long k = 0; k < len[f]; k += hbt::kCopyInChunk)
+                c->segs.push_back(hbt::CopySeg{src[f] + k, const_cast<double *>(dst[f]) + k,
+                                               std::min(hbt::kCopyInChunk, len[f] - k)});
+        }
+        CU(hbt::launch_copy_in(c->segs.data(), (int)c->segs.size(), cs));
+    }
+    // otherwise columns laid out in host memory as they will be on the device
+    // (each a multiple of 32 doubles, back to back) go over in one copy per run
+    for (int f = c->reads_host ? ncols : 0; f < ncols;) {
         if (len[f] <= 0) {
             f++;
             continue;
@@ -816,6 +833,7 @@ static void fill_tile_screen(const Grid &g, Screen &s) {
     s.sc_nk1 = f(-8.3 * u * std::max(2.0 * inv * Q * 0.53 * 1.06, 10.0) * up);
     s.sc_nk2 = f(-2.0 * inv * 4.1 * u * up);
     s.sc_nk3 = f(-2.0 * inv * (g.boost ? 4.1 : 2.1) * u * up);
+    s.sc_nkq = f(-2.0 * inv * up);
     // the outer limits lie 8 u (n + 1) inside the margin, so that a
     // coordinate they keep, however they round, has its rint on the grid or
     // is undecided
@@ -926,6 +944,11 @@ hbt_status ctx_create(const hbt_params *p, int device, cudaMemPool_t pool, hbt_c
         int sms = 0;
         CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         c->sms = sms;
+        int pageable = 0, tables = 0;
+        CU(cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device));
+        CU(cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables,
+                                  device));
+        c->reads_host = pageable && tables;
         c->max_blocks_per_sm = hbt::persistent_blocks_per_sm();
         c->persistent_grid = sms * c->max_blocks_per_sm;
     }

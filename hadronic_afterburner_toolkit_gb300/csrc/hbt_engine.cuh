@@ -127,6 +127,8 @@ struct Screen {
     // sc_nk3, the grid's outer limits sc_top - h and sc_bot + h, qnpts^2,
     // the offset of the flat bin and qnpts^3 (bins a decided pair can have)
     float sc_c0, sc_h0, sc_nk1, sc_nk2, sc_nk3, sc_top, sc_bot;
+    // the margin's coefficient of the q_inv error
+    float sc_nkq;
     unsigned sc_n2, sc_bin0, sc_q3;
     // K_T (slot_of): bin coordinate 2 K_T sk_half_inv + sk_c0 and its margin
     float sk_half_inv, sk_c0, sk_h0, sk_nkA, sk_nkk, sk_top;
@@ -214,6 +216,16 @@ cudaError_t launch_jobs_straddle(const Device &d, const StraddleJob *jobs, int n
 cudaError_t launch_defer_count(const Device &d, long long rows, long long cols, int n_res,
                                cudaStream_t st);
 cudaError_t launch_counters(const Device &d, unsigned long long *out, cudaStream_t st);
+// Copies n segments of doubles; the table and the sources may lie in host
+// memory that the GPU can read (kCopyInChunk: the largest segment that one
+// block should get).
+struct CopySeg {
+    const double *src;
+    double *dst;
+    long long n;
+};
+constexpr long long kCopyInChunk = 4096;
+cudaError_t launch_copy_in(const CopySeg *segs, int n, cudaStream_t st);
 // One output array of hbt_read_hist as FP64 in `out` (nbins doubles):
 // field 0..3 = q_out, q_side, q_long, cos sums; 4 = numerator count;
 // 5 = denominator count.

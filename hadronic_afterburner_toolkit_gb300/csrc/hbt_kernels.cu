@@ -401,6 +401,24 @@ __global__ void __launch_bounds__(256) k_export(Device d, int field, double *out
     }
 }
 
+// One segment per block: read across the CPU link, whose latency (1 to 2 us)
+// sets how much must be in flight.  One launch takes a batch's 880 columns
+// (12.8 MB) over in 85 us, 150 GB/s, where one cudaMemcpyAsync per column
+// took 1.9 ms, 2 us each.
+__global__ void __launch_bounds__(256) k_copy_in(const CopySeg *segs, int n) {
+    for (int s = blockIdx.x; s < n; s += gridDim.x) {
+        const CopySeg g = segs[s];
+#pragma unroll 4
+        for (long long k = threadIdx.x; k < g.n; k += blockDim.x) g.dst[k] = g.src[k];
+    }
+}
+
+cudaError_t launch_copy_in(const CopySeg *segs, int n, cudaStream_t st) {
+    if (n < 1) return cudaSuccess;
+    k_copy_in<<<std::min(n, 152 * 8), 256, 0, st>>>(segs, n);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_export(const Device &d, int field, double *out, long long nbins,
                           cudaStream_t st) {
     const long long blocks = std::min<long long>((nbins + 255) / 256, 152 * 16);

@@ -7,6 +7,8 @@
 // hbt_persist_qinv.cu (fast binning with the q_inv histograms).
 #pragma once
 
+#include <algorithm>
+
 #include "hbt_batch.cuh"
 #include "hbt_tile.cuh"
 
@@ -78,33 +80,11 @@ struct SameCtas {
 #endif
 constexpr int kMixedCtas = HBT_MIXED_CTAS;
 
-// One item: the tile pair, with or without the q_inv histograms by the type
-// of its shared memory.
-template <bool AZ, bool BOOST, int PREC, int MODE>
-__device__ __forceinline__ void same_item(const Device &d, SameSmem &sm, const void *cs,
-                                          const ListRows &l, const Item &it) {
-    same_tile_pair<AZ, BOOST, PREC, MODE>(d, sm, static_cast<const double *>(cs), l, (long long)it.ti * FT,
-                                          (long long)it.tj * FT);
-}
-template <bool AZ, bool BOOST, int PREC, int MODE>
-__device__ __forceinline__ void same_item(const Device &d, QinvSmem &sm, const void *cs,
-                                          const ListRows &l, const Item &it) {
-    same_tile_pair_qinv<AZ, BOOST, PREC, MODE>(d, sm, static_cast<const double2 *>(cs), l.c, l.orig, l.n,
-                                               (long long)it.ti * FT, (long long)it.tj * FT);
-}
-template <bool AZ, bool BOOST, int MODE>
-__device__ __forceinline__ void mixed_item(const Device &d, MixedSmem &sm, const ListRows &l1,
-                                           const ListRows &l2, const Item &it,
-                                           long long row_base) {
-    mixed_tile_pair<AZ, BOOST, MODE>(d, sm, l1, l2, (long long)it.ti * FT, (long long)it.tj * FT,
-                                     row_base);
-}
-template <bool AZ, bool BOOST, int MODE>
-__device__ __forceinline__ void mixed_item(const Device &d, QinvSmem &sm, const ListRows &l1,
-                                           const ListRows &l2, const Item &it,
-                                           long long row_base) {
-    mixed_tile_pair_qinv<AZ, BOOST, MODE>(d, sm, l1.c, l1.n, l2.c, l2.n, (long long)it.ti * FT,
-                                          (long long)it.tj * FT, l1.orig, l2.orig, row_base);
+// Parts of a tile pair (ranges of its j-tile) that its items are split into:
+// with fewer items than CTAs, a pair's 64 steps on one CTA are the launch's
+// whole time, so up to four CTAs share it.
+__device__ __forceinline__ unsigned item_parts(unsigned n_items) {
+    return n_items <= gridDim.x / 4u ? 4u : (n_items <= gridDim.x / 2u ? 2u : 1u);
 }
 
 // A list of the batch as the tile kernels read it (c: its column pointers).
@@ -120,20 +100,17 @@ __device__ __forceinline__ ListRows rows_of(const BatchDev &b, const BatchList &
 template <bool AZ, bool BOOST, int PREC, int MODE, bool QINV, bool MANY>
 __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(Device d, BatchDev b, unsigned base,
                                                            unsigned end) {
-    __shared__ typename std::conditional<QINV, QinvSmem, SameSmem>::type sm;
+    __shared__ SameSmem sm;
     __shared__ unsigned item;
-    // the form's cos table
-    constexpr int kTable =
-        PREC == 0 ? (QINV ? COS_TABLE : (kCosEntries + 1) / 2) : (PREC == 2 ? DF_TABLE : 1);
-    __shared__ double2 cs[kTable];
-    if (PREC == 0 && QINV) fill_cos_table(cs);
-    if (PREC == 0 && !QINV) fill_cos_entries(reinterpret_cast<double *>(cs));
-    if (PREC == 2) fill_df_table(reinterpret_cast<float4 *>(cs));
+    __shared__ double cs[PREC == 0 ? kCosEntries : 1];  // the form's cos table
+    if (PREC == 0) fill_cos_entries(cs);
     const unsigned stop = min(end, min(b.n_items[0], b.same_cap));
+    const unsigned parts = item_parts(stop > base ? stop - base : 0u), rows = FT / parts;
     for (;;) {
-        if (threadIdx.x == 0) item = base + atomicAdd(b.item_next, 1u);
+        if (threadIdx.x == 0) item = atomicAdd(b.item_next, 1u);
         __syncthreads();
-        const unsigned k = item;
+        const unsigned k = base + item / parts;
+        const int jb = (int)((item % parts) * rows), je = jb + (int)rows;
         if (k >= stop) break;
         const Item it = b.items[b.order_items ? b.item_pos_out[k] : k];
         const BatchJob &job = b.jobs[it.job];
@@ -144,9 +121,13 @@ __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(D
         if constexpr (MANY) {
             __shared__ Device dsm;
             load_device(b, job, dsm);
-            same_item<AZ, BOOST, PREC, MODE>(dsm, sm, cs, rows_of(b, la, c), it);
+            same_tile_pair<AZ, BOOST, PREC, MODE, QINV>(dsm, sm, cs, rows_of(b, la, c),
+                                                        (long long)it.ti * FT,
+                                                        (long long)it.tj * FT, jb, je);
         } else {
-            same_item<AZ, BOOST, PREC, MODE>(d, sm, cs, rows_of(b, la, c), it);
+            same_tile_pair<AZ, BOOST, PREC, MODE, QINV>(d, sm, cs, rows_of(b, la, c),
+                                                        (long long)it.ti * FT,
+                                                        (long long)it.tj * FT, jb, je);
         }
         __syncthreads();
     }
@@ -155,13 +136,15 @@ __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(D
 // Mixed-event items, all in one launch.
 template <bool AZ, bool BOOST, int MODE, bool QINV, bool MANY>
 __global__ void __launch_bounds__(FT, kMixedCtas) k_persistent_mixed(Device d, BatchDev b) {
-    __shared__ typename std::conditional<QINV, QinvSmem, MixedSmem>::type sm;
+    __shared__ MixedSmem sm;
     __shared__ unsigned item;
     const unsigned stop = min(b.n_items[1], b.mixed_cap);
+    const unsigned parts = item_parts(stop), rows = FT / parts;
     for (;;) {
         if (threadIdx.x == 0) item = atomicAdd(b.item_next + 1, 1u);
         __syncthreads();
-        const unsigned k = item;
+        const unsigned k = item / parts;
+        const int jb = (int)((item % parts) * rows), je = jb + (int)rows;
         if (k >= stop) break;
         const Item it = b.items[b.same_cap + k];
         const BatchJob &job = b.jobs[it.job];
@@ -175,11 +158,13 @@ __global__ void __launch_bounds__(FT, kMixedCtas) k_persistent_mixed(Device d, B
         if constexpr (MANY) {
             __shared__ Device dsm;
             load_device(b, job, dsm);
-            mixed_item<AZ, BOOST, MODE>(dsm, sm, rows_of(b, la, c1), rows_of(b, lb, c2), it,
-                                        job.row_base);
+            mixed_tile_pair<AZ, BOOST, MODE, QINV>(
+                dsm, sm, rows_of(b, la, c1), rows_of(b, lb, c2), (long long)it.ti * FT,
+                (long long)it.tj * FT, job.row_base, jb, je);
         } else {
-            mixed_item<AZ, BOOST, MODE>(d, sm, rows_of(b, la, c1), rows_of(b, lb, c2), it,
-                                        job.row_base);
+            mixed_tile_pair<AZ, BOOST, MODE, QINV>(
+                d, sm, rows_of(b, la, c1), rows_of(b, lb, c2), (long long)it.ti * FT,
+                (long long)it.tj * FT, job.row_base, jb, je);
         }
         __syncthreads();
     }
@@ -196,14 +181,18 @@ inline int sm_count() {
     return sms;
 }
 
-// grid > 0: that many CTAs; otherwise one CTA per resident slot.
+// grid > 0: that many CTAs; otherwise one CTA per resident slot; never more
+// than the candidate items make parts (item_parts).
 template <class K>
-int persistent_grid(K kernel, int grid) {
-    if (grid > 0) return grid;
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, FT, 0) != cudaSuccess || nb < 1)
-        nb = 4;
-    return sm_count() * nb;
+int persistent_grid(K kernel, int grid, unsigned items) {
+    if (grid <= 0) {
+        int nb = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, FT, 0) != cudaSuccess ||
+            nb < 1)
+            nb = 4;
+        grid = sm_count() * nb;
+    }
+    return (int)std::max(1ll, std::min((long long)grid, 4ll * items));
 }
 
 // The kernel for one analysis, or (b.devs, fast binning only) for many.
@@ -212,14 +201,16 @@ cudaError_t launch_same_items(const Device &d, const BatchDev &b, unsigned base,
                               int grid, cudaStream_t st) {
     if (b.devs) {
         if constexpr (MODE == MODE_FAST) {
-            grid = persistent_grid(k_persistent_same<AZ, BOOST, PREC, MODE, QINV, true>, grid);
+            grid = persistent_grid(k_persistent_same<AZ, BOOST, PREC, MODE, QINV, true>, grid,
+                                   b.same_cap);
             k_persistent_same<AZ, BOOST, PREC, MODE, QINV, true><<<grid, FT, 0, st>>>(d, b, base,
                                                                                      end);
             return cudaGetLastError();
         }
         return cudaErrorNotSupported;
     }
-    grid = persistent_grid(k_persistent_same<AZ, BOOST, PREC, MODE, QINV, false>, grid);
+    grid = persistent_grid(k_persistent_same<AZ, BOOST, PREC, MODE, QINV, false>, grid,
+                           b.same_cap);
     k_persistent_same<AZ, BOOST, PREC, MODE, QINV, false><<<grid, FT, 0, st>>>(d, b, base, end);
     return cudaGetLastError();
 }
@@ -228,13 +219,14 @@ template <bool AZ, bool BOOST, int MODE, bool QINV>
 cudaError_t launch_mixed_items(const Device &d, const BatchDev &b, int grid, cudaStream_t st) {
     if (b.devs) {
         if constexpr (MODE == MODE_FAST) {
-            grid = persistent_grid(k_persistent_mixed<AZ, BOOST, MODE, QINV, true>, grid);
+            grid = persistent_grid(k_persistent_mixed<AZ, BOOST, MODE, QINV, true>, grid,
+                                   b.mixed_cap);
             k_persistent_mixed<AZ, BOOST, MODE, QINV, true><<<grid, FT, 0, st>>>(d, b);
             return cudaGetLastError();
         }
         return cudaErrorNotSupported;
     }
-    grid = persistent_grid(k_persistent_mixed<AZ, BOOST, MODE, QINV, false>, grid);
+    grid = persistent_grid(k_persistent_mixed<AZ, BOOST, MODE, QINV, false>, grid, b.mixed_cap);
     k_persistent_mixed<AZ, BOOST, MODE, QINV, false><<<grid, FT, 0, st>>>(d, b);
     return cudaGetLastError();
 }
@@ -246,12 +238,11 @@ template <int MODE, bool QINV>
 cudaError_t launch_same_mode(const Device &d, const BatchDev &b, unsigned base, unsigned end,
                              int grid, cudaStream_t st) {
     const bool az = d.g.azimuthal, boost = d.g.boost;
-    // the forms this mode instantiates: FP64 only for COUNT; the double-float
-    // form runs the FP64 form's kernel (same bins, closer values, and faster
-    // than double-float arithmetic since those come from fixed-point columns:
-    // central group 50.7 against 79.7 ms), except with q_inv histograms
-    constexpr int P1 = MODE == MODE_COUNT ? 0 : 1, P2 = QINV && MODE != MODE_COUNT ? 2 : 0;
-    const int prec = MODE == MODE_COUNT ? 0 : (d.precision == 2 ? P2 : d.precision);
+    // the COUNT pass runs the FP64 form's kernel, and so does the double-float
+    // form: same bins, closer values, and faster than double-float arithmetic
+    // (central group 50.8 against 79.7 ms)
+    constexpr int P1 = MODE == MODE_COUNT ? 0 : 1;
+    const int prec = MODE == MODE_COUNT || d.precision != 1 ? 0 : 1;
 #define HBT_P(AZ_, BO_, PR_) \
     return launch_same_items<AZ_, BO_, PR_, MODE, QINV>(d, b, base, end, grid, st)
     if (prec == 0) {
@@ -260,16 +251,10 @@ cudaError_t launch_same_mode(const Device &d, const BatchDev &b, unsigned base, 
         if (boost) HBT_P(false, true, 0);
         HBT_P(false, false, 0);
     }
-    if (prec == 1) {
-        if (az && boost) HBT_P(true, true, P1);
-        if (az) HBT_P(true, false, P1);
-        if (boost) HBT_P(false, true, P1);
-        HBT_P(false, false, P1);
-    }
-    if (az && boost) HBT_P(true, true, P2);
-    if (az) HBT_P(true, false, P2);
-    if (boost) HBT_P(false, true, P2);
-    HBT_P(false, false, P2);
+    if (az && boost) HBT_P(true, true, P1);
+    if (az) HBT_P(true, false, P1);
+    if (boost) HBT_P(false, true, P1);
+    HBT_P(false, false, P1);
 #undef HBT_P
 }
 

@@ -11,7 +11,7 @@ BatchRunner::~BatchRunner() {
     if (exec_) cudaGraphExecDestroy(exec_);
     for (cudaEvent_t e : marks_)
         if (e) cudaEventDestroy(e);
-    Buf *all[] = {&lists_, &jobs_, &offs_, &table_, &keys_, &vals_, &sort_temp_, &boxes_,
+    Buf *all[] = {&tables_, &orig_, &table_, &keys_, &vals_, &sort_temp_, &boxes_,
                   &items_, &counters_, &devs_, &item_order_, &item_sort_temp_, &fixed_, &terms_};
     for (Buf *b : all)
         if (b->p) cudaFree(b->p);
@@ -172,7 +172,7 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
     std::vector<BatchList> lists;
     std::vector<BatchJob> bj;
     std::vector<long long> list_off, tile_off, pair_off;
-    long long total = 0, tiles = 0, pairs = 0, same_pairs = 0, mixed_pairs = 0;
+    long long total = 0, tiles = 0, pairs = 0, same_pairs = 0, mixed_pairs = 0, max_list = 0;
     auto add_list = [&](const double *const *src, int ncols, long long n) {
         BatchList l = {};
         for (int f = 0; f < 8; f++) l.src[f] = f < ncols ? src[f] : nullptr;
@@ -184,6 +184,7 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
         list_off.push_back(total);
         tile_off.push_back(tiles);
         total += n;
+        max_list = std::max(max_list, n);
         tiles += l.tiles;
         lists.push_back(l);
         return (int)lists.size() - 1;
@@ -224,40 +225,58 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
         err = "batch too large (tile pairs or particles)";
         return false;
     }
-    const size_t sort_bytes = batch_sort_temp_bytes(total);
-    if (!grow(lists_, lists.size() * sizeof(BatchList), err) ||
-        !grow(jobs_, bj.size() * sizeof(BatchJob), err) ||
-        !grow(offs_, (2 * lists.size() + bj.size()) * sizeof(long long), err) ||
-        !grow(table_, (size_t)8 * total * sizeof(double), err) ||
+    // small lists are sorted by one block each (k_prepare), others by CUB
+    const bool small = max_list <= kSmallList;
+    const size_t sort_bytes = small ? 0 : batch_sort_temp_bytes(total);
+    if (!grow(table_, (size_t)8 * total * sizeof(double), err) ||
         !grow(fixed_, (size_t)kFixedEntries * total * sizeof(int4), err) ||
         !grow(terms_, (size_t)total * (sizeof(float4) + sizeof(float2)), err) ||
-        !grow(keys_, (size_t)2 * total * sizeof(unsigned long long), err) ||
-        !grow(vals_, (size_t)3 * total * sizeof(unsigned), err) ||
-        !grow(sort_temp_, sort_bytes, err) || !grow(boxes_, (size_t)tiles * sizeof(Box), err) ||
+        !grow(orig_, (size_t)total * sizeof(unsigned), err) ||
+        (!small && (!grow(keys_, (size_t)2 * total * sizeof(unsigned long long), err) ||
+                    !grow(vals_, (size_t)2 * total * sizeof(unsigned), err) ||
+                    !grow(sort_temp_, sort_bytes, err))) || !grow(boxes_, (size_t)tiles * sizeof(Box), err) ||
         !grow(items_, (size_t)pairs * sizeof(Item), err) ||
         !grow(counters_, 4 * sizeof(unsigned), err))
         return false;
-    if (t.order_items && same_pairs > 0 &&
+    // Item order: it keeps the histogram slots in use in L2, so it is for
+    // histograms that do not fit there (the central group's 238 MB: 3.3x less
+    // DRAM traffic); those below half of L2 (129 MB) save its sort's launches.
+    // It does not change the kernels' time (central 50.8 ms either way).
+    size_t hist_bytes = 0;
+    for (int k = 0; k < std::max(n_devs, 1); k++) {
+        const Grid &g = n_devs > 0 ? devs_host[k].g : d.g;
+        hist_bytes += (size_t)g.n_slots * g.q3 * (sizeof(Sums) + 2 * sizeof(u64));
+    }
+    const bool order = t.order_items && same_pairs > 0 && hist_bytes > (64u << 20);
+    if (order &&
         (!grow(item_order_, (size_t)4 * same_pairs * sizeof(unsigned), err) ||
          !grow(item_sort_temp_, item_sort_temp_bytes(same_pairs), err)))
         return false;
-    std::vector<long long> offs(list_off);
-    offs.insert(offs.end(), tile_off.begin(), tile_off.end());
-    offs.insert(offs.end(), pair_off.begin(), pair_off.end());
-    if (cudaMemcpyAsync(lists_.p, lists.data(), lists.size() * sizeof(BatchList),
-                        cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(jobs_.p, bj.data(), bj.size() * sizeof(BatchJob), cudaMemcpyHostToDevice,
-                        st) != cudaSuccess ||
-        cudaMemcpyAsync(offs_.p, offs.data(), offs.size() * sizeof(long long),
-                        cudaMemcpyHostToDevice, st) != cudaSuccess) {
+    // the tables in one upload: lists, jobs, offsets (each a multiple of 8
+    // bytes)
+    static_assert(sizeof(BatchList) % 8 == 0 && sizeof(BatchJob) % 8 == 0, "table alignment");
+    const size_t at_jobs = lists.size() * sizeof(BatchList);
+    const size_t at_offs = at_jobs + bj.size() * sizeof(BatchJob);
+    tables_host_.resize(at_offs + (2 * lists.size() + bj.size()) * sizeof(long long));
+    unsigned char *th = tables_host_.data();
+    memcpy(th, lists.data(), at_jobs);
+    memcpy(th + at_jobs, bj.data(), bj.size() * sizeof(BatchJob));
+    long long *oh = reinterpret_cast<long long *>(th + at_offs);
+    std::copy(list_off.begin(), list_off.end(), oh);
+    std::copy(tile_off.begin(), tile_off.end(), oh + lists.size());
+    std::copy(pair_off.begin(), pair_off.end(), oh + 2 * lists.size());
+    if (!grow(tables_, tables_host_.size(), err)) return false;
+    if (cudaMemcpyAsync(tables_.p, th, tables_host_.size(), cudaMemcpyHostToDevice, st) !=
+        cudaSuccess) {
         err = "uploading the batch tables failed";
         return false;
     }
     BatchDev b;
     memset(&b, 0, sizeof(b));  // padding too: the bytes key the cached graph
-    const long long *o = static_cast<const long long *>(offs_.p);
-    b.lists = static_cast<const BatchList *>(lists_.p);
-    b.jobs = static_cast<const BatchJob *>(jobs_.p);
+    const unsigned char *td = static_cast<const unsigned char *>(tables_.p);
+    const long long *o = reinterpret_cast<const long long *>(td + at_offs);
+    b.lists = reinterpret_cast<const BatchList *>(td);
+    b.jobs = reinterpret_cast<const BatchJob *>(td + at_jobs);
     b.list_off = o;
     b.tile_off = o + lists.size();
     b.pair_off = o + 2 * lists.size();
@@ -271,11 +290,14 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
     b.fixed = static_cast<int4 *>(fixed_.p);
     b.terms4 = static_cast<float4 *>(terms_.p);
     b.terms2 = reinterpret_cast<float2 *>(b.terms4 + total);
-    b.keys_in = static_cast<unsigned long long *>(keys_.p);
-    b.keys_out = b.keys_in + total;
-    b.vals_in = static_cast<unsigned *>(vals_.p);
-    b.vals_out = b.vals_in + total;
-    b.orig = b.vals_in + 2 * total;
+    b.max_list = max_list;
+    b.orig = static_cast<unsigned *>(orig_.p);
+    if (!small) {
+        b.keys_in = static_cast<unsigned long long *>(keys_.p);
+        b.keys_out = b.keys_in + total;
+        b.vals_in = static_cast<unsigned *>(vals_.p);
+        b.vals_out = b.vals_in + total;
+    }
     b.sort_temp = sort_temp_.p;
     b.sort_temp_bytes = sort_temp_.bytes;
     b.boxes = static_cast<Box *>(boxes_.p);
@@ -290,7 +312,7 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
     b.inv_cell_y = 1.0 / t.cell_y;
     b.devs = devs_dev;
     b.n_devs = n_devs;
-    b.order_items = t.order_items && same_pairs > 0 ? 1 : 0;
+    b.order_items = order ? 1 : 0;
     if (b.order_items) {
         unsigned *o = static_cast<unsigned *>(item_order_.p);
         b.item_key_in = o;

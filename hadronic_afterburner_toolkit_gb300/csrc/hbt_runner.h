@@ -85,8 +85,9 @@ class BatchRunner {
     // Runs the device pipeline, through a cached CUDA graph when possible.
     cudaError_t launch(const Device &d, const BatchDev &b, const Device *devs_host, int n_devs,
                        const Tuning &t, cudaStream_t st, int mode);
-    Buf lists_, jobs_, offs_, table_, keys_, vals_, sort_temp_, boxes_, items_, counters_, devs_;
+    Buf tables_, orig_, table_, keys_, vals_, sort_temp_, boxes_, items_, counters_, devs_;
     Buf item_order_, item_sort_temp_, fixed_, terms_;
+    std::vector<unsigned char> tables_host_;
     long long last_pairs_ = 0, last_same_ = 0, last_mixed_ = 0;
     cudaStream_t last_stream_ = nullptr;
     int last_reuse_ = -1;

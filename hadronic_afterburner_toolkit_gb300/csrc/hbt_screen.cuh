@@ -108,20 +108,21 @@ __device__ __forceinline__ f2 rsqrt2(f2 v) {
     return pack2(rsqrt_approx(a), rsqrt_approx(b));
 }
 
-// A particle's screen terms (with the boost m = E - p_z, p = E + p_z,
-// t2 = m p; without m = p_z, p = |p_z|, t2 = 0).
+// A particle's screen terms: light-cone (LC: with the boost or the q_inv
+// histograms) m = E - p_z, p = E + p_z, t2 = m p; otherwise m = p_z, p =
+// |p_z|, t2 = 0.
 struct Terms {
     float x, y, m, p, r2, t2;
 };
 
 // FP32 terms of a particle from its FP64 momentum.
-template <bool BOOST>
+template <bool LC>
 __device__ __forceinline__ Terms screen_terms(double px, double py, double pz, double E) {
     Terms t;
     t.x = (float)px;
     t.y = (float)py;
     t.r2 = (float)(px * px + py * py);
-    if (BOOST) {
+    if (LC) {
         const double m = E - pz, p = E + pz;
         t.m = (float)m;
         t.p = (float)p;
@@ -162,9 +163,12 @@ constexpr unsigned kRoundBits = 0x4b400000u;
 // What the screen says about two pairs, the row a against particles 2 jp and
 // 2 jp + 1 of the j-tile: take[h] false when pair h is certainly outside,
 // bin[h] its q bin, und[h] when only the reference chain can tell.
+// With q_inv histograms takeq, undq and kq say the same of the q_inv bin.
 struct Screened {
     bool take[2], und[2];
     unsigned bin[2];
+    bool takeq[2], undq[2];
+    unsigned kq[2];
 };
 
 // The row of one lane, in packed form (both halves alike).
@@ -176,11 +180,57 @@ __device__ __forceinline__ Row row_of(const Terms &a) {
                both(-a.m),       both(a.p),        both(a.r2),        both(a.t2)};
 }
 
+// The q_inv bin of two pairs (src/HBT_correlation.cpp:331-356, :595-607):
+// q_inv^2 = |a_T - b_T|^2 - (m_a - m_b)(p_a - p_b).  With w = s2 / k >=
+// sqrt(s2 / 2), each difference within 2.01 u of its operands' sum:
+//   transverse part      8.1 u (|d_x| + |d_y|) w
+//   longitudinal part    2.1 u (s_m |d_p| + s_p |d_m|)
+//   roundings            4 u (|d_T|^2 + |d_m d_p|)
+// and |sqrt(t) - sqrt(T)| <= |t - T| / sqrt(t), plus 4 u of it for the
+// reciprocal root and the product.  q_inv^2 certainly negative: no event (the
+// reference's NaN fails both bounds).
+__device__ __forceinline__ void screen_qinv(const Screen &S, const Row &a, const f2 *v, f2 w,
+                                            Screened &r) {
+    const f2 dx = fma2(v[0], both(-2.0f), a.x2), dy = fma2(v[1], both(-2.0f), a.y2);  // twice
+    const f2 qt = fma2(dx, dx, mul2(dy, dy));                                        // 4 times
+    const f2 dm = add2(v[2], a.nm), dp = fma2(v[3], both(-1.0f), a.p);               // -d_m, d_p
+    const f2 lg = mul2(dm, dp);
+    const f2 sm = add2(v[2], a.m), sp = add2(v[3], a.p);
+    const f2 t2 = fma2(qt, both(0.25f), lg);
+    float x[2], y[2], m[2], p[2], g[2], t[2], q[2], M[2], P[2], W[2];
+    unpack2(dx, x[0], x[1]);
+    unpack2(dy, y[0], y[1]);
+    unpack2(dm, m[0], m[1]);
+    unpack2(dp, p[0], p[1]);
+    unpack2(lg, g[0], g[1]);
+    unpack2(t2, t[0], t[1]);
+    unpack2(qt, q[0], q[1]);
+    unpack2(sm, M[0], M[1]);
+    unpack2(sp, P[0], P[1]);
+    unpack2(w, W[0], W[1]);
+    constexpr float U = 5.9604645e-8f;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const float e = U * __fmaf_rn(4.1f * (fabsf(x[k]) + fabsf(y[k])), W[k],
+                                      __fmaf_rn(2.1f, __fmaf_rn(M[k], fabsf(p[k]),
+                                                                P[k] * fabsf(m[k])),
+                                                q[k] + 4.0f * fabsf(g[k])));
+        const float rs = rsqrt_approx(t[k]), qi = t[k] * rs;
+        const float h = __fmaf_rn(__fmaf_rn(e, rs, 4.0f * U * qi), S.sc_nkq, S.sc_h0);
+        const float tq = __fmaf_rn(qi, S.inv_dq, S.sc_c0);
+        const float kr = tq + kRound;
+        r.takeq[k] = !(t[k] + e < 0.0f) && !(tq > S.sc_top - h) && !(tq < S.sc_bot + h);
+        r.undq[k] = !(fabsf(tq - (kr - kRound)) < h);
+        r.kq[k] = __float_as_uint(kr) - kRoundBits;
+    }
+}
+
 // Screens two pairs.  `inv_dq`: 1 / bin width for each pair, negative when b
 // is the pair's first particle in the caller's order (every component of q
 // then changes sign).  False when neither pair of any lane passes the
-// transverse test (warp-uniform).
-template <bool BOOST>
+// transverse test (warp-uniform; never with q_inv histograms, whose window
+// that test does not cover).
+template <bool BOOST, bool QINV>
 __device__ __forceinline__ bool screen_two(const Screen &S, const Row &a, const TermsPair &b,
                                            f2 inv_dq, Screened &r) {
     const f2 *v = reinterpret_cast<const f2 *>(&b);
@@ -194,7 +244,7 @@ __device__ __forceinline__ bool screen_two(const Screen &S, const Row &a, const 
     unpack2(thr, ta, tb);
     r.take[0] = !(ka < ta);
     r.take[1] = !(kb < tb);
-    if (!__any_sync(0xffffffffu, r.take[0] || r.take[1])) return false;
+    if (!QINV && !__any_sync(0xffffffffu, r.take[0] || r.take[1])) return false;
     const f2 inv = pack2(rsqrt_approx(ka), rsqrt_approx(kb));
     const f2 w = mul2(s2, inv);
     const f2 qo = mul2(fma2(v[4], both(-1.0f), a.r2), inv);
@@ -206,10 +256,15 @@ __device__ __forceinline__ bool screen_two(const Screen &S, const Row &a, const 
         const f2 rl = rsqrt2(add2(sum, add2(a.t2, v[5])));
         ql = mul2(D, rl);
         el = mul2(sum, rl);
+    } else if (QINV) {
+        // z = (p - m) / 2, the sums E in the place of |z|
+        ql = mul2(both(0.5f), fma2(fma2(bp, both(-1.0f), a.p), both(1.0f), add2(bm, a.nm)));
+        el = mul2(both(0.5f), add2(add2(a.m, bm), add2(a.p, bp)));
     } else {
         ql = fma2(bm, both(-1.0f), a.m);
         el = add2(a.p, bp);
     }
+    if (QINV) screen_qinv(S, a, v, w, r);
     // h = 0.5 - et
     const f2 h = fma2(w, fma2(inv, both(S.sc_nk1), both(S.sc_nk2)),
                       fma2(el, both(S.sc_nk3), both(S.sc_h0)));
@@ -262,8 +317,10 @@ __device__ __forceinline__ bool screen_two(const Screen &S, const Row &a, const 
 // Bin edges are at multiples of the bin width from psi, the wrap included,
 // so one test of the distance to the rint covers them all.  All bounds are
 // doubled.
+// iK: the K_T bin, valid when the result is >= 0.
 template <bool AZ>
-__device__ __forceinline__ int slot_of(const Screen &S, float ax, float ay, float bx, float by) {
+__device__ __forceinline__ int slot_of(const Screen &S, float ax, float ay, float bx, float by,
+                                       int &iK) {
     const float sx = ax + bx, sy = ay + by;
     const float A = (fabsf(ax) + fabsf(ay)) + (fabsf(bx) + fabsf(by));
     const float k2 = __fmaf_rn(sx, sx, sy * sy);
@@ -275,6 +332,7 @@ __device__ __forceinline__ int slot_of(const Screen &S, float ax, float ay, floa
     const float kr = t + kRound;
     bool sure = fabsf(t - (kr - kRound)) < h;
     int slot = (int)(__float_as_uint(kr) - kRoundBits);
+    iK = slot;
     if (AZ) {
         const float cx = __fmaf_rn(sy, S.sp_sin, sx * S.sp_cos);
         const float cy = __fmaf_rn(sy, S.sp_cos, -(sx * S.sp_sin));
