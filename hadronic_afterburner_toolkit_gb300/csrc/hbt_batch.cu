@@ -509,6 +509,10 @@ cudaError_t run_batch(const Device &d, const BatchDev &b, int grid, unsigned chu
         e = persistent_mixed(d, b, grid, st, mode);
         if (e != cudaSuccess) return e;
     }
+    if (d.g.qinv && mode == MODE_FAST) {
+        for (int k = 0; k < (b.devs ? n_host_devs : 1); k++)
+            if ((e = launch_qinv_merge(b.devs ? host_devs[k] : d, st)) != cudaSuccess) return e;
+    }
     if (marks && (e = cudaEventRecord(marks[3], st)) != cudaSuccess) return e;
     return cudaSuccess;
 }

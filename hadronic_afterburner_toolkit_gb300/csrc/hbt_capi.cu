@@ -59,7 +59,7 @@ struct hbt_ctx {
     u64 cap = 0, cap_qinv = 0;
     int n_stream = 0;  // 3-D slots + q_inv K_T bins
     // histograms
-    DevBuf sums, cnt, den, qi_sums, qi_cnt, qi_den, stats, defer, n_defer;
+    DevBuf sums, cnt, den, qi_sums, qi_cnt, qi_den, qi_part, stats, defer, n_defer;
     // FP32-weight form: partial sums and Kahan compensation
     DevBuf part, comp;
     // batched path: tables, sorted particle table, sort scratch, boxes, queue
@@ -168,6 +168,7 @@ void refresh_device(hbt_ctx *c) {
     c->d.h.qi_sums = ptr<hbt::QiSums>(c->qi_sums);
     c->d.h.qi_cnt = ptr<u64>(c->qi_cnt);
     c->d.h.qi_den = ptr<u64>(c->qi_den);
+    c->d.h.qi_part = ptr<hbt::QiPart>(c->qi_part);
     c->d.stats = ptr<u64>(c->stats);
     c->d.defer = ptr<hbt::Deferral>(c->defer);
     c->d.n_defer = ptr<unsigned>(c->n_defer);
@@ -961,6 +962,8 @@ hbt_status ctx_create(const hbt_params *p, int device, cudaMemPool_t pool, hbt_c
         (s = dalloc(c, c->qi_sums, nq * sizeof(hbt::QiSums))) != HBT_OK ||
         (s = dalloc(c, c->qi_cnt, nq * sizeof(u64))) != HBT_OK ||
         (s = dalloc(c, c->qi_den, nq * sizeof(u64))) != HBT_OK ||
+        (g.qinv &&
+         (s = dalloc(c, c->qi_part, hbt::kQiCopies * nq * sizeof(hbt::QiPart))) != HBT_OK) ||
         (s = dalloc(c, c->stats, hbt::STAT_N * sizeof(u64))) != HBT_OK ||
         (s = dalloc(c, c->defer, kDeferCap * sizeof(hbt::Deferral))) != HBT_OK ||
         (s = dalloc(c, c->n_defer, sizeof(unsigned))) != HBT_OK ||
@@ -983,7 +986,7 @@ void hbt_destroy(hbt_ctx *c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     DevBuf *bufs[] = {&c->sums,   &c->cnt,     &c->den,       &c->qi_sums,  &c->qi_cnt,
-                      &c->qi_den, &c->stats,   &c->defer,     &c->n_defer,  &c->rowcnt,
+                      &c->qi_den, &c->qi_part, &c->stats,   &c->defer,     &c->n_defer,  &c->rowcnt,
                       &c->row_cut, &c->quota,  &c->remaining, &c->resolved, &c->counters,
                       &c->apply_iphi, &c->straddle_jobs, &c->slot_full, &c->in[0], &c->in[1],
                       &c->part, &c->comp, &c->exp};
@@ -1031,6 +1034,7 @@ hbt_status hbt_reset(hbt_ctx *c) {
     CU(cudaMemsetAsync(c->qi_sums.p, 0, c->qi_sums.bytes, c->stream));
     CU(cudaMemsetAsync(c->qi_cnt.p, 0, c->qi_cnt.bytes, c->stream));
     CU(cudaMemsetAsync(c->qi_den.p, 0, c->qi_den.bytes, c->stream));
+    if (c->qi_part.p) CU(cudaMemsetAsync(c->qi_part.p, 0, c->qi_part.bytes, c->stream));
     CU(cudaMemsetAsync(c->stats.p, 0, c->stats.bytes, c->stream));
     if (c->part.p) CU(cudaMemsetAsync(c->part.p, 0, c->part.bytes, c->stream));
     if (c->comp.p) CU(cudaMemsetAsync(c->comp.p, 0, c->comp.bytes, c->stream));
@@ -1507,7 +1511,8 @@ size_t ctx_device_bytes(const hbt_params &p) {
     const size_t nb = slots * p.qnpts * p.qnpts * p.qnpts, nq = (size_t)p.n_KT * p.qnpts;
     // bins, counts, the readback buffers, the q_inv bins, the deferrals
     size_t bytes = nb * (sizeof(Sums) + 2 * sizeof(u64) + 2 * sizeof(double)) +
-                   nq * (sizeof(QiSums) + 2 * sizeof(u64)) + kDeferCap * sizeof(Deferral) + 4096;
+                   nq * (sizeof(QiSums) + 2 * sizeof(u64) +
+                         (p.invariant_radius_flag == 1 ? kQiCopies * sizeof(QiPart) : 0)) + kDeferCap * sizeof(Deferral) + 4096;
     if (p.precision == HBT_PRECISION_FP32W) bytes += nb * (2 * sizeof(float4) + sizeof(Sums));
     return bytes;
 }

@@ -38,6 +38,15 @@ struct __align__(16) QiSums {
     double q, w;
 };
 
+// Private copies of the q_inv histograms: a kernel's CTAs add to copy
+// (block % kQiCopies), merged into the histogram after it (launch_qinv_merge).
+// The histogram has only n_KT x qnpts bins, and all CTAs adding to them
+// directly held the kernel up at those few addresses.
+struct __align__(32) QiPart {
+    double q, w, n, den;  // sum of q_inv, of cos(q.dx), numerator and denominator counts
+};
+constexpr int kQiCopies = 128;
+
 // Device histogram storage.
 //  sums  [n_slots*q3] {q_out, q_side, q_long, cos(q.dx)} - one 32-byte sector
 //  cnt   [n_slots*q3] numerator pair count
@@ -50,6 +59,7 @@ struct Hist {
     QiSums *qi_sums;  // {q_inv, cos(q.dx)}
     u64 *qi_cnt;
     u64 *qi_den;
+    QiPart *qi_part;  // [kQiCopies][n_KT * qnpts], zero between launches
 };
 
 // Pair whose K_phi bin sits within kphi_tol of a bin edge: its azimuthal
@@ -226,6 +236,8 @@ struct CopySeg {
 };
 constexpr long long kCopyInChunk = 4096;
 cudaError_t launch_copy_in(const CopySeg *segs, int n, cudaStream_t st);
+// Adds the private q_inv copies to the histogram and clears them.
+cudaError_t launch_qinv_merge(const Device &d, cudaStream_t st);
 // One output array of hbt_read_hist as FP64 in `out` (nbins doubles):
 // field 0..3 = q_out, q_side, q_long, cos sums; 4 = numerator count;
 // 5 = denominator count.

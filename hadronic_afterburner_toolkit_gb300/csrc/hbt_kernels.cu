@@ -401,6 +401,40 @@ __global__ void __launch_bounds__(256) k_export(Device d, int field, double *out
     }
 }
 
+// One warp per q_inv bin; the copies are added in lane order (the same sum on
+// every run for the same copies).
+__global__ void __launch_bounds__(256) k_qinv_merge(Device d, int nq) {
+    const int bin = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (bin >= nq) return;
+    QiPart s = {0.0, 0.0, 0.0, 0.0};
+    for (int c = lane; c < kQiCopies; c += 32) {
+        QiPart &p = d.h.qi_part[(long long)c * nq + bin];
+        s.q += p.q;
+        s.w += p.w;
+        s.n += p.n;
+        s.den += p.den;
+        p = QiPart{0.0, 0.0, 0.0, 0.0};
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        s.q += __shfl_down_sync(0xffffffffu, s.q, o);
+        s.w += __shfl_down_sync(0xffffffffu, s.w, o);
+        s.n += __shfl_down_sync(0xffffffffu, s.n, o);
+        s.den += __shfl_down_sync(0xffffffffu, s.den, o);
+    }
+    if (lane == 0) {
+        d.h.qi_sums[bin].q += s.q;
+        d.h.qi_sums[bin].w += s.w;
+        d.h.qi_cnt[bin] += (u64)s.n;
+        d.h.qi_den[bin] += (u64)s.den;
+    }
+}
+
+cudaError_t launch_qinv_merge(const Device &d, cudaStream_t st) {
+    const int nq = d.g.n_KT * d.g.qnpts;
+    k_qinv_merge<<<(nq * 32 + 255) / 256, 256, 0, st>>>(d, nq);
+    return cudaGetLastError();
+}
+
 // One segment per block: read across the CPU link, whose latency (1 to 2 us)
 // sets how much must be in flight.  One launch takes a batch's 880 columns
 // (12.8 MB) over in 85 us, 150 GB/s, where one cudaMemcpyAsync per column

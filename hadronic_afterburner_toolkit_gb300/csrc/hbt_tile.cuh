@@ -610,22 +610,25 @@ __device__ __forceinline__ double sum_peers(unsigned peers, double x) {
 // One q_inv histogram update per group of lanes with the same bin (`key`,
 // 0xffffffff: no update): the q_inv histogram has only n_KT x qnpts bins,
 // which the pairs of a warp share, so per-pair atomics would queue on a few
-// addresses.  num: add q_inv and cos (numerator, same-event) or only the
+// addresses; the groups' updates go to the CTA's private copy (QiPart), one
+// sector each.  num: add q_inv and cos (numerator, same-event) or only the
 // count (denominator, mixed-event).  Called by all 32 lanes.
 __device__ __forceinline__ void qinv_update(const Device &d, unsigned key, double qv, double wv,
                                             bool num) {
     const unsigned peers = __match_any_sync(0xffffffffu, key);
     const int lane = threadIdx.x & 31;
     const bool leader = (peers & ((1u << lane) - 1u)) == 0u && key != 0xffffffffu;
+    QiPart *p = d.h.qi_part +
+                (long long)(blockIdx.x % kQiCopies) * (d.g.n_KT * d.g.qnpts) + (leader ? key : 0u);
     if (num) {
         const double sq = sum_peers(peers, qv), sw = sum_peers(peers, wv);
         if (leader) {
-            atomicAdd(&d.h.qi_sums[key].q, sq);
-            atomicAdd(&d.h.qi_sums[key].w, sw);
-            atomicAdd(d.h.qi_cnt + key, (unsigned long long)__popc(peers));
+            atomicAdd(&p->q, sq);
+            atomicAdd(&p->w, sw);
+            atomicAdd(&p->n, (double)__popc(peers));
         }
     } else if (leader) {
-        atomicAdd(d.h.qi_den + key, (unsigned long long)__popc(peers));
+        atomicAdd(&p->den, (double)__popc(peers));
     }
 }
 
