@@ -4,10 +4,10 @@
 // and mixed-event jobs (list 1 x list 2).  When no pair cap can bind, the
 // order of the pairs does not matter, and the batch is run as:
 //
-//  1. k_keys + CUB radix sort + k_gather: every list is reordered by a
+//  1. k_keys + CUB radix sort, or k_order: every list is reordered by a
 //     Morton key of (p_x, p_y, rapidity) cells into a sorted particle table,
 //     so that 128-particle tiles are compact in momentum space;
-//  2. k_boxes: per tile, the ranges of p_x, p_y, rapidity y and the
+//  2. k_tiles: per tile, the sorted rows and the ranges of p_x, p_y, rapidity y and the
 //     smallest m_T = sqrt(E^2 - p_z^2);
 //  3. k_cull: every tile pair of every job is kept unless no pair in it can
 //     pass the q windows.  The test is rigorous: the reference's q_out and
@@ -63,11 +63,22 @@ __device__ __forceinline__ int find_range(const long long *off, int n, long long
     return lo;
 }
 
-__device__ __forceinline__ unsigned cell(double v, double origin, double inv_h) {
-    const double c = (v - origin) * inv_h;
-    if (!(c > 0.0)) return 0u;
-    if (c >= 1023.0) return 1023u;
-    return (unsigned)c;
+// Cell of v (in cells from the first one), 0 to `last`.
+__device__ __forceinline__ unsigned cell(float v, float last) {
+    return v > 0.0f ? (unsigned)fminf(v, last) : 0u;
+}
+
+// Morton code of a particle's (p_x, p_y, rapidity) cells, `half` cells either
+// side of zero, the outermost taking what lies beyond.  FP32: the key only
+// orders the list.
+__device__ __forceinline__ unsigned morton_key(const BatchDev &b, const BatchList &l, long long k,
+                                               float half, float last) {
+    const float px = (float)l.src[0][k], py = (float)l.src[1][k];
+    const double pz = l.src[2][k], E = l.src[3][k];
+    const float y = 0.5f * __logf((float)(E + pz) / (float)(E - pz));
+    return spread10(cell(fmaf(px, (float)b.inv_cell_pt, half), last)) |
+           (spread10(cell(fmaf(py, (float)b.inv_cell_pt, half), last)) << 1) |
+           (spread10(cell(fmaf(y == y ? y : 0.0f, (float)b.inv_cell_y, half), last)) << 2);
 }
 
 // The queues start empty (the first kernel of a batch clears their counters).
@@ -84,121 +95,21 @@ __global__ void k_keys(BatchDev b) {
          g += (long long)gridDim.x * blockDim.x) {
         const int L = find_range(b.list_off, b.n_lists, g);
         const BatchList &l = b.lists[L];
-        const long long k = g - l.off;
-        const double px = l.src[0][k], py = l.src[1][k], pz = l.src[2][k], E = l.src[3][k];
-        const double y = 0.5 * log((E + pz) / (E - pz));
-        const unsigned key = spread10(cell(px, -b.p_extent, b.inv_cell_pt)) |
-                             (spread10(cell(py, -b.p_extent, b.inv_cell_pt)) << 1) |
-                             (spread10(cell(y == y ? y : 0.0, -b.y_extent, b.inv_cell_y)) << 2);
-        b.keys_in[g] = ((unsigned long long)L << 32) | key;
+        b.keys_in[g] = ((unsigned long long)L << 32) | morton_key(b, l, g - l.off, 512.0f, 1023.0f);
         b.vals_in[g] = (unsigned)g;
     }
 }
 
-// Row s of the sorted table from row k of list l: its columns, screen terms
-// and fixed-point columns (once per particle here; a tile pair would convert
-// its 256 particles again each time it is taken) and its position in the
-// caller's list.
-template <bool LC>
-__device__ __forceinline__ void put_row(const BatchDev &b, const Grid &g, const BatchList &l,
-                                        long long s, long long k) {
-    double v[8];
-#pragma unroll
-    for (int f = 0; f < 8; f++)
-        if (f < l.ncols) {
-            v[f] = l.src[f][k];
-            b.table[(long long)f * b.cap + s] = v[f];
-        }
-    const Terms t = screen_terms<LC>(v[0], v[1], v[2], v[3]);
-    b.terms4[s] = make_float4(t.x, t.y, t.m, t.p);
-    b.terms2[s] = make_float2(t.r2, t.t2);
-    if (l.ncols == 8) {
-        const FixedCols c = fixed_cols(g, v);
-#pragma unroll
-        for (int f = 0; f < kFixedCols; f++) b.fixed[(long long)f * b.cap + s] = c.c[f];
-    }
-    b.orig[s] = (unsigned)k;
-}
-
-template <bool LC>
-__global__ void k_gather(BatchDev b, Grid g) {
-    for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < b.total;
-         s += (long long)gridDim.x * blockDim.x) {
-        const int L = (int)(b.keys_out[s] >> 32);
-        const BatchList &l = b.lists[L];
-        put_row<LC>(b, g, l, s, (long long)b.vals_out[s] - l.off);
-    }
-}
-
-// Momentum-space box of tile t of list l, by one warp.
-__device__ __forceinline__ void put_box(const BatchDev &b, const BatchList &l, long long t) {
-    const int lane = threadIdx.x & 31;
-    const long long s0 = l.off + t * FT, s1 = min(l.off + (t + 1) * FT, l.off + l.n);
-    double x0 = 1e300, x1 = -1e300, y0 = 1e300, y1 = -1e300, Y0 = 1e300, Y1 = -1e300, m0 = 1e300;
-    double z0 = 1e300, z1 = -1e300, mm0 = 1e300, mm1 = -1e300;
-    for (long long s = s0 + lane; s < s1; s += 32) {
-        const double px = b.table[s], py = b.table[b.cap + s];
-        const double pz = b.table[2 * b.cap + s], E = b.table[3 * b.cap + s];
-        const double y = 0.5 * log((E + pz) / (E - pz));
-        const double m2 = (E - pz) * (E + pz);
-        x0 = fmin(x0, px);
-        x1 = fmax(x1, px);
-        y0 = fmin(y0, py);
-        y1 = fmax(y1, py);
-        z0 = fmin(z0, pz);
-        z1 = fmax(z1, pz);
-        if (y == y) {
-            Y0 = fmin(Y0, y);
-            Y1 = fmax(Y1, y);
-        } else {
-            Y0 = -1e300;  // not a physical momentum: never cull on rapidity
-            Y1 = 1e300;
-        }
-        m0 = fmin(m0, m2 > 0.0 ? sqrt(m2) : 0.0);
-        const double mm = m2 - (px * px + py * py);
-        if (mm == mm) {
-            mm0 = fmin(mm0, mm);
-            mm1 = fmax(mm1, mm);
-        } else {
-            mm0 = -1e300;  // never treated as one mass
-            mm1 = 1e300;
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        x0 = fmin(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-        x1 = fmax(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-        y0 = fmin(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-        y1 = fmax(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-        Y0 = fmin(Y0, __shfl_xor_sync(0xffffffffu, Y0, o));
-        Y1 = fmax(Y1, __shfl_xor_sync(0xffffffffu, Y1, o));
-        m0 = fmin(m0, __shfl_xor_sync(0xffffffffu, m0, o));
-        z0 = fmin(z0, __shfl_xor_sync(0xffffffffu, z0, o));
-        z1 = fmax(z1, __shfl_xor_sync(0xffffffffu, z1, o));
-        mm0 = fmin(mm0, __shfl_xor_sync(0xffffffffu, mm0, o));
-        mm1 = fmax(mm1, __shfl_xor_sync(0xffffffffu, mm1, o));
-    }
-    if (lane == 0) b.boxes[l.tile_off + t] = Box{x0, x1, y0, y1, Y0, Y1, m0, z0, z1, mm0, mm1};
-}
-
-// One warp per tile.
-__global__ void k_boxes(BatchDev b) {
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp >= b.total_tiles) return;
-    const BatchList &l = b.lists[find_range(b.tile_off, b.n_lists, warp)];
-    put_box(b, l, warp - l.tile_off);
-}
-
-// Sort, gather and boxes of one list of at most kThreads x kItems particles
-// by one block, for batches of short lists: one launch in the place of keys,
-// the device-wide radix sort's 6 to 8, gather and boxes, whose launches and
-// gaps cost such a batch more than its pairs do.  The key is k_keys' with 8
-// bits to a dimension (cells 2.56 GeV and 6.4 units of rapidity either side
-// of zero at the default sizes, values beyond in the outermost), which orders
-// the list alike: 6 passes of the block's sort.  (Cells scaled to the list's
+// Order of one list of at most kThreads x kItems particles, by one block, for
+// batches of short lists: one launch in the place of keys and the device-wide
+// radix sort's 6 to 8, whose launches and gaps cost such a batch more than
+// its pairs do.  The key has 8 bits to a dimension (2.56 GeV and 6.4 units of
+// rapidity either side of zero at the default cells), which orders the list
+// as 10 bits do: 6 passes of the block's sort.  (Cells scaled to the list's
 // own ranges, which the few largest momenta set, made tiles wide in p_x, p_y
 // and culled less.)
-template <bool LC, int kThreads, int kItems>
-__global__ void __launch_bounds__(kThreads) k_prepare(BatchDev b, Grid g) {
+template <int kThreads, int kItems>
+__global__ void __launch_bounds__(kThreads) k_order(BatchDev b) {
     typedef cub::BlockRadixSort<unsigned, kThreads, kItems, unsigned short> Sort;
     __shared__ typename Sort::TempStorage tmp;
     clear_queues(b);
@@ -210,30 +121,118 @@ __global__ void __launch_bounds__(kThreads) k_prepare(BatchDev b, Grid g) {
     for (int i = 0; i < kItems; i++) {
         const int k = i * kThreads + threadIdx.x;
         row[i] = (unsigned short)k;
-        key[i] = 0xffffffffu;  // past the end: sorts behind every row
-        if (k < n) {
-            const double pz = l.src[2][k], E = l.src[3][k];
-            const double y = 0.5 * log((E + pz) / (E - pz));
-            const double c[3] = {l.src[0][k] * b.inv_cell_pt, l.src[1][k] * b.inv_cell_pt,
-                                 (y == y ? y : 0.0) * b.inv_cell_y};
-            unsigned v = 0;
-#pragma unroll
-            for (int f = 0; f < 3; f++) {
-                // (254 at most: no key equals the padding's 24 bits)
-                const double x = c[f] + 128.0;
-                v |= spread10(x > 0.0 ? (unsigned)fmin(x, 254.0) : 0u) << f;
-            }
-            key[i] = v;
-        }
+        // past the end: behind every row (whose cells are 254 at most, so
+        // that no key equals the padding's 24 bits)
+        key[i] = k < n ? morton_key(b, l, k, 128.0f, 254.0f) : 0xffffffffu;
     }
     Sort(tmp).SortBlockedToStriped(key, row, 0, 24);
 #pragma unroll
     for (int i = 0; i < kItems; i++) {
         const int s = i * kThreads + threadIdx.x;
-        if (s < n) put_row<LC>(b, g, l, l.off + s, row[i]);
+        if (s < n) b.orig[l.off + s] = row[i];
     }
-    __syncthreads();  // the boxes read this block's rows
-    for (long long t = threadIdx.x >> 5; t < l.tiles; t += kThreads / 32) put_box(b, l, t);
+}
+
+__device__ __forceinline__ float warp_min(float v) {
+    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ double warp_min(double v) {
+    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// One block per tile: its sorted rows (columns, screen terms, fixed-point
+// columns: converted once per particle here, as a tile pair would convert its
+// 256 particles again each time it is taken) and its box.  One tile to a
+// block, so that the conversions' FP64 work, 2 instructions a cycle on an SM,
+// spreads over the SMs: by one block per list it took 78 us for a list of
+// 1000.  The box is FP32 where the cull's bounds allow (rapidity: logarithm
+// of the light-cone terms' ratio, within 2e-6).
+template <bool LC>
+__global__ void __launch_bounds__(FT) k_tiles(BatchDev b, Grid g) {
+    __shared__ float part[FT / 32][9];
+    __shared__ double part2[FT / 32][2];
+    const long long tile = blockIdx.x;
+    const BatchList &l = b.lists[find_range(b.tile_off, b.n_lists, tile)];
+    const long long t = tile - l.tile_off, r = t * FT + threadIdx.x, s = l.off + r;
+    const float inf = __int_as_float(0x7f800000);
+    // minima of x, y, Y, z, of their negatives, and of m_T
+    float q[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) q[k] = inf;
+    double mm0 = 1e300, mm1 = 1e300;
+    if (r < l.n) {
+        long long k;
+        if (b.vals_out) {
+            k = (long long)b.vals_out[s] - l.off;
+            b.orig[s] = (unsigned)k;
+        } else {
+            k = b.orig[s];
+        }
+        double v[8];
+#pragma unroll
+        for (int f = 0; f < 8; f++)
+            if (f < l.ncols) {
+                v[f] = l.src[f][k];
+                b.table[(long long)f * b.cap + s] = v[f];
+            }
+        const Terms w = screen_terms<LC>(v[0], v[1], v[2], v[3]);
+        b.terms4[s] = make_float4(w.x, w.y, w.m, w.p);
+        b.terms2[s] = make_float2(w.r2, w.t2);
+        if (l.ncols == 8) {
+            const FixedCols c = fixed_cols(g, v);
+#pragma unroll
+            for (int f = 0; f < kFixedCols; f++) b.fixed[(long long)f * b.cap + s] = c.c[f];
+        }
+        q[0] = __double2float_rd(v[0]);
+        q[1] = __double2float_rd(v[1]);
+        q[3] = __double2float_rd(v[2]);
+        q[4] = -__double2float_ru(v[0]);
+        q[5] = -__double2float_ru(v[1]);
+        q[7] = -__double2float_ru(v[2]);
+        q[2] = q[6] = -inf;  // no sound rapidity: never cull on it
+        q[8] = 0.0f;
+        mm0 = mm1 = -1e300;  // never treated as one mass
+        if (LC && w.x == w.x) {
+            const float y = 0.5f * logf(w.p / w.m), e = 2e-6f + 1e-6f * fabsf(y);
+            q[2] = y - e;
+            q[6] = -(y + e);
+            q[8] = sqrtf(fmaxf(w.t2, 0.0f)) * (1.0f - 1e-6f);
+            if (g.qinv) {
+                const double mm = (v[3] - v[2]) * (v[3] + v[2]) - (v[0] * v[0] + v[1] * v[1]);
+                if (mm == mm) {
+                    mm0 = mm;
+                    mm1 = -mm;
+                }
+            }
+        }
+    }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        q[k] = warp_min(q[k]);
+        if (lane == 0) part[w][k] = q[k];
+    }
+    if (g.qinv) {
+        mm0 = warp_min(mm0);
+        mm1 = warp_min(mm1);
+        if (lane == 0) {
+            part2[w][0] = mm0;
+            part2[w][1] = mm1;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x > 0) return;
+    for (int o = 1; o < FT / 32; o++) {
+#pragma unroll
+        for (int k = 0; k < 9; k++) q[k] = fminf(q[k], part[o][k]);
+        if (g.qinv) {
+            mm0 = fmin(mm0, part2[o][0]);
+            mm1 = fmin(mm1, part2[o][1]);
+        }
+    }
+    b.boxes[tile] = Box{q[0], -q[4], q[1], -q[5], q[2], -q[6], q[8], q[3], -q[7], mm0, -mm1};
 }
 
 // Can a pair with one particle in box a and one in box b pass the windows?
@@ -245,28 +244,35 @@ __global__ void __launch_bounds__(kThreads) k_prepare(BatchDev b, Grid g) {
 // for two particles of one mass q.K = 0, so in the LCMS
 // q_inv^2 = q_out^2 (1 - beta_T^2) + q_side^2 + q_long^2 >= q_long^2, and
 // only the q_long bound culls (tiles whose masses differ keep every pair).
+// In FP32 with every bound rounded so that it stays one: gaps and squares
+// rounded down, sinh below 1 by its series cut (a lower bound), and 2e-5 taken
+// off the quotient, far above the rounding of exp, the root and the products.
 __device__ __forceinline__ bool boxes_may_pair(const BatchJob &b, const Box &a, const Box &c) {
-    const double gY = fmax(0.0, fmax(a.Y0 - c.Y1, c.Y0 - a.Y1));
-    double qlong_lcms = 0.0;  // lower bound of |q_long| in the LCMS
-    if (gY > 0.0) {
-        const double m1 = a.m0, m2 = c.m0;
-        qlong_lcms = 2.0 * m1 * m2 * sinh(gY) /
-                     sqrt(m1 * m1 + m2 * m2 + 2.0 * m1 * m2 * cosh(gY));
+    const float gY = fmaxf(0.0f, fmaxf(__fsub_rd(a.Y0, c.Y1), __fsub_rd(c.Y0, a.Y1)));
+    float qlong = 0.0f;  // lower bound of |q_long| in the LCMS
+    if (gY > 0.0f) {
+        const float m1 = a.m0, m2 = c.m0, g = fminf(gY, 40.0f);
+        const float e = expf(g), i = 1.0f / e;
+        const float sh = g < 1.0f ? g * (1.0f + g * g * (1.0f / 6.0f)) : 0.5f * (e - i);
+        const float ch = 0.5f * (e + i);
+        qlong = (1.0f - 2e-5f) * 2.0f * m1 * m2 * sh *
+                rsqrtf(m1 * m1 + m2 * m2 + 2.0f * m1 * m2 * ch);
+        if (!(qlong == qlong)) qlong = 0.0f;  // both masses zero
     }
-    const double gx = fmax(0.0, fmax(a.x0 - c.x1, c.x0 - a.x1));
-    const double gy = fmax(0.0, fmax(a.y0 - c.y1, c.y0 - a.y1));
-    bool pass3 = !(gx * gx + gy * gy > b.qt2_max);
+    const float gx = fmaxf(0.0f, fmaxf(__fsub_rd(a.x0, c.x1), __fsub_rd(c.x0, a.x1)));
+    const float gy = fmaxf(0.0f, fmaxf(__fsub_rd(a.y0, c.y1), __fsub_rd(c.y0, a.y1)));
+    bool pass3 = !((double)__fadd_rd(__fmul_rd(gx, gx), __fmul_rd(gy, gy)) > b.qt2_max);
     if (b.boost) {
-        pass3 = pass3 && !(qlong_lcms > b.ql_max);
+        pass3 = pass3 && !((double)qlong > b.ql_max);
     } else {
         // q_long = q_z
-        const double gz = fmax(0.0, fmax(a.z0 - c.z1, c.z0 - a.z1));
-        pass3 = pass3 && !(gz > b.ql_max);
+        const float gz = fmaxf(0.0f, fmaxf(__fsub_rd(a.z0, c.z1), __fsub_rd(c.z0, a.z1)));
+        pass3 = pass3 && !((double)gz > b.ql_max);
     }
     if (pass3 || !b.qinv) return pass3;
     const double lo = fmin(a.mm0, c.mm0), hi = fmax(a.mm1, c.mm1);
     if (!(hi - lo <= 1e-9 * fabs(hi))) return true;
-    return !(qlong_lcms > b.ql_max);
+    return !((double)qlong > b.ql_max);
 }
 
 // Momentum-space region of a tile pair's pairs: K = (p_1 + p_2) / 2 at the
@@ -274,12 +280,12 @@ __device__ __forceinline__ bool boxes_may_pair(const BatchJob &b, const Box &a, 
 // sectors, above the analysis index (serving).  Items of one region update
 // the same few histogram slots.
 __device__ __forceinline__ unsigned region_key(const BatchJob &job, const Box &a, const Box &c) {
-    const double kx = 0.25 * (a.x0 + a.x1 + c.x0 + c.x1);
-    const double ky = 0.25 * (a.y0 + a.y1 + c.y0 + c.y1);
-    const double kt = sqrt(kx * kx + ky * ky);
-    const unsigned kc = kt < 2.0 ? (unsigned)(kt * 32.0) : 63u;
-    double ph = atan2(ky, kx) * (16.0 / 3.141592653589793) + 16.0;  // [0, 32]
-    const unsigned pc = ph >= 0.0 && ph < 32.0 ? (unsigned)ph : 0u;
+    const float kx = 0.25f * (a.x0 + a.x1 + c.x0 + c.x1);
+    const float ky = 0.25f * (a.y0 + a.y1 + c.y0 + c.y1);
+    const float kt = sqrtf(kx * kx + ky * ky);
+    const unsigned kc = kt < 2.0f ? (unsigned)(kt * 32.0f) : 63u;
+    const float ph = atan2f(ky, kx) * (16.0f / 3.14159265f) + 16.0f;  // [0, 32]
+    const unsigned pc = ph >= 0.0f && ph < 32.0f ? (unsigned)ph : 0u;
     // (below 0x1FFFFF, so that no key equals the unused entries' 0xffffffff)
     const unsigned dev = job.dev < 0x1FFFFE ? (unsigned)job.dev : 0x1FFFFEu;
     return (dev << 11) | (kc << 5) | pc;
@@ -304,8 +310,8 @@ struct SlotCull {
 // admits nothing more in a full slot, so such a tile pair needs neither the
 // count nor the order pass.
 __device__ bool slots_all_full(const SlotCull &sc, const Box &a, const Box &c) {
-    const double x0 = 0.5 * (a.x0 + c.x0), x1 = 0.5 * (a.x1 + c.x1);
-    const double y0 = 0.5 * (a.y0 + c.y0), y1 = 0.5 * (a.y1 + c.y1);
+    const double x0 = 0.5 * ((double)a.x0 + c.x0), x1 = 0.5 * ((double)a.x1 + c.x1);
+    const double y0 = 0.5 * ((double)a.y0 + c.y0), y1 = 0.5 * ((double)a.y1 + c.y1);
     if (x0 <= 0.0 && x1 >= 0.0 && y0 <= 0.0 && y1 >= 0.0) return false;
     const double nx = x0 > 0.0 ? x0 : (x1 < 0.0 ? x1 : 0.0);
     const double ny = y0 > 0.0 ? y0 : (y1 < 0.0 ? y1 : 0.0);
@@ -422,18 +428,10 @@ cudaError_t run_batch(const Device &d, const BatchDev &b, int grid, unsigned chu
     const int gs = 152 * 8;
     const bool lc = d.g.boost || d.g.qinv;  // light-cone screen terms
     if (b.max_list <= kSmallList) {
-        // (1024-particle lists: 64 threads of 16 rows would leave the sort's
-        // latency bare; 256 of 4 measured fastest)
-        if (b.max_list <= 1024) {
-            if (lc)
-                k_prepare<true, 256, 4><<<b.n_lists, 256, 0, st>>>(b, d.g);
-            else
-                k_prepare<false, 256, 4><<<b.n_lists, 256, 0, st>>>(b, d.g);
-        } else if (lc) {
-            k_prepare<true, 1024, 8><<<b.n_lists, 1024, 0, st>>>(b, d.g);
-        } else {
-            k_prepare<false, 1024, 8><<<b.n_lists, 1024, 0, st>>>(b, d.g);
-        }
+        if (b.max_list <= 1024)
+            k_order<256, 4><<<b.n_lists, 256, 0, st>>>(b);
+        else
+            k_order<1024, 8><<<b.n_lists, 1024, 0, st>>>(b);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     } else {
         k_keys<<<gs, 256, 0, st>>>(b);
@@ -444,14 +442,12 @@ cudaError_t run_batch(const Device &d, const BatchDev &b, int grid, unsigned chu
         e = cub::DeviceRadixSort::SortPairs(b.sort_temp, bytes, b.keys_in, b.keys_out, b.vals_in,
                                             b.vals_out, (int)b.total, 0, end_bit, st);
         if (e != cudaSuccess) return e;
-        if (lc)
-            k_gather<true><<<gs, 256, 0, st>>>(b, d.g);
-        else
-            k_gather<false><<<gs, 256, 0, st>>>(b, d.g);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        k_boxes<<<(unsigned)((b.total_tiles * 32 + 255) / 256), 256, 0, st>>>(b);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
+    if (lc)
+        k_tiles<true><<<(unsigned)b.total_tiles, FT, 0, st>>>(b, d.g);
+    else
+        k_tiles<false><<<(unsigned)b.total_tiles, FT, 0, st>>>(b, d.g);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (b.order_items && b.same_cap > 0 &&
         (e = cudaMemsetAsync(b.item_key_in, 0xff, (size_t)b.same_cap * sizeof(unsigned), st)) !=
             cudaSuccess)

@@ -44,13 +44,13 @@ struct BatchJob {
     long long row_base;
 };
 
-// Momentum-space box of a 128-particle tile.
+// Momentum-space box of a 128-particle tile, FP32 ranges rounded outwards.
 struct Box {
-    double x0, x1, y0, y1;  // p_x, p_y ranges
-    double Y0, Y1;          // rapidity range
-    double m0;              // smallest m_T = sqrt(E^2 - p_z^2)
-    double z0, z1;          // p_z range
-    double mm0, mm1;        // range of the mass squared E^2 - |p|^2
+    float x0, x1, y0, y1;  // p_x, p_y ranges
+    float Y0, Y1;          // rapidity range
+    float m0;              // lower bound of m_T = sqrt(E^2 - p_z^2)
+    float z0, z1;          // p_z range
+    double mm0, mm1;       // range of the mass squared E^2 - |p|^2
 };
 
 struct Item {
@@ -96,7 +96,8 @@ struct BatchDev {
     void *item_sort_temp;
     size_t item_sort_temp_bytes;
     // cell sizes of the sort key
-    double p_extent, inv_cell_pt, y_extent, inv_cell_y;
+    double inv_cell_pt, inv_cell_y;
+    const double *cos;  // the cosine table (cos_entries), read by every CTA
     // Several analyses in one launch (the serving loop): each job's engine
     // descriptor (grid, screen constants, histograms) is devs[job.dev];
     // nullptr: every job belongs to the launch's own descriptor.

@@ -103,7 +103,8 @@ __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(D
     __shared__ SameSmem sm;
     __shared__ unsigned item;
     __shared__ double cs[PREC == 0 ? kCosEntries : 1];  // the form's cos table
-    if (PREC == 0) fill_cos_entries(cs);
+    if (PREC == 0)
+        for (int k = threadIdx.x; k < kCosEntries; k += FT) cs[k] = b.cos[k];
     const unsigned stop = min(end, min(b.n_items[0], b.same_cap));
     const unsigned parts = item_parts(stop > base ? stop - base : 0u), rows = FT / parts;
     for (;;) {

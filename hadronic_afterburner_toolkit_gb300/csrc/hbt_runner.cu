@@ -7,12 +7,26 @@
 
 namespace hbt {
 
+namespace {
+
+// The table of cos_fixed (hbt_fixed.cuh): cos(2 pi k / 2048), k = 0..512, the
+// last one a number too small to matter in the place of zero.
+std::vector<double> cos_entries() {
+    std::vector<double> t(513);
+    for (int k = 0; k < 512; k++)
+        t[k] = (double)cosl(3.14159265358979323846264338327950288L * k / 1024.0L);
+    t[512] = std::ldexp(1.0, -100);
+    return t;
+}
+
+}  // namespace
+
 BatchRunner::~BatchRunner() {
     if (exec_) cudaGraphExecDestroy(exec_);
     for (cudaEvent_t e : marks_)
         if (e) cudaEventDestroy(e);
     Buf *all[] = {&tables_, &orig_, &table_, &keys_, &vals_, &sort_temp_, &boxes_,
-                  &items_, &counters_, &devs_, &item_order_, &item_sort_temp_, &fixed_, &terms_};
+                  &items_, &counters_, &devs_, &item_order_, &item_sort_temp_, &fixed_, &terms_, &cos_};
     for (Buf *b : all)
         if (b->p) cudaFree(b->p);
 }
@@ -225,6 +239,20 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
         err = "batch too large (tile pairs or particles)";
         return false;
     }
+    // the cosine table, once (each CTA computing its 513 entries took 4 us of
+    // a launch, most of it for the smallest)
+    if (!cos_.p) {
+        const std::vector<double> table = cos_entries();
+        if (!grow(cos_, table.size() * sizeof(double), err)) return false;
+        if (cudaMemcpyAsync(cos_.p, table.data(), table.size() * sizeof(double),
+                            cudaMemcpyHostToDevice, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess) {
+            cudaFree(cos_.p);
+            cos_ = Buf();
+            err = "uploading the cosine table failed";
+            return false;
+        }
+    }
     // small lists are sorted by one block each (k_prepare), others by CUB
     const bool small = max_list <= kSmallList;
     const size_t sort_bytes = small ? 0 : batch_sort_temp_bytes(total);
@@ -306,10 +334,9 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
     b.mixed_cap = (unsigned)mixed_pairs;
     b.n_items = static_cast<unsigned *>(counters_.p);
     b.item_next = b.n_items + 2;
-    b.p_extent = 1024 * t.cell_pt / 2;
     b.inv_cell_pt = 1.0 / t.cell_pt;
-    b.y_extent = 1024 * t.cell_y / 2;
     b.inv_cell_y = 1.0 / t.cell_y;
+    b.cos = static_cast<const double *>(cos_.p);
     b.devs = devs_dev;
     b.n_devs = n_devs;
     b.order_items = order ? 1 : 0;

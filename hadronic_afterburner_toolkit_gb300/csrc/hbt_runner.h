@@ -86,7 +86,7 @@ class BatchRunner {
     cudaError_t launch(const Device &d, const BatchDev &b, const Device *devs_host, int n_devs,
                        const Tuning &t, cudaStream_t st, int mode);
     Buf tables_, orig_, table_, keys_, vals_, sort_temp_, boxes_, items_, counters_, devs_;
-    Buf item_order_, item_sort_temp_, fixed_, terms_;
+    Buf item_order_, item_sort_temp_, fixed_, terms_, cos_;
     std::vector<unsigned char> tables_host_;
     long long last_pairs_ = 0, last_same_ = 0, last_mixed_ = 0;
     cudaStream_t last_stream_ = nullptr;
