@@ -238,6 +238,15 @@ constexpr long long kCopyInChunk = 4096;
 cudaError_t launch_copy_in(const CopySeg *segs, int n, cudaStream_t st);
 // Adds the private q_inv copies to the histogram and clears them.
 cudaError_t launch_qinv_merge(const Device &d, cudaStream_t st);
+// Arrays to export into: q_out, q_side, q_long, cos sums, numerator and
+// denominator counts (qinv: the sums of q_inv and cos, the two counts), and
+// the STAT_N status words.
+struct HistOut {
+    double *v[6];
+    u64 *stats;
+};
+cudaError_t launch_export_all(const Device &d, const HistOut &o, long long nbins, bool qinv,
+                              cudaStream_t st);
 // One output array of hbt_read_hist as FP64 in `out` (nbins doubles):
 // field 0..3 = q_out, q_side, q_long, cos sums; 4 = numerator count;
 // 5 = denominator count.

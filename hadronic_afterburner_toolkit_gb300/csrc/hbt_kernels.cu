@@ -260,9 +260,12 @@ __global__ void k_defer_count(Device d, long long rows, long long cols, int n_re
 // Pair counters = sums of the count histograms (each counter is
 // incremented exactly when a pair is binned).  out: [num slots][den
 // slots][num q_inv][den q_inv].
+// kCounterParts blocks per counter, each adding its part of the bins (one
+// block alone took 42 us for the 68,921 bins of a slot).
+constexpr int kCounterParts = 16;
 __global__ void __launch_bounds__(256) k_counters(Device d, unsigned long long *out) {
     const int ns = d.g.n_slots, nk = d.g.n_KT;
-    const int b = blockIdx.x;
+    const int b = blockIdx.x / kCounterParts, part = blockIdx.x % kCounterParts;
     const u64 *src;
     long long len;
     if (b < ns) {
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(256) k_counters(Device d, unsigned long long *
         len = d.g.qnpts;
     }
     unsigned long long s = 0;
-    for (long long k = threadIdx.x; k < len; k += blockDim.x) s += src[k];
+    for (long long k = part * 256 + threadIdx.x; k < len; k += kCounterParts * 256) s += src[k];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     __shared__ unsigned long long ws[8];
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(256) k_counters(Device d, unsigned long long *
     if (threadIdx.x == 0) {
         unsigned long long t = 0;
         for (int k = 0; k < 8; k++) t += ws[k];
-        out[b] = t;
+        if (t) atomicAdd(out + b, t);
     }
 }
 
@@ -401,6 +404,46 @@ __global__ void __launch_bounds__(256) k_export(Device d, int field, double *out
     }
 }
 
+// The six arrays of hbt_read_hist (any may be null) in one pass over the
+// histograms, with the status words: into host memory where the GPU writes
+// it.  Six kernels and copies took 127 us for the smallest histograms.
+__global__ void __launch_bounds__(256) k_export_all(Device d, HistOut o, long long nbins) {
+    if (blockIdx.x == 0 && threadIdx.x < STAT_N) o.stats[threadIdx.x] = d.stats[threadIdx.x];
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nbins;
+         k += (long long)gridDim.x * blockDim.x) {
+        const Sums s = d.h.sums[k];
+        if (o.v[0]) o.v[0][k] = s.qo;
+        if (o.v[1]) o.v[1][k] = s.qs;
+        if (o.v[2]) o.v[2][k] = s.ql;
+        if (o.v[3]) o.v[3][k] = s.w;
+        if (o.v[4]) o.v[4][k] = (double)d.h.cnt[k];
+        if (o.v[5]) o.v[5][k] = (double)d.h.den[k];
+    }
+}
+
+// The four arrays of hbt_read_qinv (any may be null) and the status words.
+__global__ void __launch_bounds__(256) k_export_qinv(Device d, HistOut o, long long nbins) {
+    if (blockIdx.x == 0 && threadIdx.x < STAT_N) o.stats[threadIdx.x] = d.stats[threadIdx.x];
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nbins;
+         k += (long long)gridDim.x * blockDim.x) {
+        if (o.v[0]) o.v[0][k] = d.h.qi_sums[k].q;
+        if (o.v[1]) o.v[1][k] = d.h.qi_sums[k].w;
+        if (o.v[2]) o.v[2][k] = (double)d.h.qi_cnt[k];
+        if (o.v[3]) o.v[3][k] = (double)d.h.qi_den[k];
+    }
+}
+
+cudaError_t launch_export_all(const Device &d, const HistOut &o, long long nbins, bool qinv,
+                              cudaStream_t st) {
+    const unsigned blocks =
+        (unsigned)std::max<long long>(1, std::min<long long>((nbins + 255) / 256, 152 * 8));
+    if (qinv)
+        k_export_qinv<<<blocks, 256, 0, st>>>(d, o, nbins);
+    else
+        k_export_all<<<blocks, 256, 0, st>>>(d, o, nbins);
+    return cudaGetLastError();
+}
+
 // One warp per q_inv bin; the copies are added in lane order (the same sum on
 // every run for the same copies).
 __global__ void __launch_bounds__(256) k_qinv_merge(Device d, int nq) {
@@ -461,7 +504,10 @@ cudaError_t launch_export(const Device &d, int field, double *out, long long nbi
 }
 
 cudaError_t launch_counters(const Device &d, unsigned long long *out, cudaStream_t st) {
-    k_counters<<<2 * d.g.n_slots + 2 * d.g.n_KT, 256, 0, st>>>(d, out);
+    const int n = 2 * d.g.n_slots + 2 * d.g.n_KT;
+    const cudaError_t e = cudaMemsetAsync(out, 0, n * sizeof(unsigned long long), st);
+    if (e != cudaSuccess) return e;
+    k_counters<<<n * kCounterParts, 256, 0, st>>>(d, out);
     return cudaGetLastError();
 }
 
