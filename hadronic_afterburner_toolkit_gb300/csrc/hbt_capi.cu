@@ -17,7 +17,6 @@
 #include <thread>
 #include <vector>
 
-#include <sys/mman.h>
 #include <unistd.h>
 
 #include "../../include/hbt_gpu.h"
@@ -1351,12 +1350,13 @@ int64_t hbt_n_bins(const hbt_ctx *c) { return c ? (int64_t)c->d.g.n_slots * c->d
 namespace {
 
 // Maps the pages of the output arrays before the results arrive, while the
-// binning still runs: left to the GPU's copy, the first touch of a page took
-// up to 48 us (a 16 MB read 12 ms).  MADV_POPULATE_WRITE maps a range in one
-// call and leaves its contents; where the system lacks it, or for the edges, an
-// atomic addition of zero does (a plain read would first map the shared zero
-// page, and replacing that page costs 25 us where the GPU shares the page
-// tables).  Large arrays by several threads.
+// binning still runs, by a store to each (every element is written later):
+// left to the GPU's copy, the first touch of a page took up to 48 us (a 16 MB
+// read 12 ms).  Large arrays by several threads: 238 MB in fresh memory take
+// 8.1 ms by one, 2.0 ms by eight.  (MADV_POPULATE_WRITE keeps the contents,
+// but took 6 ms by eight threads and 2 ms for mapped pages; a read or an
+// atomic before the store maps the shared zero page first, whose replacement
+// costs 25 us where the GPU shares the page tables.)
 void map_pages(double *const *dst, int n, size_t count) {
     const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
     struct Range {
@@ -1372,21 +1372,14 @@ void map_pages(double *const *dst, int n, size_t count) {
             parts.push_back(Range{std::max(p, a), std::min(p + most, b)});
         total += b - a;
     }
-    auto run = [&](const Range &r) {
-#ifdef MADV_POPULATE_WRITE
-        const uintptr_t p = r.a & ~(page - 1);
-        if (madvise(reinterpret_cast<void *>(p), r.b - p, MADV_POPULATE_WRITE) == 0) return;
-#endif
-        for (uintptr_t q = r.a; q < r.b; q = (q & ~(page - 1)) + page)
-            __atomic_fetch_add(reinterpret_cast<u64 *>((q + 7) & ~(uintptr_t)7), 0,
-                               __ATOMIC_RELAXED);
+    std::atomic<size_t> next{0};
+    auto work = [&] {
+        for (size_t k; (k = next.fetch_add(1)) < parts.size();)
+            for (uintptr_t q = parts[k].a; q < parts[k].b; q = (q & ~(page - 1)) + page)
+                *reinterpret_cast<volatile char *>(q) = 0;
     };
     const size_t threads = std::min<size_t>(
         {8, std::max(1u, std::thread::hardware_concurrency()), 1 + total / (16u << 20)});
-    std::atomic<size_t> next{0};
-    auto work = [&] {
-        for (size_t k; (k = next.fetch_add(1)) < parts.size();) run(parts[k]);
-    };
     std::vector<std::thread> pool;
     try {
         for (size_t t = 1; t < threads; t++) pool.emplace_back(work);

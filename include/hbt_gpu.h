@@ -48,10 +48,11 @@ typedef enum hbt_precision {
     HBT_PRECISION_FP32W = 1, /* cos(q.dx) weight and q sums in FP32 partials,
                                 merged into FP64 bins with Kahan compensation;
                                 bins and counts stay exact */
-    HBT_PRECISION_DF64 = 2   /* same-event weight and q sums computed in
-                                double-float arithmetic (value = hi + lo, two
-                                FP32 numbers) on the FP32 pipe and added to
-                                the FP64 bins; bins and counts stay exact */
+    HBT_PRECISION_DF64 = 2   /* same-event weight and q sums to 1e-11 per pair
+                                into the FP64 bins; bins and counts stay
+                                exact.  Runs the FP64 form's kernels, whose
+                                fixed-point and double-float values are both
+                                closer and faster than 48-bit ones */
 } hbt_precision;
 
 /* The HBT keys of parameters.dat that shape the histograms
@@ -234,7 +235,8 @@ int64_t hbt_n_bins(const hbt_ctx *ctx);
  * numerator, denominator pair count.  These are the arrays the reference's
  * writer reads (correl_3d_num_count, q_out_mean, q_side_mean, q_long_mean,
  * correl_3d_num, correl_3d_denorm and their K_phi twins,
- * src/HBT_correlation.h:55-61). */
+ * src/HBT_correlation.h:55-61).  When the call fails, the arrays' contents
+ * are unspecified. */
 hbt_status hbt_read_hist(hbt_ctx *ctx, double *num_count, double *q_out_sum,
                          double *q_side_sum, double *q_long_sum, double *num,
                          double *den);
