@@ -74,6 +74,7 @@ struct hbt_ctx {
     hbt_tuning tune = {0, 0.02, 0.05, kMergeChunk, 1, 0, 1};
     // ordered admission scratch
     DevBuf rowcnt, row_cut, quota, remaining, resolved, counters, apply_iphi, straddle_jobs,
+        straddle_bits,
         slot_full;
     // input staging, two buffers in turn: the host-to-device copy of a call
     // runs on `copy_in` while the binning of the previous call still reads
@@ -399,6 +400,17 @@ hbt_status set_slot_full(hbt_ctx *c, const std::vector<u64> &rem) {
     return HBT_OK;
 }
 
+// Scratch of the cut rows' admission over up to `cols` columns.
+hbt_status set_straddle(hbt_ctx *c, long long cols) {
+    const size_t chunks = (size_t)((cols + hbt::kStraddleCols - 1) / hbt::kStraddleCols);
+    const size_t per = hbt::kStraddleCols / 32, n = (size_t)c->n_stream * chunks;
+    TRY(dalloc(c, c->straddle_bits, n * (per + 1) * sizeof(unsigned)));
+    c->d.caps.straddle_bits = ptr<unsigned>(c->straddle_bits);
+    c->d.caps.straddle_count = c->d.caps.straddle_bits + n * per;
+    c->d.caps.straddle_chunks = (int)chunks;
+    return HBT_OK;
+}
+
 // Clears Caps::slot_full when an ordered pass ends, on every return path.
 struct SlotFullScope {
     hbt::Caps &caps;
@@ -432,6 +444,7 @@ hbt_status ordered_launch(hbt_ctx *c, int mixed, long long rows, long long cols,
     TRY(dalloc(c, c->row_cut, nst * sizeof(long long)));
     TRY(dalloc(c, c->quota, nst * sizeof(u64)));
     TRY(dalloc(c, c->remaining, nst * sizeof(u64)));
+    TRY(set_straddle(c, cols));
     refresh_device(c);
     // the batched passes skip tile pairs that reach only full slots
     SlotFullScope slot_scope{c->d.caps};
@@ -513,6 +526,7 @@ hbt_status ordered_launch_mixed_jobs(hbt_ctx *c, const std::vector<hbt::FastJob>
     TRY(dalloc(c, c->row_cut, nst * sizeof(long long)));
     TRY(dalloc(c, c->quota, nst * sizeof(u64)));
     TRY(dalloc(c, c->remaining, nst * sizeof(u64)));
+    TRY(set_straddle(c, cols));
     TRY(dalloc(c, c->straddle_jobs, sj.size() * sizeof(hbt::StraddleJob)));
     refresh_device(c);
     // the joint row numbering holds for the two passes and the straddle only
@@ -992,7 +1006,7 @@ void hbt_destroy(hbt_ctx *c) {
     DevBuf *bufs[] = {&c->sums,   &c->cnt,     &c->den,       &c->qi_sums,  &c->qi_cnt,
                       &c->qi_den, &c->qi_part, &c->stats,   &c->defer,     &c->n_defer,  &c->rowcnt,
                       &c->row_cut, &c->quota,  &c->remaining, &c->resolved, &c->counters,
-                      &c->apply_iphi, &c->straddle_jobs, &c->slot_full, &c->in[0], &c->in[1],
+                      &c->apply_iphi, &c->straddle_jobs, &c->straddle_bits, &c->slot_full, &c->in[0], &c->in[1],
                       &c->part, &c->comp, &c->exp};
     if (c->copy) cudaStreamSynchronize(c->copy);
     for (DevBuf *b : bufs) dfree(c, *b);

@@ -106,7 +106,12 @@ struct Caps {
     // (n_slots bytes), so that the batched passes skip tile pairs that can
     // reach no other slot; nullptr: none
     const unsigned char *slot_full;
+    // the cut rows' pairs, in chunks of kStraddleCols columns: survivors'
+    // bits [n_stream][chunks][kStraddleCols / 32] and counts [n_stream][chunks]
+    unsigned *straddle_bits, *straddle_count;
+    int straddle_chunks;
 };
+constexpr int kStraddleCols = 256;
 
 // FP32 copies of the constants used by the FP32 pair screen (hbt_fast.cu),
 // each with the bound on its rounding (slack) relative to the FP64 value.

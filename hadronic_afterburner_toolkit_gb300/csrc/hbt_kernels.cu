@@ -71,93 +71,35 @@ __global__ void __launch_bounds__(TILE) k_mixed(Device d, long long n1, Cols4 l1
     }
 }
 
-// Ordered admission of stream bin b's cut row (row r of the list a8, whose
-// pairs run over cols particles: a8 itself after r for same-event lists,
-// b4 for mixed-event lists): the first `quota` survivors in pair order, by
-// one warp.  A deferred K_phi bin is looked up under key_row * key_cols + j.
-template <bool MIXED>
-__device__ __forceinline__ void straddle_row(const Device &d, int b, long long r,
-                                             long long key_row, long long key_cols,
-                                             long long cols, const double *const *a8,
-                                             const double *const *b4) {
-    const unsigned long long quota = d.caps.quota[b];
-    const int lane = threadIdx.x;
-    const int ns = d.g.n_slots;
-    unsigned long long admitted = 0;
-    const double apx = a8[0][r], apy = a8[1][r], apz = a8[2][r], aE = a8[3][r];
-    double ax[4] = {0, 0, 0, 0};
-    if (!MIXED) {
-        ax[0] = a8[4][r];
-        ax[1] = a8[5][r];
-        ax[2] = a8[6][r];
-        ax[3] = a8[7][r];
-    }
-    const long long jstart = MIXED ? 0 : r + 1;
-    for (long long j0 = jstart; j0 < cols && admitted < quota; j0 += 32) {
-        const long long j = j0 + lane;
-        Chain c;
-        c.iK = -1;
-        bool has = false;
-        int slot = -1;
-        if (j < cols) {
-            double bx[4] = {0, 0, 0, 0};
-            if (!MIXED) {
-                bx[0] = a8[4][j];
-                bx[1] = a8[5][j];
-                bx[2] = a8[6][j];
-                bx[3] = a8[7][j];
-            }
-            const double *const *src = MIXED ? b4 : a8;
-            c = pair_chain<MIXED>(d.g, apx, apy, apz, aE, src[0][j], src[1][j], src[2][j],
-                                  src[3][j], ax, bx);
-            if (c.iK >= 0) {
-                if (b >= ns) {
-                    has = c.qi_k >= 0 && ns + c.iK == b;
-                } else if (c.ev3 == 1) {
-                    slot = c.slot;
-                    has = slot == b;
-                } else if (c.ev3 == 2) {
-                    slot = resolved_slot(d, key_row * key_cols + j, c.iK);
-                    has = slot == b;
-                }
-            }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, has);
-        const unsigned long long rank =
-            admitted + __popc(m & ((1u << lane) - 1u));
-        if (has && rank < quota) {
-            if (b >= ns) {
-                if (MIXED)
-                    bin_den_qinv(d, c);
-                else
-                    bin_num_qinv(d, c);
-            } else {
-                if (MIXED)
-                    bin_den3(d, slot, c.bin);
-                else
-                    bin_num3(d, slot, c.bin, c);
-            }
-        }
-        admitted += __popc(m);
-    }
-}
+// Admission of a stream bin's cut row, pair by pair in column order, by many
+// blocks: straddle_mark runs the reference chain on the row's pairs and
+// leaves the survivors' bits and each block's count, straddle_admit bins the
+// survivors whose rank is below the bin's quota (their chain again).  One
+// warp per stream bin walking the row is bound by its serial chain of pairs: it
+// took 9.6 ms for 60,000 columns (and 2.1 ms over mixed jobs); with the columns
+// spread over blocks a capped run of that size went from 28.3 to 18.3 ms.
 
-// One launch's cut rows, one warp per stream bin.
+// The cut row of stream bin b: the first particle's columns and row, the row
+// and column stride of the deferrals' keys, and the second particles.
+struct CutRow {
+    const double *const *a, *const *b;
+    long long r, key_row, key_cols, first, cols;
+};
 template <bool MIXED>
-__global__ void k_straddle(Device d, long long rows, long long cols, Cols8 a8, Cols4 b4) {
-    const int b = blockIdx.x;
+__device__ __forceinline__ bool cut_row(const Device &d, int b, long long rows, long long cols,
+                                        const double *const *a8, const double *const *b4,
+                                        CutRow &t) {
     const long long r = d.caps.row_cut[b];
-    if (r >= rows) return;
-    straddle_row<MIXED>(d, b, r, r, cols, cols, a8.p, b4.p);
+    if (r >= rows || d.caps.quota[b] == 0ull) return false;
+    t = CutRow{a8, MIXED ? b4 : a8, r, r, cols, MIXED ? 0 : r + 1, cols};
+    return true;
 }
-
-// The cut rows of several mixed-event jobs admitted together: a stream
-// bin's cut row r (in the jobs' joint row order) belongs to the last job
-// whose row_base is at most r.
-__global__ void k_straddle_jobs(Device d, const StraddleJob *jobs, int n_jobs, long long rows) {
-    const int b = blockIdx.x;
+// The jobs' joint row order: row r belongs to the last job whose row_base is
+// at most r.
+__device__ __forceinline__ bool cut_row_jobs(const Device &d, int b, const StraddleJob *jobs,
+                                             int n_jobs, long long rows, CutRow &t) {
     const long long r = d.caps.row_cut[b];
-    if (r >= rows) return;
+    if (r >= rows || d.caps.quota[b] == 0ull) return false;
     int lo = 0, hi = n_jobs - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -167,7 +109,120 @@ __global__ void k_straddle_jobs(Device d, const StraddleJob *jobs, int n_jobs, l
             hi = mid - 1;
     }
     const StraddleJob &job = jobs[lo];
-    straddle_row<true>(d, b, r - job.row_base, r, d.caps.cols_key, job.n2, job.a, job.b);
+    t = CutRow{job.a, job.b, r - job.row_base, r, d.caps.cols_key, 0, job.n2};
+    return true;
+}
+
+// Does column j's pair fall in stream bin b (3-D slots first, then the q_inv
+// K_T bins)?  Fills the chain and the slot.
+template <bool MIXED>
+__device__ __forceinline__ bool cut_pair(const Device &d, int b, const CutRow &t, long long j,
+                                         Chain &c, int &slot) {
+    if (j < t.first || j >= t.cols) return false;
+    const int ns = d.g.n_slots;
+    const double apx = t.a[0][t.r], apy = t.a[1][t.r], bpx = t.b[0][j], bpy = t.b[1][j];
+    double ax[4] = {0, 0, 0, 0}, bx[4] = {0, 0, 0, 0};
+    if (!MIXED)
+        for (int f = 0; f < 4; f++) {
+            ax[f] = t.a[4 + f][t.r];
+            bx[f] = t.b[4 + f][j];
+        }
+    c = pair_chain<MIXED>(d.g, apx, apy, t.a[2][t.r], t.a[3][t.r], bpx, bpy, t.b[2][j], t.b[3][j],
+                          ax, bx);
+    if (c.iK < 0) return false;
+    if (b >= ns) return c.qi_k >= 0 && ns + c.iK == b;
+    slot = -1;
+    if (c.ev3 == 1)
+        slot = c.slot;
+    else if (c.ev3 == 2)
+        slot = resolved_slot(d, t.key_row * t.key_cols + j, c.iK);
+    return slot == b;
+}
+
+template <bool MIXED>
+__device__ __forceinline__ void straddle_mark(const Device &d, int b, const CutRow &t) {
+    const int chunk = blockIdx.x % d.caps.straddle_chunks;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    Chain c;
+    int slot;
+    const bool has =
+        cut_pair<MIXED>(d, b, t, (long long)chunk * kStraddleCols + threadIdx.x, c, slot);
+    const unsigned m = __ballot_sync(0xffffffffu, has);
+    __shared__ unsigned cnt[kStraddleCols / 32];
+    const long long at = (long long)b * d.caps.straddle_chunks + chunk;
+    if (lane == 0) {
+        d.caps.straddle_bits[at * (kStraddleCols / 32) + w] = m;
+        cnt[w] = __popc(m);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned n = 0;
+        for (int k = 0; k < kStraddleCols / 32; k++) n += cnt[k];
+        d.caps.straddle_count[at] = n;
+    }
+}
+
+template <bool MIXED>
+__device__ __forceinline__ void straddle_admit(const Device &d, int b, const CutRow &t) {
+    const int chunk = blockIdx.x % d.caps.straddle_chunks;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned *count = d.caps.straddle_count + (long long)b * d.caps.straddle_chunks;
+    const unsigned long long quota = d.caps.quota[b];
+    __shared__ unsigned long long before;
+    if (threadIdx.x == 0) before = 0ull;
+    __syncthreads();
+    unsigned long long n = 0;
+    for (int k = threadIdx.x; k < chunk; k += kStraddleCols) n += count[k];
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    if (lane == 0 && n) atomicAdd(&before, n);
+    __syncthreads();
+    if (before >= quota) return;
+    const unsigned *bits = d.caps.straddle_bits +
+                           ((long long)b * d.caps.straddle_chunks + chunk) * (kStraddleCols / 32);
+    unsigned long long rank = before;
+    for (int k = 0; k < w; k++) rank += __popc(bits[k]);
+    rank += __popc(bits[w] & ((1u << lane) - 1u));
+    if (!((bits[w] >> lane) & 1u) || rank >= quota) return;
+    Chain c;
+    int slot;
+    if (!cut_pair<MIXED>(d, b, t, (long long)chunk * kStraddleCols + threadIdx.x, c, slot)) return;
+    if (b >= d.g.n_slots) {
+        if (MIXED)
+            bin_den_qinv(d, c);
+        else
+            bin_num_qinv(d, c);
+    } else {
+        if (MIXED)
+            bin_den3(d, slot, c.bin);
+        else
+            bin_num3(d, slot, c.bin, c);
+    }
+}
+
+// One launch's cut rows (a block for each stream bin's chunk of columns).
+template <bool MIXED, bool ADMIT>
+__global__ void __launch_bounds__(kStraddleCols) k_straddle(Device d, long long rows,
+                                                            long long cols, Cols8 a8, Cols4 b4) {
+    const int b = blockIdx.x / d.caps.straddle_chunks;
+    CutRow t;
+    if (!cut_row<MIXED>(d, b, rows, cols, a8.p, b4.p, t)) return;
+    if (ADMIT)
+        straddle_admit<MIXED>(d, b, t);
+    else
+        straddle_mark<MIXED>(d, b, t);
+}
+
+// The cut rows of several mixed-event jobs admitted together.
+template <bool ADMIT>
+__global__ void __launch_bounds__(kStraddleCols) k_straddle_jobs(Device d, const StraddleJob *jobs,
+                                                                 int n_jobs, long long rows) {
+    const int b = blockIdx.x / d.caps.straddle_chunks;
+    CutRow t;
+    if (!cut_row_jobs(d, b, jobs, n_jobs, rows, t)) return;
+    if (ADMIT)
+        straddle_admit<true>(d, b, t);
+    else
+        straddle_mark<true>(d, b, t);
 }
 
 // Per stream bin: first row at which the running survivor count exceeds
@@ -341,7 +396,11 @@ cudaError_t launch_mixed(const Device &d, int mode, long long n1, const double *
 
 cudaError_t launch_same_straddle(const Device &d, long long n, const double *const *c8,
                                  int n_stream, cudaStream_t st) {
-    k_straddle<false><<<n_stream, 32, 0, st>>>(d, n, n, cols8(c8), cols4(nullptr));
+    const long long grid = (long long)d.caps.straddle_chunks * n_stream;
+    if (grid < 1) return cudaSuccess;
+    if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
+    k_straddle<false, false><<<(unsigned)grid, kStraddleCols, 0, st>>>(d, n, n, cols8(c8), cols4(nullptr));
+    k_straddle<false, true><<<(unsigned)grid, kStraddleCols, 0, st>>>(d, n, n, cols8(c8), cols4(nullptr));
     return cudaGetLastError();
 }
 
@@ -350,14 +409,22 @@ cudaError_t launch_mixed_straddle(const Device &d, long long n1, const double *c
                                   cudaStream_t st) {
     Cols8 a;
     for (int f = 0; f < 8; f++) a.p[f] = f < 4 ? l1[f] : nullptr;
-    k_straddle<true><<<n_stream, 32, 0, st>>>(d, n1, n2, a, cols4(l2));
+    const long long grid = (long long)d.caps.straddle_chunks * n_stream;
+    if (grid < 1) return cudaSuccess;
+    if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
+    k_straddle<true, false><<<(unsigned)grid, kStraddleCols, 0, st>>>(d, n1, n2, a, cols4(l2));
+    k_straddle<true, true><<<(unsigned)grid, kStraddleCols, 0, st>>>(d, n1, n2, a, cols4(l2));
     return cudaGetLastError();
 }
 
 cudaError_t launch_jobs_straddle(const Device &d, const StraddleJob *jobs, int n_jobs,
                                  long long rows, int n_stream, cudaStream_t st) {
     if (n_jobs < 1) return cudaSuccess;
-    k_straddle_jobs<<<n_stream, 32, 0, st>>>(d, jobs, n_jobs, rows);
+    const long long grid = (long long)d.caps.straddle_chunks * n_stream;
+    if (grid < 1) return cudaSuccess;
+    if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
+    k_straddle_jobs<false><<<(unsigned)grid, kStraddleCols, 0, st>>>(d, jobs, n_jobs, rows);
+    k_straddle_jobs<true><<<(unsigned)grid, kStraddleCols, 0, st>>>(d, jobs, n_jobs, rows);
     return cudaGetLastError();
 }
 
