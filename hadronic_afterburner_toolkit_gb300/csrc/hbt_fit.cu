@@ -4,29 +4,31 @@
 // table and one q_cut at a time (ebe_scripts/fit_HBT_radii.py:60-92).  Here
 // all fits of a batch of tables advance together:
 //
-//  * k_fit_select (one CTA per table) applies the script's preprocessing
-//    (numpy nan_to_num, C_err + 1e-15, weight 1 / sigma) and keeps the rows
-//    with q_cut_min < |q| < the largest cut, ordered by the smallest cut
-//    they pass, so the rows of cut k are a prefix of the table's kept rows.
-//    Per row it stores the five q products of the exponent (FP64 and FP32),
-//    C and the weight.
-//  * Each fit's rows are cut into work items of up to 8192 rows.  A pass
-//    (k_fit_pass, one CTA per item) sums chi^2, J^T r and J^T J of every
-//    active fit's items at its trial point; a step (k_fit_step, one thread
-//    per fit) adds its items' sums and makes one Levenberg-Marquardt step:
-//    damped 6 x 6 system by Cholesky, accept or reject, next trial point.
-//    Passes and steps alternate until no fit has a trial point; work is
-//    balanced over the GPU whatever the fits' sizes, and finished fits cost
-//    nothing in later passes.
+//  * k_fit_count and k_fit_select (a block for each 4096 rows of a table)
+//    apply the script's preprocessing (numpy nan_to_num, C_err + 1e-15, weight
+//    1 / sigma) and keep the rows with q_cut_min < |q| < the largest cut,
+//    ordered by the smallest cut they pass, so the rows of cut k are a prefix
+//    of the table's kept rows.  Per row they store the five q products of the
+//    exponent (FP64 and FP32), C and the weight.
+//  * Each fit's rows are cut into work items of up to 8192 rows, four units
+//    each.  A pass (k_fit_pass, a block per unit) sums chi^2, J^T r and J^T J
+//    of every active fit's units at its trial point; the block that finishes a
+//    fit's last unit adds them and makes one Levenberg-Marquardt step: damped
+//    6 x 6 system by Cholesky, accept or reject, next trial point.  Passes
+//    repeat until no fit has a trial point; work is balanced over the GPU
+//    whatever the fits' sizes, and finished fits are passed over.
 //  * A last pass sums J^T J in FP64 at each minimum; k_fit_finish inverts
 //    it for the errors sqrt(diag((J^T J)^-1)) (curve_fit, absolute_sigma).
 //
-// A pass reads 76 bytes per row against about 35 FP64 operations (exp
-// table-driven, hbt_math.cuh): the fits are bound by the FP64 pipe.
+// A pass reads 76 bytes per row against 32 FP64 operations (exp table-driven,
+// hbt_math.cuh): the fits are bound by the FP64 pipe.  The order in which a
+// fit's rows are added is fixed (lane, unit, item), so a fit's result does not
+// depend on the other fits of the call.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -40,8 +42,16 @@ constexpr double kHbarC = 0.19733;  // fit_HBT_radii.py:10
 constexpr double kEps = 1e-15;      // fit_HBT_radii.py:11
 constexpr int kMaxCuts = 16;
 constexpr int kSelThreads = 512;
+constexpr int kSelRows = 4096;  // a selection block's rows
 constexpr int kFitThreads = 128;
 constexpr int kSums = 28;  // chi2, J^T r (6), J^T J (21, packed lower)
+// A work item: up to kItemRows consecutive kept rows of one fit, in kItemUnits
+// units of 32 lanes: lane l of unit w takes every kItemStride-th row from
+// 32 w + l on.
+constexpr int kItemRows = 8192;
+constexpr int kItemUnits = 4;
+constexpr int kItemStride = 32 * kItemUnits;
+constexpr int kItemWarps = kFitThreads / 32;  // warps to a unit
 
 // Resident pass CTAs per SM the pass kernel is compiled for.
 #ifndef HBT_FIT_MIN_BLOCKS
@@ -50,6 +60,9 @@ constexpr int kSums = 28;  // chi2, J^T r (6), J^T J (21, packed lower)
 
 struct FitConst {
     double cut_sorted[kMaxCuts];  // ascending
+    // the cuts on |q|^2 as bits of doubles: sqrt(s) < cut_sorted[c] exactly
+    // when s < cut_sq[c], sqrt(s) > q_cut_min exactly when s > min_sq
+    long long cut_sq[kMaxCuts], min_sq;
     int rank[kMaxCuts];           // position of cut k in cut_sorted
     int by_rank[kMaxCuts];        // the cut at position s of cut_sorted
     int n_cuts;
@@ -80,33 +93,77 @@ struct Rows {
 constexpr int kColC = 5, kColW = 6;
 
 __device__ __forceinline__ double nan_to_num(double v) {
-    if (isnan(v)) return 0.0;
-    if (isinf(v)) return v > 0 ? DBL_MAX : -DBL_MAX;
-    return v;
+    const int hi = __double2hiint(v);
+    if ((hi & 0x7ff00000) != 0x7ff00000) return v;
+    if ((hi & 0xfffff) | __double2loint(v)) return 0.0;
+    return hi > 0 ? DBL_MAX : -DBL_MAX;
 }
 
-// numpy's sqrt(q_out**2. + q_side**2. + q_long**2.), without contraction.
-__device__ __forceinline__ double qabs(double qo, double qs, double ql) {
-    return sqrt(__dadd_rn(__dadd_rn(__dmul_rn(qo, qo), __dmul_rn(qs, qs)), __dmul_rn(ql, ql)));
-}
-
-__device__ __forceinline__ int cut_class(const FitConst &fc, double r) {
-    if (!(r > fc.q_cut_min)) return -1;
+// The smallest cut that |q| = sqrt(q_out**2. + q_side**2. + q_long**2.)
+// passes (numpy's sum, without contraction), -1 for none.  The cuts are
+// compared on the sum itself, as integers (it is never negative or NaN).
+__device__ __forceinline__ int cut_class(const FitConst &fc, double qo, double qs, double ql) {
+    const long long s = __double_as_longlong(
+        __dadd_rn(__dadd_rn(__dmul_rn(qo, qo), __dmul_rn(qs, qs)), __dmul_rn(ql, ql)));
+    if (!(s > fc.min_sq)) return -1;
     for (int c = 0; c < fc.n_cuts; c++)
-        if (r < fc.cut_sorted[c]) return c;
+        if (s < fc.cut_sq[c]) return c;
     return -1;
 }
 
-// Two sweeps over a table's rows: the first counts the rows of each cut
-// class (the smallest cut a row passes, or none), the second writes every
-// kept row at its class's running position: within a class, rows keep
-// their table order (the same arrays and sums on every run).
+// A selection block's rows: part p of table t.
+struct SelPart {
+    int t, p;
+};
+
+// Row selection, sweep 1: the rows of each cut class (the smallest cut a row
+// passes) in each part of kSelRows rows, part_cls[block][c].
+//
+// Both sweeps read 24 or 40 bytes a row against the few FP64 operations of
+// |q|^2; with one block for a whole table and square roots in FP64 they took
+// 1.59 ms for 64 tables of 41^3 rows (64 of 152 SMs), now 65 + 190 us.
+__global__ void __launch_bounds__(kSelThreads)
+    k_fit_count(FitConst fc, const long long *tab_off, const TabDesc *desc, const double *in,
+                const SelPart *parts, int *part_cls) {
+    __shared__ int cnt[kMaxCuts];
+    const SelPart P = parts[blockIdx.x];
+    const TabDesc d = desc[P.t];
+    const long long i0 = (long long)P.p * kSelRows;
+    const long long i1 = min(i0 + kSelRows, tab_off[P.t + 1] - tab_off[P.t]);
+    const double *qo_in = in + d.base + d.col[0], *qs_in = in + d.base + d.col[1],
+                 *ql_in = in + d.base + d.col[2];
+    if (threadIdx.x < kMaxCuts) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    int mine[kMaxCuts];
+#pragma unroll
+    for (int c = 0; c < kMaxCuts; c++) mine[c] = 0;
+    for (long long i = i0 + threadIdx.x; i < i1; i += kSelThreads) {
+        const int c = cut_class(fc, nan_to_num(qo_in[i * d.stride]), nan_to_num(qs_in[i * d.stride]),
+                                nan_to_num(ql_in[i * d.stride]));
+#pragma unroll
+        for (int k = 0; k < kMaxCuts; k++) mine[k] += (c == k);
+    }
+#pragma unroll
+    for (int k = 0; k < kMaxCuts; k++) {
+        if (k >= fc.n_cuts) break;
+        const int v = __reduce_add_sync(0xffffffffu, mine[k]);
+        if ((threadIdx.x & 31) == 0 && v) atomicAdd(&cnt[k], v);
+    }
+    __syncthreads();
+    if (threadIdx.x < fc.n_cuts)
+        part_cls[(long long)blockIdx.x * fc.n_cuts + threadIdx.x] = cnt[threadIdx.x];
+}
+
+// Sweep 2 writes every kept row at its class's running position: within a
+// class, rows keep their table order (the same arrays and sums on every run).
+// first[t] is table t's first part; part 0 leaves the table's class counts.
 __global__ void __launch_bounds__(kSelThreads)
     k_fit_select(FitConst fc, const long long *tab_off, const TabDesc *desc, const double *in,
-                 Rows out, int *cls) {
+                 const SelPart *parts, const int *first, const int *part_cls, Rows out, int *cls) {
     __shared__ int cnt[kSelThreads / 32][kMaxCuts];
-    __shared__ int base[kMaxCuts];
-    const int t = blockIdx.x;
+    __shared__ int base[kMaxCuts], total[kMaxCuts];
+    const SelPart P = parts[blockIdx.x];
+    const int t = P.t;
     const long long r0 = tab_off[t], n = tab_off[t + 1] - r0;
     const TabDesc d = desc[t];
     const double *qo_in = in + d.base + d.col[0], *qs_in = in + d.base + d.col[1],
@@ -114,47 +171,43 @@ __global__ void __launch_bounds__(kSelThreads)
                  *e_in = in + d.base + d.col[4];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nc = fc.n_cuts;
     const unsigned below = (1u << lane) - 1u;
-    // sweep 1: rows per class (per-thread counters, then the block's sums)
-    int mine[kMaxCuts];
-#pragma unroll
-    for (int c = 0; c < kMaxCuts; c++) mine[c] = 0;
-    for (long long i = threadIdx.x; i < n; i += kSelThreads) {
-        const int c = cut_class(fc, qabs(nan_to_num(qo_in[i * d.stride]),
-                                         nan_to_num(qs_in[i * d.stride]),
-                                         nan_to_num(ql_in[i * d.stride])));
-#pragma unroll
-        for (int k = 0; k < kMaxCuts; k++) mine[k] += (c == k);
-    }
-#pragma unroll
-    for (int k = 0; k < kMaxCuts; k++) {
-        if (k >= nc) break;
-        int v = mine[k];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) cnt[warp][k] = v;
+    // a class's rows in the parts before this one and in the whole table
+    for (int c = warp; c < nc; c += kSelThreads / 32) {
+        int before = 0, all = 0;
+        for (int b = first[t] + lane; b < first[t + 1]; b += 32) {
+            const int v = part_cls[(long long)b * nc + c];
+            all += v;
+            if (b < (int)blockIdx.x) before += v;
+        }
+        before = __reduce_add_sync(0xffffffffu, before);
+        all = __reduce_add_sync(0xffffffffu, all);
+        if (lane == 0) {
+            base[c] = before;
+            total[c] = all;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         int run = 0;
-        for (int k = 0; k < nc; k++) {
-            int tot = 0;
-            for (int w = 0; w < kSelThreads / 32; w++) tot += cnt[w][k];
-            base[k] = run;
-            cls[t * (nc + 1) + k] = tot;
-            run += tot;
+        for (int c = 0; c < nc; c++) {
+            base[c] += run;
+            run += total[c];
+            if (P.p == 0) cls[t * (nc + 1) + c] = total[c];
         }
-        cls[t * (nc + 1) + nc] = run;
+        if (P.p == 0) cls[t * (nc + 1) + nc] = run;
     }
     __syncthreads();
-    // sweep 2: chunk by chunk, rank each row among its class in row order
-    for (long long i0 = 0; i0 < n; i0 += kSelThreads) {
+    // chunk by chunk, rank each row among its class in row order
+    const long long i1 = min(((long long)P.p + 1) * kSelRows, n);
+    for (long long i0 = (long long)P.p * kSelRows; i0 < i1; i0 += kSelThreads) {
         const long long i = i0 + threadIdx.x;
         double qo = 0, qs = 0, ql = 0;
         int c = -1;
-        if (i < n) {
+        if (i < i1) {
             qo = nan_to_num(qo_in[i * d.stride]);
             qs = nan_to_num(qs_in[i * d.stride]);
             ql = nan_to_num(ql_in[i * d.stride]);
-            c = cut_class(fc, qabs(qo, qs, ql));
+            c = cut_class(fc, qo, qs, ql);
         }
         // this warp's rows per class: zeroed, then each class group's first
         // lane writes the group's size
@@ -187,100 +240,200 @@ __global__ void __launch_bounds__(kSelThreads)
     }
 }
 
-// One pass at parameters p: chi^2, J^T r, J^T J of the rows [0, n) of the
-// fit, reduced over the block into red[0..27] (valid in thread 0).
+// Sums each of v[0..7] over the warp's lanes: every halving exchanges the half
+// a lane gives up, 9 adds instead of 5 for each value (and the same pairs as
+// the tree of one value, so the same result).  Lane l returns sum l / 4.
+__device__ __forceinline__ double warp_sums(double (&v)[8]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int h = 4, o = 16; h >= 1; h /= 2, o /= 2) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < h; i++) {
+            const double give = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    return v[0];
+}
+
+__device__ __forceinline__ double fma_rn(double a, double b, double c) {
+    return __fma_rn(a, b, c);
+}
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
+// A step's row of one lane, as the columns give it.
+struct RowIn {
+    double q[5], w, c;
+    float f[5];
+};
+__device__ __forceinline__ void load_row(const Rows &rw, long long o, bool in, RowIn &x) {
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        x.q[k] = in ? rw.d[k * rw.ld + o] : 0.0;
+        x.f[k] = in ? rw.f[k * rw.ld + o] : 0.f;
+    }
+    x.w = in ? rw.d[kColW * rw.ld + o] : 0.0;
+    x.c = in ? rw.d[kColC * rw.ld + o] : 0.0;
+}
+
+// The steps of a batch in shared memory: v[0..5], r, and the FP32 J.
+constexpr int kBatchSteps = 8;
+struct StepBuf {
+    double v[kBatchSteps][7][32];
+    float j[kBatchSteps][6][32];
+};
+
+// The chains of warp G of a pass's block: s and sa by number.
+template <int G>
+struct Chains {
+    static constexpr int s0 = 2 * G, ns = G == 3 ? 1 : 2;   // of chi^2, J^T r
+    static constexpr int a0 = 5 * G, na = G == 3 ? 6 : 5;   // of J^T J
+};
+// J^T J's element m is the product of columns col_j(m) and col_k(m).
+__host__ __device__ constexpr int col_j(int m) {
+    int j = 0;
+    while ((j + 1) * (j + 2) / 2 <= m) j++;
+    return j;
+}
+__host__ __device__ constexpr int col_k(int m) { return m - col_j(m) * (col_j(m) + 1) / 2; }
+
+template <int G, class AccT>
+__device__ __forceinline__ void add_steps(const StepBuf &b, int lane, double (&s)[2],
+                                          AccT (&sa)[6]) {
+    using C = Chains<G>;
+#pragma unroll
+    for (int t = 0; t < kBatchSteps; t++) {
+        const double r = b.v[t][6][lane];
+#pragma unroll
+        for (int k = 0; k < C::ns; k++) {
+            const int n = C::s0 + k;
+            s[k] = __fma_rn(n == 0 ? r : b.v[t][n == 0 ? 6 : n - 1][lane], r, s[k]);
+        }
+        AccT v[6];
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            if constexpr (std::is_same<AccT, double>::value)
+                v[k] = b.v[t][k][lane];
+            else
+                v[k] = b.j[t][k][lane];
+        }
+#pragma unroll
+        for (int k = 0; k < C::na; k++) {
+            sa[k] = fma_rn(v[col_j(C::a0 + k)], v[col_k(C::a0 + k)], sa[k]);
+        }
+    }
+}
+
+// A trial point's constants: lambda, a_k^2 and the factors of the 28 sums.
+struct PassConst {
+    double lam, a2[5], factor[kSums];
+};
+
+// A warp's chains summed over its lanes, with J's constant factors: lane 4 k
+// leaves its sum k.
+template <int G, class AccT>
+__device__ __forceinline__ void store_chains(const double (&s)[2], const AccT (&sa)[6],
+                                             const PassConst &pc, double *out) {
+    using C = Chains<G>;
+    double tot[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < C::ns; k++) tot[k] = C::s0 + k == 0 ? s[k] : s[k] * pc.factor[C::s0 + k];
+#pragma unroll
+    for (int k = 0; k < C::na; k++) tot[C::ns + k] = (double)sa[k] * pc.factor[7 + C::a0 + k];
+    const double x = warp_sums(tot);
+    const int lane = threadIdx.x & 31, k = lane >> 2;
+    if ((lane & 3) == 0 && k < C::ns + C::na)
+        __stcg(out + (k < C::ns ? C::s0 + k : 7 + C::a0 + k - C::ns), x);
+}
+
+#define FIT_BY_WARP(g, call)      \
+    switch (g) {                  \
+        case 0: call(0); break;   \
+        case 1: call(1); break;   \
+        case 2: call(2); break;   \
+        default: call(3); break;  \
+    }
+
+// One pass at parameters p: chi^2, J^T r, J^T J of the rows first, first +
+// kItemStride, ... below n of an item, for 32 neighbouring `first` (a unit)
+// by the block, to out[0..27].
 // Residual r = w (f - C), J = w df/dp with f = lambda exp(-E),
 // E = sum_k a_k^2 Q_k over the five q products Q_k (a_k = R_k / hbar c), so
 // J_0 = w e and J_k = -w f (2 a_k / hbar c) Q_k: the constant factors
 // 2 a_k / hbar c are applied after the sums.  chi^2 and J^T r, which fix
 // where the minimum is, are summed in FP64.  J^T J only shapes the steps
-// while iterating (kExact = false: FP32 products and per-thread sums over
-// at most a few hundred rows, 1e-5 relative); the pass at the minimum that
-// gives the covariance sums it in FP64 (kExact = true).
+// while iterating (kExact = false: FP32 products and sums over a lane's at
+// most 64 rows, 1e-5 relative); the pass at the minimum that gives the
+// covariance sums it in FP64 (kExact = true).
+//
+// A lane's rows add up in row order.  The block's four warps evaluate two
+// steps each of eight (a step: one row a lane), then each adds the eight
+// steps to its share of the 28 sums: an SM sub-partition gives one FP64 warp
+// instruction in 64 clocks, so one warp alone needs 150 us for the 64 steps of
+// a full unit, however few fits are still active, and four of them a quarter.
 template <bool kExact>
-__device__ void fit_pass(const Rows &rw, long long r0, int n, const double *p, const double *etab,
-                         double *red) {
+__device__ __forceinline__ void fit_unit(const Rows &rw, long long r0, int first, int n,
+                                         const PassConst &pc, const double *etab, StepBuf *buf,
+                                         double *out) {
     using AccT = typename std::conditional<kExact, double, float>::type;
-    __shared__ double part[kFitThreads / 32][kSums];
-    double a2[5], cdf[7];
-    cdf[0] = 1.0;
-    for (int k = 0; k < 5; k++) {
-        const double a = p[k + 1] / kHbarC;
-        a2[k] = a * a;
-        cdf[k + 1] = -2.0 * a / kHbarC;
-    }
-    const double lam = p[0];
-    double s[7];
-    AccT sa[21];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    double a2[5];
 #pragma unroll
-    for (int k = 0; k < 7; k++) s[k] = 0.0;
+    for (int k = 0; k < 5; k++) a2[k] = pc.a2[k];
+    const double lam = pc.lam;
+    double s[2] = {0.0, 0.0};
+    AccT sa[6] = {0, 0, 0, 0, 0, 0};
+    constexpr int kMine = kBatchSteps / kItemWarps;  // steps of a warp in a batch
+    RowIn x[kMine];
+    auto load = [&](int b) {
 #pragma unroll
-    for (int k = 0; k < 21; k++) sa[k] = 0;
-    for (int i = threadIdx.x; i < n; i += kFitThreads) {
-        const long long o = r0 + i;
-        const double *dp = rw.d + o;
-        double q[5];
-#pragma unroll
-        for (int k = 0; k < 5; k++) q[k] = dp[k * rw.ld];
-        const double w = dp[kColW * rw.ld];
-        double E = 0.0;
-#pragma unroll
-        for (int k = 0; k < 5; k++) E += a2[k] * q[k];
-        const double e = table_exp(etab, -E);
-        const double f = lam * e;
-        const double r = w * (f - dp[kColC * rw.ld]);
-        const double u = w * f;
-        double v[6];  // J without its constant factors
-        v[0] = w * e;
-#pragma unroll
-        for (int k = 0; k < 5; k++) v[k + 1] = u * q[k];
-        s[0] += r * r;
-#pragma unroll
-        for (int k = 0; k < 6; k++) s[1 + k] += v[k] * r;
-        AccT va[6];
-        if (kExact) {
-#pragma unroll
-            for (int k = 0; k < 6; k++) va[k] = (AccT)v[k];
-        } else {
-            const float uf = (float)u;
-            va[0] = (AccT)v[0];
-#pragma unroll
-            for (int k = 0; k < 5; k++) va[k + 1] = (AccT)(uf * rw.f[k * rw.ld + o]);
+        for (int m = 0; m < kMine; m++) {
+            const int i = first + lane + (b + g * kMine + m) * kItemStride;
+            load_row(rw, r0 + i, i < n, x[m]);
         }
-        int m = 0;
+    };
+    load(0);
+    for (int b = 0, at = 0; first + b * kItemStride < n; b += kBatchSteps, at ^= 1) {
+        StepBuf &sb = buf[at];
 #pragma unroll
-        for (int j = 0; j < 6; j++)
+        for (int m = 0; m < kMine; m++) {
+            const int t = g * kMine + m;
+            const RowIn &y = x[m];
+            double E = 0.0;
 #pragma unroll
-            for (int k = 0; k <= j; k++) sa[m++] += va[j] * va[k];
+            for (int k = 0; k < 5; k++) E = __fma_rn(a2[k], y.q[k], E);
+            const double e = table_exp(etab, -E);
+            const double f = lam * e;
+            // a lane past the item's end adds zeros
+            const bool in = first + lane + (b + t) * kItemStride < n;
+            const double r = in ? __dmul_rn(y.w, __dsub_rn(f, y.c)) : 0.0;
+            const double u = in ? y.w * f : 0.0;
+            const double v0 = in ? y.w * e : 0.0;
+            sb.v[t][0][lane] = v0;
+#pragma unroll
+            for (int k = 0; k < 5; k++) sb.v[t][k + 1][lane] = u * y.q[k];
+            sb.v[t][6][lane] = r;
+            if (!kExact) {
+                const float uf = to_float_rn(u);
+                sb.j[t][0][lane] = to_float_rn(v0);
+#pragma unroll
+                for (int k = 0; k < 5; k++) sb.j[t][k + 1][lane] = uf * y.f[k];
+            }
+        }
+        load(b + kBatchSteps);
+        __syncthreads();
+#define FIT_ADD(G) add_steps<G>(sb, lane, s, sa)
+        FIT_BY_WARP(g, FIT_ADD)
+#undef FIT_ADD
     }
-    double tot[kSums];
-    tot[0] = s[0];
-#pragma unroll
-    for (int k = 0; k < 6; k++) tot[1 + k] = s[1 + k] * cdf[k];
-    {
-        int m = 0;
-#pragma unroll
-        for (int j = 0; j < 6; j++)
-#pragma unroll
-            for (int k = 0; k <= j; k++, m++) tot[7 + m] = (double)sa[m] * (cdf[j] * cdf[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < kSums; k++) {
-        double x = tot[k];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        tot[k] = x;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0)
-        for (int k = 0; k < kSums; k++) part[warp][k] = tot[k];
-    __syncthreads();
-    if (threadIdx.x < kSums) {
-        double x = 0.0;
-        for (int w = 0; w < kFitThreads / 32; w++) x += part[w][threadIdx.x];
-        red[threadIdx.x] = x;
-    }
-    __syncthreads();
+#define FIT_STORE(G) store_chains<G>(s, sa, pc, out)
+    FIT_BY_WARP(g, FIT_STORE)
+#undef FIT_STORE
 }
+#undef FIT_BY_WARP
 
 // Cholesky of the packed symmetric 6 x 6 matrix M (lower, row-major
 // packed: M[j(j+1)/2 + k], k <= j) in place; false if not positive definite.
@@ -316,12 +469,13 @@ __device__ void chol_solve6(const double *L, const double *b, double *x) {
 }
 
 // Levenberg-Marquardt state of one fit, in device memory, advanced by one
-// thread (k_fit_step) between the passes over the fit's rows.
+// thread of the block that finishes the fit's last unit of a pass, between the passes over the fit's rows.
 struct LmState {
     double x[6], trial[6];
     double S, g[6], A[21], D[6], mu, nu;
     int iter, status, stop, go;
     int use_x;  // the next pass evaluates x (the start point), not trial
+    int done;   // units finished in the current pass
     long long passes;
 };
 
@@ -420,17 +574,24 @@ struct FitInfo {
     int t, k, n, item0, item1;
 };
 
-// A work item: up to kItemRows consecutive kept rows of one fit.
+// A work item's fit, rows and place: unit w's sums are at
+// partial[(kItemUnits slot + w) * kSums].
 struct FitItem {
-    int fit, rows;
+    int fit, rows, slot, pad;
     long long row0;
 };
-constexpr int kItemRows = 8192;
+
+// Per pass of a check interval: the next (item, unit) to take, and whether any fit
+// has another trial point.
+struct PassCtl {
+    int next, active;
+};
 
 __global__ void k_fit_init(FitConst fc, const FitInfo *fits, int n_fits, LmState *st) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= n_fits) return;
     LmState &s = st[f];
+    s.done = 0;
     for (int j = 0; j < 6; j++) s.x[j] = s.trial[j] = fc.p0[j];
     s.use_x = 1;
     s.iter = 0;
@@ -442,97 +603,161 @@ __global__ void k_fit_init(FitConst fc, const FitInfo *fits, int n_fits, LmState
     s.status = enough ? HBT_FIT_CONVERGED : HBT_FIT_TOO_FEW;
 }
 
-// One pass over every active fit's rows: each item's chi^2, J^T r and
-// J^T J (at the fit's trial point, its start point on the first pass, or
-// with kExact at its minimum for the covariance) into partial[item].
-// Items of finished fits return at once.
+// Sum k of a fit: its items' units' partials in order.  They come from other
+// SMs: read past L1.
+__device__ __forceinline__ double fit_sum(const FitInfo &fi, const double *partial, int k) {
+    double x = 0.0;
+    for (int it = fi.item0; it < fi.item1; it++) {
+        double y = 0.0;
+#pragma unroll
+        for (int w = 0; w < kItemUnits; w++)
+            y += __ldcg(partial + ((long long)it * kItemUnits + w) * kSums + k);
+        x += y;
+    }
+    return x;
+}
+
+// One pass over every active fit's rows: the chi^2, J^T r and J^T J of each
+// item's units (at the fit's trial point, its start point on the first pass,
+// or with kExact at its minimum for the covariance) into `partial`.
+// Blocks take units in turn, the largest first; finished fits' are skipped.
+// The block that finishes a fit's last unit of an iterating pass makes its
+// Levenberg-Marquardt step, so the fit's state only changes once all its units
+// of the pass are done; `active` is set while any fit has another trial point.
+//
+// Bound by the FP64 pipe (2 lanes a clock and SM): 32 operations a row, 36
+// issued with a unit's constants and reduction, the conversions by the integer
+// pipe.  The first pass over 64 tables of 41^3 rows, five cuts: 349 us, FP64
+// pipe 82 % busy (474 us as a block per item with 39 operations a row); a late
+// pass with few active fits 110 us (180 us with a warp per unit); over four
+// tables 52 us (168 us).
 template <bool kExact>
 __global__ void __launch_bounds__(kFitThreads, HBT_FIT_MIN_BLOCKS)
-    k_fit_pass(const FitItem *items, int n_items, Rows rw, const LmState *st, double *partial) {
+    k_fit_pass(FitConst fc, const FitItem *items, int n_items, Rows rw, const FitInfo *fits,
+               LmState *st, double *partial, PassCtl *ctl) {
     __shared__ double etab[EXP_TABLE];
+    __shared__ StepBuf buf[2];
     __shared__ double red[kSums];
-    __shared__ double p[6];
+    __shared__ PassConst pc;
+    __shared__ int next, last;
+    const int n_units = n_items * kItemUnits;
+    // warp 0 takes the next active unit; units of finished fits are passed
+    // over up to 32 at a time
+    auto take = [&] {
+        const int lane = threadIdx.x;
+        int u = 0;
+        while (true) {
+            if (lane == 0) u = atomicAdd(&ctl->next, 1);
+            u = __shfl_sync(0xffffffffu, u, 0);
+            if (u >= n_units) break;
+            bool on = true;  // past the last unit: nothing to pass over
+            if (u + lane < n_units) {
+                const LmState &s = st[items[(u + lane) / kItemUnits].fit];
+                on = kExact ? s.status != HBT_FIT_TOO_FEW : s.go;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, on);
+            if (m & 1u) break;
+            if (lane == 0) atomicMax(&ctl->next, u + (m ? __ffs(m) - 1 : 32));
+        }
+        if (lane == 0) next = u;
+    };
+    if (threadIdx.x < 32) take();
     fill_exp_table(etab);
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-        const FitItem I = items[it];
-        const LmState &s = st[I.fit];
-        if (kExact ? s.status == HBT_FIT_TOO_FEW : !s.go) continue;  // uniform in the block
-        __syncthreads();  // the previous item's p and red are read
-        if (threadIdx.x < 6) p[threadIdx.x] = (kExact || s.use_x) ? s.x[threadIdx.x] : s.trial[threadIdx.x];
+    __syncthreads();
+    while (next < n_units) {
+        const FitItem I = items[next / kItemUnits];
+        const int w = next % kItemUnits;
+        LmState &s = st[I.fit];
+        if (threadIdx.x < 32) {
+            // lane k forms parameter k's constants, lane k the factor of sum k:
+            // 1 + j carries J's column j, 7 + m the columns of element m
+            const int k = threadIdx.x;
+            const double pk = k < 6 ? ((kExact || s.use_x) ? s.x[k] : s.trial[k]) : 0.0;
+            const double a = pk / kHbarC;
+            const double cdf = k ? -2.0 * a / kHbarC : 1.0;
+            if (k == 0) pc.lam = pk;
+            if (k >= 1 && k < 6) pc.a2[k - 1] = a * a;
+            int j = 0;
+            while (k >= 7 && (j + 1) * (j + 2) / 2 <= k - 7) j++;
+            const int l = k >= 7 ? k - 7 - j * (j + 1) / 2 : 0;
+            const double cj = __shfl_sync(0xffffffffu, cdf, k >= 7 ? j : max(k - 1, 0));
+            const double cl = __shfl_sync(0xffffffffu, cdf, l);
+            if (k < kSums) pc.factor[k] = k >= 7 ? cj * cl : cj;
+        }
         __syncthreads();
-        fit_pass<kExact>(rw, I.row0, I.rows, p, etab, red);
-        if (threadIdx.x < kSums) partial[(long long)it * kSums + threadIdx.x] = red[threadIdx.x];
+        fit_unit<kExact>(rw, I.row0, 32 * w, I.rows, pc, etab, buf,
+                         partial + ((long long)I.slot * kItemUnits + w) * kSums);
+        __threadfence();
+        __syncthreads();
+        if (!kExact) {
+            const FitInfo fi = fits[I.fit];
+            if (threadIdx.x == 0)
+                last = atomicAdd(&s.done, 1) == (fi.item1 - fi.item0) * kItemUnits - 1;
+            __syncthreads();
+            if (last) {
+                __threadfence();
+                if (threadIdx.x < kSums) red[threadIdx.x] = fit_sum(fi, partial, threadIdx.x);
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    s.done = 0;
+                    if (s.use_x) {
+                        lm_init(s, red);
+                        s.use_x = 0;
+                    } else {
+                        lm_update(s, red);
+                    }
+                    lm_propose(s, fc.max_iter);
+                    if (s.go) atomicOr(&ctl->active, 1);
+                }
+            }
+        }
+        if (threadIdx.x < 32) take();
+        __syncthreads();
     }
-}
-
-// The fit's sums: its items' partials added in item order.
-__device__ __forceinline__ void fit_sums(const FitInfo &fi, const double *partial, double *red) {
-    for (int k = 0; k < kSums; k++) red[k] = 0.0;
-    for (int it = fi.item0; it < fi.item1; it++)
-        for (int k = 0; k < kSums; k++) red[k] += partial[(long long)it * kSums + k];
-}
-
-// One Levenberg-Marquardt step of every active fit (one thread per fit);
-// `active` is set while any fit has another trial point.
-__global__ void k_fit_step(FitConst fc, const FitInfo *fits, int n_fits, LmState *st,
-                           const double *partial, int *active) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= n_fits) return;
-    LmState &s = st[f];
-    if (!s.go) return;
-    double red[kSums];
-    fit_sums(fits[f], partial, red);
-    if (s.use_x) {
-        lm_init(s, red);
-        s.use_x = 0;
-    } else {
-        lm_update(s, red);
-    }
-    lm_propose(s, fc.max_iter);
-    if (s.go) atomicOr(active, 1);
 }
 
 // Results: the point, chi^2, the errors sqrt(diag((J^T J)^-1)) from the
 // exact pass at the minimum (inf and the singular status when J^T J is not
-// positive definite), rows, iterations, status.
-__global__ void k_fit_finish(FitConst fc, int first_table, const FitInfo *fits, int n_fits,
+// positive definite), rows, iterations, status.  One warp per fit: a lane per
+// sum, then a lane per column of the inverse.
+__global__ void __launch_bounds__(32) k_fit_finish(FitConst fc, int first_table, const FitInfo *fits, int n_fits,
                              const LmState *st, const double *partial, hbt_fit_result *res,
                              unsigned long long *n_passes) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    const int f = blockIdx.x, j = threadIdx.x;
     if (f >= n_fits) return;
     const FitInfo fi = fits[f];
     const LmState &s = st[f];
     hbt_fit_result *out = res + (long long)(first_table + fi.t) * fc.n_cuts + fi.k;
-    out->q_cut = fc.cut_sorted[fc.rank[fi.k]];
-    out->n_points = fi.n;
-    out->iterations = s.iter;
-    out->reserved = 0;
-    if (s.status == HBT_FIT_TOO_FEW) {
-        for (int j = 0; j < 6; j++) out->p[j] = out->err[j] = NAN;
-        out->chi2 = NAN;
-        out->status = HBT_FIT_TOO_FEW;
+    const bool few = s.status == HBT_FIT_TOO_FEW;
+    if (j == 0) {
+        out->q_cut = fc.cut_sorted[fc.rank[fi.k]];
+        out->n_points = fi.n;
+        out->iterations = s.iter;
+        out->reserved = 0;
+        out->chi2 = few ? NAN : s.S;
+    }
+    if (j < 6) out->p[j] = few ? NAN : s.x[j];
+    if (few) {
+        if (j < 6) out->err[j] = NAN;
+        if (j == 0) out->status = HBT_FIT_TOO_FEW;
         return;
     }
-    for (int j = 0; j < 6; j++) out->p[j] = s.x[j];
-    out->chi2 = s.S;
-    int status = s.status;
-    double red[kSums];
-    fit_sums(fi, partial, red);
-    double L[21];
-    for (int j = 0; j < 21; j++) L[j] = red[7 + j];
-    if (cholesky6(L)) {
-        for (int j = 0; j < 6; j++) {
-            double e[6] = {0, 0, 0, 0, 0, 0}, col[6];
-            e[j] = 1.0;
-            chol_solve6(L, e, col);
-            out->err[j] = sqrt(col[j]);
-        }
-    } else {
-        for (int j = 0; j < 6; j++) out->err[j] = INFINITY;
-        if (status == HBT_FIT_CONVERGED) status = HBT_FIT_SINGULAR;
+    __shared__ double L[21];
+    __shared__ int definite;
+    if (j >= 7 && j < kSums) L[j - 7] = fit_sum(fi, partial, j);
+    __syncwarp();
+    if (j == 0) definite = cholesky6(L);
+    __syncwarp();
+    if (j < 6) {
+        double e[6] = {0, 0, 0, 0, 0, 0}, col[6];
+        e[j] = 1.0;
+        chol_solve6(L, e, col);
+        out->err[j] = definite ? sqrt(col[j]) : INFINITY;
     }
-    out->status = status;
-    atomicAdd(n_passes, (unsigned long long)s.passes + 1);
+    if (j == 0) {
+        out->status = !definite && s.status == HBT_FIT_CONVERGED ? HBT_FIT_SINGULAR : s.status;
+        atomicAdd(n_passes, (unsigned long long)s.passes + 1);
+    }
 }
 
 struct Buf {
@@ -562,6 +787,39 @@ constexpr long long kBatchIn = 256LL << 20;
 // Iterations launched between two reads of the any-fit-active flag.
 constexpr int kStepsPerCheck = 4;
 
+// The cuts on |q| as cuts on its square (FitConst): the square root is
+// monotone, so each is the neighbour of the cut's square at which the
+// comparison turns.
+void set_cut_squares(FitConst &fc) {
+    auto bits = [](double v) {
+        long long b;
+        std::memcpy(&b, &v, sizeof(b));
+        return b;
+    };
+    for (int k = 0; k < fc.n_cuts; k++) {
+        const double cut = fc.cut_sorted[k];
+        double z = 0.0;  // nothing is below a cut that is 0, negative or NaN
+        if (cut > 0.0) {
+            z = cut * cut;
+            while (std::sqrt(z) < cut) z = std::nextafter(z, HUGE_VAL);
+            while (z > 0.0 && !(std::sqrt(std::nextafter(z, 0.0)) < cut)) z = std::nextafter(z, 0.0);
+        }
+        fc.cut_sq[k] = bits(z);
+    }
+    const double lo = fc.q_cut_min;
+    if (std::isnan(lo)) {
+        fc.min_sq = bits(HUGE_VAL);
+    } else if (lo < 0.0) {
+        fc.min_sq = -1;  // every row is above
+    } else {
+        double z = lo * lo;
+        while (z > 0.0 && std::sqrt(z) > lo) z = std::nextafter(z, 0.0);
+        while (std::sqrt(std::nextafter(z, HUGE_VAL)) <= lo && z < HUGE_VAL)
+            z = std::nextafter(z, HUGE_VAL);
+        fc.min_sq = bits(z);
+    }
+}
+
 // The input doubles of a table and, for an interleaved one, where its
 // block starts: the five columns within one row-major block of n rows.
 long long table_span(const hbt_fit_table &T, const double **lo_out) {
@@ -590,7 +848,9 @@ struct hbt_fit_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-    Buf in, rows, frows, tab_off, desc, cls, fits, items, state, partial, res, counter, active;
+    Buf in, rows, frows, tab_off, desc, parts, first, part_cls, cls, fits, items, state, partial,
+        res, counter, ctl;
+    int sms = 0;
     int *active_host = nullptr;  // pinned
     std::vector<double> packed;
     hbt_fit_stats stats{};
@@ -617,8 +877,12 @@ hbt_status hbt_fit_create(int device, hbt_fit_ctx **out) {
         cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ev[0]) != cudaSuccess || cudaEventCreate(&c->ev[1]) != cudaSuccess ||
         cudaEventCreate(&c->ev[2]) != cudaSuccess || !grow(c->counter, 8) ||
-        !grow(c->active, sizeof(int)) ||
+        !grow(c->ctl, (kStepsPerCheck + 1) * sizeof(PassCtl)) ||
         cudaMallocHost(&c->active_host, sizeof(int)) != cudaSuccess) {
+        hbt_fit_destroy(c);
+        return HBT_ERR_CUDA;
+    }
+    if (cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
         hbt_fit_destroy(c);
         return HBT_ERR_CUDA;
     }
@@ -630,8 +894,9 @@ void hbt_fit_destroy(hbt_fit_ctx *c) {
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (Buf *b : {&c->in, &c->rows, &c->frows, &c->tab_off, &c->desc, &c->cls, &c->fits,
-                   &c->items, &c->state, &c->partial, &c->res, &c->counter, &c->active})
+    for (Buf *b : {&c->in, &c->rows, &c->frows, &c->tab_off, &c->desc, &c->parts, &c->first,
+                   &c->part_cls, &c->cls, &c->fits, &c->items, &c->state, &c->partial, &c->res,
+                   &c->counter, &c->ctl})
         if (b->p) cudaFree(b->p);
     for (cudaEvent_t e : c->ev)
         if (e) cudaEventDestroy(e);
@@ -668,6 +933,7 @@ hbt_status hbt_fit_radii(hbt_fit_ctx *c, int32_t n_tables, const hbt_fit_table *
         fc.rank[order[s]] = s;
         fc.by_rank[s] = order[s];
     }
+    set_cut_squares(fc);
     for (int t = 0; t < n_tables; t++) {
         const hbt_fit_table &T = tables[t];
         if (T.n_rows < 0 || T.stride < 1 ||
@@ -691,7 +957,8 @@ hbt_status hbt_fit_radii(hbt_fit_ctx *c, int32_t n_tables, const hbt_fit_table *
     std::vector<TabDesc> desc;
     std::vector<const double *> block;
     std::vector<long long> packed_at;
-    std::vector<int> cls_h;
+    std::vector<int> cls_h, first;
+    std::vector<SelPart> parts;
     std::vector<FitInfo> fits;
     std::vector<FitItem> items;
     for (int t0 = 0; t0 < n_tables && e == cudaSuccess;) {
@@ -701,6 +968,8 @@ hbt_status hbt_fit_radii(hbt_fit_ctx *c, int32_t n_tables, const hbt_fit_table *
         off.assign(1, 0);
         desc.clear();
         block.clear();
+        parts.clear();
+        first.assign(1, 0);
         while (t1 < n_tables) {
             const hbt_fit_table &T = tables[t1];
             const double *lo = nullptr;
@@ -722,12 +991,19 @@ hbt_status hbt_fit_radii(hbt_fit_ctx *c, int32_t n_tables, const hbt_fit_table *
             in_total += span;
             rows += T.n_rows;
             off.push_back(rows);
+            // a table without rows has one part, which leaves its counts
+            const int np = (int)std::max<long long>(1, (T.n_rows + kSelRows - 1) / kSelRows);
+            for (int p = 0; p < np; p++) parts.push_back(SelPart{t1 - t0, p});
+            first.push_back((int)parts.size());
             t1++;
         }
         const int nt = t1 - t0;
         bool ok = grow(c->tab_off, (nt + 1) * sizeof(long long)) &&
                   grow(c->desc, nt * sizeof(TabDesc)) &&
                   grow(c->cls, (size_t)nt * (nc + 1) * sizeof(int)) &&
+                  grow(c->parts, parts.size() * sizeof(SelPart)) &&
+                  grow(c->first, first.size() * sizeof(int)) &&
+                  grow(c->part_cls, parts.size() * nc * sizeof(int)) &&
                   grow(c->in, in_total * sizeof(double)) &&
                   grow(c->rows, 7 * rows * sizeof(double)) &&
                   grow(c->frows, 5 * rows * sizeof(float));
@@ -751,6 +1027,10 @@ hbt_status hbt_fit_radii(hbt_fit_ctx *c, int32_t n_tables, const hbt_fit_table *
             (e = cudaMemcpyAsync(c->tab_off.p, off.data(), off.size() * sizeof(long long),
                                  cudaMemcpyHostToDevice, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(c->desc.p, desc.data(), desc.size() * sizeof(TabDesc),
+                                 cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(c->parts.p, parts.data(), parts.size() * sizeof(SelPart),
+                                 cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(c->first.p, first.data(), first.size() * sizeof(int),
                                  cudaMemcpyHostToDevice, st)) != cudaSuccess)
             break;
         // all copies first (copies from pageable memory wait for the stream's
@@ -765,8 +1045,14 @@ hbt_status hbt_fit_radii(hbt_fit_ctx *c, int32_t n_tables, const hbt_fit_table *
                                 cudaMemcpyHostToDevice, st);
         }
         if (e != cudaSuccess) break;
-        k_fit_select<<<nt, kSelThreads, 0, st>>>(fc, d_off, static_cast<const TabDesc *>(c->desc.p),
-                                                din, rw, static_cast<int *>(c->cls.p));
+        const TabDesc *d_desc = static_cast<const TabDesc *>(c->desc.p);
+        const SelPart *d_parts = static_cast<const SelPart *>(c->parts.p);
+        const unsigned sb = (unsigned)parts.size();
+        k_fit_count<<<sb, kSelThreads, 0, st>>>(fc, d_off, d_desc, din, d_parts,
+                                                static_cast<int *>(c->part_cls.p));
+        k_fit_select<<<sb, kSelThreads, 0, st>>>(
+            fc, d_off, d_desc, din, d_parts, static_cast<const int *>(c->first.p),
+            static_cast<const int *>(c->part_cls.p), rw, static_cast<int *>(c->cls.p));
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         // the fits and their work items, from the selected row counts
         cls_h.resize((size_t)nt * (nc + 1));
@@ -777,21 +1063,36 @@ hbt_status hbt_fit_radii(hbt_fit_ctx *c, int32_t n_tables, const hbt_fit_table *
             break;
         fits.clear();
         items.clear();
-        for (int t = 0; t < nt; t++)
+        int slots = 0;
+        for (int t = 0; t < nt; t++) {
+            const int f0 = (int)fits.size();
+            int most = 0;
             for (int k = 0; k < nc; k++) {
-                FitInfo fi{t, k, 0, (int)items.size(), 0};
+                FitInfo fi{t, k, 0, slots, 0};
                 for (int r = 0; r <= fc.rank[k]; r++) fi.n += cls_h[(size_t)t * (nc + 1) + r];
-                if (fi.n >= 6)
-                    for (int r = 0; r < fi.n; r += kItemRows)
-                        items.push_back(FitItem{(int)fits.size(), std::min(kItemRows, fi.n - r),
-                                                off[t] + r});
-                fi.item1 = (int)items.size();
+                if (fi.n >= 6) {
+                    slots += (fi.n + kItemRows - 1) / kItemRows;
+                    most = std::max(most, fi.n);
+                }
+                fi.item1 = slots;
                 fits.push_back(fi);
             }
+            for (int r = 0; r < most; r += kItemRows)
+                for (int k = 0; k < nc; k++) {
+                    const FitInfo &fi = fits[f0 + k];
+                    if (fi.n >= 6 && r < fi.n)
+                        items.push_back(FitItem{f0 + k, std::min(kItemRows, fi.n - r),
+                                                fi.item0 + r / kItemRows, 0, off[t] + r});
+                }
+        }
+        // the largest items first (the blocks take their units in turn); items of the
+        // same size stay in row order, so fits that share rows find them in L2
+        std::stable_sort(items.begin(), items.end(),
+                         [](const FitItem &a, const FitItem &b) { return a.rows > b.rows; });
         const int nf = (int)fits.size(), ni = (int)items.size();
         ok = grow(c->fits, nf * sizeof(FitInfo)) && grow(c->items, std::max(ni, 1) * sizeof(FitItem)) &&
              grow(c->state, nf * sizeof(LmState)) &&
-             grow(c->partial, (size_t)std::max(ni, 1) * kSums * sizeof(double));
+             grow(c->partial, (size_t)std::max(slots, 1) * kItemUnits * kSums * sizeof(double));
         if (!ok) return fit_fail(c, HBT_ERR_NOMEM, "device allocation failed");
         if ((e = cudaMemcpyAsync(c->fits.p, fits.data(), nf * sizeof(FitInfo),
                                  cudaMemcpyHostToDevice, st)) != cudaSuccess ||
@@ -802,33 +1103,43 @@ hbt_status hbt_fit_radii(hbt_fit_ctx *c, int32_t n_tables, const hbt_fit_table *
         const FitItem *d_items = static_cast<const FitItem *>(c->items.p);
         LmState *d_state = static_cast<LmState *>(c->state.p);
         double *d_part = static_cast<double *>(c->partial.p);
-        int *d_active = static_cast<int *>(c->active.p);
-        const unsigned fb = (unsigned)((nf + 127) / 128);
-        const unsigned pg = (unsigned)std::max(1, std::min(ni, 152 * HBT_FIT_MIN_BLOCKS * 8));
-        k_fit_init<<<fb, 128, 0, st>>>(fc, d_fits, nf, d_state);
+        PassCtl *d_ctl = static_cast<PassCtl *>(c->ctl.p);
+        // resident pass blocks: with few units two an SM, so that the small
+        // units come after the large ones (16 tables of 23^3 rows: 2.15 ms a
+        // call against 2.39 ms at four); with many four, which fill the FP64
+        // pipe (64 tables of 41^3 rows: 9.4 ms against 9.9 ms at two)
+        const int units = ni * kItemUnits;
+        const int per_sm = units < 8 * c->sms ? 2 : HBT_FIT_MIN_BLOCKS;
+        const unsigned pg = (unsigned)std::max(1, std::min(units, c->sms * per_sm));
+        k_fit_init<<<(unsigned)((nf + 127) / 128), 128, 0, st>>>(fc, d_fits, nf, d_state);
         e = cudaGetLastError();
-        // Levenberg-Marquardt: a pass over all active fits' rows, then one
-        // step of every active fit; the flag is read every few iterations
+        // Levenberg-Marquardt passes over all active fits' rows, each with
+        // the fits' steps; the flag is read every few passes
         for (int done = 0; e == cudaSuccess && ni > 0 && done <= fc.max_iter + 1;
              done += kStepsPerCheck) {
-            for (int r = 0; r < kStepsPerCheck && e == cudaSuccess; r++) {
-                if ((e = cudaMemsetAsync(d_active, 0, sizeof(int), st)) != cudaSuccess) break;
-                k_fit_pass<false><<<pg, kFitThreads, 0, st>>>(d_items, ni, rw, d_state, d_part);
-                k_fit_step<<<fb, 128, 0, st>>>(fc, d_fits, nf, d_state, d_part, d_active);
-                e = cudaGetLastError();
-            }
+            if ((e = cudaMemsetAsync(d_ctl, 0, kStepsPerCheck * sizeof(PassCtl), st)) !=
+                cudaSuccess)
+                break;
+            for (int r = 0; r < kStepsPerCheck; r++)
+                k_fit_pass<false><<<pg, kFitThreads, 0, st>>>(fc, d_items, ni, rw, d_fits,
+                                                              d_state, d_part, d_ctl + r);
+            e = cudaGetLastError();
             if (e == cudaSuccess)
-                e = cudaMemcpyAsync(c->active_host, d_active, sizeof(int), cudaMemcpyDeviceToHost,
-                                    st);
+                e = cudaMemcpyAsync(c->active_host, &d_ctl[kStepsPerCheck - 1].active, sizeof(int),
+                                    cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess || *c->active_host == 0) break;
         }
         if (e != cudaSuccess) break;
         // J^T J in FP64 at each minimum, then the results
-        if (ni > 0) k_fit_pass<true><<<pg, kFitThreads, 0, st>>>(d_items, ni, rw, d_state, d_part);
-        k_fit_finish<<<fb, 128, 0, st>>>(fc, t0, d_fits, nf, d_state, d_part,
-                                          static_cast<hbt_fit_result *>(c->res.p),
-                                          static_cast<unsigned long long *>(c->counter.p));
+        if (ni > 0) {
+            if ((e = cudaMemsetAsync(d_ctl, 0, sizeof(PassCtl), st)) != cudaSuccess) break;
+            k_fit_pass<true><<<pg, kFitThreads, 0, st>>>(fc, d_items, ni, rw, d_fits,
+                                                         d_state, d_part, d_ctl);
+        }
+        k_fit_finish<<<(unsigned)nf, 32, 0, st>>>(fc, t0, d_fits, nf, d_state, d_part,
+                                                  static_cast<hbt_fit_result *>(c->res.p),
+                                                  static_cast<unsigned long long *>(c->counter.p));
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         if ((e = cudaEventRecord(c->ev[2], st)) != cudaSuccess) break;
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;

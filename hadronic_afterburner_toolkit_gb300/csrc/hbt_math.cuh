@@ -83,6 +83,28 @@ __device__ __forceinline__ double table_cos(const double2 *cs, const CosScale &k
     return __fma_rn(e.x, cd, -(e.y * sd));
 }
 
+// Conversions with the integer pipe: the hardware's conversions to and from
+// FP64 issue on the FP64 pipe.
+
+// (float)x, rounded to nearest even; outside FP32's normal range (and for
+// values that round up out of it) the hardware's conversion.
+__device__ __forceinline__ float to_float_rn(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), e = (hi >> 20) & 0x7ffu;
+    if (e - 897u >= 253u) return (float)x;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const unsigned long long r = b + 0x0fffffffull + ((b >> 29) & 1ull);
+    const unsigned f = (unsigned)(r >> 29) - (896u << 23);
+    return __uint_as_float((f & 0x7fffffffu) | (hi & 0x80000000u));
+}
+
+// (double)n for an integer below 2^24 in magnitude.
+__device__ __forceinline__ double small_to_double(int n) {
+    const unsigned f = __float_as_uint(__int2float_rn(n));
+    const unsigned mag = f & 0x7fffffffu;
+    const unsigned hi = mag ? (f & 0x80000000u) | ((mag >> 3) + (896u << 20)) : 0u;
+    return __hiloint2double((int)hi, (int)(f << 29));
+}
+
 // Table of 2^(j / 64), j = 0..63, for table_exp, filled by each CTA that
 // uses it.
 constexpr int EXP_TABLE = 64;
@@ -98,11 +120,13 @@ __device__ __forceinline__ void fill_exp_table(double *t) {
 // (truncation below 4e-17 relative), 2^m added to the exponent field.
 // Outside |x| < 700 (where 2^m could leave the normal range) it calls exp().
 __device__ __forceinline__ double table_exp(const double *t, double x) {
-    if (!(fabs(x) < 700.0)) return exp(x);
-    const double nd = rint(x * 92.33248261689366);             // 64 / ln 2
+    if (!((unsigned)(__double2hiint(x) & 0x7fffffff) < 0x4085e000u)) return exp(x);  // |x| < 700
+    // rounded by an addition of 1.5 2^52, whose low word then holds n
+    const int n = __double2loint(__dadd_rn(__dmul_rn(x, 92.33248261689366),  // 64 / ln 2
+                                           6755399441055744.0));
+    const double nd = small_to_double(n);
     double r = __fma_rn(-nd, 0x1.62e42ff000000p-7, x);         // leading part
     r = __fma_rn(-nd, -6.563929801064195e-13, r);              // ln 2 / 64 - leading part
-    const int n = __double2int_rn(nd);
     double p = __fma_rn(r, 1.0 / 120.0, 1.0 / 24.0);
     p = __fma_rn(p, r, 1.0 / 6.0);
     p = __fma_rn(p, r, 0.5);
