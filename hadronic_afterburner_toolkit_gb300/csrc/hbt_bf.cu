@@ -19,15 +19,28 @@
 #include <vector>
 
 #include "../../include/hbt_bf.h"
+#include "hbt_engine.cuh"
+#include "hbt_screen.cuh"
 
 namespace {
 
+using hbt::tile::add2;
+using hbt::tile::f2;
+using hbt::tile::fma2;
+using hbt::tile::pack2;
+using hbt::tile::unpack2;
+
 constexpr int kTile = 128;
+#ifndef HBT_BF_STAGE
+#define HBT_BF_STAGE 256
+#endif
+constexpr int kStage = HBT_BF_STAGE;  // particles of list B staged at a time
+constexpr int kGroup = 4;  // pairs of a thread between two branches
 constexpr int kNphi = HBT_BF_NPHI;
 
 // Resident CTAs per SM the kernel is compiled for (register budget).
 #ifndef HBT_BF_MIN_BLOCKS
-#define HBT_BF_MIN_BLOCKS 10
+#define HBT_BF_MIN_BLOCKS 8
 #endif
 
 // A job with its particle ranges resolved in the concatenated arrays.
@@ -42,6 +55,7 @@ struct BfJob {
 struct BfConst {
     double drap, Brap_min, dphi, Bphi_min;
     double inv_drap, inv_dphi;
+    double phi0;  // -Bphi_min / dphi, in [0, 20)
     int Bnpts;
 };
 
@@ -78,18 +92,21 @@ __device__ __noinline__ int bin_slow(const BfConst &c, const double *phi, const 
 //   T_y   = (y_a - y_b - Brap_min) / drap              (T_y < 0 is the
 //           reference's dy < Brap_min cut),
 // each the difference of a term of particle a and a term of particle b.
-// The terms are computed once per particle in FP64, the phi term reduced
-// mod 20 into [0, 20), and rounded to FP32 (error <= u |term|, u = 2^-24),
-// so a pair costs one FP32 subtraction per quotient (error <= u (|term a| +
-// |term b|)).  Each term carries a bound: 2.0001 u |term| for those
-// roundings, 2^-46 times the magnitudes it was made of for the FP64
-// arithmetic here and in the reference's own quotient, and on particle a
-// 2e-7 for the FP32 rounding of 1 - bound.  When the fraction of both FP32
-// differences clears the summed bounds, their floors are the reference's.
-// A term of magnitude >= 1e9 (or NaN) becomes NaN: every pair of that
-// particle then fails the screen and takes the FP64 path.
+// The terms are computed once per particle and call in FP64, the phi terms
+// reduced mod 20 into [0, 20) (particle a's without the rotation, which a job
+// adds to it in two floats), and rounded to FP32 (error <= u |term|, u =
+// 2^-24), so a pair costs one FP32 subtraction per quotient (error <= u
+// (|term a| + |term b|)).  Each term carries a bound: 2.0001 u |term| for
+// those roundings, 2^-46 times the magnitudes it was made of for the FP64
+// arithmetic here and in the reference's own quotient (and, 120 units of it,
+// for the two floats), and on particle a 2e-7 for the FP32 rounding of 0.5 -
+// bound.  When the fraction of both FP32 differences clears the summed
+// bounds, their floors are the reference's.  A term of magnitude >= 5e8 (or
+// NaN) becomes NaN: every pair of that particle then fails the screen and
+// takes the FP64 path.
 constexpr double kU64 = 0x1p-24;
 constexpr float kU = 0x1p-24f;
+constexpr double kTermMax = 5e8;
 
 __device__ __forceinline__ double wrap20(double x) {
     double r = x - 20.0 * floor(x * 0.05);
@@ -98,42 +115,51 @@ __device__ __forceinline__ double wrap20(double x) {
     return r;
 }
 
-__device__ __forceinline__ float4 pack_terms(double xp, double mp, double xy, double my,
-                                             double slack) {
-    if (!(fabs(xp) < 1e9 && fabs(xy) < 1e9)) return make_float4(NAN, 0.f, NAN, 0.f);
-    const float tp = (float)wrap20(xp), ty = (float)xy;
-    const float ep = (float)(2.0001 * kU64 * fabs((double)tp) + 0x1p-46 * (mp + 40.0) + slack);
-    const float ey = (float)(2.0001 * kU64 * fabs((double)ty) + 0x1p-46 * my + slack);
-    return make_float4(tp, ep, ty, ey);
+// Particle b's terms, negated (the pair loop adds): the terms of phi / dphi
+// and y / drap, and their bounds.
+__device__ __forceinline__ float4 terms_b(const BfConst &c, double wp, double xp, double xy) {
+    if (!(fabs(xp) < kTermMax && fabs(xy) < kTermMax)) return make_float4(NAN, NAN, 0.f, 0.f);
+    const float tp = (float)wp, ty = (float)xy;
+    const float ep = (float)(2.0001 * kU64 * fabs((double)tp) + 0x1p-46 * (fabs(xp) + 40.0));
+    const float ey = (float)(2.0001 * kU64 * fabs((double)ty) + 0x1p-46 * fabs(xy));
+    return make_float4(-tp, -ty, -ep, -ey);
 }
 
-// Particle a's terms as the pair loop uses them: the azimuthal term plus
-// 19.5 and the rapidity term minus 0.5 (both shifts in FP64 before the
-// rounding to FP32, inside the bound), so that rint of a pair's difference
-// is the floor of the unshifted one (plus 20 for the azimuth: a column in
-// [0, 40) of a histogram whose columns c and c + 20 are the same bin), and
-// each bound as its distance to a half-integer, 0.5 - bound.
-__device__ __forceinline__ float4 pack_terms_a(double xp, double mp, double xy, double my) {
-    if (!(fabs(xp) < 1e9 && fabs(xy) < 1e9)) return make_float4(NAN, 0.f, NAN, 0.f);
-    const double sp = wrap20(xp) + 19.5, sy = xy - 0.5;
-    const float tp = (float)sp, ty = (float)sy;
-    const double ep = 2.0001 * kU64 * fabs((double)tp) + 0x1p-46 * (mp + 60.0) + 2e-7;
-    const double ey = 2.0001 * kU64 * fabs((double)ty) + 0x1p-46 * (my + 1.0) + 2e-7;
-    return make_float4(tp, (float)(0.5 - ep), ty, (float)(0.5 - ey));
+// Particle a's terms: of (phi - Bphi_min) / dphi, wrapped, in two floats (the
+// job's rotation and 19.5 come on top, a_terms), then of (y - Brap_min) / drap
+// less 0.5 (the shifts make rint of a pair's difference the floor of the
+// unshifted one, plus 20 for the azimuth: a column in [0, 40) of a histogram
+// whose columns c and c + 20 are the same bin), then the parts of the bounds:
+// the azimuth's without 2 u |term|, and 0.5 - bound of the rapidity's.
+struct TermsA {
+    float ph, pl, ty, ep, gy, pad;
+};
+__device__ __forceinline__ TermsA terms_a(const BfConst &c, double wp, double xp, double y) {
+    const double cp = c.Bphi_min * c.inv_dphi, xy = (y - c.Brap_min) * c.inv_drap;
+    const double my = (fabs(y) + fabs(c.Brap_min)) * c.inv_drap;
+    TermsA t = {NAN, 0.f, NAN, 0.f, 0.f, 0.f};
+    if (!(fabs(xp) < kTermMax && fabs(xy) < kTermMax)) return t;
+    double s = wp + c.phi0;
+    if (s >= 20.0) s -= 20.0;
+    t.ph = (float)s;
+    t.pl = (float)(s - (double)t.ph);
+    t.ty = (float)(xy - 0.5);
+    t.ep = (float)(0x1p-46 * (fabs(xp) + fabs(cp) + 200.0) + 2e-7);
+    t.gy = (float)(0.5 - (2.0001 * kU64 * fabs((double)t.ty) + 0x1p-46 * (my + 1.0) + 2e-7));
+    return t;
 }
 
-// Particle a: (phi + rot - Bphi_min) / dphi and (y - Brap_min) / drap,
-// shifted (pack_terms_a).
-__device__ __forceinline__ float4 terms_a(const BfConst &c, double phi, double y, double rot) {
-    return pack_terms_a(((phi + rot) - c.Bphi_min) * c.inv_dphi,
-                        (fabs(phi) + fabs(rot) + fabs(c.Bphi_min)) * c.inv_dphi,
-                        (y - c.Brap_min) * c.inv_drap, (fabs(y) + fabs(c.Brap_min)) * c.inv_drap);
-}
-
-// Particle b: phi / dphi and y / drap.
-__device__ __forceinline__ float4 terms_b(const BfConst &c, double phi, double y) {
-    return pack_terms(phi * c.inv_dphi, fabs(phi) * c.inv_dphi, y * c.inv_drap,
-                      fabs(y) * c.inv_drap, 0.0);
+// A job's rotation as the terms take it: wrapped, in two floats, and its part
+// of the bound.
+struct Rotation {
+    float h, l, e;
+};
+__device__ __forceinline__ Rotation rotation_of(const BfConst &c, double rot) {
+    const double x = rot * c.inv_dphi;
+    if (!(fabs(x) < kTermMax)) return Rotation{NAN, 0.f, 0.f};
+    const double w = wrap20(x);
+    const float h = (float)w;
+    return Rotation{h, (float)(w - (double)h), (float)(0x1p-46 * (fabs(x) + 1.0))};
 }
 
 // The |dy| < 1e-10 cut: |dy| from FP32 copies errs by at most u (|y_a| +
@@ -144,14 +170,76 @@ __device__ __forceinline__ float2 dy_terms(double y, float slack) {
     return make_float2(fy, 7.0f * kU * fabsf(fy) + slack);
 }
 
-// Every particle's b terms, once per call.
+// Particle a in a job, as the pair loop uses it: {t_phi, t_y}, {0.5 - bound of
+// each}, {y, slack}.
+struct ParticleA {
+    f2 t, g, y;
+};
+__device__ __forceinline__ ParticleA a_terms(const TermsA &a, const float2 &yb,
+                                             const Rotation &r) {
+    // (ph + pl) + (h + l) + 19.5, less 20 from 20 on; two_sum each
+    auto two_sum = [](float x, float y, float &err) {
+        const float s = __fadd_rn(x, y), v = __fsub_rn(s, x);
+        err = __fadd_rn(__fsub_rn(x, __fsub_rn(s, v)), __fsub_rn(y, v));
+        return s;
+    };
+    float e1, e2;
+    float s = two_sum(a.ph, r.h, e1);
+    const float low = __fadd_rn(e1, __fadd_rn(a.pl, r.l));
+    s = two_sum(s, s >= 20.f ? -0.5f : 19.5f, e2);
+    const float tp = __fadd_rn(s, __fadd_rn(e2, low));
+    const float ep = __fmaf_rn(2.0002f * kU, fabsf(tp), __fadd_rn(a.ep, r.e));
+    return ParticleA{pack2(tp, a.ty), pack2(0.5f - ep, a.gy), pack2(yb.x, yb.y + 1.0001e-10f)};
+}
+
+// Every particle's terms, once per call: a dozen FP64 operations and the
+// conversions a particle, which a job's every block made again before (57 us
+// of FP64 for 1,600 jobs of 385 x 385 particles).
 __global__ void k_bf_terms(long long n, const double *phi, const double *y, BfConst c,
-                           float4 *tb, float2 *yb) {
+                           float4 *tb, float2 *yb, TermsA *ta) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
-        tb[i] = terms_b(c, phi[i], y[i]);
-        yb[i] = dy_terms(y[i], 0.f);
+        const double p = phi[i], yi = y[i], xp = p * c.inv_dphi;
+        const double wp = wrap20(xp);
+        tb[i] = terms_b(c, wp, xp, yi * c.inv_drap);
+        ta[i] = terms_a(c, wp, xp, yi);
+        const float2 d = dy_terms(yi, 0.f);
+        yb[i] = make_float2(-d.x, d.y);
     }
+}
+
+// A pair's place in the shared histogram, and whether the screen is sure of it.
+struct Decision {
+    unsigned k;
+    bool sure;
+};
+__device__ __forceinline__ Decision decide(const ParticleA &A, const float4 &B, const float2 &By) {
+    constexpr float kMagic = 12582912.0f;  // 1.5 2^23
+    constexpr unsigned kOff = 0x4b400000u * (2u * kNphi + 1u);
+    // shifted differences: rint gives the floors (the azimuth + 20); certain
+    // when their distance to the rint is below 0.5 - bound (which also keeps
+    // |t| below 2^22)
+    const f2 t = add2(A.t, pack2(B.x, B.y)), g = add2(A.g, pack2(B.z, B.w));
+    const f2 m = add2(t, pack2(kMagic, kMagic));
+    const f2 r = fma2(add2(m, pack2(-kMagic, -kMagic)), pack2(-1.f, -1.f), t);
+    const f2 dy = add2(A.y, pack2(By.x, By.y));
+    float mp, my, rp, ry, gp, gy, d, dmin;
+    unpack2(m, mp, my);
+    unpack2(r, rp, ry);
+    unpack2(g, gp, gy);
+    unpack2(dy, d, dmin);
+    // t_phi in (-0.5, 39.5): column in [0, 39]; a row beyond [0, Bnpts) puts k
+    // outside the histogram
+    return Decision{__float_as_uint(my) * (2u * kNphi) + __float_as_uint(mp) - kOff,
+                    bool((fabsf(rp) < gp) & (fabsf(ry) < gy) & (fabsf(d) > dmin))};
+}
+
+// Adds one to word k of the histogram at `at` when k < n, without a branch.
+__device__ __forceinline__ void count_one(unsigned at, unsigned k, unsigned n) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.lt.u32 p, %0, %1;\n @p red.shared.add.u32 [%2], 1;\n}" ::"r"(k),
+        "r"(n), "r"(at + 4u * k)
+        : "memory");
 }
 
 // One work item per (job, tile of up to 128 particles of list A): a job of
@@ -160,59 +248,83 @@ __global__ void k_bf_terms(long long n, const double *phi, const double *y, BfCo
 // registers (one particle per thread), B's are staged through shared memory
 // 128 at a time; the histogram is privatised in shared memory and its
 // non-zero bins are added to the global one when the item is done.
+//
+// A pair costs two broadcast reads, six packed FP32 operations (rint by the
+// addition of 1.5 2^23, whose low bits then are the bin), three comparisons
+// and the shared-memory addition; four pairs share a branch for those the
+// screen leaves open.  Bound by the issue of some 28 instructions a pair (62 %
+// of the slots) next to the shared-memory pipe (58 %): 160 million pairs of
+// 1,600 jobs in 188 us, 273 us with scalar operations, rint and a branch a
+// pair.
 __global__ void __launch_bounds__(kTile, HBT_BF_MIN_BLOCKS)
     k_bf(const BfJob *jobs, const int2 *items, long long n_items, const double *phi,
-         const double *y, const float4 *tb, const float2 *yb, BfConst c,
+         const double *y, const float4 *tb, const float2 *yb, const TermsA *ta, BfConst c,
          unsigned long long *hist, unsigned long long *n_slow) {
     extern __shared__ unsigned sh[];  // [Bnpts][2 kNphi]: columns c and c + 20 are bin c
-    __shared__ float4 sb[kTile];
-    __shared__ float2 sd[kTile];
+    __shared__ float4 sb[kStage];
+    __shared__ float2 sd[kStage];
     __shared__ BfJob sj;
+    __shared__ Rotation rot;
     const int nbins = c.Bnpts * kNphi, nsh = 2 * nbins;
+    const unsigned sh_at = (unsigned)__cvta_generic_to_shared(sh);
     unsigned slow = 0;
     for (long long it = blockIdx.x; it < n_items; it += gridDim.x) {
         const int2 item = items[it];
         for (int k = threadIdx.x; k < nsh; k += blockDim.x) sh[k] = 0u;
-        if (threadIdx.x == 0) sj = jobs[item.x];
+        if (threadIdx.x == 0) {
+            sj = jobs[item.x];
+            rot = rotation_of(c, sj.mixed ? sj.rotation : 0.0);
+        }
         __syncthreads();
         const long long ia = sj.a0 + item.y + threadIdx.x;
         const bool have = ia < sj.a1;
-        float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
-        float2 Ay = make_float2(0.f, 0.f);
+        ParticleA A = {};
+        bool self_skips = false;
         if (have) {
-            A = terms_a(c, phi[ia], y[ia], sj.mixed ? sj.rotation : 0.0);
-            Ay = dy_terms(y[ia], 1.0001e-10f);
+            const float2 ya = yb[ia];
+            A = a_terms(ta[ia], make_float2(-ya.x, ya.y), rot);
+            self_skips = fabsf(ya.x) < INFINITY;
         }
-        for (long long b = sj.b0; b < sj.b1; b += kTile) {
-            if (b + threadIdx.x < sj.b1) {
-                sb[threadIdx.x] = tb[b + threadIdx.x];
-                sd[threadIdx.x] = yb[b + threadIdx.x];
+        for (long long b = sj.b0; b < sj.b1; b += kStage) {
+            // past the end: terms that leave every pair undecided
+            for (int k = threadIdx.x; k < kStage; k += kTile) {
+                const bool in = b + k < sj.b1;
+                sb[k] = in ? tb[b + k] : make_float4(NAN, NAN, 0.f, 0.f);
+                sd[k] = in ? yb[b + k] : make_float2(0.f, 0.f);
             }
             __syncthreads();
-            const int nb = (int)min((long long)kTile, sj.b1 - b);
+            const int nb = (int)min((long long)kStage, sj.b1 - b);
             if (have) {
-#pragma unroll 2
-                for (int j = 0; j < nb; j++) {
-                    const float4 B = sb[j];
-                    const float2 By = sd[j];
-                    // shifted differences: rint gives the floors (the azimuth
-                    // + 20); certain when their distance to the rint is
-                    // below 0.5 - bound
-                    const float tp = A.x - B.x, ty = A.z - B.z;
-                    const float kp = rintf(tp), ky = rintf(ty);
-                    int k;
-                    if (fabsf(tp - kp) < A.y - B.y && fabsf(ty - ky) < A.w - B.w &&
-                        fabsf(Ay.x - By.x) > Ay.y + By.y) {
-                        // tp in (-0.5, 39.5): column kp in [0, 39]; a row ky
-                        // beyond [0, Bnpts) puts k outside the histogram
-                        // (|ty| < 2^23 here, so k fits an int)
-                        k = (int)__fmaf_rn(ky, 2.0f * kNphi, kp);
-                    } else {
-                        const int k20 = bin_slow(c, phi, y, ia, b + j, sj.mixed, sj.rotation);
-                        k = k20 < 0 ? -1 : (k20 / kNphi) * (2 * kNphi) + k20 % kNphi;
-                        slow++;
+                for (int j = 0; j < nb; j += kGroup) {
+                    unsigned k[kGroup];
+                    bool sure = true;
+#pragma unroll
+                    for (int q = 0; q < kGroup; q++) {
+                        const Decision s = decide(A, sb[j + q], sd[j + q]);
+                        k[q] = s.k;
+                        sure = sure & s.sure;
                     }
-                    if ((unsigned)k < (unsigned)nsh) atomicAdd(&sh[k], 1u);
+                    if (!sure) {
+#pragma unroll 1
+                        for (int q = 0; q < kGroup; q++) {
+                            if (decide(A, sb[j + q], sd[j + q]).sure) continue;
+                            int f = -1;
+                            if (j + q < nb) {
+                                slow++;
+                                // a particle with itself: dy = 0, skipped
+                                if (!(ia == b + j + q && self_skips))
+                                    f = bin_slow(c, phi, y, ia, b + j + q, sj.mixed, sj.rotation);
+                            }
+                            const unsigned to =
+                                f < 0 ? ~0u : (unsigned)((f / kNphi) * (2 * kNphi) + f % kNphi);
+#pragma unroll
+                            for (int p = 0; p < kGroup; p++)
+                                if (p == q) k[p] = to;
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < kGroup; q++)
+                        count_one(sh_at, k[q], (unsigned)nsh);
                 }
             }
             __syncthreads();
@@ -227,6 +339,12 @@ __global__ void __launch_bounds__(kTile, HBT_BF_MIN_BLOCKS)
     }
     for (int o = 16; o > 0; o >>= 1) slow += __shfl_xor_sync(0xffffffffu, slow, o);
     if ((threadIdx.x & 31) == 0 && slow) atomicAdd(n_slow, (unsigned long long)slow);
+}
+
+// A histogram as doubles, to memory the GPU writes (host memory too).
+__global__ void k_bf_export(const unsigned long long *h, int n, double *out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) out[k] = (double)h[k];
 }
 
 struct Buf {
@@ -255,7 +373,9 @@ struct hbt_bf_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     BfConst c;
-    Buf hist, jobs, items, phi, y, tb, yb, counter;
+    Buf hist, jobs, items, phi, y, tb, yb, ta, counter;
+    bool reads_host = false;  // the GPU reads and writes pageable host memory
+    std::vector<hbt::CopySeg> segs;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     hbt_bf_stats stats{};
     std::string err;
@@ -288,6 +408,8 @@ hbt_status hbt_bf_create(const hbt_bf_params *p, int device, hbt_bf_ctx **out) {
     c->c.Bnpts = p->Bnpts;
     c->c.inv_drap = 1.0 / c->c.drap;
     c->c.inv_dphi = 1.0 / c->c.dphi;
+    const double x0 = -c->c.Bphi_min * c->c.inv_dphi;
+    c->c.phi0 = x0 - 20.0 * std::floor(x0 * 0.05);
     if (cudaSetDevice(device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ev[0]) != cudaSuccess || cudaEventCreate(&c->ev[1]) != cudaSuccess ||
@@ -299,6 +421,10 @@ hbt_status hbt_bf_create(const hbt_bf_params *p, int device, hbt_bf_ctx **out) {
         hbt_bf_destroy(c);
         return HBT_ERR_CUDA;
     }
+    int pageable = 0, tables = 0;
+    cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device);
+    cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device);
+    c->reads_host = pageable && tables;
     const hbt_status s = hbt_bf_reset(c);
     if (s != HBT_OK) {
         hbt_bf_destroy(c);
@@ -312,7 +438,7 @@ void hbt_bf_destroy(hbt_bf_ctx *c) {
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (Buf *b : {&c->hist, &c->jobs, &c->items, &c->phi, &c->y, &c->tb, &c->yb, &c->counter})
+    for (Buf *b : {&c->hist, &c->jobs, &c->items, &c->phi, &c->y, &c->tb, &c->yb, &c->ta, &c->counter})
         if (b->p) cudaFree(b->p);
     for (cudaEvent_t e : c->ev)
         if (e) cudaEventDestroy(e);
@@ -325,8 +451,7 @@ const char *hbt_bf_last_error(const hbt_bf_ctx *c) { return c ? c->err.c_str() :
 hbt_status hbt_bf_reset(hbt_bf_ctx *c) {
     if (!c) return HBT_ERR_INVALID;
     if (cudaSetDevice(c->device) != cudaSuccess ||
-        cudaMemsetAsync(c->hist.p, 0, (size_t)8 * c->p.Bnpts * kNphi * 8, c->stream) != cudaSuccess ||
-        cudaStreamSynchronize(c->stream) != cudaSuccess)
+        cudaMemsetAsync(c->hist.p, 0, (size_t)8 * c->p.Bnpts * kNphi * 8, c->stream) != cudaSuccess)
         return bf_fail(c, HBT_ERR_CUDA, "clearing the histograms failed");
     return HBT_OK;
 }
@@ -386,43 +511,65 @@ hbt_status hbt_bf_bin(hbt_bf_ctx *c, int32_t n_lists, const hbt_bf_list *lists, 
     }
     if (!grow(c->jobs, dj.size() * sizeof(BfJob)) || !grow(c->items, items.size() * sizeof(int2)) ||
         !grow(c->phi, total * sizeof(double)) || !grow(c->y, total * sizeof(double)) ||
-        !grow(c->tb, total * sizeof(float4)) || !grow(c->yb, total * sizeof(float2)))
+        !grow(c->tb, total * sizeof(float4)) || !grow(c->yb, total * sizeof(float2)) ||
+        !grow(c->ta, total * sizeof(TermsA)))
         return bf_fail(c, HBT_ERR_NOMEM, "device allocation failed");
     cudaError_t e = cudaEventRecord(c->ev[0], c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(c->jobs.p, dj.data(), dj.size() * sizeof(BfJob),
-                            cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(c->items.p, items.data(), items.size() * sizeof(int2),
-                            cudaMemcpyHostToDevice, c->stream);
+    // where the GPU reads host memory itself, one kernel takes everything
+    c->segs.clear();
+    auto copy = [&](void *dst, const void *src, long long n_doubles) {
+        if (e != cudaSuccess) return;
+        if (!c->reads_host) {
+            e = cudaMemcpyAsync(dst, src, n_doubles * sizeof(double), cudaMemcpyHostToDevice,
+                                c->stream);
+            return;
+        }
+        double *to = static_cast<double *>(dst);
+        const double *from = static_cast<const double *>(src);
+        // a bad pointer fails here, on the host
+        const volatile char *v = static_cast<const volatile char *>(src);
+        (void)v[0];
+        (void)v[n_doubles * sizeof(double) - 1];
+        for (long long k = 0; k < n_doubles; k += hbt::kCopyInChunk)
+            c->segs.push_back(
+                hbt::CopySeg{from + k, to + k, std::min(hbt::kCopyInChunk, n_doubles - k)});
+    };
+    static_assert(sizeof(BfJob) % 8 == 0 && sizeof(int2) == 8, "copied as doubles");
+    copy(c->jobs.p, dj.data(), (long long)(dj.size() * sizeof(BfJob) / 8));
+    copy(c->items.p, items.data(), (long long)items.size());
     if (e == cudaSuccess)
         e = cudaMemsetAsync(c->counter.p, 0, sizeof(unsigned long long), c->stream);
-    for (int l = 0; l < n_lists && e == cudaSuccess; l++) {
+    for (int l = 0; l < n_lists; l++) {
         const long long n = lists[l].n_events > 0 ? lists[l].offsets[lists[l].n_events] : 0;
         if (n == 0 || copy_of[l] >= 0) continue;
-        e = cudaMemcpyAsync(static_cast<double *>(c->phi.p) + base[l], lists[l].phi,
-                            n * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(static_cast<double *>(c->y.p) + base[l], lists[l].y,
-                                n * sizeof(double), cudaMemcpyHostToDevice, c->stream);
+        copy(static_cast<double *>(c->phi.p) + base[l], lists[l].phi, n);
+        copy(static_cast<double *>(c->y.p) + base[l], lists[l].y, n);
     }
+    if (e == cudaSuccess)
+        e = hbt::launch_copy_in(c->segs.data(), (int)c->segs.size(), c->stream);
     if (e == cudaSuccess) e = cudaEventRecord(c->ev[1], c->stream);
-    if (e != cudaSuccess) return bf_fail(c, HBT_ERR_CUDA, "upload failed");
+    // a copy that was queued reads the host arrays: wait before giving up
+    auto give_up = [&](const std::string &m) {
+        cudaStreamSynchronize(c->stream);
+        return bf_fail(c, HBT_ERR_CUDA, m);
+    };
+    if (e != cudaSuccess) return give_up("upload failed");
     const double *dphi_p = static_cast<const double *>(c->phi.p);
     const double *dy_p = static_cast<const double *>(c->y.p);
     if (total > 0)
         k_bf_terms<<<(unsigned)std::min<long long>((total + 255) / 256, 152LL * 16), 256, 0,
                      c->stream>>>(total, dphi_p, dy_p, c->c, static_cast<float4 *>(c->tb.p),
-                                  static_cast<float2 *>(c->yb.p));
+                                  static_cast<float2 *>(c->yb.p),
+                                  static_cast<TermsA *>(c->ta.p));
     const long long n_items = (long long)items.size();
     const long long grid = std::min<long long>(n_items, 1LL << 30);
     k_bf<<<(unsigned)grid, kTile, (size_t)c->p.Bnpts * 2 * kNphi * sizeof(unsigned), c->stream>>>(
         static_cast<const BfJob *>(c->jobs.p), static_cast<const int2 *>(c->items.p), n_items,
         dphi_p, dy_p, static_cast<const float4 *>(c->tb.p), static_cast<const float2 *>(c->yb.p),
-        c->c, static_cast<unsigned long long *>(c->hist.p),
+        static_cast<const TermsA *>(c->ta.p), c->c, static_cast<unsigned long long *>(c->hist.p),
         static_cast<unsigned long long *>(c->counter.p));
     if ((e = cudaGetLastError()) != cudaSuccess)
-        return bf_fail(c, HBT_ERR_CUDA, std::string("k_bf: ") + cudaGetErrorString(e));
+        return give_up(std::string("k_bf: ") + cudaGetErrorString(e));
     unsigned long long slow = 0;
     if ((e = cudaEventRecord(c->ev[2], c->stream)) != cudaSuccess ||
         (e = cudaMemcpyAsync(&slow, c->counter.p, sizeof slow, cudaMemcpyDeviceToHost,
@@ -452,8 +599,19 @@ hbt_status hbt_bf_get_stats(const hbt_bf_ctx *c, hbt_bf_stats *out) {
 hbt_status hbt_bf_read(hbt_bf_ctx *c, int32_t hist, double *out) {
     if (!c || hist < 0 || hist > 7 || !out) return HBT_ERR_INVALID;
     const size_t nb = (size_t)c->p.Bnpts * kNphi;
+    if (cudaSetDevice(c->device) != cudaSuccess) return bf_fail(c, HBT_ERR_CUDA, "cudaSetDevice");
+    if (c->reads_host) {
+        // the host maps the pages, one kernel writes them
+        for (size_t k = 0; k < nb; k += 512) static_cast<volatile double *>(out)[k] = 0.0;
+        static_cast<volatile double *>(out)[nb - 1] = 0.0;
+        k_bf_export<<<(unsigned)((nb + 255) / 256), 256, 0, c->stream>>>(
+            static_cast<unsigned long long *>(c->hist.p) + hist * nb, (int)nb, out);
+        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(c->stream) != cudaSuccess)
+            return bf_fail(c, HBT_ERR_CUDA, "reading the histogram failed");
+        return HBT_OK;
+    }
     std::vector<unsigned long long> v(nb);
-    if (cudaSetDevice(c->device) != cudaSuccess ||
+    if (
         cudaMemcpyAsync(v.data(), static_cast<unsigned long long *>(c->hist.p) + hist * nb,
                         nb * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                         c->stream) != cudaSuccess ||
