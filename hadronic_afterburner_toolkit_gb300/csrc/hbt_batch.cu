@@ -428,8 +428,14 @@ cudaError_t run_batch(const Device &d, const BatchDev &b, int grid, unsigned chu
     const int gs = 152 * 8;
     const bool lc = d.g.boost || d.g.qinv;  // light-cone screen terms
     if (b.max_list <= kSmallList) {
+        // the smallest block that holds the list: its sort's time grows with
+        // the threads it synchronises and their items (10, 12, 18 and 24 us)
         if (b.max_list <= 1024)
             k_order<256, 4><<<b.n_lists, 256, 0, st>>>(b);
+        else if (b.max_list <= 2048)
+            k_order<512, 4><<<b.n_lists, 512, 0, st>>>(b);
+        else if (b.max_list <= 4096)
+            k_order<512, 8><<<b.n_lists, 512, 0, st>>>(b);
         else
             k_order<1024, 8><<<b.n_lists, 1024, 0, st>>>(b);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
