@@ -51,34 +51,37 @@ __device__ __forceinline__ void load_device(const BatchDev &b, const BatchJob &j
     __syncthreads();
 }
 
-// Resident CTAs per SM (register budget 65536 / (128 x CTAs); shared
-// memory allows 5 of the FP64 and double-float forms' 38.4 KB): measured on
-// GB300, the FP64 form of the same-event kernel is fastest at 5 (96
-// registers, no spills: 141.0 ms kernel per central group against 144.6 ms
-// at 4 with 124 registers; at 3, 164 registers, it took 173.6 ms), the
-// double-float form at 5 too (96 registers: 119.8 ms kernel against 123.1
-// ms at 4 with 128, with the descriptor read from the kernel parameter), the
-// FP32-weight form at 6 (80 registers: 94.0 ms, against 97.4 ms at 5 and,
-// before the descriptor change, 127.8 ms at 7 with 72) and the mixed-event
-// kernel at 6 (12.6 ms, against 13.0 ms at 5 and 18.3 ms at 7).
+// Resident CTAs per SM (register budget 65536 / (128 x CTAs)), measured on
+// GB300 in whole kernels.  FP64 form, central group: 5 (51.0 ms; 53.5 at 4,
+// 55.1 at 6).  FP32-weight form: 4 (37.3 ms; 41.2 at 3, 38.5 at 5, 41.5 at
+// 6).  With q_inv histograms,
+// 45,000 pions: same-event 6 (8.8 ms; 9.0 at 5, 9.7 at 4), mixed-event 7 (2.9
+// ms; 3.1 at 6, 3.2 at 5).  Mixed-event without them: 5 (uneven events 2.57
+// ms, small ones 0.34; 2.74 and 0.37 at 6, 3.03 and 0.41 at 8).
 #ifndef HBT_FP64_SAME_CTAS
-#define HBT_FP64_SAME_CTAS 5  // compile-time choice for the FP64 form (-D to measure others)
-#endif
-#ifndef HBT_DF64_SAME_CTAS
-#define HBT_DF64_SAME_CTAS 5  // the same for the double-float form
+#define HBT_FP64_SAME_CTAS 5  // compile-time choices (-D to measure others)
 #endif
 #ifndef HBT_FP32W_SAME_CTAS
-#define HBT_FP32W_SAME_CTAS 6  // and for the FP32-weight form
+#define HBT_FP32W_SAME_CTAS 4
 #endif
-template <int PREC>
+#ifndef HBT_QINV_SAME_CTAS
+#define HBT_QINV_SAME_CTAS 6
+#endif
+#ifndef HBT_MIXED_CTAS
+#define HBT_MIXED_CTAS 5
+#endif
+#ifndef HBT_QINV_MIXED_CTAS
+#define HBT_QINV_MIXED_CTAS 7
+#endif
+template <int PREC, bool QINV>
 struct SameCtas {
     static constexpr int value =
-        PREC == 1 ? HBT_FP32W_SAME_CTAS : (PREC == 2 ? HBT_DF64_SAME_CTAS : HBT_FP64_SAME_CTAS);
+        QINV ? HBT_QINV_SAME_CTAS : (PREC == 1 ? HBT_FP32W_SAME_CTAS : HBT_FP64_SAME_CTAS);
 };
-#ifndef HBT_MIXED_CTAS
-#define HBT_MIXED_CTAS 6  // the mixed-event kernel's
-#endif
-constexpr int kMixedCtas = HBT_MIXED_CTAS;
+template <bool QINV>
+struct MixedCtas {
+    static constexpr int value = QINV ? HBT_QINV_MIXED_CTAS : HBT_MIXED_CTAS;
+};
 
 // Parts of a tile pair (ranges of its j-tile) that its items are split into:
 // with fewer items than CTAs, a pair's 64 steps on one CTA are the launch's
@@ -102,8 +105,8 @@ __device__ __forceinline__ ListRows rows_of(const BatchDev &b, const BatchList &
 // MODE: fast binning, or one pass of ordered cap admission; MANY: the items
 // of many analyses (b.devs), fast binning only.
 template <bool AZ, bool BOOST, int PREC, int MODE, bool QINV, bool MANY>
-__global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(Device d, BatchDev b, unsigned base,
-                                                           unsigned end) {
+__global__ void __launch_bounds__(FT, SameCtas<PREC, QINV>::value)
+    k_persistent_same(Device d, BatchDev b, unsigned base, unsigned end) {
     __shared__ SameSmem sm;
     __shared__ unsigned item;
     __shared__ double cs[PREC == 0 ? kCosEntries : 1];  // the form's cos table
@@ -140,7 +143,8 @@ __global__ void __launch_bounds__(FT, SameCtas<PREC>::value) k_persistent_same(D
 
 // Mixed-event items, all in one launch.
 template <bool AZ, bool BOOST, int MODE, bool QINV, bool MANY>
-__global__ void __launch_bounds__(FT, kMixedCtas) k_persistent_mixed(Device d, BatchDev b) {
+__global__ void __launch_bounds__(FT, MixedCtas<QINV>::value)
+    k_persistent_mixed(Device d, BatchDev b) {
     __shared__ MixedSmem sm;
     __shared__ unsigned item;
     const unsigned stop = min(b.n_items[1], b.mixed_cap);
