@@ -7,8 +7,9 @@
 //  1. k_keys + CUB radix sort, or k_order: every list is reordered by a
 //     Morton key of (p_x, p_y, rapidity) cells into a sorted particle table,
 //     so that 128-particle tiles are compact in momentum space;
-//  2. k_tiles: per tile, the sorted rows and the ranges of p_x, p_y, rapidity y and the
-//     smallest m_T = sqrt(E^2 - p_z^2);
+//  2. k_tiles: per tile, the sorted rows with their screen terms and
+//     fixed-point columns, and the tile's FP32 box: ranges of p_x, p_y,
+//     rapidity y, p_z, and the smallest m_T = sqrt(E^2 - p_z^2);
 //  3. k_cull: every tile pair of every job is kept unless no pair in it can
 //     pass the q windows.  The test is rigorous: the reference's q_out and
 //     q_side satisfy q_out^2 + q_side^2 = q_x^2 + q_y^2, and both lie within
@@ -19,8 +20,7 @@
 //     which grows with m_T1, m_T2 and |y1 - y2|, so its smallest value over
 //     two tiles bounds |q_long| from below; without the boost q_long = q_z.
 //     With q_inv histograms the LCMS q_long bound alone also keeps a tile
-//     pair (boxes_may_pair).  Each bound carries a 1e-6 relative margin for
-//     rounding;
+//     pair (boxes_may_pair).  FP32, every step rounded outwards;
 //  4. k_persistent_same / k_persistent_mixed (hbt_persist.cuh): persistent
 //     CTAs (4 to 6 per SM) pull (job, i-tile, j-tile) items from the culled
 //     same-event and mixed-event queues and run the screened tile-pair

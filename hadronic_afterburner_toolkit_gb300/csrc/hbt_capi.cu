@@ -882,30 +882,11 @@ static void fill_tile_screen(const Grid &g, Screen &s) {
 }
 
 void screen_from_grid(const Grid &g, Screen &s) {
-    auto f = [](double v) { return static_cast<float>(v); };
-    auto slack = [](double v, float v32) { return std::fabs(v - static_cast<double>(v32)); };
-    const double lo4 = 4.0 * g.KT_min_sq, hi4 = 4.0 * g.KT_max_sq;
-    s.kt_lo4 = f(lo4);
-    s.kt_hi4 = f(hi4);
-    s.kt_slack = f(std::max(slack(lo4, s.kt_lo4), slack(hi4, s.kt_hi4)) + 1e-7 * hi4);
-    s.lo = f(g.q_lo);
-    s.hi = f(g.q_hi);
-    s.win_slack = f(std::max(slack(g.q_lo, s.lo), slack(g.q_hi, s.hi)) + 1e-12);
-    s.base = f(g.q_base);
-    s.inv_dq = f(1.0 / g.delta_q);
-    s.t_slack = f(slack(g.q_base, s.base) / g.delta_q + 4.0 * 5.96e-8 * g.qnpts + 1e-9);
-    s.KT_min = f(g.KT_min);
-    s.inv_dKT = f(1.0 / g.dKT);
-    s.kt_t_slack = f(slack(g.KT_min, s.KT_min) / g.dKT + 4.0 * 5.96e-8 * g.n_KT + 1e-9);
-    s.psi = f(g.psi_ref);
-    s.psi_slack = f(slack(g.psi_ref, s.psi));
-    s.two_pi = f(g.two_pi);
-    s.inv_dKphi = f(1.0 / g.dKphi);
-    s.kphi_tol = std::nextafter(f(g.kphi_tol), INFINITY);
+    const double Q = (std::max(-g.q_lo, g.q_hi) + 1e-7) * (1.0 + 1e-6);
+    s.inv_dq = static_cast<float>(1.0 / g.delta_q);
+    s.pqt2 = static_cast<float>(2.0 * Q * Q * (1.0 + 2e-4));
     s.qnpts = g.qnpts;
-    s.n_KT = g.n_KT;
     s.n_Kphi = g.n_Kphi;
-    fill_prefilter(s);
     fill_tile_screen(g, s);
 }
 

@@ -116,27 +116,9 @@ constexpr int kStraddleCols = 256;
 // FP32 copies of the constants used by the FP32 pair screen (hbt_fast.cu),
 // each with the bound on its rounding (slack) relative to the FP64 value.
 struct Screen {
-    float kt_lo4, kt_hi4, kt_slack;  // 4 KT_min^2, 4 KT_max^2 (0: no lower cut)
-    float lo, hi, win_slack;         // q window bounds
-    float base, inv_dq, t_slack;     // bin origin, 1/delta_q, slack in bin units
-    float KT_min, inv_dKT, kt_t_slack;
-    float psi, psi_slack, two_pi, inv_dKphi;
-    int qnpts, n_KT, n_Kphi;
-    // prefilter (hbt_tile.cuh prefilter()): Q = max(-lo, hi) + win_slack
-    // with margin, Q^2, 2 Q^2 and the coefficient of the input-rounding term
-    // of the q_T test
-    float pq, pq2, pqt2, pqt_c;
-    // 1 / hbarC as a double-float pair (FP32-weight phase)
-    float hc_h, hc_l;
-    // q_inv prefilter (invariant_radius_flag): square of the upper window
-    // bound with its slack and a margin; -1 when no q_inv >= 0 can pass
-    float qi_hi2;
-    // Grid::kphi_tol rounded up: the K_phi screen leaves pairs this close to
-    // an edge (plus its error bound) to the reference chain, which hands
-    // them to the host, so that every pass that meets such a pair (the
-    // screened kernels and the pair-by-pair cut rows of cap admission)
-    // decides it the same way
-    float kphi_tol;
+    float inv_dq;         // 1 / delta_q
+    float pqt2;           // above the window: 2 Q^2, Q = max(-q_lo, q_hi), with margin
+    int qnpts, n_Kphi;
     // tile screen (hbt_screen.cuh screen_two): bin coordinate q / bin width +
     // sc_c0, its margin 0.5 - et = sc_h0 + w (sc_nk1 / k + sc_nk2) + e_long
     // sc_nk3, the grid's outer limits sc_top - h and sc_bot + h, qnpts^2,
@@ -151,22 +133,6 @@ struct Screen {
     // quarter turn, margin
     float sp_cos, sp_sin, sp_scale, sp_quarter, sp_h0, sp_nkA;
 };
-
-// Host: the prefilter constants of a screen whose window is filled in.
-inline void fill_prefilter(Screen &s) {
-    const double U = 5.9604644775390625e-8;  // 2^-24
-    const double Q = ((double)(-s.lo > s.hi ? -s.lo : s.hi) + (double)s.win_slack) * (1.0 + 1e-6);
-    s.pq = (float)(Q * (1.0 + 1e-5));
-    s.pq2 = (float)(Q * Q * (1.0 + 2e-4));
-    s.pqt2 = (float)(2.0 * Q * Q * (1.0 + 2e-4));
-    // (c + e)^2 <= c^2 + 2 c e (1 + 1e-4), c = sqrt(2) Q, e = 2.01 u L
-    s.pqt_c = (float)(2.0 * 1.4142135623730951 * Q * 2.01 * U * (1.0 + 2e-4));
-    const double hc = 1.0 / 0.197327053;  // 1 / hbarC [1 / (GeV fm)]
-    s.hc_h = (float)hc;
-    s.hc_l = (float)(hc - (double)s.hc_h);
-    const double qh = ((double)s.hi + (double)s.win_slack) * (1.0 + 1e-6);
-    s.qi_hi2 = qh > 0.0 ? (float)(qh * qh * (1.0 + 2e-4)) : -1.0f;
-}
 
 struct Device {
     Grid g;

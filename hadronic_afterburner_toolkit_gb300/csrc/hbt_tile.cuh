@@ -18,14 +18,14 @@
 //                    (q_out = (q_x S_x + q_y S_y) / |S|, ...) in double-float
 //                    on the FP32 pipe; pairs of particles outside the
 //                    columns' range in FP64 (values64);
-//       FP32W form - each FP64 column split once per tile into hi + lo
-//                    FP32 parts; differences and the phase in double-float
-//                    arithmetic on the FP32 pipe, q values in FP32, cos by
-//                    quadrant reduction and FP32 Taylor polynomials
-//                    (values32_split); added with one float4 vector atomic
-//                    into FP32 partial bins (two arrays, even and odd warps:
-//                    partials_of) that are merged into the FP64 bins with
-//                    Kahan compensation.
+//       FP32W form - differences and the phase from the same fixed-point
+//                    columns, q values in FP32, cos by quadrant reduction and
+//                    FP32 Taylor polynomials (values32_fixed); added with one
+//                    float4 vector atomic into FP32 partial bins (two
+//                    arrays, even and odd warps: partials_of) that are
+//                    merged into the FP64 bins with Kahan compensation.
+//       The double-float form runs the FP64 form's kernels, which are faster
+//       than double-float values were and more precise.
 //     In the FP32-weight form a pair is evaluated as stored (i, j) and
 //     oriented afterwards: swapping first and second negates every momentum
 //     and position difference, so it negates q_out, q_side, q_long exactly
@@ -34,23 +34,15 @@
 //  D. Pairs left undecided by A or B go to another per-warp queue; the
 //     reference chain runs on them 32 at a time.
 //
-// Measured on the central group (150k pions, 5.4e9 pairs in the kept tile
-// pairs, 1.94e9 binned), whole passes, against a scalar prefilter, a queue
-// and a scalar window test with per-component bounds: FP32-weight form 118.0
-// -> 70.6 ms, FP64 form (still with FP64 values) 143.6 -> 134.7 ms, bound by
-// the FP64 pipe, so the issue slots saved showed less.
+// With q_inv histograms the same screen decides the q_inv bin too
+// (screen_qinv) and a pair stays when it is inside either window.
 //
-// The forms with q_inv histograms (same_tile_pair_qinv,
-// mixed_tile_pair_qinv) screen in two steps, a prefilter and a window test
-// on queued pairs, in scalar FP32.  Error analysis of that screen (u = 2^-24).  Inputs are FP64 values v
-// rounded once to FP32: |v32 - v| <= u|v|.  For s = a +- b in FP32, |s - S|
-// <= 2.01 u A with A = |a| + |b| and S the exact sum of the FP64 inputs.
-// Products, sums, the reciprocal square root (rsqrtf: at most 2 ulp) and the
-// approximate divisions used only inside the bounds (__fdividef: at most 2
-// ulp, the bounds carry a 1e-4 relative margin for it) propagate this as
-// coded in screen_lcms() and decide_bins(); every bound is then doubled and
-// widened by the rounding of the FP32 copies of the constants, which also
-// covers the FP64 reference's own rounding (2^-29 times smaller).
+// Measured on the central group (150k pions, 5.4e9 pairs in the kept tile
+// pairs, 1.94e9 binned), the same-event kernel: FP64 form 121.7 -> 51.1 ms,
+// FP32-weight form 94.0 -> 41.7 ms, against a scalar prefilter, a queue, a
+// scalar window test with per-component bounds and FP64 (or split FP32)
+// values.  The FP64 form now keeps the shared-memory and atomics pipe 76 %,
+// the issue slots 66 % and the FP64 pipe 56 % busy.
 #pragma once
 
 #include <type_traits>

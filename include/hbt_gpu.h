@@ -188,7 +188,9 @@ typedef struct hbt_tuning {
     int32_t blocks_per_sm;  /* persistent CTAs per SM, at most 8 (0: each kernel at
                                its occupancy limit) */
     double cell_pt;         /* sort cell of p_x and p_y in GeV (0: 0.02) */
-    double cell_y;          /* sort cell of rapidity (0: 0.05) */
+    double cell_y;          /* sort cell of rapidity (0: 0.05); lists of at most
+                               8192 rows take 128 cells either side of zero, what
+                               lies beyond in the outermost */
     int32_t merge_chunk;    /* FP32-weight form: same-event tile pairs between two
                                merges of the partials, <= 8192 (0: 8192; the
                                bound keeps the numerator within 1e-6 per pair) */
@@ -204,6 +206,8 @@ typedef struct hbt_tuning {
                                CTAs running at any time update few histogram
                                slots (on the central workload 3.3x less DRAM
                                traffic); 0: in the order the cull found them.
+                               Analyses whose histograms are at most 64 MB stay
+                               in L2 whatever the order: they are not ordered.
                                The FP32-weight form always takes the cull's
                                order (its FP32 partials' bound needs the pairs of
                                a merge chunk spread over many bins) */
