@@ -150,7 +150,7 @@ __device__ __forceinline__ double warp_min(double v) {
 // 1000.  The box is FP32 where the cull's bounds allow (rapidity: logarithm
 // of the light-cone terms' ratio, within 2e-6).
 template <bool LC>
-__global__ void __launch_bounds__(FT) k_tiles(BatchDev b, Grid g) {
+__global__ void __launch_bounds__(FT) k_tiles(BatchDev b, Grid g, bool split) {
     __shared__ float part[FT / 32][9];
     __shared__ double part2[FT / 32][2];
     const long long tile = blockIdx.x;
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(FT) k_tiles(BatchDev b, Grid g) {
         b.terms4[s] = make_float4(w.x, w.y, w.m, w.p);
         b.terms2[s] = make_float2(w.r2, w.t2);
         if (l.ncols == 8) {
-            const FixedCols c = fixed_cols(g, v);
+            const FixedCols c = split ? split_cols(v) : fixed_cols(g, v);
 #pragma unroll
             for (int f = 0; f < kFixedCols; f++) b.fixed[(long long)f * b.cap + s] = c.c[f];
         }
@@ -449,10 +449,11 @@ cudaError_t run_batch(const Device &d, const BatchDev &b, int grid, unsigned chu
                                             b.vals_out, (int)b.total, 0, end_bit, st);
         if (e != cudaSuccess) return e;
     }
+    const bool split = d.precision == 1;  // the FP32-weight form's columns
     if (lc)
-        k_tiles<true><<<(unsigned)b.total_tiles, FT, 0, st>>>(b, d.g);
+        k_tiles<true><<<(unsigned)b.total_tiles, FT, 0, st>>>(b, d.g, split);
     else
-        k_tiles<false><<<(unsigned)b.total_tiles, FT, 0, st>>>(b, d.g);
+        k_tiles<false><<<(unsigned)b.total_tiles, FT, 0, st>>>(b, d.g, split);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (b.order_items && b.same_cap > 0 &&
         (e = cudaMemsetAsync(b.item_key_in, 0xff, (size_t)b.same_cap * sizeof(unsigned), st)) !=

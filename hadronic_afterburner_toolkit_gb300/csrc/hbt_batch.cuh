@@ -9,7 +9,7 @@ namespace hbt {
 // Fixed-point columns of a same-event row, in entries of two (hbt_fixed.cuh).
 constexpr int kFixedEntries = 4;
 
-// Lists up to this length are sorted by one block each (k_prepare).
+// Lists up to this length are ordered by one block each (k_order).
 constexpr long long kSmallList = 8192;
 
 // One particle list of a batch, as the caller passed it.

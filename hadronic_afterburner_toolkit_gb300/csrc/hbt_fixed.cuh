@@ -26,7 +26,7 @@
 // high bits, the table point and the remainder are bit fields, and the
 // remainder enters the cosine as an exact FP64 integer.  A particle outside
 // those ranges (or not finite) carries kFar, and its pairs take the FP64
-// values (values64).
+// values (values64_rows).
 //
 // Of the FP64 pipe a binned pair takes 5 instructions, all for the cosine,
 // where the FP64 differences, phase, table reduction and sums took 29.

@@ -253,7 +253,7 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
             return false;
         }
     }
-    // small lists are sorted by one block each (k_prepare), others by CUB
+    // small lists are ordered by one block each (k_order), others by CUB
     const bool small = max_list <= kSmallList;
     const size_t sort_bytes = small ? 0 : batch_sort_temp_bytes(total);
     if (!grow(table_, (size_t)8 * total * sizeof(double), err) ||

@@ -17,13 +17,15 @@
 //                    q_side, q_long from algebraically identical expressions
 //                    (q_out = (q_x S_x + q_y S_y) / |S|, ...) in double-float
 //                    on the FP32 pipe; pairs of particles outside the
-//                    columns' range in FP64 (values64);
-//       FP32W form - differences and the phase from the same fixed-point
-//                    columns, q values in FP32, cos by quadrant reduction and
-//                    FP32 Taylor polynomials (values32_fixed); added with one
-//                    float4 vector atomic into FP32 partial bins (two
-//                    arrays, even and odd warps: partials_of) that are
-//                    merged into the FP64 bins with Kahan compensation.
+//                    columns' range in FP64 (values64_rows);
+//       FP32W form - each FP64 column split once per particle into hi + lo
+//                    FP32 parts; differences and the phase in double-float
+//                    arithmetic on the FP32 pipe, q values in FP32, cos by
+//                    quadrant reduction and FP32 Taylor polynomials
+//                    (values32_split); added with one float4 vector atomic
+//                    into FP32 partial bins (two arrays, even and odd warps:
+//                    partials_of) that are merged into the FP64 bins with
+//                    Kahan compensation.
 //       The double-float form runs the FP64 form's kernels, which are faster
 //       than double-float values were and more precise.
 //     In the FP32-weight form a pair is evaluated as stored (i, j) and
@@ -39,8 +41,8 @@
 //
 // Measured on the central group (150k pions, 5.4e9 pairs in the kept tile
 // pairs, 1.94e9 binned), the same-event kernel: FP64 form 121.7 -> 51.1 ms,
-// FP32-weight form 94.0 -> 41.7 ms, against a scalar prefilter, a queue, a
-// scalar window test with per-component bounds and FP64 (or split FP32)
+// FP32-weight form 94.0 -> 46.2 ms, against a scalar prefilter, a queue, a
+// scalar window test with per-component bounds and, in the FP64 form, FP64
 // values.  The FP64 form now keeps the shared-memory and atomics pipe 76 %,
 // the issue slots 66 % and the FP64 pipe 56 % busy.
 #pragma once
@@ -142,6 +144,14 @@ __device__ __forceinline__ FF fast_two_sum(float a, float b) {
     return FF{s, __fsub_rn(b, __fsub_rn(s, a))};
 }
 
+// (ah + al) - (bh + bl) of two split FP64 values.  A split holds its value
+// to 2^-48 relative; the high parts' difference is exact (two-sum) and the
+// low parts add one FP32 rounding of a term below 2^-47 of the inputs.
+__device__ __forceinline__ FF ff_diff(float2 a, float2 b) {
+    const FF s = two_sum(a.x, -b.x);
+    return two_sum(s.h, __fadd_rn(s.l, __fsub_rn(a.y, b.y)));
+}
+
 __device__ __forceinline__ FF ff_mul(FF a, FF b) {
     const float p = __fmul_rn(a.h, b.h);
     float e = __fmaf_rn(a.h, b.h, -p);
@@ -162,6 +172,26 @@ __device__ __forceinline__ FF ff_neg(FF a) { return FF{-a.h, -a.l}; }
 __device__ __forceinline__ float2 split(double x) {
     const float h = (float)x;
     return make_float2(h, (float)(x - (double)h));
+}
+
+// The eight columns of a particle split, two to an entry of the fixed-point
+// columns' arrays, and back.
+__device__ __forceinline__ FixedCols split_cols(const double *v) {
+    FixedCols r;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 a = split(v[2 * k]), b = split(v[2 * k + 1]);
+        r.c[k] = make_int4(__float_as_int(a.x), __float_as_int(a.y), __float_as_int(b.x),
+                           __float_as_int(b.y));
+    }
+    return r;
+}
+__device__ __forceinline__ void columns_of(const FixedCols &r, float2 *c) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        c[2 * k] = make_float2(__int_as_float(r.c[k].x), __int_as_float(r.c[k].y));
+        c[2 * k + 1] = make_float2(__int_as_float(r.c[k].z), __int_as_float(r.c[k].w));
+    }
 }
 
 // a + b of two split values.
@@ -233,11 +263,12 @@ __device__ __forceinline__ void ff_lcms(const FF *dp, const FF *sp, FF &vo, FF &
     }
 }
 
-// FP64 summed values of an accepted same-event pair (algebraically the
+// FP64 summed values of an accepted same-event pair of particles outside the
+// fixed-point columns' range (algebraically the
 // reference's q_out, q_side, q_long and cos(q.dx / hbarC)).  The momentum
 // differences and sums are FP64 (one rounding each, so that cancelling sums
 // stay exact to the last bits), and so are the phase q.dx and its cos
-// (table_cos of the unrounded product with 1/hbarC, 3e-16).  q_out, q_side
+// (of the unrounded product with 1/hbarC).  q_out, q_side
 // and the boosted q_long, which are only summed, follow in double-float on
 // the FP32 pipe (ff_lcms: about 1e-14 relative) from the FP64 sums and
 // differences split on the integer pipe, and come back as FP64 with one
@@ -245,8 +276,7 @@ __device__ __forceinline__ void ff_lcms(const FF *dp, const FF *sp, FF &vo, FF &
 // (used with the boost only) come in as double-float sums of the particles'
 // split values (2^-47 of the sum: sE does not cancel, and sz enters q_long
 // through sz dE and M_T^2 = (sE - sz)(sE + sz), where its absolute error
-// stays below 1e-14 GeV).  Of the FP64 pipe, which bounds this form, a
-// binned pair then takes 27 to 29 instructions instead of 55.
+// stays below 1e-14 GeV).
 template <bool BOOST>
 __device__ __forceinline__ void lcms64(const double *a, const double *b, FF sz, FF sE, double &qo,
                                        double &qs, double &ql, double &ph) {
@@ -418,89 +448,70 @@ static __device__ __noinline__ double qinv64_rows(const double *const *c, long l
     return sqrt(-(q[3] * q[3] - q[0] * q[0] - q[1] * q[1] - q[2] * q[2]));
 }
 
-// Limbs (h, l) of a difference or sum in FP32, in units of h.
-__device__ __forceinline__ float limbs_f(int h, int l) {
-    return __fmaf_rn(__int2float_rn(l), 0x1p-30f, __int2float_rn(h));
-}
-
-// Summed values of the FP32-weight form from the fixed-point columns, for
-// the pair as stored, negated in q when `swap`: q_out, q_side, q_long in FP32
-// from exact differences and sums (a few 1e-7 relative; q_long = (s(m) d(p) -
-// s(p) d(m)) / (2 sqrt(s(m) s(p))), whose two terms add up); the phase as in
-// values_fixed without the products of the low limbs (below 1e-13 rad), its
-// cos by the quarter period's Taylor polynomials of ff_cos (below 2e-7).
-template <bool BOOST>
-__device__ __forceinline__ float4 values32_fixed(const FixedCols &a, const FixedCols &b,
-                                                 bool swap) {
-    int h[8], l[8];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        h[2 * k] = a.c[k].x - b.c[k].x;
-        l[2 * k] = a.c[k].y - b.c[k].y;
-        h[2 * k + 1] = a.c[k].z - b.c[k].z;
-        l[2 * k + 1] = a.c[k].w - b.c[k].w;
-    }
-    long long hh = 0, hl = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        hh += (long long)h[k] * h[k + 4];
-        hl += (long long)h[k] * l[k + 4];
-        hl += (long long)l[k] * h[k + 4];
-    }
-    hh += hl >> 30;
-    const float unit = swap ? -0x1p-26f : 0x1p-26f;  // GeV
-    const float dx = limbs_f(h[0], l[0]), dy = limbs_f(h[1], l[1]);
-    const float dm = limbs_f(h[2], l[2]), dp = limbs_f(h[3], l[3]);
-    const float sx = limbs_f(a.c[0].x + b.c[0].x, a.c[0].y + b.c[0].y);
-    const float sy = limbs_f(a.c[0].z + b.c[0].z, a.c[0].w + b.c[0].w);
-    const float inv = rsqrt_approx(__fmaf_rn(sx, sx, sy * sy)) * unit;
-    float4 v;
-    v.x = __fmaf_rn(dx, sx, dy * sy) * inv;
-    v.y = __fmaf_rn(dy, sx, -(dx * sy)) * inv;
-    if (BOOST) {
-        // (the low limbs change these sums by 2^-27 GeV at most)
-        const float sm = __uint2float_rn((unsigned)a.c[1].x + (unsigned)b.c[1].x);
-        const float sp = __uint2float_rn((unsigned)a.c[1].z + (unsigned)b.c[1].z);
-        v.z = __fmaf_rn(sm, dp, -(sp * dm)) * (rsqrt_approx(sm * sp) * (0.5f * unit));
+// cos of a phase given as a double-float: reduction by quadrant with pi/2
+// split into three parts (12 + 12 significant bits and the rest, so that
+// j times either leading part is exact for |j| < 2^11), then the FP32
+// Taylor polynomials of values32.  Absolute error below 2e-7.
+__device__ __forceinline__ float ff_cos(FF ph) {
+    const float j = rintf(ph.h * 0.63661977f);  // 2 / pi
+    float x;
+    if (fabsf(j) < 2048.0f) {
+        const float t1 = __fmaf_rn(-j, 1.57080078125f, ph.h);       // exact
+        const FF t2 = two_sum(t1, __fmul_rn(-j, -4.453584551811218e-06f));
+        x = __fadd_rn(t2.h, __fadd_rn(t2.l, __fmaf_rn(-j, -8.705515752716053e-10f, ph.l)));
     } else {
-        v.z = (dp - dm) * (0.5f * unit);
+        // never on this path (|q.dx| / hbarC is a few hundred at most)
+        const double r = (double)ph.h + (double)ph.l;
+        const double k = rint(r * 0.6366197723675814);
+        x = (float)(r - k * 1.5707963267948966);
+        return cosf(x + (float)(fmod(k, 4.0)) * 1.5707964f);
     }
-    // period 2^46 units of hh: quarter and remainder, the latter in 2^-34
-    // periods
-    const int top = (int)(hh >> 32) + 2048;  // + half a quarter
-    const int r = (top & 4095) - 2048, quad = top >> 12;
-    const float x = __int2float_rn((int)__funnelshift_r((unsigned)hh, (unsigned)r, 12)) *
-                    (float)(6.283185307179586 / 17179869184.0);
-    const float x2 = x * x;
+    const float x2 = __fmul_rn(x, x);
     const float c = __fmaf_rn(x2, __fmaf_rn(x2, __fmaf_rn(x2, __fmaf_rn(x2, 2.48015873e-5f,
-                                                                      -1.38888889e-3f),
-                                                          4.16666667e-2f),
-                                            -0.5f),
+                                                                    -1.38888889e-3f),
+                                                        4.16666667e-2f),
+                                          -0.5f),
                               1.0f);
     const float s = x * __fmaf_rn(x2, __fmaf_rn(x2, __fmaf_rn(x2, __fmaf_rn(x2, 2.75573192e-6f,
-                                                                          -1.98412698e-4f),
-                                                              8.33333333e-3f),
-                                                -1.66666667e-1f),
-                                  1.0f);
-    // cos(x + quad pi / 2): c, -s, -c, s
-    v.w = __uint_as_float(__float_as_uint(quad & 1 ? s : c) ^
-                          ((unsigned)((quad + 1) & 2) << 30));
-    return v;
+                                                                        -1.98412698e-4f),
+                                                            8.33333333e-3f),
+                                              -1.66666667e-1f),
+                                1.0f);
+    const int quad = ((int)j) & 3;  // cos(x + j pi/2)
+    return quad == 0 ? c : quad == 1 ? -s : quad == 2 ? -c : s;
 }
 
-// values32 from the FP64 columns of rows i and j (pairs of particles that do
-// not fit the fixed-point columns; out of line, as values64_rows).
+// Summed values of the FP32-weight form from split FP64 inputs, all on the
+// FP32 pipe: momentum and position differences in double-float (their
+// rounding relative to the difference, not to the momenta), q_out, q_side,
+// q_long in FP32 (a few 1e-7 relative), the phase (q.dx)/hbarC in
+// double-float and its cos by ff_cos.  a, b: the eight split columns of the
+// pair's first and second particle.
 template <bool BOOST>
-__device__ __noinline__ float4 values32_rows(const Grid &g, const double *const *c, long long i,
-                                             long long j, bool swap) {
-    double a[8], b[8];
-#pragma unroll
-    for (int f = 0; f < 8; f++) {
-        const double u = c[f][i], v = c[f][j];
-        a[f] = swap ? v : u;
-        b[f] = swap ? u : v;
+__device__ __forceinline__ float4 values32_split(const float2 *a, const float2 *b) {
+    const FF dx = ff_diff(a[0], b[0]), dy = ff_diff(a[1], b[1]);
+    const FF dz = ff_diff(a[2], b[2]), dE = ff_diff(a[3], b[3]);
+    const float sx = __fadd_rn(__fadd_rn(a[0].x, b[0].x), __fadd_rn(a[0].y, b[0].y));
+    const float sy = __fadd_rn(__fadd_rn(a[1].x, b[1].x), __fadd_rn(a[1].y, b[1].y));
+    const float inv = rsqrtf(__fmaf_rn(sx, sx, sy * sy));
+    float4 v;
+    v.x = __fmaf_rn(dx.h, sx, dy.h * sy) * inv;
+    v.y = __fmaf_rn(dy.h, sx, -(dx.h * sy)) * inv;
+    if (BOOST) {
+        const float sE = __fadd_rn(__fadd_rn(a[3].x, b[3].x), __fadd_rn(a[3].y, b[3].y));
+        const float sz = __fadd_rn(__fadd_rn(a[2].x, b[2].x), __fadd_rn(a[2].y, b[2].y));
+        v.z = __fmaf_rn(sE, dz.h, -(sz * dE.h)) * rsqrtf((sE - sz) * (sE + sz));
+    } else {
+        v.z = dz.h;
     }
-    return values32<BOOST>(g, a, b);
+    FF ph = ff_mul(dE, ff_diff(a[7], b[7]));
+    ph = ff_add(ph, ff_neg(ff_mul(dx, ff_diff(a[4], b[4]))));
+    ph = ff_add(ph, ff_neg(ff_mul(dy, ff_diff(a[5], b[5]))));
+    ph = ff_add(ph, ff_neg(ff_mul(dz, ff_diff(a[6], b[6]))));
+    constexpr double hc = 1.0 / kHbarC;  // split
+    ph = ff_mul(ph, FF{(float)hc, (float)(hc - (double)(float)hc)});
+    v.w = ff_cos(ph);
+    return v;
 }
 
 // Shared memory of a same-event tile pair.  The i-tile's arrays hold row r at
@@ -701,19 +712,21 @@ __device__ __forceinline__ Terms load_terms(const ListRows &l, long long k, floa
     return Terms{a.x, a.y, a.z, a.w, b.x, b.y};
 }
 
-// Fixed-point columns of row k.
-__device__ __forceinline__ FixedCols load_fixed(const Grid &g, const ListRows &l, long long k) {
+// Row k's columns for the values of a form (zero past the list's end): the
+// fixed-point ones, or the split ones of the FP32-weight form.
+template <int PREC>
+__device__ __forceinline__ FixedCols load_cols(const Grid &g, const ListRows &l, long long k) {
     FixedCols r = {};
     if (k >= l.n) return r;
     if (l.fixed) {
 #pragma unroll
-            for (int f = 0; f < kFixedCols; f++) r.c[f] = l.fixed[f * l.stride + k];
+        for (int f = 0; f < kFixedCols; f++) r.c[f] = l.fixed[f * l.stride + k];
         return r;
     }
     double v[8];
 #pragma unroll
     for (int f = 0; f < 8; f++) v[f] = l.c[f][k];
-    return fixed_cols(g, v);
+    return PREC == 1 ? split_cols(v) : fixed_cols(g, v);
 }
 
 // The pair loop: screens this lane's row against particles [jbegin, jend) of
@@ -825,7 +838,8 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
     const long long n = l.n;
     const double *const *c = l.c;
     {
-        const FixedCols a = load_fixed(d.g, l, i0 + tid), b = load_fixed(d.g, l, j0 + tid);
+        const FixedCols a = load_cols<PREC>(d.g, l, i0 + tid),
+                        b = load_cols<PREC>(d.g, l, j0 + tid);
 #pragma unroll
         for (int f = 0; f < kFixedCols; f++) {
             sm.xi[f][at_i] = a.c[f];
@@ -892,19 +906,26 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
             a.c[f] = sm.xi[f][qi];
             b.c[f] = sm.xj[f][qj];
         }
-        const bool far = a.c[1].x == kFar || b.c[1].x == kFar;
-        if (QINV && hasq)
-            vq = far ? qinv64_rows(c, i0 + row_at(qi), j0 + qj, swap) : qinv_fixed(a, b);
         if (PREC == 1) {
-            float4 v;
-            if (far)
-                v = values32_rows<BOOST>(d.g, c, i0 + row_at(qi), j0 + qj, swap);
-            else
-                v = values32_fixed<BOOST>(a, b, swap);
+            if (QINV && hasq) vq = qinv64_rows(c, i0 + row_at(qi), j0 + qj, swap);
+            // the pair as stored (i, j); swapping first and second negates
+            // q_out, q_side, q_long exactly and leaves the phase unchanged
+            float2 sa[8], sb[8];
+            columns_of(a, sa);
+            columns_of(b, sb);
+            float4 v = values32_split<BOOST>(sa, sb);
+            if (swap) {
+                v.x = -v.x;
+                v.y = -v.y;
+                v.z = -v.z;
+            }
             if (!QINV || has3) atomicAdd(partials_of(d) + at, v);
             if (QINV) vw = (double)v.w;
             return nullptr;
         }
+        const bool far = a.c[1].x == kFar || b.c[1].x == kFar;
+        if (QINV && hasq)
+            vq = far ? qinv64_rows(c, i0 + row_at(qi), j0 + qj, swap) : qinv_fixed(a, b);
         if (far)
             values64_rows<BOOST>(d.g, c, i0 + row_at(qi), j0 + qj, swap, vo, vs, vl, vw);
         else
