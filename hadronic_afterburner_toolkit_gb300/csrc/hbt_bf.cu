@@ -246,7 +246,7 @@ __device__ __forceinline__ void count_one(unsigned at, unsigned k, unsigned n) {
 // n_a particles is ceil(n_a / 128) items, so the grid holds several waves
 // of similar items instead of one CTA per event pair.  A's terms sit in
 // registers (one particle per thread), B's are staged through shared memory
-// 128 at a time; the histogram is privatised in shared memory and its
+// 256 at a time; the histogram is privatised in shared memory and its
 // non-zero bins are added to the global one when the item is done.
 //
 // A pair costs two broadcast reads, six packed FP32 operations (rint by the
