@@ -186,9 +186,10 @@ __device__ __forceinline__ Row row_of(const Terms &a) {
 //   transverse part      8.1 u (|d_x| + |d_y|) w
 //   longitudinal part    2.1 u (s_m |d_p| + s_p |d_m|)
 //   roundings            4 u (|d_T|^2 + |d_m d_p|)
-// and |sqrt(t) - sqrt(T)| <= |t - T| / sqrt(t), plus 4 u of it for the
-// reciprocal root and the product.  q_inv^2 certainly negative: no event (the
-// reference's NaN fails both bounds).
+// and, T not negative, |sqrt(t) - sqrt(T)| <= |t - T| / sqrt(t), plus 4 u of it
+// for the reciprocal root and the product.  q_inv^2 certainly negative: no
+// event (the reference's NaN fails both bounds); its sign not certain (t up to
+// twice the bound): undecided, as a T below zero has no root to be near to.
 __device__ __forceinline__ void screen_qinv(const Screen &S, const Row &a, const f2 *v, f2 w,
                                             Screened &r) {
     const f2 dx = fma2(v[0], both(-2.0f), a.x2), dy = fma2(v[1], both(-2.0f), a.y2);  // twice
@@ -220,7 +221,7 @@ __device__ __forceinline__ void screen_qinv(const Screen &S, const Row &a, const
         const float tq = __fmaf_rn(qi, S.inv_dq, S.sc_c0);
         const float kr = tq + kRound;
         r.takeq[k] = !(t[k] + e < 0.0f) && !(tq > S.sc_top - h) && !(tq < S.sc_bot + h);
-        r.undq[k] = !(fabsf(tq - (kr - kRound)) < h);
+        r.undq[k] = !(t[k] > 2.0f * e) || !(fabsf(tq - (kr - kRound)) < h);
         r.kq[k] = __float_as_uint(kr) - kRoundBits;
     }
 }
