@@ -425,23 +425,15 @@ __device__ __forceinline__ void values_fixed(const Grid &g, const double *t, con
     w = cos_fixed(g, t, hh + (hl >> 30), (unsigned)hl);
 }
 
-// q_inv of a pair inside the q_inv window, from its fixed-point columns:
-// q_x^2 + q_y^2 - d(m) d(p) and its root in double-float (about 1e-14
-// relative; the reference's FP64 expression rounds q_E^2 and so has 1e-16
-// GeV^2 in q_inv^2).
-__device__ __forceinline__ double qinv_fixed(const FixedCols &a, const FixedCols &b) {
-    const FF dx = limbs_ff(a.c[0].x - b.c[0].x, a.c[0].y - b.c[0].y);
-    const FF dy = limbs_ff(a.c[0].z - b.c[0].z, a.c[0].w - b.c[0].w);
-    const FF dm = limbs_ff(a.c[1].x - b.c[1].x, a.c[1].y - b.c[1].y);
-    const FF dp = limbs_ff(a.c[1].z - b.c[1].z, a.c[1].w - b.c[1].w);
-    const FF t = ff_add(ff_dot(dx, dx, dy, dy), ff_neg(ff_mul(dm, dp)));
-    return ff_scaled(ff_mul(t, ff_rsqrt_fast(t)), 0u, -26);
-}
-
-// The reference's FP64 expression (src/HBT_correlation.cpp:334-337) from the
-// columns of rows i and j, for the pairs outside the fixed-point range.
-static __device__ __noinline__ double qinv64_rows(const double *const *c, long long i, long long j,
-                                                  bool swap) {
+// q_inv by the reference's FP64 expression (src/HBT_correlation.cpp:334-337),
+// from the FP64 columns of rows i and j: bound by its 20 FP64 instructions
+// (45,000 pions 18.9 ms a call; 19.1 ms with the momenta in shared memory, 18.3
+// ms with the root by a corrected estimate).  From the fixed-point columns it
+// cannot have the expression's precision: in double-float it took 12.6 ms, but
+// had 6e-15 rms of relative error in the place of 1e-16, and their 2^-57 GeV
+// alone are 1e-15 of a q_inv of 5 MeV.
+__device__ __forceinline__ double qinv64(const double *const *c, long long i, long long j,
+                                         bool swap) {
     double q[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) q[f] = swap ? c[f][j] - c[f][i] : c[f][i] - c[f][j];
@@ -906,8 +898,8 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
             a.c[f] = sm.xi[f][qi];
             b.c[f] = sm.xj[f][qj];
         }
+        if (QINV && hasq) vq = qinv64(c, i0 + row_at(qi), j0 + qj, swap);
         if (PREC == 1) {
-            if (QINV && hasq) vq = qinv64_rows(c, i0 + row_at(qi), j0 + qj, swap);
             // the pair as stored (i, j); swapping first and second negates
             // q_out, q_side, q_long exactly and leaves the phase unchanged
             float2 sa[8], sb[8];
@@ -924,8 +916,6 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
             return nullptr;
         }
         const bool far = a.c[1].x == kFar || b.c[1].x == kFar;
-        if (QINV && hasq)
-            vq = far ? qinv64_rows(c, i0 + row_at(qi), j0 + qj, swap) : qinv_fixed(a, b);
         if (far)
             values64_rows<BOOST>(d.g, c, i0 + row_at(qi), j0 + qj, swap, vo, vs, vl, vw);
         else
