@@ -20,6 +20,7 @@
 
 #include "../../include/hbt_bf.h"
 #include "hbt_engine.cuh"
+#include "hbt_hostmem.h"
 #include "hbt_screen.cuh"
 
 namespace {
@@ -519,7 +520,7 @@ hbt_status hbt_bf_bin(hbt_bf_ctx *c, int32_t n_lists, const hbt_bf_list *lists, 
     c->segs.clear();
     auto copy = [&](void *dst, const void *src, long long n_doubles) {
         if (e != cudaSuccess) return;
-        if (!c->reads_host) {
+        if (!c->reads_host || hbt::host_route(src) != hbt::HostRoute::kKernel) {
             e = cudaMemcpyAsync(dst, src, n_doubles * sizeof(double), cudaMemcpyHostToDevice,
                                 c->stream);
             return;
@@ -600,7 +601,7 @@ hbt_status hbt_bf_read(hbt_bf_ctx *c, int32_t hist, double *out) {
     if (!c || hist < 0 || hist > 7 || !out) return HBT_ERR_INVALID;
     const size_t nb = (size_t)c->p.Bnpts * kNphi;
     if (cudaSetDevice(c->device) != cudaSuccess) return bf_fail(c, HBT_ERR_CUDA, "cudaSetDevice");
-    if (c->reads_host) {
+    if (c->reads_host && hbt::host_route(out) == hbt::HostRoute::kKernel) {
         // the host maps the pages, one kernel writes them
         for (size_t k = 0; k < nb; k += 512) static_cast<volatile double *>(out)[k] = 0.0;
         static_cast<volatile double *>(out)[nb - 1] = 0.0;

@@ -22,6 +22,7 @@
 #include "../../include/hbt_gpu.h"
 #include "hbt_batch.cuh"
 #include "hbt_engine.cuh"
+#include "hbt_hostmem.h"
 #include "hbt_internal.h"
 #include "hbt_runner.h"
 
@@ -745,7 +746,10 @@ hbt_status stage(hbt_ctx *c, const double *const *src, const long long *len, int
         off += (size_t)((len[f] + 31) / 32 * 32);
     }
     // where the GPU reads host memory itself, one kernel takes all columns
-    if (c->reads_host) {
+    bool kernel = c->reads_host;
+    for (int f = 0; f < ncols && kernel; f++)
+        kernel = len[f] <= 0 || hbt::host_route(src[f]) == hbt::HostRoute::kKernel;
+    if (kernel) {
         c->segs.clear();
         for (int f = 0; f < ncols; f++) {
             if (len[f] <= 0) continue;
@@ -761,7 +765,7 @@ hbt_status stage(hbt_ctx *c, const double *const *src, const long long *len, int
     }
     // otherwise columns laid out in host memory as they will be on the device
     // (each a multiple of 32 doubles, back to back) go over in one copy per run
-    for (int f = c->reads_host ? ncols : 0; f < ncols;) {
+    for (int f = kernel ? ncols : 0; f < ncols;) {
         if (len[f] <= 0) {
             f++;
             continue;
@@ -1384,6 +1388,14 @@ void map_pages(double *const *dst, int n, size_t count) {
     for (std::thread &t : pool) t.join();
 }
 
+// Can a kernel write the caller's arrays (any may be null)?
+bool exports(const hbt_ctx *c, double *const *dst, int n) {
+    bool kernel = c->reads_host;
+    for (int f = 0; f < n; f++)
+        kernel = kernel && hbt::host_route(dst[f]) == hbt::HostRoute::kKernel;
+    return kernel;
+}
+
 // Exports the arrays to host memory by a kernel and waits for it.
 hbt_status export_to_host(hbt_ctx *c, double *const *dst, int n, size_t count, bool qinv) {
     hbt::HistOut o = {};
@@ -1411,7 +1423,7 @@ hbt_status hbt_read_hist(hbt_ctx *c, double *num_count, double *q_out_sum, doubl
     TRY(drain_deferrals(c));
     // small histograms by one kernel that writes host memory; for large ones
     // the copy engine is faster (238 MB: 1.5 against 2.2 ms)
-    if (c->reads_host && 6 * nb * sizeof(double) <= (16u << 20))
+    if (exports(c, dst, 6) && 6 * nb * sizeof(double) <= (16u << 20))
         return export_to_host(c, dst, 6, nb, false);
     TRY(hbt_sync(c, 0));
     // each array is laid out as FP64 on the device (k_export), then copied
@@ -1484,8 +1496,8 @@ hbt_status hbt_read_qinv(hbt_ctx *c, double *qinv_sum, double *num, double *num_
     if (!c) return HBT_ERR_INVALID;
     CU(cudaSetDevice(c->device));
     const size_t nq = (size_t)c->d.g.n_KT * c->d.g.qnpts;
-    if (c->reads_host) {
-        double *dst[4] = {qinv_sum, num, num_count, den};
+    double *dst[4] = {qinv_sum, num, num_count, den};
+    if (exports(c, dst, 4)) {
         map_pages(dst, 4, nq);
         return export_to_host(c, dst, 4, nq, true);
     }

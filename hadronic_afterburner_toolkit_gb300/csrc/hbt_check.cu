@@ -1,6 +1,7 @@
 // Device evaluation of the table-driven FP64 functions and of the
 // double-float cos of the pair kernels (include/hbt_check.h).
 #include "../../include/hbt_check.h"
+#include "hbt_hostmem.h"
 #include "hbt_math.cuh"
 #include "hbt_tile.cuh"
 
@@ -133,4 +134,8 @@ extern "C" hbt_status hbt_check_math(int device, int32_t which, int64_t n, const
     if (e == cudaSuccess) e = cudaMemcpy(out, d + n, n * sizeof(double), cudaMemcpyDeviceToHost);
     cudaFree(d);
     return e == cudaSuccess ? HBT_OK : HBT_ERR_CUDA;
+}
+
+extern "C" int32_t hbt_check_host_route(const void *p) {
+    return static_cast<int32_t>(hbt::host_route(p));
 }

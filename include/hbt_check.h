@@ -26,6 +26,10 @@ extern "C" {
 /* out[i] = f(x[i]) on `device` for the function `which`; host arrays. */
 hbt_status hbt_check_math(int device, int32_t which, int64_t n, const double *x, double *out);
 
+/* How the library reads or writes a caller's array of doubles at p where the
+ * GPU reaches host memory itself: 2 by a kernel, 1 by copies.  No device call. */
+int32_t hbt_check_host_route(const void *p);
+
 #ifdef __cplusplus
 }
 #endif
