@@ -60,13 +60,16 @@ void hbt_bf_destroy(hbt_bf_ctx *ctx);
 const char *hbt_bf_last_error(const hbt_bf_ctx *ctx);
 hbt_status hbt_bf_reset(hbt_bf_ctx *ctx);
 
-/* Bins the jobs over `n_lists` species lists (host arrays, copied during the
- * call) in one launch; counts add to the histograms. */
+/* Bins the jobs over `n_lists` species lists (host arrays at any address, every
+ * element readable by the process, copied during the call) in one launch;
+ * counts add to the histograms. */
 hbt_status hbt_bf_bin(hbt_bf_ctx *ctx, int32_t n_lists, const hbt_bf_list *lists,
                       int32_t n_jobs, const hbt_bf_job *jobs);
 
 /* Counts of histogram `hist`, Bnpts x HBT_BF_NPHI doubles, [y bin][phi bin]
- * (the reference's C_ab ... C_mixed_abarb arrays). */
+ * (the reference's C_ab ... C_mixed_abarb arrays).  Every element must be
+ * writable by the process; when the call fails, the array's contents are
+ * unspecified. */
 hbt_status hbt_bf_read(hbt_bf_ctx *ctx, int32_t hist, double *out);
 
 /* What the last hbt_bf_bin did: candidate pairs, bytes copied to the device

@@ -142,8 +142,9 @@ hbt_status hbt_set_psi_ref(hbt_ctx *ctx, double psi_ref);
 /* Zeroes histograms, pair counters and statistics. */
 hbt_status hbt_reset(hbt_ctx *ctx);
 
-/* Same-event pairs i < j of one gathered buffer, host arrays
- * (replaces the pair loop of HBT_correlation::combine_and_bin_particle_pairs,
+/* Same-event pairs i < j of one gathered buffer, host arrays (of this call and
+ * the host calls below: at any address, every element readable by the process;
+ * a pointer to anything else ends it) (replaces the pair loop of HBT_correlation::combine_and_bin_particle_pairs,
  * src/HBT_correlation.cpp:282-461). */
 hbt_status hbt_bin_same(hbt_ctx *ctx, int64_t n, const hbt_soa8 *list);
 
@@ -239,8 +240,8 @@ int64_t hbt_n_bins(const hbt_ctx *ctx);
  * numerator, denominator pair count.  These are the arrays the reference's
  * writer reads (correl_3d_num_count, q_out_mean, q_side_mean, q_long_mean,
  * correl_3d_num, correl_3d_denorm and their K_phi twins,
- * src/HBT_correlation.h:55-61).  When the call fails, the arrays' contents
- * are unspecified. */
+ * src/HBT_correlation.h:55-61).  Every element must be writable by the process;
+ * when the call fails, the arrays' contents are unspecified. */
 hbt_status hbt_read_hist(hbt_ctx *ctx, double *num_count, double *q_out_sum,
                          double *q_side_sum, double *q_long_sum, double *num,
                          double *den);
@@ -259,7 +260,8 @@ hbt_status hbt_read_hist_async(hbt_ctx *ctx, double *num_count, double *q_out_su
 hbt_status hbt_read_hist_wait(hbt_ctx *ctx);
 
 /* q_inv histograms, n_KT * qnpts doubles each (q_inv_mean,
- * correl_1d_inv_num, correl_1d_inv_num_count, correl_1d_inv_denorm). */
+ * correl_1d_inv_num, correl_1d_inv_num_count, correl_1d_inv_denorm); the
+ * arrays as for hbt_read_hist. */
 hbt_status hbt_read_qinv(hbt_ctx *ctx, double *qinv_sum, double *num,
                          double *num_count, double *den);
 
