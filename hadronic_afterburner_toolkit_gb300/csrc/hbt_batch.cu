@@ -194,11 +194,14 @@ __global__ void __launch_bounds__(FT) k_tiles(BatchDev b, Grid g, bool split) {
         q[2] = q[6] = -inf;  // no sound rapidity: never cull on it
         q[8] = 0.0f;
         mm0 = mm1 = -1e300;  // never treated as one mass
-        if (LC && w.x == w.x) {
-            const float y = 0.5f * logf(w.p / w.m), e = 2e-6f + 1e-6f * fabsf(y);
+        // up to rapidity 10.7 the reference's q_long stays within the cull's
+        // margin (1e-6) of the bound: 3 2^-53 of gamma^2
+        const float m = (float)(v[3] - v[2]), p = (float)(v[3] + v[2]);
+        if (LC && m * 0x1p31f > p && p * 0x1p31f > m) {
+            const float y = 0.5f * logf(p / m), e = 2e-6f + 1e-6f * fabsf(y);
             q[2] = y - e;
             q[6] = -(y + e);
-            q[8] = sqrtf(fmaxf(w.t2, 0.0f)) * (1.0f - 1e-6f);
+            q[8] = sqrtf(m * p) * (1.0f - 1e-6f);
             if (g.qinv) {
                 const double mm = (v[3] - v[2]) * (v[3] + v[2]) - (v[0] * v[0] + v[1] * v[1]);
                 if (mm == mm) {

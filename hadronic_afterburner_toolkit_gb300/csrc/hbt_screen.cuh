@@ -41,9 +41,13 @@
 // In units of the bin width, doubled, plus the rounding of the conversion
 // to bins and the distance of the window's bounds from the outer bin edges
 // (1e-8 GeV), this is the one margin et of a pair's three bins.  The
-// reference's own FP64 rounding is 2^-29 times smaller (particles with
-// p > 2^19 m or m > 2^19 p, where it is not, and unphysical ones get NaN
-// terms: all their pairs are undecided).  A pair is outside when a bin coordinate
+// reference's own FP64 rounding is 2^-29 times smaller but for that of q_long,
+// which cancels from E and p_z: some 20 2^-53 gamma^2 of Q, at p = 2^28 m
+// (rapidity 9.7) a third of this bound.  Particles beyond get a NaN t2,
+// unphysical ones NaN for all longitudinal terms: their pairs that pass the
+// transverse test are undecided (with NaN for all terms from rapidity 6.6 on,
+// 30,000 particles spread to 8 took 28.6 ms in the place of 1.0).  A pair is
+// outside when a bin coordinate
 // lies beyond the grid by more than et, decided when all three lie farther
 // than et from a bin edge, undecided otherwise; a NaN or infinite margin
 // (k = 0, an overflow) leaves it undecided.  The coefficient of w / k is at
@@ -127,9 +131,9 @@ __device__ __forceinline__ Terms screen_terms(double px, double py, double pz, d
         t.m = (float)m;
         t.p = (float)p;
         t.t2 = (float)(m * p);
-        // |rapidity| below 6.6; false for NaN too
-        const bool sound = t.m * 524288.0f > t.p && t.p * 524288.0f > t.m;
-        if (!sound) t.x = t.y = t.r2 = t.m = t.p = t.t2 = __int_as_float(0x7fffffff);
+        const float nan = __int_as_float(0x7fffffff);
+        if (!(t.m * 0x1p28f > t.p && t.p * 0x1p28f > t.m)) t.t2 = nan;  // rapidity past 9.7
+        if (!(t.m > 0.0f && t.p > 0.0f)) t.m = t.p = nan;               // E <= |p_z|, NaN
     } else {
         t.m = (float)pz;
         t.p = fabsf(t.m);
@@ -186,10 +190,13 @@ __device__ __forceinline__ Row row_of(const Terms &a) {
 //   transverse part      8.1 u (|d_x| + |d_y|) w
 //   longitudinal part    2.1 u (s_m |d_p| + s_p |d_m|)
 //   roundings            4 u (|d_T|^2 + |d_m d_p|)
+//   the reference's q_E^2 - q_z^2 in FP64
+//                        2^-51 (d_m^2 + d_p^2) = 2.1 u (2^-28 d_m^2 + 2^-28 d_p^2)
 // and, T not negative, |sqrt(t) - sqrt(T)| <= |t - T| / sqrt(t), plus 4 u of it
 // for the reciprocal root and the product.  q_inv^2 certainly negative: no
-// event (the reference's NaN fails both bounds); its sign not certain (t up to
-// twice the bound): undecided, as a T below zero has no root to be near to.
+// event (the reference's NaN fails both bounds); its sign not certain (within
+// twice the bound of zero): undecided, as a T below zero has no root to be near
+// to.
 __device__ __forceinline__ void screen_qinv(const Screen &S, const Row &a, const f2 *v, f2 w,
                                             Screened &r) {
     const f2 dx = fma2(v[0], both(-2.0f), a.x2), dy = fma2(v[1], both(-2.0f), a.y2);  // twice
@@ -212,15 +219,16 @@ __device__ __forceinline__ void screen_qinv(const Screen &S, const Row &a, const
     constexpr float U = 5.9604645e-8f;
 #pragma unroll
     for (int k = 0; k < 2; k++) {
+        const float Mp = __fmaf_rn(0x1p-28f, fabsf(p[k]), M[k]);
+        const float Pm = __fmaf_rn(0x1p-28f, fabsf(m[k]), P[k]);
         const float e = U * __fmaf_rn(4.1f * (fabsf(x[k]) + fabsf(y[k])), W[k],
-                                      __fmaf_rn(2.1f, __fmaf_rn(M[k], fabsf(p[k]),
-                                                                P[k] * fabsf(m[k])),
+                                      __fmaf_rn(2.1f, __fmaf_rn(Mp, fabsf(p[k]), Pm * fabsf(m[k])),
                                                 q[k] + 4.0f * fabsf(g[k])));
         const float rs = rsqrt_approx(t[k]), qi = t[k] * rs;
         const float h = __fmaf_rn(__fmaf_rn(e, rs, 4.0f * U * qi), S.sc_nkq, S.sc_h0);
         const float tq = __fmaf_rn(qi, S.inv_dq, S.sc_c0);
         const float kr = tq + kRound;
-        r.takeq[k] = !(t[k] + e < 0.0f) && !(tq > S.sc_top - h) && !(tq < S.sc_bot + h);
+        r.takeq[k] = !(t[k] + 2.0f * e < 0.0f) && !(tq > S.sc_top - h) && !(tq < S.sc_bot + h);
         r.undq[k] = !(t[k] > 2.0f * e) || !(fabsf(tq - (kr - kRound)) < h);
         r.kq[k] = __float_as_uint(kr) - kRoundBits;
     }
