@@ -25,8 +25,8 @@
 // sum of four rounded products has about 5e-15).  Whole periods drop out as
 // high bits, the table point and the remainder are bit fields, and the
 // remainder enters the cosine as an exact FP64 integer.  A particle outside
-// those ranges (or not finite) carries kFar, and its pairs take the FP64
-// values (values64_rows).
+// those ranges (or not finite) carries kFar in v, and in m where its momentum is
+// outside; its pairs take the FP64 phase, or all values in FP64 (far_values).
 //
 // Of the FP64 pipe a binned pair takes 5 instructions, all for the cosine,
 // where the FP64 differences, phase, table reduction and sums took 29.
@@ -37,7 +37,7 @@
 namespace hbt {
 namespace tile {
 
-constexpr int kFar = (int)0x80000000;  // h limb of E: not representable
+constexpr int kFar = (int)0x80000000;  // h limb of m or v: not representable
 
 // hi + lo (|hi| < 2^31, in units of h) as limbs.
 __device__ __forceinline__ int2 to_limbs(double hi, double lo) {
@@ -66,22 +66,22 @@ struct FixedCols {
 // v: px py pz E x y z t.
 __device__ __forceinline__ FixedCols fixed_cols(const Grid &g, const double *v) {
     int2 q[8];
-    bool near = true;
+    bool near_p = true, near_x = true;
 #pragma unroll
     for (int f = 0; f < 8; f++) {
         double hi, lo = 0.0;
         if (f < 4) {
-            near = near && fabs(v[f]) < 8.0;
+            near_p = near_p && fabs(v[f]) < 8.0;
             hi = v[f] * 67108864.0;  // 2^26
         } else {
             hi = v[f] * g.pos_h;
             lo = __fma_rn(v[f], g.pos_h, -hi) + v[f] * g.pos_l;
-            near = near && fabs(hi) < 536870912.0;  // 2^18 2^11
+            near_x = near_x && fabs(hi) < 536870912.0;  // 2^18 2^11
         }
         q[f] = to_limbs(hi, lo);
     }
     // E > |p_z|: m and p positive, their sums below 2^31 as unsigned h
-    near = near && v[3] > fabs(v[2]);
+    near_p = near_p && v[3] > fabs(v[2]);
     const long long E = join_limbs(q[3]), z = join_limbs(q[2]);
     const long long T = join_limbs(q[7]), Z = join_limbs(q[6]);
     const int2 m = split_limbs(E - z), p = split_limbs(E + z);
@@ -89,21 +89,10 @@ __device__ __forceinline__ FixedCols fixed_cols(const Grid &g, const double *v) 
     const int2 X = split_limbs(-join_limbs(q[4])), Y = split_limbs(-join_limbs(q[5]));
     FixedCols r;
     r.c[0] = make_int4(q[0].x, q[0].y, q[1].x, q[1].y);
-    r.c[1] = make_int4(near ? m.x : kFar, m.y, p.x, p.y);
+    r.c[1] = make_int4(near_p ? m.x : kFar, m.y, p.x, p.y);
     r.c[2] = make_int4(X.x, X.y, Y.x, Y.y);
-    r.c[3] = make_int4(vv.x, vv.y, uu.x, uu.y);
+    r.c[3] = make_int4(near_p && near_x ? vv.x : kFar, vv.y, uu.x, uu.y);
     return r;
-}
-
-// Cosine table of the fixed-point values: cos(2 pi k / 2048) for a quarter
-// period, k = 0..512, filled by each CTA (FP64 alone: with an FP32 copy beside
-// each entry, the random reads took twice the shared-memory wavefronts).  The
-// last entry, zero, is a number too small to matter whose exponent fits FP32
-// (cos_fixed takes FP32 values from the bits).
-constexpr int kCosEntries = 513;
-__device__ __forceinline__ void fill_cos_entries(double *t) {
-    for (int k = threadIdx.x; k < kCosEntries; k += blockDim.x)
-        t[k] = k < kCosEntries - 1 ? cospi(k / 1024.0) : 0x1p-100;
 }
 
 // The FP32 value of the leading 24 bits of a normal FP64 one within FP32's

@@ -8,16 +8,24 @@
 #include <cmath>
 #include <cstring>
 
-// Table of cos and sin of 2 pi k / 512, k = 0..511, for table_cos, filled
-// by each CTA of the FP64-form same-event kernels.
-constexpr int COS_TABLE = 512;
-__device__ __forceinline__ void fill_cos_table(double2 *cs) {
-    for (int k = threadIdx.x; k < COS_TABLE; k += blockDim.x) {
-        double sn, cn;
-        sincospi(k / 256.0, &sn, &cn);
-        cs[k] = make_double2(cn, sn);
-    }
+// Cosine table of the pair kernels: cos(2 pi k / 2048) for a quarter period, k =
+// 0..512 (FP64 alone: with an FP32 copy beside each entry, the random reads took
+// twice the shared-memory wavefronts).  The last entry, zero, is a number too
+// small to matter whose exponent fits FP32 (cos_fixed takes FP32 values from the
+// bits).  Made on the host for the batched path, by each CTA elsewhere.
+constexpr int kCosEntries = 513;
+static inline void cos_entries(double *t) {
+    for (int k = 0; k < kCosEntries - 1; k++)
+        t[k] = (double)cosl(3.14159265358979323846264338327950288L * k / 1024.0L);
+    t[kCosEntries - 1] = std::ldexp(1.0, -100);
 }
+__device__ __forceinline__ void fill_cos_entries(double *t) {
+    for (int k = threadIdx.x; k < kCosEntries; k += blockDim.x)
+        t[k] = k < kCosEntries - 1 ? cospi(k / 1024.0) : 0x1p-100;
+}
+
+// Points of a period that table_cos takes from it.
+constexpr int COS_POINTS = 512;
 
 // Constants of table_cos for one scale h: it returns cos(h ph) of a phase
 // ph (h = 1 / hbarC for the pair numerators, h = 1 for a plain cos), with
@@ -69,18 +77,26 @@ static inline CosScale make_cos_scale(double h) {
 // (truncation below 1e-16 and 1e-18).  |ph| >= L (k could reach 2^27;
 // never on the pair path, where |q.dx| / hbarC is a few hundred at most) and
 // NaN fall back to cos(h ph).
-__device__ __forceinline__ double table_cos(const double2 *cs, const CosScale &k, double ph) {
+__device__ __forceinline__ double table_cos(const double *t, const CosScale &k, double ph) {
     if (!(((unsigned)__double2hiint(ph) & 0x7fffffffu) < k.lim_hi)) return cos(k.h * ph);
-    const double t = __fma_rn(ph, k.c1, 6755399441055744.0);  // 1.5 2^52
-    const double kd = t - 6755399441055744.0;
+    const double n = __fma_rn(ph, k.c1, 6755399441055744.0);  // 1.5 2^52
+    const double kd = n - 6755399441055744.0;
     double d = __fma_rn(-kd, k.s1, ph);
     d = __fma_rn(-kd, k.s2, d);
-    const int j = __double2loint(t) & (COS_TABLE - 1);
+    // point j of the quarter's table (every fourth of its entries): signs of
+    // the quadrant, cos and sin swapped in odd ones
+    const int j = __double2loint(n), odd = j & (COS_POINTS / 4);
+    const int at = (j & (COS_POINTS / 4 - 1)) * (2048 / COS_POINTS);
+    const int iu = odd ? 512 - at : at;
+    const unsigned turned = (unsigned)((j + COS_POINTS / 4) & (COS_POINTS / 2)) << 23;
+    const double U = t[iu], V = t[512 - iu];
+    const double cj = __hiloint2double(__double2hiint(U) ^ (int)turned, __double2loint(U));
+    const double sj = __hiloint2double(
+        __double2hiint(V) ^ (int)(turned ^ ((unsigned)odd << 24)), __double2loint(V));
     const double d2 = d * d;
     const double cd = __fma_rn(d2, __fma_rn(d2, k.c4, k.c2), 1.0);
     const double sd = d * __fma_rn(d2, __fma_rn(d2, k.s5, k.s3), k.h);
-    const double2 e = cs[j];
-    return __fma_rn(e.x, cd, -(e.y * sd));
+    return __fma_rn(cj, cd, -(sj * sd));
 }
 
 // Conversions with the integer pipe: the hardware's conversions to and from

@@ -7,20 +7,6 @@
 
 namespace hbt {
 
-namespace {
-
-// The table of cos_fixed (hbt_fixed.cuh): cos(2 pi k / 2048), k = 0..512, the
-// last one a number too small to matter in the place of zero.
-std::vector<double> cos_entries() {
-    std::vector<double> t(513);
-    for (int k = 0; k < 512; k++)
-        t[k] = (double)cosl(3.14159265358979323846264338327950288L * k / 1024.0L);
-    t[512] = std::ldexp(1.0, -100);
-    return t;
-}
-
-}  // namespace
-
 BatchRunner::~BatchRunner() {
     if (exec_) cudaGraphExecDestroy(exec_);
     for (cudaEvent_t e : marks_)
@@ -242,7 +228,8 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
     // the cosine table, once (each CTA computing its 513 entries took 4 us of
     // a launch, most of it for the smallest)
     if (!cos_.p) {
-        const std::vector<double> table = cos_entries();
+        std::vector<double> table(kCosEntries);
+        cos_entries(table.data());
         if (!grow(cos_, table.size() * sizeof(double), err)) return false;
         if (cudaMemcpyAsync(cos_.p, table.data(), table.size() * sizeof(double),
                             cudaMemcpyHostToDevice, st) != cudaSuccess ||

@@ -17,7 +17,7 @@
 //                    q_side, q_long from algebraically identical expressions
 //                    (q_out = (q_x S_x + q_y S_y) / |S|, ...) in double-float
 //                    on the FP32 pipe; pairs of particles outside the
-//                    columns' range in FP64 (values64_rows);
+//                    columns' range in FP64 (far_values), 32 at a time;
 //       FP32W form - each FP64 column split once per particle into hi + lo
 //                    FP32 parts; differences and the phase in double-float
 //                    arithmetic on the FP32 pipe, q values in FP32, cos by
@@ -117,20 +117,6 @@ struct FF {
     float h, l;
 };
 
-// Exact FP32 -> FP64 conversion of a normal FP32 value or zero through its
-// bits, on the integer pipe (the conversion instruction runs on the FP64
-// pipe): the exponent
-// rebiased by 1023 - 127 = 896, the significand moved up by 29 bits.  FP32
-// subnormals (below 1.2e-38, which the low parts of these values never
-// reach but at zero) give a signed zero; infinities and NaN are not
-// handled (the values of binned pairs are finite).
-__device__ __forceinline__ double f32_to_f64_bits(float f) {
-    const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu, sign = u & 0x80000000u;
-    const bool normal = m >= 0x00800000u;
-    const unsigned hi = normal ? ((m >> 3) + (896u << 20)) | sign : sign;
-    return __hiloint2double((int)hi, normal ? (int)(m << 29) : 0);
-}
-
 __device__ __forceinline__ FF two_sum(float a, float b) {
     const float s = __fadd_rn(a, b);
     const float bb = __fsub_rn(s, a);
@@ -194,33 +180,6 @@ __device__ __forceinline__ void columns_of(const FixedCols &r, float2 *c) {
     }
 }
 
-// a + b of two split values.
-__device__ __forceinline__ FF ff_sum(float2 a, float2 b) {
-    const FF s = two_sum(a.x, b.x);
-    return two_sum(s.h, __fadd_rn(s.l, __fadd_rn(a.y, b.y)));
-}
-
-__device__ __forceinline__ FF ff_mul_f(FF a, float b) {
-    const float p = __fmul_rn(a.h, b);
-    float e = __fmaf_rn(a.h, b, -p);
-    e = __fmaf_rn(a.l, b, e);
-    return fast_two_sum(p, e);
-}
-
-// 1 / sqrt(x): the FP32 estimate y0 and one Newton step carried in
-// double-float.  With u = x y0^2 = 1 + e (|e| ~ 2^-22, u.h - 1 exact),
-// 1 / sqrt(x) = y0 (1 - e / 2 + 3 e^2 / 8 - ...): relative error about 2^-46.
-__device__ __forceinline__ FF ff_rsqrt(FF x) {
-    const float y0 = rsqrtf(x.h);
-    const FF u = ff_mul_f(ff_mul_f(x, y0), y0);
-    const float e = __fadd_rn(__fsub_rn(u.h, 1.0f), u.l);
-    return fast_two_sum(y0, __fmul_rn(__fmul_rn(y0, e), __fmaf_rn(0.375f, e, -0.5f)));
-}
-
-__device__ __forceinline__ double ff_double_bits(FF a) {
-    return f32_to_f64_bits(a.h) + f32_to_f64_bits(a.l);
-}
-
 // x as hi + lo, two FP32 values formed from its bits on the integer pipe:
 // hi is x with the significand truncated to 24 bits, lo the remaining 29
 // bits truncated to 24, so that |x - hi - lo| < 2^-46 |x| (both parts carry
@@ -242,88 +201,6 @@ __device__ __forceinline__ FF f64_to_ff_bits(double x) {
                             ? ((unsigned)e << 23) | (((r << (lz & 31)) >> 8) & 0x7fffffu) | sign
                             : sign;
     return in_range ? FF{__uint_as_float(hb), __uint_as_float(lb)} : FF{0.0f, 0.0f};
-}
-
-// q_out, q_side, q_long of a pair in double-float arithmetic from its
-// momentum differences dp and sums sp (px, py, pz, E; sp[2], sp[3] only
-// with the boost): q_out = (dx sx + dy sy) / |s_T|, q_side = (dy sx - dx sy)
-// / |s_T| and, with the longitudinal boost, q_long = (sE dz - sz dE) /
-// sqrt(sE^2 - sz^2) (algebraically the reference's expressions), each
-// operation in double-float: about 1e-14 relative, or 2^-45 of |dp_T| in
-// absolute terms where q_out or q_side cancels.
-template <bool BOOST>
-__device__ __forceinline__ void ff_lcms(const FF *dp, const FF *sp, FF &vo, FF &vs, FF &vl) {
-    const FF inv = ff_rsqrt(ff_add(ff_mul(sp[0], sp[0]), ff_mul(sp[1], sp[1])));
-    vo = ff_mul(ff_add(ff_mul(dp[0], sp[0]), ff_mul(dp[1], sp[1])), inv);
-    vs = ff_mul(ff_add(ff_mul(dp[1], sp[0]), ff_neg(ff_mul(dp[0], sp[1]))), inv);
-    vl = dp[2];
-    if (BOOST) {
-        const FF m2 = ff_mul(ff_add(sp[3], ff_neg(sp[2])), ff_add(sp[3], sp[2]));
-        vl = ff_mul(ff_add(ff_mul(sp[3], dp[2]), ff_neg(ff_mul(sp[2], dp[3]))), ff_rsqrt(m2));
-    }
-}
-
-// FP64 summed values of an accepted same-event pair of particles outside the
-// fixed-point columns' range (algebraically the
-// reference's q_out, q_side, q_long and cos(q.dx / hbarC)).  The momentum
-// differences and sums are FP64 (one rounding each, so that cancelling sums
-// stay exact to the last bits), and so are the phase q.dx and its cos
-// (of the unrounded product with 1/hbarC).  q_out, q_side
-// and the boosted q_long, which are only summed, follow in double-float on
-// the FP32 pipe (ff_lcms: about 1e-14 relative) from the FP64 sums and
-// differences split on the integer pipe, and come back as FP64 with one
-// addition each.  The longitudinal sums sz = p_z1 + p_z2 and sE = E_1 + E_2
-// (used with the boost only) come in as double-float sums of the particles'
-// split values (2^-47 of the sum: sE does not cancel, and sz enters q_long
-// through sz dE and M_T^2 = (sE - sz)(sE + sz), where its absolute error
-// stays below 1e-14 GeV).
-template <bool BOOST>
-__device__ __forceinline__ void lcms64(const double *a, const double *b, FF sz, FF sE, double &qo,
-                                       double &qs, double &ql, double &ph) {
-    const double dx = a[0] - b[0], dy = a[1] - b[1];
-    const double dz = a[2] - b[2], dE = a[3] - b[3];
-    FF dp[4] = {f64_to_ff_bits(dx), f64_to_ff_bits(dy), f64_to_ff_bits(dz), f64_to_ff_bits(dE)};
-    FF sp[4];
-    sp[0] = f64_to_ff_bits(a[0] + b[0]);
-    sp[1] = f64_to_ff_bits(a[1] + b[1]);
-    sp[2] = sz;
-    sp[3] = sE;
-    FF vo, vs, vl;
-    ff_lcms<BOOST>(dp, sp, vo, vs, vl);
-    qo = ff_double_bits(vo);
-    qs = ff_double_bits(vs);
-    ql = BOOST ? ff_double_bits(vl) : dz;
-    // q.dx = dE dt - dx dX - dy dY - dz dZ, accumulated with fused
-    // multiply-adds (one rounding per term)
-    ph = dE * (a[7] - b[7]);
-    ph = __fma_rn(-dx, a[4] - b[4], ph);
-    ph = __fma_rn(-dy, a[5] - b[5], ph);
-    ph = __fma_rn(-dz, a[6] - b[6], ph);
-}
-// The values of a pair from the FP64 columns of rows i and j, in the
-// reference's orientation (`swap`: j first): momentum sums and differences
-// and the phase in FP64, q_out, q_side and q_long in double-float (ff_lcms).
-// For the pairs of particles whose values do not fit the fixed-point
-// columns; out of line to keep its registers out of the pair loop.  The
-// product of the phase with 1 / hbarC enters the cosine unrounded.
-template <bool BOOST>
-__device__ __noinline__ void values64_rows(const Grid &g, const double *const *c, long long i,
-                                           long long j, bool swap, double &qo, double &qs,
-                                           double &ql, double &w) {
-    double a[8], b[8];
-#pragma unroll
-    for (int f = 0; f < 8; f++) {
-        const double u = c[f][i], v = c[f][j];
-        a[f] = swap ? v : u;
-        b[f] = swap ? u : v;
-    }
-    double ph;
-    lcms64<BOOST>(a, b, ff_sum(split(a[2]), split(b[2])), ff_sum(split(a[3]), split(b[3])), qo, qs,
-                  ql, ph);
-    const double p = g.hbarC_inv * ph, e = __fma_rn(g.hbarC_inv, ph, -p);
-    double sn, cn;
-    sincos(p, &sn, &cn);
-    w = __fma_rn(-e, sn, cn);
 }
 
 // Limbs (h, l) of a difference or sum as a double-float in units of h: h in
@@ -374,25 +251,54 @@ __device__ __forceinline__ double ff_scaled(FF a, unsigned neg, int shift) {
     return conv(a.h) + conv(a.l);
 }
 
-// Summed values of an accepted same-event pair from its fixed-point columns
-// (hbt_fixed.cuh), a from the i-tile, b from the j-tile, negated in q when
-// `swap` (b is the pair's first particle).  The differences and sums are
-// exact; q_out, q_side and the boosted q_long, which are only summed, follow
-// in double-float (about 1e-14 relative).  The phase is summed from 32 x 32
-// bit products: with the limbs (h, l) of a difference, sum of h h' (unit
-// 2^-37 table steps), h l' + l h' (2^-67) and l l' (2^-97).
+// q_out, q_side and q_long of a pair from its fixed-point momenta (hbt_fixed.cuh):
+// the columns (p_x, p_y) and (m, p) of both particles, the limbs h, l of their
+// differences, the results' sign.  The differences and sums are exact, the rest
+// in double-float (about 1e-14 relative).
+template <bool BOOST>
+__device__ __forceinline__ void lcms_fixed(const int4 *a, const int4 *b, const int *h,
+                                           const int *l, unsigned neg, double &qo, double &qs,
+                                           double &ql) {
+    const FF dx = limbs_ff(h[0], l[0]), dy = limbs_ff(h[1], l[1]);
+    const FF sx = limbs_ff(a[0].x + b[0].x, a[0].y + b[0].y);
+    const FF sy = limbs_ff(a[0].z + b[0].z, a[0].w + b[0].w);
+    const FF inv = ff_rsqrt_fast(ff_dot(sx, sx, sy, sy));
+    qo = ff_scaled(ff_mul(ff_dot(dx, sx, dy, sy), inv), neg, -26);
+    qs = ff_scaled(ff_mul(ff_dot(dy, sx, ff_neg(dx), sy), inv), neg, -26);
+    const FF dm = limbs_ff(h[2], l[2]), dp = limbs_ff(h[3], l[3]);
+    if (BOOST) {
+        const FF sm = limbs_ff((unsigned)a[1].x + (unsigned)b[1].x, a[1].y + b[1].y);
+        const FF sp = limbs_ff((unsigned)a[1].z + (unsigned)b[1].z, a[1].w + b[1].w);
+        const FF n = ff_dot(sm, dp, ff_neg(sp), dm);
+        ql = ff_scaled(ff_mul(n, ff_rsqrt_fast(ff_mul(sm, sp))), neg, -27);
+    } else {
+        ql = ff_scaled(ff_add(dp, ff_neg(dm)), neg, -27);
+    }
+}
+
+// The limbs of the differences of a pair's columns [0, N).
+template <int N>
+__device__ __forceinline__ void limb_differences(const int4 *a, const int4 *b, int *h, int *l) {
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        h[2 * k] = a[k].x - b[k].x;
+        l[2 * k] = a[k].y - b[k].y;
+        h[2 * k + 1] = a[k].z - b[k].z;
+        l[2 * k + 1] = a[k].w - b[k].w;
+    }
+}
+
+// Summed values of an accepted same-event pair from its fixed-point columns, a
+// from the i-tile, b from the j-tile, negated in q when `swap` (b is the pair's
+// first particle).  The phase is summed from 32 x 32 bit products: with the
+// limbs (h, l) of a difference, sum of h h' (unit 2^-37 table steps), h l' + l h'
+// (2^-67) and l l' (2^-97).
 template <bool BOOST>
 __device__ __forceinline__ void values_fixed(const Grid &g, const double *t, const FixedCols &a,
                                              const FixedCols &b, bool swap, double &qo,
                                              double &qs, double &ql, double &w) {
     int h[8], l[8];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        h[2 * k] = a.c[k].x - b.c[k].x;
-        l[2 * k] = a.c[k].y - b.c[k].y;
-        h[2 * k + 1] = a.c[k].z - b.c[k].z;
-        l[2 * k + 1] = a.c[k].w - b.c[k].w;
-    }
+    limb_differences<4>(a.c, b.c, h, l);
     long long hh = 0, hl = 0, ll = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -401,28 +307,63 @@ __device__ __forceinline__ void values_fixed(const Grid &g, const double *t, con
         hl += (long long)l[k] * h[k + 4];
         ll += (long long)l[k] * l[k + 4];
     }
-    const unsigned neg = swap ? 0x80000000u : 0u;
-    {
-        const FF dx = limbs_ff(h[0], l[0]), dy = limbs_ff(h[1], l[1]);
-        const FF sx = limbs_ff(a.c[0].x + b.c[0].x, a.c[0].y + b.c[0].y);
-        const FF sy = limbs_ff(a.c[0].z + b.c[0].z, a.c[0].w + b.c[0].w);
-        const FF inv = ff_rsqrt_fast(ff_dot(sx, sx, sy, sy));
-        qo = ff_scaled(ff_mul(ff_dot(dx, sx, dy, sy), inv), neg, -26);
-        qs = ff_scaled(ff_mul(ff_dot(dy, sx, ff_neg(dx), sy), inv), neg, -26);
-        const FF dm = limbs_ff(h[2], l[2]), dp = limbs_ff(h[3], l[3]);
-        if (BOOST) {
-            const FF sm = limbs_ff((unsigned)a.c[1].x + (unsigned)b.c[1].x,
-                                   a.c[1].y + b.c[1].y);
-            const FF sp = limbs_ff((unsigned)a.c[1].z + (unsigned)b.c[1].z,
-                                   a.c[1].w + b.c[1].w);
-            const FF n = ff_dot(sm, dp, ff_neg(sp), dm);
-            ql = ff_scaled(ff_mul(n, ff_rsqrt_fast(ff_mul(sm, sp))), neg, -27);
-        } else {
-            ql = ff_scaled(ff_add(dp, ff_neg(dm)), neg, -27);
-        }
-    }
+    lcms_fixed<BOOST>(a.c, b.c, h, l, swap ? 0x80000000u : 0u, qo, qs, ql);
     hl += ll >> 30;
     w = cos_fixed(g, t, hh + (hl >> 30), (unsigned)hl);
+}
+
+// Summed values of an accepted same-event pair of particles outside the
+// fixed-point columns' range, negated in q when `swap` (algebraically the
+// reference's q_out, q_side, q_long and cos(q.dx / hbarC)).  c: the FP64 columns,
+// of which the pair's rows are i and j; a, b: its fixed-point momenta, which hold
+// the q values where only a position is out of range.  The phase q.dx and its
+// cos (table_cos: of the unrounded product with 1 / hbarC) are FP64, and so are
+// the transverse differences and sums where a momentum is out of range (one
+// rounding each, so that cancelling sums stay exact to the last bits).  The q
+// values, which are only summed, follow in double-float on the FP32 pipe (about
+// 1e-14 relative), the boosted q_long as (m_j p_i - m_i p_j) / sqrt(s_m s_p) of
+// the particles' m = E - p_z, p = E + p_z, which unlike s_E d_z - s_z d_E does
+// not lose digits to the pair's rapidity.  The FP64 numbers are split on the
+// integer pipe, and the q values come back with one addition each: 27 or 33 FP64
+// instructions, which bound it (60 with sincos and the hardware's conversions:
+// 6e7 binned pairs of particles spread over 1000 fm 3.9 ms, 7.6 that way; over 300
+// fm, where most pairs of a warp are of near ones, 2.6 and 8.2).  Out of line to
+// keep its registers out of the pair loop.
+template <bool BOOST>
+__device__ __noinline__ void far_values(const Grid &g, const double *t, const double *const *c,
+                                        long long i, long long j, const int4 (*a)[FT],
+                                        const int4 (*b)[FT], int qi, int qj, bool swap,
+                                        double &qo, double &qs, double &ql, double &w) {
+    const double dx = c[0][i] - c[0][j], dy = c[1][i] - c[1][j];
+    const double dz = c[2][i] - c[2][j], dE = c[3][i] - c[3][j];
+    const unsigned neg = swap ? 0x80000000u : 0u;
+    const int4 u[2] = {a[0][qi], a[1][qi]}, v[2] = {b[0][qj], b[1][qj]};
+    if (u[1].x != kFar && v[1].x != kFar) {
+        int h[4], l[4];
+        limb_differences<2>(u, v, h, l);
+        lcms_fixed<BOOST>(u, v, h, l, neg, qo, qs, ql);
+    } else {
+        const FF fx = f64_to_ff_bits(dx), fy = f64_to_ff_bits(dy);
+        const FF sx = f64_to_ff_bits(c[0][i] + c[0][j]), sy = f64_to_ff_bits(c[1][i] + c[1][j]);
+        const FF inv = ff_rsqrt_fast(ff_dot(sx, sx, sy, sy));
+        qo = ff_scaled(ff_mul(ff_dot(fx, sx, fy, sy), inv), neg, 0);
+        qs = ff_scaled(ff_mul(ff_dot(fy, sx, ff_neg(fx), sy), inv), neg, 0);
+        if (BOOST) {
+            const FF mi = f64_to_ff_bits(c[3][i] - c[2][i]), pi = f64_to_ff_bits(c[3][i] + c[2][i]);
+            const FF mj = f64_to_ff_bits(c[3][j] - c[2][j]), pj = f64_to_ff_bits(c[3][j] + c[2][j]);
+            const FF r = ff_rsqrt_fast(ff_mul(ff_add(mi, mj), ff_add(pi, pj)));
+            ql = ff_scaled(ff_mul(ff_dot(mj, pi, ff_neg(mi), pj), r), neg, 0);
+        } else {
+            ql = swap ? -dz : dz;
+        }
+    }
+    // q.dx = dE dt - dx dX - dy dY - dz dZ, accumulated with fused
+    // multiply-adds (one rounding per term)
+    double ph = dE * (c[7][i] - c[7][j]);
+    ph = __fma_rn(-dx, c[4][i] - c[4][j], ph);
+    ph = __fma_rn(-dy, c[5][i] - c[5][j], ph);
+    ph = __fma_rn(-dz, c[6][i] - c[6][j], ph);
+    w = table_cos(t, g.cph, ph);
 }
 
 // q_inv by the reference's FP64 expression (src/HBT_correlation.cpp:334-337),
@@ -523,6 +464,10 @@ struct __align__(16) SameSmem {
     // undecided pairs, (i, j) bits: the reference chain runs on them 32 at a
     // time (inline, a warp would run it for the one or two lanes holding one)
     unsigned queue3[FT / 32][QCAP];
+    // FP64 form: pairs of far particles (far_values), x = (i, j) bits | slot <<
+    // 16, y = q bin; 32 at a time, as few of a list's pairs in each warp's 32
+    // would make all warps run both kinds of values
+    uint2 queue4[FT / 32][QCAP];
     unsigned oi[FT], oj[FT];  // original list positions (pair orientation)
     // FP64 form: 32 pairs' sums and bins on their way out
     // (add_sums)
@@ -882,8 +827,9 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
 
     // one pair with its bins decided: its values; has3: its 3-D bin's record
     // (the FP32-weight form adds it here and returns none), hasq: q_inv too
+    // (of far particles: far, without sums; q_inv's form takes them here)
     auto decided = [&](unsigned e, int slot, unsigned bin, bool has3, bool hasq, double &vo,
-                       double &vs, double &vl, double &vw, double &vq) -> Sums * {
+                       double &vs, double &vl, double &vw, double &vq, bool &far) -> Sums * {
         const int qi = e & 0xff, qj = (e >> 8) & 0xff;
         const unsigned oa = sm.oi[qi], ob = sm.oj[qj];
         const bool swap = oa > ob;
@@ -915,12 +861,30 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
             if (QINV) vw = (double)v.w;
             return nullptr;
         }
-        const bool far = a.c[1].x == kFar || b.c[1].x == kFar;
-        if (far)
-            values64_rows<BOOST>(d.g, c, i0 + row_at(qi), j0 + qj, swap, vo, vs, vl, vw);
-        else
+        far = a.c[3].x == kFar || b.c[3].x == kFar;
+        if (far) {
+            if (!QINV) return nullptr;
+            far_values<BOOST>(d.g, cs, c, i0 + row_at(qi), j0 + qj, sm.xi, sm.xj, qi, qj, swap, vo,
+                              vs, vl, vw);
+        } else
             values_fixed<BOOST>(d.g, cs, a, b, swap, vo, vs, vl, vw);
         return !QINV || has3 ? d.h.sums + at : nullptr;
+    };
+
+    // 32 decided pairs of far particles
+    constexpr bool kFarQueue = PREC == 0 && !QINV && MODE != MODE_COUNT;
+    uint2 *q4 = sm.queue4[w];
+    int count4 = 0;
+    auto fars = [&](uint2 f, bool valid) {
+        double vo = 0.0, vs = 0.0, vl = 0.0, vw = 0.0;
+        if (valid) {
+            const int qi = f.x & 0xff, qj = (f.x >> 8) & 0xff;
+            far_values<BOOST>(d.g, cs, c, i0 + row_at(qi), j0 + qj, sm.xi, sm.xj, qi, qj,
+                              sm.oi[qi] > sm.oj[qj], vo, vs, vl, vw);
+        }
+        add_sums(sm.sums[w], sm.bins[w],
+                 valid ? d.h.sums + ((long long)(f.x >> 16) * d.g.q3 + f.y) : nullptr, vo, vs, vl,
+                 vw);
     };
 
     // 32 pairs that passed the screen (all lanes of the warp in step): their
@@ -941,13 +905,16 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
         }
         double vo = 0.0, vs = 0.0, vl = 0.0, vw = 0.0, vq = 0.0;
         Sums *bin = nullptr;
-        if (slot >= 0) bin = decided(e, slot, e2.y, has3, hasq, vo, vs, vl, vw, vq);
+        bool far = false;
+        if (slot >= 0) bin = decided(e, slot, e2.y, has3, hasq, vo, vs, vl, vw, vq, far);
         if (PREC != 1 && MODE != MODE_COUNT)
             add_sums(sm.sums[w], sm.bins[w], bin, vo, vs, vl, vw);
         if (QINV)
             qinv_update(d,
                         slot >= 0 && hasq ? (unsigned)(iK * d.g.qnpts) + (e2.x >> 20) : 0xffffffffu,
                         vq, vw, true);
+        if constexpr (kFarQueue)
+            enqueue(q4, count4, far, make_uint2(e | (unsigned)slot << 16, e2.y), lane, fars);
         enqueue(q3, count3, slot == -1, e, lane, chains);
     };
 
@@ -956,6 +923,7 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
     const float2 tb = sm.tb[tid];
     screen_loop<BOOST, true, QINV>(S, Terms{ta.x, ta.y, ta.z, ta.w, tb.x, tb.y}, sm.tj,
                                    sm.oi[tid], sm.oj, jmin, jb, jend, sm.queue[w], process);
+    if constexpr (kFarQueue) drain(q4, count4, lane, fars);
     drain(q3, count3, lane, chains);
 }
 

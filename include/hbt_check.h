@@ -1,8 +1,7 @@
 /*
  * hbt_check.h - device checks of the engine's own FP64 elementary functions
  * (libhbt_gpu.so).  The pair kernels and the radii fits evaluate cos and
- * exp with table-driven implementations of their own (csrc/hbt_math.cuh,
- * and the double-float cos of csrc/hbt_tile.cuh);
+ * exp with table-driven implementations of their own (csrc/hbt_math.cuh);
  * this entry point runs them on the device over caller-given arguments so
  * that tests can compare them with the host's libm.  Not part of the
  * reference's interface.
@@ -16,10 +15,12 @@
 extern "C" {
 #endif
 
-#define HBT_CHECK_COS 0 /* the pair kernels' table_cos at scale 1: cos(x) */
+#define HBT_CHECK_COS 0 /* table_cos, the cosine of the pairs of far particles,
+                           at scale 1: cos(x) */
 #define HBT_CHECK_EXP 1 /* the radii fits' table_exp */
-#define HBT_CHECK_DFCOS 2 /* the double-float form's df_cos, of x split into
-                             hi = (float)x and lo = (float)(x - hi) */
+#define HBT_CHECK_DFCOS 2 /* the same of x rounded to hi = (float)x and lo =
+                             (float)(x - hi): the double-float form runs the
+                             FP64 form's kernels */
 #define HBT_CHECK_COS_PHASE 3 /* table_cos with the pair kernels' scale:
                                  cos(x / hbarC), the product never rounded */
 
