@@ -27,6 +27,11 @@ extern "C" {
 /* out[i] = f(x[i]) on `device` for the function `which`; host arrays. */
 hbt_status hbt_check_math(int device, int32_t which, int64_t n, const double *x, double *out);
 
+/* The pair kernels' cosine of fixed-point phases on `device`: out[i] = cos(2 pi /
+ * 512 (steps[2 i] 2^-37 + steps[2 i + 1] 2^-67)), |steps[2 i]| < 2^62 and 0 <=
+ * steps[2 i + 1] < 2^30. */
+hbt_status hbt_check_cos_fixed(int device, int64_t n, const int64_t *steps, double *out);
+
 /* How the library reads or writes a caller's array of doubles at p where the
  * GPU reaches host memory itself: 2 by a kernel, 1 by copies.  No device call. */
 int32_t hbt_check_host_route(const void *p);
