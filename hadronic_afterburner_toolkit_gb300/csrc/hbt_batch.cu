@@ -183,7 +183,8 @@ __global__ void __launch_bounds__(FT) k_tiles(BatchDev b, Grid g, bool split) {
         if (l.ncols == 8) {
             const FixedCols c = split ? split_cols(v) : fixed_cols(g, v);
 #pragma unroll
-            for (int f = 0; f < kFixedCols; f++) b.fixed[(long long)f * b.cap + s] = c.c[f];
+            for (int f = 0; f < kFixedCols; f++)
+                b.fixed[(long long)f * b.fixed_cap + l.fixed_off + r] = c.c[f];
         }
         q[0] = __double2float_rd(v[0]);
         q[1] = __double2float_rd(v[1]);

@@ -19,6 +19,7 @@ struct BatchList {
     long long off;         // first row in the sorted table
     long long tiles;       // ceil(n / 128)
     long long tile_off;    // first box of this list
+    long long fixed_off;   // same-event: first row in the fixed-point columns
     int ncols;             // 8 (same-event) or 4 (mixed-event)
     int pad;
 };
@@ -71,10 +72,13 @@ struct BatchDev {
     long long max_list;     // particles of the longest list
     double *table;          // [8][cap] sorted particle table
     unsigned *orig;         // [cap] each row's position in the caller's list
-    // per row: the fixed-point columns of same-event lists ([kFixedEntries][cap],
-    // hbt_fixed.cuh) and the screen's terms (x, y, m, p) and (r2, t2)
+    // per row: the fixed-point columns of same-event lists
+    // ([kFixedEntries][fixed_cap], their rows alone: 64 bytes of a row that
+    // mixed-event lists, most of a batch, do not have; hbt_fixed.cuh) and the
+    // screen's terms (x, y, m, p) and (r2, t2)
     // (hbt_screen.cuh), converted once per batch
     int4 *fixed;
+    long long fixed_cap;
     float4 *terms4;
     float2 *terms2;
     unsigned long long *keys_in, *keys_out;

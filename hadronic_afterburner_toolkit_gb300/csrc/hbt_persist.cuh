@@ -97,8 +97,8 @@ __device__ __forceinline__ unsigned item_parts(unsigned n_items) {
 // A list of the batch as the tile kernels read it (c: its column pointers).
 __device__ __forceinline__ ListRows rows_of(const BatchDev &b, const BatchList &l,
                                             const double *const *c) {
-    return ListRows{c,    b.orig + l.off, b.fixed + l.off, b.terms4 + l.off, b.terms2 + l.off,
-                    b.cap, l.n};
+    return ListRows{c,           b.orig + l.off, b.fixed + l.fixed_off, b.terms4 + l.off,
+                    b.terms2 + l.off, b.fixed_cap, l.n};
 }
 
 // Same-event items [base, min(end, queued)) pulled by persistent CTAs.

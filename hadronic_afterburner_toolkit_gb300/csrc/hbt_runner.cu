@@ -173,6 +173,7 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
     std::vector<BatchJob> bj;
     std::vector<long long> list_off, tile_off, pair_off;
     long long total = 0, tiles = 0, pairs = 0, same_pairs = 0, mixed_pairs = 0, max_list = 0;
+    long long fixed_rows = 0;  // of same-event lists
     auto add_list = [&](const double *const *src, int ncols, long long n) {
         BatchList l = {};
         for (int f = 0; f < 8; f++) l.src[f] = f < ncols ? src[f] : nullptr;
@@ -181,6 +182,10 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
         l.tiles = (n + 127) / 128;
         l.tile_off = tiles;
         l.ncols = ncols;
+        if (ncols == 8) {
+            l.fixed_off = fixed_rows;
+            fixed_rows += n;
+        }
         list_off.push_back(total);
         tile_off.push_back(tiles);
         total += n;
@@ -244,7 +249,7 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
     const bool small = max_list <= kSmallList;
     const size_t sort_bytes = small ? 0 : batch_sort_temp_bytes(total);
     if (!grow(table_, (size_t)8 * total * sizeof(double), err) ||
-        !grow(fixed_, (size_t)kFixedEntries * total * sizeof(int4), err) ||
+        !grow(fixed_, (size_t)kFixedEntries * std::max(fixed_rows, 1LL) * sizeof(int4), err) ||
         !grow(terms_, (size_t)total * (sizeof(float4) + sizeof(float2)), err) ||
         !grow(orig_, (size_t)total * sizeof(unsigned), err) ||
         (!small && (!grow(keys_, (size_t)2 * total * sizeof(unsigned long long), err) ||
@@ -303,6 +308,7 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
     b.cap = total;
     b.table = static_cast<double *>(table_.p);
     b.fixed = static_cast<int4 *>(fixed_.p);
+    b.fixed_cap = fixed_rows;
     b.terms4 = static_cast<float4 *>(terms_.p);
     b.terms2 = reinterpret_cast<float2 *>(b.terms4 + total);
     b.max_list = max_list;
