@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(FT) k_tiles(BatchDev b, Grid g, bool split) {
         b.terms4[s] = make_float4(w.x, w.y, w.m, w.p);
         b.terms2[s] = make_float2(w.r2, w.t2);
         if (l.ncols == 8) {
-            const FixedCols c = split ? split_cols(v) : fixed_cols(g, v);
+            const FixedCols c = split ? split_cols(v) : fixed_cols(g, l.fixed_p, v);
 #pragma unroll
             for (int f = 0; f < kFixedCols; f++)
                 b.fixed[(long long)f * b.fixed_cap + l.fixed_off + r] = c.c[f];

@@ -21,7 +21,7 @@ struct BatchList {
     long long tile_off;    // first box of this list
     long long fixed_off;   // same-event: first row in the fixed-point columns
     int ncols;             // 8 (same-event) or 4 (mixed-event)
-    int pad;
+    int fixed_p;           // of the job's analysis (Grid::fixed_p)
 };
 
 // One job: same-event pairs of list la (kind 0) or la x lb (kind 1).

@@ -839,6 +839,7 @@ void grid_from_params(const hbt_params &p, Grid &g) {
     g.pos_h = std::ldexp(turns, 20);
     g.pos_l = std::ldexp(rest, 20);
     g.cfx_half = std::ldexp(6.283185307179586 / 2048.0, -53);
+    g.fixed_p = std::fabs(g.delta_q) >= std::ldexp(1.0, -11);
 }
 
 // The margins of the tile screen (hbt_screen.cuh derives them).

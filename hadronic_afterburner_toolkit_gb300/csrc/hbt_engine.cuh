@@ -28,6 +28,7 @@ struct Grid {
     // fixed-point pair values (hbt_fixed.cuh): 2^20 / (2 pi hbarC) in two
     // parts, and half a 2^-52 of the cos table's step in rad
     double pos_h, pos_l, cfx_half;
+    int fixed_p;  // bins wide enough for fixed-point momenta
 };
 
 // Per-bin numerator sums, one 32-byte L2 sector per bin.

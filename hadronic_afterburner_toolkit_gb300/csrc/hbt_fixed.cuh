@@ -24,9 +24,13 @@
 // 2^-57 |dx| steps: about 1e-15 rad for |q| = 0.2 GeV, dx = 50 fm; the FP64
 // sum of four rounded products has about 5e-15).  Whole periods drop out as
 // high bits, the table point and the remainder are bit fields, and the
-// remainder enters the cosine as an exact FP64 integer.  A particle outside
-// those ranges (or not finite) carries kFar in v, and in m where its momentum is
-// outside; its pairs take the FP64 phase, or all values in FP64 (far_values).
+// remainder enters the cosine as an exact FP64 integer.
+//
+// A particle outside those ranges (or not finite) carries kFar in v, and in m
+// where its momentum is outside; its pairs take the FP64 phase, or all values in
+// FP64 (far_values).  On grids with bins below 2^-11 GeV the momenta's 2^-57 GeV
+// would exceed the 2^-46 of a q value that double-float keeps: there no momentum
+// is taken (Grid::fixed_p).
 //
 // Of the FP64 pipe a binned pair takes 5 instructions, all for the cosine,
 // where the FP64 differences, phase, table reduction and sums took 29.
@@ -63,10 +67,10 @@ struct FixedCols {
     int4 c[kFixedCols];
 };
 
-// v: px py pz E x y z t.
-__device__ __forceinline__ FixedCols fixed_cols(const Grid &g, const double *v) {
+// v: px py pz E x y z t; fixed_p: may the momenta be taken (Grid::fixed_p)?
+__device__ __forceinline__ FixedCols fixed_cols(const Grid &g, bool fixed_p, const double *v) {
     int2 q[8];
-    bool near_p = true, near_x = true;
+    bool near_p = fixed_p, near_x = true;
 #pragma unroll
     for (int f = 0; f < 8; f++) {
         double hi, lo = 0.0;

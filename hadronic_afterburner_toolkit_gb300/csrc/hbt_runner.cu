@@ -200,6 +200,7 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
         if (j.kind == 0) {
             if (j.na < 2) continue;
             b.la = b.lb = add_list(j.a, 8, j.na);
+            lists[b.la].fixed_p = (n_devs > 0 ? devs_host[j.dev].g : d.g).fixed_p;
             const long long t = lists[b.la].tiles;
             b.n_pairs = t * (t + 1) / 2;
             same_pairs += b.n_pairs;

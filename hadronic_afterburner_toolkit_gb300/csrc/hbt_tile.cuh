@@ -321,11 +321,11 @@ __device__ __forceinline__ void values_fixed(const Grid &g, const double *t, con
 // the transverse differences and sums where a momentum is out of range (one
 // rounding each, so that cancelling sums stay exact to the last bits).  The q
 // values, which are only summed, follow in double-float on the FP32 pipe (about
-// 1e-14 relative), the boosted q_long as (m_j p_i - m_i p_j) / sqrt(s_m s_p) of
-// the particles' m = E - p_z, p = E + p_z, which unlike s_E d_z - s_z d_E does
-// not lose digits to the pair's rapidity.  The FP64 numbers are split on the
-// integer pipe, and the q values come back with one addition each: 27 or 33 FP64
-// instructions, which bound it (60 with sincos and the hardware's conversions:
+// 1e-14 relative), the boosted q_long as (s_m d_p - s_p d_m) / (2 sqrt(s_m s_p))
+// of m = E - p_z, p = E + p_z: s_E d_z - s_z d_E loses digits to the pair's
+// rapidity, and m_j p_i - m_i p_j, without differences of near numbers, to a small
+// q_long.  The FP64 numbers are split on the integer pipe, and the q values come
+// back with one addition each: 27 or 35 FP64 instructions, which bound it (60 with sincos and the hardware's conversions:
 // 6e7 binned pairs of particles spread over 1000 fm 3.9 ms, 7.6 that way; over 300
 // fm, where most pairs of a warp are of near ones, 2.6 and 8.2).  Out of line to
 // keep its registers out of the pair loop.
@@ -349,10 +349,11 @@ __device__ __noinline__ void far_values(const Grid &g, const double *t, const do
         qo = ff_scaled(ff_mul(ff_dot(fx, sx, fy, sy), inv), neg, 0);
         qs = ff_scaled(ff_mul(ff_dot(fy, sx, ff_neg(fx), sy), inv), neg, 0);
         if (BOOST) {
-            const FF mi = f64_to_ff_bits(c[3][i] - c[2][i]), pi = f64_to_ff_bits(c[3][i] + c[2][i]);
-            const FF mj = f64_to_ff_bits(c[3][j] - c[2][j]), pj = f64_to_ff_bits(c[3][j] + c[2][j]);
-            const FF r = ff_rsqrt_fast(ff_mul(ff_add(mi, mj), ff_add(pi, pj)));
-            ql = ff_scaled(ff_mul(ff_dot(mj, pi, ff_neg(mi), pj), r), neg, 0);
+            const FF dm = f64_to_ff_bits(dE - dz), dp = f64_to_ff_bits(dE + dz);
+            const FF sm = ff_add(f64_to_ff_bits(c[3][i] - c[2][i]), f64_to_ff_bits(c[3][j] - c[2][j]));
+            const FF sp = ff_add(f64_to_ff_bits(c[3][i] + c[2][i]), f64_to_ff_bits(c[3][j] + c[2][j]));
+            const FF n = ff_dot(sm, dp, ff_neg(sp), dm);
+            ql = ff_scaled(ff_mul(n, ff_rsqrt_fast(ff_mul(sm, sp))), neg, -1);
         } else {
             ql = swap ? -dz : dz;
         }
@@ -663,7 +664,7 @@ __device__ __forceinline__ FixedCols load_cols(const Grid &g, const ListRows &l,
     double v[8];
 #pragma unroll
     for (int f = 0; f < 8; f++) v[f] = l.c[f][k];
-    return PREC == 1 ? split_cols(v) : fixed_cols(g, v);
+    return PREC == 1 ? split_cols(v) : fixed_cols(g, g.fixed_p, v);
 }
 
 // The pair loop: screens this lane's row against particles [jbegin, jend) of
