@@ -38,6 +38,8 @@ constexpr int kTile = 128;
 constexpr int kStage = HBT_BF_STAGE;  // particles of list B staged at a time
 constexpr int kGroup = 4;  // pairs of a thread between two branches
 constexpr int kNphi = HBT_BF_NPHI;
+// bytes of the largest shared-memory histogram (Bnpts x 40 counts)
+constexpr int kMaxSharedHist = 96 * 1024;
 
 // Resident CTAs per SM the kernel is compiled for (register budget).
 #ifndef HBT_BF_MIN_BLOCKS
@@ -396,8 +398,8 @@ extern "C" {
 hbt_status hbt_bf_create(const hbt_bf_params *p, int device, hbt_bf_ctx **out) {
     if (!p || !out) return HBT_ERR_INVALID;
     *out = nullptr;
-    // the shared-memory histogram holds Bnpts x 40 counts (at most 96 KB)
-    if (p->Bnpts < 2 || p->Bnpts * kNphi * 4 > 48 * 1024) return HBT_ERR_INVALID;
+    if (p->Bnpts < 2 || p->Bnpts > kMaxSharedHist / (2 * kNphi * (int)sizeof(unsigned)))
+        return HBT_ERR_INVALID;
     hbt_bf_ctx *c = new hbt_bf_ctx();
     c->p = *p;
     c->device = device;
@@ -417,8 +419,9 @@ hbt_status hbt_bf_create(const hbt_bf_params *p, int device, hbt_bf_ctx **out) {
         cudaEventCreate(&c->ev[2]) != cudaSuccess ||
         !grow(c->hist, (size_t)8 * p->Bnpts * kNphi * sizeof(unsigned long long)) ||
         !grow(c->counter, sizeof(unsigned long long)) ||
-        cudaFuncSetAttribute(k_bf, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             p->Bnpts * 2 * kNphi * (int)sizeof(unsigned)) != cudaSuccess) {
+        // the same for every context: the limit is the kernel's, not a launch's
+        cudaFuncSetAttribute(k_bf, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSharedHist) !=
+            cudaSuccess) {
         hbt_bf_destroy(c);
         return HBT_ERR_CUDA;
     }
