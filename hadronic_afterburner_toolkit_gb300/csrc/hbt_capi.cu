@@ -1422,9 +1422,11 @@ hbt_status hbt_read_hist(hbt_ctx *c, double *num_count, double *q_out_sum, doubl
     double *dst[6] = {q_out_sum, q_side_sum, q_long_sum, num, num_count, den};
     map_pages(dst, 6, nb);
     TRY(drain_deferrals(c));
-    // small histograms by one kernel that writes host memory; for large ones
-    // the copy engine is faster (238 MB: 1.5 against 2.2 ms)
-    if (exports(c, dst, 6) && 6 * nb * sizeof(double) <= (16u << 20))
+    // up to 32 MB by one kernel that writes host memory, larger ones by the copy
+    // engine: reads into fresh arrays of 0.26 MB 0.05 against 0.14 ms, 16.5 MB 0.81
+    // against 0.87, 30 MB 1.3 both (again into the same arrays 0.27 against 0.34),
+    // 60 MB 1.9 against 1.8, 238 MB 5.6 against 5.3
+    if (exports(c, dst, 6) && 6 * nb * sizeof(double) <= (32u << 20))
         return export_to_host(c, dst, 6, nb, false);
     TRY(hbt_sync(c, 0));
     // each array is laid out as FP64 on the device (k_export), then copied

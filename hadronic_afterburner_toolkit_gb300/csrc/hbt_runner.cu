@@ -259,16 +259,17 @@ bool BatchRunner::run_impl(const std::vector<FastJob> &jobs, const Device &d,
         !grow(items_, (size_t)pairs * sizeof(Item), err) ||
         !grow(counters_, 4 * sizeof(unsigned), err))
         return false;
-    // Item order: it keeps the histogram slots in use in L2, so it is for
-    // histograms that do not fit there (the central group's 238 MB: 3.3x less
-    // DRAM traffic); those below half of L2 (129 MB) save its sort's launches.
-    // It does not change the kernels' time (central 50.8 ms either way).
+    // Item order: it keeps the histogram slots in use in L2 (129 MB), so it is for
+    // histograms that do not fit there: for 90,000 pions and 238 or 458 MB it
+    // saves DRAM traffic (3.3x less on the central group) at no cost in time (18.49
+    // ms a call either way); for 119 MB, which L2 keeps, its key sort is all it
+    // adds (18.55 against 18.46 ms).
     size_t hist_bytes = 0;
     for (int k = 0; k < std::max(n_devs, 1); k++) {
         const Grid &g = n_devs > 0 ? devs_host[k].g : d.g;
         hist_bytes += (size_t)g.n_slots * g.q3 * (sizeof(Sums) + 2 * sizeof(u64));
     }
-    const bool order = t.order_items && same_pairs > 0 && hist_bytes > (64u << 20);
+    const bool order = t.order_items && same_pairs > 0 && hist_bytes > (128u << 20);
     if (order &&
         (!grow(item_order_, (size_t)4 * same_pairs * sizeof(unsigned), err) ||
          !grow(item_sort_temp_, item_sort_temp_bytes(same_pairs), err)))

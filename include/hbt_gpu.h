@@ -207,7 +207,7 @@ typedef struct hbt_tuning {
                                CTAs running at any time update few histogram
                                slots (on the central workload 3.3x less DRAM
                                traffic); 0: in the order the cull found them.
-                               Analyses whose histograms are at most 64 MB stay
+                               Analyses whose histograms are at most 128 MB stay
                                in L2 whatever the order: they are not ordered.
                                The FP32-weight form always takes the cull's
                                order (its FP32 partials' bound needs the pairs of
