@@ -16,7 +16,7 @@ using namespace tile;
 
 template <bool AZ, bool BOOST, int PREC>
 __global__ void __launch_bounds__(FT) k_same_screened(Device d, long long n, Cols8 c) {
-    __shared__ SameSmem sm;
+    __shared__ SameSmem<PREC, false> sm;
     __shared__ double cs[PREC == 0 ? kCosEntries : 1];
     if (PREC == 0) fill_cos_entries(cs);
     long long ti, tj;

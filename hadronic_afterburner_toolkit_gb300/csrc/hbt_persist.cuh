@@ -107,7 +107,7 @@ __device__ __forceinline__ ListRows rows_of(const BatchDev &b, const BatchList &
 template <bool AZ, bool BOOST, int PREC, int MODE, bool QINV, bool MANY>
 __global__ void __launch_bounds__(FT, SameCtas<PREC, QINV>::value)
     k_persistent_same(Device d, BatchDev b, unsigned base, unsigned end) {
-    __shared__ SameSmem sm;
+    __shared__ SameSmem<PREC, QINV> sm;
     __shared__ unsigned item;
     __shared__ double cs[PREC == 0 ? kCosEntries : 1];  // the form's cos table
     if (PREC == 0)

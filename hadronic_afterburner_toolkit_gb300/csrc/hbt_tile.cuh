@@ -453,7 +453,8 @@ __device__ __forceinline__ float4 values32_split(const float2 *a, const float2 *
 // momentum space, so interleaving evens out the binned pairs between warps),
 // and lane k of it finds its row, and later the rows of neighbouring queue
 // entries, at consecutive places, without bank conflicts.
-struct __align__(16) SameSmem {
+template <bool FAR>
+struct __align__(16) SameSmemT {
     // fixed-point columns
     int4 xi[kFixedCols][FT];
     int4 xj[kFixedCols][FT];
@@ -465,16 +466,19 @@ struct __align__(16) SameSmem {
     // undecided pairs, (i, j) bits: the reference chain runs on them 32 at a
     // time (inline, a warp would run it for the one or two lanes holding one)
     unsigned queue3[FT / 32][QCAP];
-    // FP64 form: pairs of far particles (far_values), x = (i, j) bits | slot <<
-    // 16, y = q bin; 32 at a time, as few of a list's pairs in each warp's 32
-    // would make all warps run both kinds of values
-    uint2 queue4[FT / 32][QCAP];
+    // FAR (the FP64 form without q_inv histograms): pairs of far particles
+    // (far_values), x = (i, j) bits | slot << 16, y = q bin; 32 at a time, as few
+    // of a list's pairs in each warp's 32 would make all warps run both kinds of
+    // values
+    uint2 queue4[FAR ? FT / 32 : 1][FAR ? QCAP : 1];
     unsigned oi[FT], oj[FT];  // original list positions (pair orientation)
     // FP64 form: 32 pairs' sums and bins on their way out
     // (add_sums)
     double2 sums[FT / 32][2][32];
     Sums *bins[FT / 32][32];
 };
+template <int PREC, bool QINV>
+using SameSmem = SameSmemT<PREC == 0 && !QINV>;
 // Place of row r in the i-tile's arrays, and back.
 __device__ __forceinline__ int place_of(int r) { return (r >> 2) | ((r & 3) << 5); }
 __device__ __forceinline__ int row_at(int s) { return ((s & 31) << 2) | (s >> 5); }
@@ -767,8 +771,8 @@ __device__ __forceinline__ void add_sums(double2 (*sums)[32], Sums **bins, Sums 
 // [jb, je) of the j-tile's rows to take (jb even).
 // Called by all FT threads of the CTA; the caller syncs before reusing `sm`.
 template <bool AZ, bool BOOST, int PREC, int MODE = MODE_FAST, bool QINV = false>
-__device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, const double *cs,
-                                               const ListRows &l, long long i0, long long j0,
+__device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem<PREC, QINV> &sm,
+                                               const double *cs, const ListRows &l, long long i0, long long j0,
                                                int jb = 0, int je = FT) {
     constexpr bool LC = BOOST || QINV;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -874,7 +878,7 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem &sm, co
 
     // 32 decided pairs of far particles
     constexpr bool kFarQueue = PREC == 0 && !QINV && MODE != MODE_COUNT;
-    uint2 *q4 = sm.queue4[w];
+    uint2 *q4 = sm.queue4[kFarQueue ? w : 0];
     int count4 = 0;
     auto fars = [&](uint2 f, bool valid) {
         double vo = 0.0, vs = 0.0, vl = 0.0, vw = 0.0;
