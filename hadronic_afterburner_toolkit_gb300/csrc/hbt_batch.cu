@@ -22,7 +22,7 @@
 //     With q_inv histograms the LCMS q_long bound alone also keeps a tile
 //     pair (boxes_may_pair).  FP32, every step rounded outwards;
 //  4. k_persistent_same / k_persistent_mixed (hbt_persist.cuh): persistent
-//     CTAs (4 to 6 per SM) pull (job, i-tile, j-tile) items from the culled
+//     CTAs (5 to 7 per SM) pull (job, i-tile, j-tile) items from the culled
 //     same-event and mixed-event queues and run the screened tile-pair
 //     bodies of hbt_tile.cuh.  The FP32-weight form runs the same-event
 //     queue in chunks and merges the FP32 partials between them.

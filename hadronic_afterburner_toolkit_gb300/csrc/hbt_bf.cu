@@ -1,13 +1,13 @@
 // Balance-function pair binning (include/hbt_bf.h).
 //
-// One CTA per event pair (job): the particles of list A in registers (one
-// per thread), those of list B staged through shared memory in tiles of
-// 128.  Every pair is binned in FP32 with rigorous error bounds (bin32);
-// the pairs within those bounds of a bin edge or a cut run the reference's
-// FP64 expressions (bin64, src/BalanceFunction.cpp:136-160 and :183-204;
-// this unit is compiled with --fmad=false), so every bin is the
-// reference's.  Counts go to a shared-memory histogram of Bnpts x 20,
-// whose non-zero bins are added to the global histogram when the job is
+// One CTA per event pair (job) and 128 particles of list A, in registers (one
+// per thread); those of list B are staged through shared memory 256 at a time.
+// Every pair is binned in FP32 with rigorous error bounds (decide); the pairs
+// within those bounds of a bin edge or a cut run the reference's FP64
+// expressions (bin_slow, src/BalanceFunction.cpp:136-160 and :183-204; this unit
+// is compiled with --fmad=false), so every bin is the reference's.  Counts go to
+// a shared-memory histogram of Bnpts x 40 (columns c and c + 20 are one bin),
+// whose non-zero bins are added to the global histogram when the item is
 // done.  The bins are few and every pair lands in one, so privatising the
 // histogram in shared memory turns the pair rate's worth of global atomics
 // into one per non-zero bin and job.

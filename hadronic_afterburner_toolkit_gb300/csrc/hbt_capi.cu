@@ -68,7 +68,6 @@ struct hbt_ctx {
     DevBuf part, comp;
     // batched path: tables, sorted particle table, sort scratch, boxes, queue
     hbt::BatchRunner runner;
-    int persistent_grid = 152 * 4;
     u64 stats_host[hbt::STAT_N] = {};  // status words as the exports leave them
     bool reads_host = false;  // the GPU reads pageable host memory through the host's page tables
     int sms = 152, max_blocks_per_sm = 5;
@@ -955,7 +954,6 @@ hbt_status ctx_create(const hbt_params *p, int device, cudaMemPool_t pool, hbt_c
                                   device));
         c->reads_host = pageable && tables;
         c->max_blocks_per_sm = hbt::persistent_blocks_per_sm();
-        c->persistent_grid = sms * c->max_blocks_per_sm;
     }
 
     const size_t nb = (size_t)g.n_slots * g.q3, nq = (size_t)g.n_KT * g.qnpts;
@@ -1576,8 +1574,6 @@ hbt_status hbt_get_stats(hbt_ctx *c, hbt_stats *out) {
 namespace hbt {
 
 const Device &ctx_device(const hbt_ctx *c) { return c->d; }
-
-int ctx_persistent_grid(const hbt_ctx *c) { return c->persistent_grid; }
 
 cudaStream_t ctx_stream(const hbt_ctx *c) { return c->own; }
 

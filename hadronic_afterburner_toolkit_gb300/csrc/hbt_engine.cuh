@@ -114,8 +114,8 @@ struct Caps {
 };
 constexpr int kStraddleCols = 256;
 
-// FP32 copies of the constants used by the FP32 pair screen (hbt_fast.cu),
-// each with the bound on its rounding (slack) relative to the FP64 value.
+// Constants of the FP32 pair screen (hbt_screen.cuh), rounded to the safe side
+// where they are bounds.
 struct Screen {
     float inv_dq;         // 1 / delta_q
     float pqt2;           // above the window: 2 Q^2, Q = max(-q_lo, q_hi), with margin

@@ -64,7 +64,6 @@ struct FitConst {
     // when s < cut_sq[c], sqrt(s) > q_cut_min exactly when s > min_sq
     long long cut_sq[kMaxCuts], min_sq;
     int rank[kMaxCuts];           // position of cut k in cut_sorted
-    int by_rank[kMaxCuts];        // the cut at position s of cut_sorted
     int n_cuts;
     double q_cut_min;
     double p0[6];
@@ -469,7 +468,7 @@ __device__ void chol_solve6(const double *L, const double *b, double *x) {
 }
 
 // Levenberg-Marquardt state of one fit, in device memory, advanced by one
-// thread of the block that finishes the fit's last unit of a pass, between the passes over the fit's rows.
+// thread of the block that finishes the fit's last unit of a pass.
 struct LmState {
     double x[6], trial[6];
     double S, g[6], A[21], D[6], mu, nu;
@@ -931,7 +930,6 @@ hbt_status hbt_fit_radii(hbt_fit_ctx *c, int32_t n_tables, const hbt_fit_table *
     for (int s = 0; s < opt->n_cuts; s++) {
         fc.cut_sorted[s] = opt->q_cut_max[order[s]];
         fc.rank[order[s]] = s;
-        fc.by_rank[s] = order[s];
     }
     set_cut_squares(fc);
     for (int t = 0; t < n_tables; t++) {

@@ -16,10 +16,10 @@
 // is a sum of four products, and q_long = (s(m) d(p) - s(p) d(m)) /
 // (2 sqrt(s(m) s(p))) needs no sums of E and p_z (s: sums over the pair).
 // (q_out as the difference of p_x^2 + p_y^2 over |s_T| loses its digits for
-// small |s_T|: it is formed from the differences and sums.)  Differences of limbs stay below 2^30 (l) and, for
-// |p_x|, |p_y|, E < 8 GeV and positions within 2^18 steps per GeV (634 fm),
-// below 2^30 (h), so the products' high, cross and low parts accumulate in
-// 64 bits without overflow: 16 multiply-adds of 32 x 32 -> 64 bits for the
+// small |s_T|: it is formed from the differences and sums.)  Differences of
+// limbs stay below 2^30 (l) and, for |p_x|, |p_y|, E < 8 GeV and positions within
+// 2^18 steps per GeV (634 fm), below 2^30 (h), so the products' high, cross and
+// low parts accumulate in 64 bits without overflow: 16 multiply-adds of 32 x 32 -> 64 bits for the
 // phase, whose rounding is that of the stored values alone (2^-42 |q| +
 // 2^-57 |dx| steps: about 1e-15 rad for |q| = 0.2 GeV, dx = 50 fm; the FP64
 // sum of four rounded products has about 5e-15).  Whole periods drop out as
@@ -32,8 +32,10 @@
 // would exceed the 2^-46 of a q value that double-float keeps: there no momentum
 // is taken (Grid::fixed_p).
 //
-// Of the FP64 pipe a binned pair takes 5 instructions, all for the cosine,
-// where the FP64 differences, phase, table reduction and sums took 29.
+// Of the FP64 pipe a binned pair takes 8 instructions, 5 for the cosine and an
+// addition for each of the three q values (9 to 10 counted, with the undecided
+// pairs' chains), where the FP64 differences, phase, table reduction and sums
+// took 29.
 #pragma once
 
 #include "hbt_engine.cuh"

@@ -25,8 +25,6 @@ cudaStream_t ctx_stream(const hbt_ctx *c);
 
 // The context's engine descriptor (grid, screen constants, histograms).
 const Device &ctx_device(const hbt_ctx *c);
-// Persistent-kernel grid for the context's device.
-int ctx_persistent_grid(const hbt_ctx *c);
 // Adds candidate pairs binned on the context's behalf to its statistics.
 void ctx_add_pairs(hbt_ctx *c, u64 same, u64 mixed);
 // Merges the FP32-weight partials into the FP64 bins on `st` (no-op for
