@@ -53,10 +53,11 @@ __device__ __forceinline__ void load_device(const BatchDev &b, const BatchJob &j
 
 // Resident CTAs per SM (register budget 65536 / (128 x CTAs)), measured on
 // GB300 in whole kernels.  FP64 form, central group: 5 (51.0 ms; 53.5 at 4,
-// 55.1 at 6).  FP32-weight form: 5 (46.2 ms; 50.6 at 3, 47.8 at 4, 48.1 at
-// 6).  With q_inv histograms, 45,000 pions: same-event 6 (18.8 ms a call; the same
-// at 5, 19.4 at 4), mixed-event 7 (2.9 ms; 3.1 at 6, 3.2 at 5).  Mixed-event without them: 5 (uneven events 2.57
-// ms, small ones 0.34; 2.74 and 0.37 at 6, 3.03 and 0.41 at 8).
+// 55.1 at 6).  FP32-weight form: 5 (46.2 ms; 50.6 at 3, 47.8 at 4, 48.1 at 6).
+// With q_inv histograms, 45,000 pions: same-event 5, what shared memory holds
+// (17.0 ms a call; 17.1 at 4), mixed-event 7 (2.9 ms; 3.1 at 6, 3.2 at 5).
+// Mixed-event without them: 5 (uneven events 2.57 ms, small ones 0.34; 2.74 and
+// 0.37 at 6, 3.03 and 0.41 at 8).
 #ifndef HBT_FP64_SAME_CTAS
 #define HBT_FP64_SAME_CTAS 5  // compile-time choices (-D to measure others)
 #endif
@@ -64,7 +65,7 @@ __device__ __forceinline__ void load_device(const BatchDev &b, const BatchJob &j
 #define HBT_FP32W_SAME_CTAS 5
 #endif
 #ifndef HBT_QINV_SAME_CTAS
-#define HBT_QINV_SAME_CTAS 6
+#define HBT_QINV_SAME_CTAS 5
 #endif
 #ifndef HBT_MIXED_CTAS
 #define HBT_MIXED_CTAS 5

@@ -368,12 +368,11 @@ __device__ __noinline__ void far_values(const Grid &g, const double *t, const do
 }
 
 // q_inv by the reference's FP64 expression (src/HBT_correlation.cpp:334-337),
-// from the FP64 columns of rows i and j: bound by its 20 FP64 instructions
-// (45,000 pions 18.9 ms a call; 19.1 ms with the momenta in shared memory, 18.3
-// ms with the root by a corrected estimate).  From the fixed-point columns it
-// cannot have the expression's precision: in double-float it took 12.6 ms, but
-// had 6e-15 rms of relative error in the place of 1e-16, and their 2^-57 GeV
-// alone are 1e-15 of a q_inv of 5 MeV.
+// from the FP64 columns of rows i and j: bound by its 20 FP64 instructions.  (The
+// momenta from shared memory changed nothing.)  From the fixed-point columns it
+// cannot have the expression's precision: in double-float 45,000 pions took 12.6
+// ms in the place of 17.0, but had 6e-15 rms of relative error in the place of
+// 1e-16, and their 2^-57 GeV alone are 1e-15 of a q_inv of 5 MeV.
 __device__ __forceinline__ double qinv64(const double *const *c, long long i, long long j,
                                          bool swap) {
     double q[4];
@@ -453,7 +452,7 @@ __device__ __forceinline__ float4 values32_split(const float2 *a, const float2 *
 // momentum space, so interleaving evens out the binned pairs between warps),
 // and lane k of it finds its row, and later the rows of neighbouring queue
 // entries, at consecutive places, without bank conflicts.
-template <bool FAR>
+template <bool FAR, bool QINV>
 struct __align__(16) SameSmemT {
     // fixed-point columns
     int4 xi[kFixedCols][FT];
@@ -471,6 +470,9 @@ struct __align__(16) SameSmemT {
     // of a list's pairs in each warp's 32 would make all warps run both kinds of
     // values
     uint2 queue4[FAR ? FT / 32 : 1][FAR ? QCAP : 1];
+    // with q_inv histograms: q_inv events, x = (i, j) bits, y = bin, (z, w) = the
+    // pair's cosine
+    uint4 queue5[QINV ? FT / 32 : 1][QINV ? QCAP : 1];
     unsigned oi[FT], oj[FT];  // original list positions (pair orientation)
     // FP64 form: 32 pairs' sums and bins on their way out
     // (add_sums)
@@ -478,7 +480,7 @@ struct __align__(16) SameSmemT {
     Sums *bins[FT / 32][32];
 };
 template <int PREC, bool QINV>
-using SameSmem = SameSmemT<PREC == 0 && !QINV>;
+using SameSmem = SameSmemT<PREC == 0 && !QINV, QINV>;
 // Place of row r in the i-tile's arrays, and back.
 __device__ __forceinline__ int place_of(int r) { return (r >> 2) | ((r & 3) << 5); }
 __device__ __forceinline__ int row_at(int s) { return ((s & 31) << 2) | (s >> 5); }
@@ -831,10 +833,10 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem<PREC, Q
     };
 
     // one pair with its bins decided: its values; has3: its 3-D bin's record
-    // (the FP32-weight form adds it here and returns none), hasq: q_inv too
+    // (the FP32-weight form adds it here and returns none)
     // (of far particles: far, without sums; q_inv's form takes them here)
-    auto decided = [&](unsigned e, int slot, unsigned bin, bool has3, bool hasq, double &vo,
-                       double &vs, double &vl, double &vw, double &vq, bool &far) -> Sums * {
+    auto decided = [&](unsigned e, int slot, unsigned bin, bool has3, double &vo, double &vs,
+                       double &vl, double &vw, bool &far) -> Sums * {
         const int qi = e & 0xff, qj = (e >> 8) & 0xff;
         const unsigned oa = sm.oi[qi], ob = sm.oj[qj];
         const bool swap = oa > ob;
@@ -849,7 +851,6 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem<PREC, Q
             a.c[f] = sm.xi[f][qi];
             b.c[f] = sm.xj[f][qj];
         }
-        if (QINV && hasq) vq = qinv64(c, i0 + row_at(qi), j0 + qj, swap);
         if (PREC == 1) {
             // the pair as stored (i, j); swapping first and second negates
             // q_out, q_side, q_long exactly and leaves the phase unchanged
@@ -892,6 +893,18 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem<PREC, Q
                  vw);
     };
 
+    // 32 q_inv events: half of the pairs that pass the screen have one, and
+    // their FP64 instructions bind this form (45,000 pions 18.8 ms a call with
+    // the events taken in place, 17.0 ms with full warps of them)
+    uint4 *q5 = sm.queue5[QINV ? w : 0];
+    int count5 = 0;
+    auto qinvs = [&](uint4 f, bool valid) {
+        const int qi = f.x & 0xff, qj = (f.x >> 8) & 0xff;
+        const double vq =
+            valid ? qinv64(c, i0 + row_at(qi), j0 + qj, sm.oi[qi] > sm.oj[qj]) : 0.0;
+        qinv_update(d, valid ? f.y : 0xffffffffu, vq, __hiloint2double((int)f.w, (int)f.z), true);
+    };
+
     // 32 pairs that passed the screen (all lanes of the warp in step): their
     // slot, the decided pairs' values, then the undecided ones to the last
     // queue (last, so that the chain runs with nothing of the values live)
@@ -908,16 +921,17 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem<PREC, Q
                                (hasq && (int)(e2.x >> 20) >= S.qnpts)))
                 slot = -1;
         }
-        double vo = 0.0, vs = 0.0, vl = 0.0, vw = 0.0, vq = 0.0;
+        double vo = 0.0, vs = 0.0, vl = 0.0, vw = 0.0;
         Sums *bin = nullptr;
         bool far = false;
-        if (slot >= 0) bin = decided(e, slot, e2.y, has3, hasq, vo, vs, vl, vw, vq, far);
+        if (slot >= 0) bin = decided(e, slot, e2.y, has3, vo, vs, vl, vw, far);
         if (PREC != 1 && MODE != MODE_COUNT)
             add_sums(sm.sums[w], sm.bins[w], bin, vo, vs, vl, vw);
-        if (QINV)
-            qinv_update(d,
-                        slot >= 0 && hasq ? (unsigned)(iK * d.g.qnpts) + (e2.x >> 20) : 0xffffffffu,
-                        vq, vw, true);
+        if constexpr (QINV)
+            enqueue(q5, count5, slot >= 0 && hasq,
+                    make_uint4(e, (unsigned)(iK * d.g.qnpts) + (e2.x >> 20),
+                               (unsigned)__double2loint(vw), (unsigned)__double2hiint(vw)),
+                    lane, qinvs);
         if constexpr (kFarQueue)
             enqueue(q4, count4, far, make_uint2(e | (unsigned)slot << 16, e2.y), lane, fars);
         enqueue(q3, count3, slot == -1, e, lane, chains);
@@ -929,6 +943,7 @@ __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem<PREC, Q
     screen_loop<BOOST, true, QINV>(S, Terms{ta.x, ta.y, ta.z, ta.w, tb.x, tb.y}, sm.tj,
                                    sm.oi[tid], sm.oj, jmin, jb, jend, sm.queue[w], process);
     if constexpr (kFarQueue) drain(q4, count4, lane, fars);
+    if constexpr (QINV) drain(q5, count5, lane, qinvs);
     drain(q3, count3, lane, chains);
 }
 
