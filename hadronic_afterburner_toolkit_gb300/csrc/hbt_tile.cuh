@@ -40,11 +40,11 @@
 // (screen_qinv) and a pair stays when it is inside either window.
 //
 // Measured on the central group (150k pions, 5.4e9 pairs in the kept tile
-// pairs, 1.94e9 binned), the same-event kernel: FP64 form 121.7 -> 51.1 ms,
+// pairs, 1.94e9 binned), the same-event kernel: FP64 form 121.7 -> 49.7 ms,
 // FP32-weight form 94.0 -> 46.2 ms, against a scalar prefilter, a queue, a
 // scalar window test with per-component bounds and, in the FP64 form, FP64
-// values.  The FP64 form now keeps the shared-memory and atomics pipe 76 %,
-// the issue slots 66 % and the FP64 pipe 56 % busy.
+// values.  The FP64 form now keeps the shared-memory and atomics pipe 70 %,
+// the issue slots 70 % and the FP64 pipe 59 % busy.
 #pragma once
 
 #include <type_traits>
