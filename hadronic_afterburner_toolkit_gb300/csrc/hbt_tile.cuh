@@ -325,10 +325,11 @@ __device__ __forceinline__ void values_fixed(const Grid &g, const double *t, con
 // of m = E - p_z, p = E + p_z: s_E d_z - s_z d_E loses digits to the pair's
 // rapidity, and m_j p_i - m_i p_j, without differences of near numbers, to a small
 // q_long.  The FP64 numbers are split on the integer pipe, and the q values come
-// back with one addition each: 27 or 35 FP64 instructions, which bound it (60 with sincos and the hardware's conversions:
-// 6e7 binned pairs of particles spread over 1000 fm 3.9 ms, 7.6 that way; over 300
-// fm, where most pairs of a warp are of near ones, 2.6 and 8.2).  Out of line to
-// keep its registers out of the pair loop.
+// back with one addition each: 27 or 35 FP64 instructions, which bound it (60
+// with sincos and the hardware's conversions: 6e7 binned pairs of particles
+// spread over 1000 fm 3.9 ms, 7.6 that way; over 300 fm, where most pairs of a
+// warp are of near ones, 2.6 and 8.2).  Out of line to keep its registers out of
+// the pair loop.
 template <bool BOOST>
 __device__ __noinline__ void far_values(const Grid &g, const double *t, const double *const *c,
                                         long long i, long long j, const int4 (*a)[FT],
@@ -774,7 +775,8 @@ __device__ __forceinline__ void add_sums(double2 (*sums)[32], Sums **bins, Sums 
 // Called by all FT threads of the CTA; the caller syncs before reusing `sm`.
 template <bool AZ, bool BOOST, int PREC, int MODE = MODE_FAST, bool QINV = false>
 __device__ __forceinline__ void same_tile_pair(const Device &d, SameSmem<PREC, QINV> &sm,
-                                               const double *cs, const ListRows &l, long long i0, long long j0,
+                                               const double *cs, const ListRows &l,
+                                               long long i0, long long j0,
                                                int jb = 0, int je = FT) {
     constexpr bool LC = BOOST || QINV;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
